@@ -61,173 +61,175 @@ __device__ __forceinline__ T* at(char* base, int64_t off) {
 }
 
 // ---------------------------------------------------------------------------
-// block reductions of K values per thread (deterministic order)
-// ---------------------------------------------------------------------------
-enum { RED_SUM = 0, RED_MAX = 1, RED_MIN = 2 };
-
-__device__ __forceinline__ double red_op(double a, double b, int op) {
-  return op == RED_SUM ? a + b : (op == RED_MAX ? fmax(a, b) : fmin(a, b));
-}
-
-// Reduce v[0..K) over the block; result valid in every thread's out[].
-// scratch: (blockDim.x / 32) * K doubles of shared memory.
-template <int K>
-__device__ __forceinline__ void block_reduce(const double (&v)[K], const int (&op)[K],
-                                             double (&out)[K], double* scratch) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-  for (int k = 0; k < K; ++k) {
-    double a = v[k];
-#pragma unroll
-    for (int s = 16; s > 0; s >>= 1) a = red_op(a, __shfl_xor_sync(0xffffffffu, a, s), op[k]);
-    if (lane == 0) scratch[wid * K + k] = a;
-  }
-  __syncthreads();
-#pragma unroll
-  for (int k = 0; k < K; ++k) {
-    double a = scratch[k];
-    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) a = red_op(a, scratch[w * K + k], op[k]);
-    out[k] = a;
-  }
-  __syncthreads();
-}
-
-// ---------------------------------------------------------------------------
 // Group context: the CTAs that cooperate on one problem.
 // ---------------------------------------------------------------------------
 struct GroupCtx {
   int rank, G;
-  unsigned* bar;       // [0] arrival counter, [1] generation
-  double* red_part;    // [G][SMILI_REDK] partials
-  double* red_out;     // [SMILI_REDK] reduced values
+  unsigned* bar;       // arrivals of the group's CTAs since the launch began (never reset)
+  unsigned target;     // arrival count that completed the last barrier
+  double* red_part;    // [2][G][redk] partials of the group reductions, used in turn
+  int redk;            // values one CTA may contribute to a reduction
+  int parity;          // half of red_part the next reduction uses
   int* abort_flag;     // global abort (set on a barrier timeout)
   long long spin_limit;
 };
+
+// largest reduction: the Gram blocks of formk, 2 m (m + 1) / 2 + 2 m m at m = 6
+#define SMILI_REDK 128
+// reductions of one evaluation (no L-BFGS-B step): at most 16 sums and 3 maxima
+#define SMILI_REDK_FG 32
 
 // Spin budget of one barrier wait.  A healthy barrier completes in
 // microseconds; the limit only ends a wait that can never complete.
 #define SMILI_SPIN_LIMIT (1LL << 24)
 
-__device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
+__device__ __forceinline__ unsigned ld_relaxed(const unsigned* p) {
   unsigned v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
 
 __device__ __forceinline__ void red_release_add(unsigned* p, unsigned v) {
   asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
-__device__ __forceinline__ unsigned atom_acqrel_add(unsigned* p, unsigned v) {
-  unsigned old;
-  asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
-  return old;
-}
 
-// Wait until the generation counter moves past gen.  Polls without sleeping
-// for a short while (barriers normally complete within microseconds), then
-// backs off; gives up after spin_limit polls or when another CTA aborted.
-__device__ __forceinline__ bool wait_generation(GroupCtx& g, unsigned gen) {
+// Wait until the group's arrival count reaches g.target (compared modulo
+// 2^32).  The polls are relaxed and one fence follows them: an acquire load
+// per poll would drop the SM's L1 lines each time, also those of the other
+// CTA on the SM (an FP32 batch ran 4 % slower).  Polls without sleeping for a short while (barriers normally
+// complete within microseconds), then backs off; gives up after spin_limit
+// polls or when another CTA aborted.
+__device__ __forceinline__ bool wait_arrivals(GroupCtx& g) {
   long long spins = 0;
-  while (ld_acquire(&g.bar[1]) == gen) {
-    if (++spins > g.spin_limit || *((volatile int*)g.abort_flag)) {
+  while ((int)(ld_relaxed(g.bar) - g.target) < 0) {
+    ++spins;
+    if (spins > g.spin_limit || ((spins & 63) == 0 && *((volatile int*)g.abort_flag))) {
       atomicExch(g.abort_flag, 1);
       return false;
     }
     if (spins > 4096) __nanosleep(64);
   }
+  asm volatile("fence.acq_rel.gpu;" ::: "memory");
   return true;
 }
 
-// Returns false when the wait timed out (abort flag set): callers stop work.
-// Arrival is an acquire-release atomic on the group's counter (it orders this
-// CTA's earlier writes before the arrival and the last arriver's reads after
-// it); the last arriver resets the counter and releases the generation.
+// Group barrier.  Returns false when the wait timed out (abort flag set):
+// callers stop work.  The count only grows, so a CTA's arrival is one release
+// reduction (cumulative over the block's earlier writes, which bar.sync
+// orders before it) and the wait polls that same count: two trips to L2.  A
+// barrier whose last arriver resets a counter and then releases a generation
+// takes four: 2.4 against 1.2 us at 2 to 64 CTAs, 2.8 against 1.5 at 296 (B200).
 __device__ bool group_sync(GroupCtx& g) {
   __syncthreads();
   if (g.G == 1) return true;
   __shared__ int ok_s;
+  g.target += (unsigned)g.G;
   if (threadIdx.x == 0) {
-    int ok = 1;
-    __threadfence();  // writes of the whole block (ordered by bar.sync) before the arrival
-    const unsigned gen = ld_acquire(&g.bar[1]);
-    const unsigned arrived = atom_acqrel_add(&g.bar[0], 1u);
-    if (arrived == (unsigned)(g.G - 1)) {
-      g.bar[0] = 0;
-      red_release_add(&g.bar[1], 1u);
-    } else {
-      ok = wait_generation(g, gen) ? 1 : 0;
-    }
-    ok_s = ok;
+    red_release_add(g.bar, 1u);
+    ok_s = wait_arrivals(g) ? 1 : 0;
   }
   __syncthreads();
   return ok_s != 0;
 }
 
-// Group-wide reduction of K values held in shared memory (vals[0..K),
-// already reduced over the block).  Every CTA passes its partials; the last
-// CTA to arrive combines them in rank order and publishes the result, so the
-// value is identical in every CTA and independent of arrival order.  On
-// return vals[] holds the group result in every CTA.  K <= SMILI_REDK.
-#define SMILI_REDK 128
-__device__ bool group_reduce(GroupCtx& g, double* vals, const unsigned char* ops, int K) {
+// ---------------------------------------------------------------------------
+// Reductions over the group (deterministic, the same value in every CTA)
+// ---------------------------------------------------------------------------
+// Sums of N values (N a power of two up to 32) over a warp: every butterfly
+// step halves the values a lane carries, so N = 16 takes 16 exchanges instead
+// of 80.  Lane l returns the total of value l / (32 / N).
+template <int N>
+__device__ __forceinline__ double warp_fold(double (&v)[N], int lane) {
+  int b = 16;
+#pragma unroll
+  for (int h = N / 2; h >= 1; h >>= 1, b >>= 1) {
+    const bool up = (lane & b) != 0;
+#pragma unroll
+    for (int i = 0; i < h; ++i) {
+      const double send = up ? v[i] : v[i + h], keep = up ? v[i + h] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, b);
+    }
+  }
+#pragma unroll
+  for (int q = 16 / N; q >= 1; q >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], q);
+  return v[0];
+}
+
+// Second half of a group reduction: every CTA has its partials (ns sums,
+// then maxima, K in all) in its row of the current half of red_part, or in
+// out when G == 1.  After the barrier each CTA combines all rows itself, in
+// the same order: T / Kp slices of ranks in parallel, then the slices.  (A
+// last arriver that combines the rows one after another and publishes the
+// result adds a second barrier trip and a load latency per row.)  The halves
+// alternate, so a row is rewritten only after a later barrier has shown that
+// every CTA has read it.  scratch: blockDim.x doubles of shared memory.
+__device__ __noinline__ bool group_combine(GroupCtx& g, int K, int ns, double* out, double* scratch) {
   if (g.G == 1) {
     __syncthreads();
     return true;
   }
-  __shared__ int last_s, ok_s;
-  for (int k = threadIdx.x; k < K; k += blockDim.x) g.red_part[(size_t)g.rank * SMILI_REDK + k] = vals[k];
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    ok_s = 1;
-    last_s = 0;
-    __threadfence();  // the block's partials (written by other threads) before the arrival
-    const unsigned gen = ld_acquire(&g.bar[1]);
-    const unsigned arrived = atom_acqrel_add(&g.bar[0], 1u);
-    if (arrived == (unsigned)(g.G - 1)) {
-      last_s = 1;
-    } else {
-      ok_s = wait_generation(g, gen) ? 1 : 0;
+  const double* part = g.red_part + (size_t)g.parity * g.G * g.redk;
+  g.parity ^= 1;
+  if (!group_sync(g)) return false;
+  const int sh = K <= 16 ? 4 : (K <= 32 ? 5 : (K <= 64 ? 6 : 7));
+  const int k = threadIdx.x & ((1 << sh) - 1), sl = threadIdx.x >> sh, S = blockDim.x >> sh;
+  const bool sum = k < ns;
+  double a = sum ? 0.0 : -INFINITY;
+  if (k < K) {
+#pragma unroll 4
+    for (int r = sl; r < g.G; r += S) {
+      const double v = __ldcg(part + (size_t)r * g.redk + k);
+      a = sum ? a + v : fmax(a, v);
     }
   }
+  scratch[threadIdx.x] = a;
   __syncthreads();
-  if (last_s) {
-    for (int k = threadIdx.x; k < K; k += blockDim.x) {
-      const volatile double* rp = g.red_part;
-      double a = rp[k];
-      for (int r = 1; r < g.G; ++r) a = red_op(a, rp[(size_t)r * SMILI_REDK + k], ops[k]);
-      g.red_out[k] = a;
+  if (threadIdx.x < K) {
+    const int n = min(S, g.G);
+    double t = scratch[threadIdx.x];
+#pragma unroll 4
+    for (int q = 1; q < n; ++q) {
+      const double v = scratch[(q << sh) + threadIdx.x];
+      t = sum ? t + v : fmax(t, v);
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      __threadfence();  // the reduced values before the release
-      g.bar[0] = 0;
-      red_release_add(&g.bar[1], 1u);
-    }
+    out[threadIdx.x] = t;
   }
   __syncthreads();
-  for (int k = threadIdx.x; k < K; k += blockDim.x) vals[k] = ((const volatile double*)g.red_out)[k];
-  __syncthreads();
-  return ok_s != 0;
+  return true;
 }
 
-// Block reduction of K per-thread values (v[k] in each thread, op per entry)
-// into shared out[0..K).  scratch: (blockDim.x / 32) * K doubles.
-__device__ void block_reduce_arr(const double* v, const unsigned char* ops, int K, double* out,
-                                 double* scratch) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  for (int k = 0; k < K; ++k) {
-    double a = v[k];
-    const int op = ops[k];
-    for (int s = 16; s > 0; s >>= 1) a = red_op(a, __shfl_xor_sync(0xffffffffu, a, s), op);
-    if (lane == 0) scratch[wid * K + k] = a;
+// the row this CTA writes before group_combine
+__device__ __forceinline__ double* group_row(GroupCtx& g, double* out) {
+  return g.G == 1 ? out : g.red_part + ((size_t)g.parity * g.G + g.rank) * g.redk;
+}
+
+// Group-wide sums of s[0..NS) and maxima of x[0..NX) over all threads:
+// out[0..NS) and out[NS..NS+NX) (shared) in every CTA.  s is clobbered.
+// scratch: max(blockDim.x, warps * (NS + NX)) doubles of shared memory.
+template <int NS, int NX>
+__device__ __noinline__ bool group_reduce(GroupCtx& g, double (&s)[NS], const double (&x)[NX], double* out, double* scratch) {
+  constexpr int K = NS + NX, L = 32 / NS;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const double v = warp_fold<NS>(s, lane);
+  if (lane % L == 0) scratch[wid * K + lane / L] = v;
+#pragma unroll
+  for (int q = 0; q < NX; ++q) {
+    double a = x[q];
+#pragma unroll
+    for (int b = 16; b >= 1; b >>= 1) a = fmax(a, __shfl_xor_sync(0xffffffffu, a, b));
+    if (lane == 0) scratch[wid * K + NS + q] = a;
   }
   __syncthreads();
-  for (int k = threadIdx.x; k < K; k += blockDim.x) {
-    double a = scratch[k];
-    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) a = red_op(a, scratch[w * K + k], ops[k]);
-    out[k] = a;
+  if (threadIdx.x < K) {
+    double a = scratch[threadIdx.x];
+#pragma unroll 4
+    for (int w = 1; w < nw; ++w) {
+      const double b = scratch[w * K + threadIdx.x];
+      a = (int)threadIdx.x < NS ? a + b : fmax(a, b);
+    }
+    group_row(g, out)[threadIdx.x] = a;
   }
-  __syncthreads();
+  return group_combine(g, K, NS, out, scratch);
 }
 
 // ---------------------------------------------------------------------------

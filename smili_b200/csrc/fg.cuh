@@ -105,7 +105,7 @@ constexpr int DFT_KC = 32;  // image columns per staged chunk in F1
 // chunks of DFT_KC columns (rows padded by one element against bank
 // conflicts).
 template <typename R>
-__device__ void dft_t2_rows(FgCtx<R>& c, const GroupCtx& g, double (&mom)[10]) {
+__device__ __noinline__ void dft_t2_rows(FgCtx<R>& c, const GroupCtx& g, double (&mom)[10]) {
   const ProbDesc& P = *c.P;
   const double* x = at<double>(c.base, P.o_x);
   const int* inv = at<int>(c.base, P.o_inv);
@@ -192,7 +192,7 @@ __device__ void dft_t2_rows(FgCtx<R>& c, const GroupCtx& g, double (&mom)[10]) {
 // F2 on the DFT path: one band cell per thread and pass; tmpA and Ey staged
 // in chunks of DFT_KC rows.
 template <typename R>
-__device__ void dft_t2_cols(FgCtx<R>& c, const GroupCtx& g) {
+__device__ __noinline__ void dft_t2_cols(FgCtx<R>& c, const GroupCtx& g) {
   const ProbDesc& P = *c.P;
   const cpx<R>* Ey = at<cpx<R>>(c.base, P.o_ey);
   const cpx<R>* tmpA = at<cpx<R>>(c.base, P.o_tmpA);
@@ -231,7 +231,7 @@ __device__ void dft_t2_cols(FgCtx<R>& c, const GroupCtx& g) {
 // F6 on the DFT path: bandC staged whole; a thread takes one image column
 // and up to 8 band rows, streaming its column of Ex.
 template <typename R>
-__device__ void dft_t1_rows(FgCtx<R>& c, const GroupCtx& g) {
+__device__ __noinline__ void dft_t1_rows(FgCtx<R>& c, const GroupCtx& g) {
   const ProbDesc& P = *c.P;
   const cpx<R>* Ex = at<cpx<R>>(c.base, P.o_ex);
   const cpx<R>* bandC = at<cpx<R>>(c.base, P.o_bandC);
@@ -267,7 +267,7 @@ __device__ void dft_t1_rows(FgCtx<R>& c, const GroupCtx& g) {
 
 // F7 on the DFT path: a thread takes one image column and 4 image rows.
 template <typename R>
-__device__ void dft_t1_cols(FgCtx<R>& c, const GroupCtx& g) {
+__device__ __noinline__ void dft_t1_cols(FgCtx<R>& c, const GroupCtx& g) {
   const ProbDesc& P = *c.P;
   const cpx<R>* Ey = at<cpx<R>>(c.base, P.o_ey);
   const cpx<R>* tmpC = at<cpx<R>>(c.base, P.o_tmpC);
@@ -301,7 +301,7 @@ __device__ void dft_t1_cols(FgCtx<R>& c, const GroupCtx& g) {
 // Optionally accumulates image moments for the global regularizers.
 // ---------------------------------------------------------------------------
 template <typename R>
-__device__ void fg_t2_rows(FgCtx<R>& c, const GroupCtx& g, double (&mom)[10]) {
+__device__ __noinline__ void fg_t2_rows(FgCtx<R>& c, const GroupCtx& g, double (&mom)[10]) {
   if (c.P->dft) {
     dft_t2_rows(c, g, mom);
     return;
@@ -362,7 +362,7 @@ __device__ void fg_t2_rows(FgCtx<R>& c, const GroupCtx& g, double (&mom)[10]) {
 // F2: type-2 column pass over band columns -> bandA[b2][b1]
 // ---------------------------------------------------------------------------
 template <typename R>
-__device__ void fg_t2_cols(FgCtx<R>& c, const GroupCtx& g) {
+__device__ __noinline__ void fg_t2_cols(FgCtx<R>& c, const GroupCtx& g) {
   if (c.P->dft) {
     dft_t2_cols(c, g);
     return;
@@ -397,7 +397,7 @@ __device__ void fg_t2_cols(FgCtx<R>& c, const GroupCtx& g) {
 // The kernel width W is a template constant so both tap vectors stay in
 // registers and the W row loads of a tap row issue back to back.
 template <int W, typename R>
-__device__ __forceinline__ void interp_points(const ProbDesc& P, const R* __restrict__ xu, const R* __restrict__ xv,
+__device__ __noinline__ void interp_points(const ProbDesc& P, const R* __restrict__ xu, const R* __restrict__ xv,
                                               const cpx<R>* bandA, cpx<R>* V, cpx<R>* cacc, R beta, int j0,
                                               int dj) {
   const R half = (R)0.5 * (R)W;
@@ -492,7 +492,7 @@ __device__ __forceinline__ void acc_add(cpx<double>* p, cpx<double> v) {
 }
 
 template <typename R>
-__device__ void fg_chisq(FgCtx<R>& c, const GroupCtx& g, double (&chi)[4]) {
+__device__ __noinline__ void fg_chisq(FgCtx<R>& c, const GroupCtx& g, double (&chi)[4]) {
   const ProbDesc& P = *c.P;
   const cpx<R>* V = at<cpx<R>>(c.base, P.o_V);
   const R* dre = at<R>(c.base, P.o_dre);
@@ -704,7 +704,7 @@ __device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], 
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-__device__ void fg_spread_tc(FgCtx<float>& c, const GroupCtx& g) {
+__device__ __noinline__ void fg_spread_tc(FgCtx<float>& c, const GroupCtx& g) {
   const ProbDesc& P = *c.P;
   const float* xu = at<float>(c.base, P.o_u);
   const float* xv = at<float>(c.base, P.o_v);
@@ -825,7 +825,7 @@ __device__ void fg_spread_tc(FgCtx<float>& c, const GroupCtx& g) {
 }
 
 template <typename R>
-__device__ void fg_spread(FgCtx<R>& c, const GroupCtx& g) {
+__device__ __noinline__ void fg_spread(FgCtx<R>& c, const GroupCtx& g) {
   if constexpr (std::is_same<R, float>::value) {
     if (c.P->w <= 9 && c.P->bin == 8) {
       fg_spread_tc(c, g);
@@ -943,7 +943,7 @@ __device__ void fg_spread(FgCtx<R>& c, const GroupCtx& g) {
 // F6: type-1 row pass over band rows -> tmpC[b2][ix] (modes along axis 1)
 // ---------------------------------------------------------------------------
 template <typename R>
-__device__ void fg_t1_rows(FgCtx<R>& c, const GroupCtx& g) {
+__device__ __noinline__ void fg_t1_rows(FgCtx<R>& c, const GroupCtx& g) {
   if (c.P->dft) {
     dft_t1_rows(c, g);
     return;
@@ -977,7 +977,7 @@ __device__ void fg_t1_rows(FgCtx<R>& c, const GroupCtx& g) {
 // F7: type-1 column pass -> gchi[iy][ix] = Re(F) * dc1 * dc2
 // ---------------------------------------------------------------------------
 template <typename R>
-__device__ void fg_t1_cols(FgCtx<R>& c, const GroupCtx& g) {
+__device__ __noinline__ void fg_t1_cols(FgCtx<R>& c, const GroupCtx& g) {
   if (c.P->dft) {
     dft_t1_cols(c, g);
     return;
@@ -1252,7 +1252,7 @@ __device__ void reg_grad_loop(const ProbDesc& P, char* base, const PX& px, const
 // pixels [lo, hi); neighbours come from the dense image grid when F1 wrote
 // it in this evaluation (frames without data use the pixel map).
 template <typename T>
-__device__ void fg_reg_grad(const ProbDesc& P, char* base, const GroupCtx& g, const RegMoments& rm,
+__device__ __noinline__ void fg_reg_grad(const ProbDesc& P, char* base, const GroupCtx& g, const RegMoments& rm,
                             int lo, int hi, double (&reg)[8], double& gd, double& sbg,
                             bool opt_terms = true) {
   if (P.ident || (P.nuv > 0 && P.o_xg)) {

@@ -48,8 +48,7 @@ struct LbCtxT {
   double* lred;   // global scratch for results of the group-leader scan
   double* trace;
   double* red;    // shared [SMILI_REDK]
-  unsigned char* ops;
-  double* scratch;
+  double* scratch;  // shared, blockDim.x doubles (group_reduce)
   char* dyn;      // shared scratch (the FFT buffers)
   Prof* prof;
 };
@@ -305,17 +304,10 @@ __device__ __forceinline__ void reset_memory(LbState& S) {
   S.updatd = 0;
 }
 
-// reduce acc[0..K) over the group with the ops in c.ops; result in c.red
-template <typename SY>
-__device__ bool lb_reduce(LbCtxT<SY>& c, const double* acc, int K) {
-  block_reduce_arr(acc, c.ops, K, c.red, c.scratch);
-  return group_reduce(*c.g, c.red, c.ops, K);
-}
-
-template <typename SY>
-__device__ void set_ops(LbCtxT<SY>& c, int K, int op_default) {
-  for (int k = threadIdx.x; k < K; k += blockDim.x) c.ops[k] = (unsigned char)op_default;
-  __syncthreads();
+// Group-wide sums of s and maxima of x into c.red (sums first).
+template <int NS, int NX, typename SY>
+__device__ __forceinline__ bool lb_reduce(LbCtxT<SY>& c, double (&s)[NS], const double (&x)[NX]) {
+  return group_reduce<NS, NX>(*c.g, s, x, c.red, c.scratch);
 }
 
 // ---------------------------------------------------------------------------
@@ -425,7 +417,7 @@ __device__ __forceinline__ int bucket_of(unsigned long long k, unsigned long lon
 // by radix selection on 12-bit digits of the 96-bit composite (key, index).
 // Used for a bucket that holds more than SMILI_KC breakpoints.
 template <typename SY>
-__device__ int select_from_range(LbCtxT<SY>& c, const unsigned long long* sbk, const int* sbi, int r0,
+__device__ __noinline__ int select_from_range(LbCtxT<SY>& c, const unsigned long long* sbk, const int* sbi, int r0,
                                  int r1, u128 lo_key, u128* cand, unsigned* hist) {
   __shared__ int cnt_s, vstar_s, cum_s;
   u128 prefix = 0;
@@ -510,7 +502,7 @@ constexpr size_t SMILI_CAUCHY_SMEM =
     16 * SMILI_KC + 4 * SMILI_NBUCKET + 4 * 4096 +
     8 * (SMILI_MAX_WARPS * 32 + 2 * SMILI_MAX_THREADS + 4 * SMILI_MAXM_DEV * SMILI_MAXM_DEV + 5 + 4 * SMILI_MAXM_DEV);
 template <typename SY>
-__device__ void cauchy_scan(LbCtxT<SY>& c, double f1_0, const double* p0, int nbreak, int bnded,
+__device__ __noinline__ void cauchy_scan(LbCtxT<SY>& c, double f1_0, const double* p0, int nbreak, int bnded,
                             const unsigned long long* sbk, const int* sbi, const int* ghist) {
   LbState& S = *c.S;
   const int m = c.m, col = S.col, col2 = 2 * col, n = c.n;
@@ -794,7 +786,7 @@ __device__ void cauchy_scan(LbCtxT<SY>& c, double f1_0, const double* p0, int nb
 
 // Returns 0 on success, -1 when bmv failed (info != 0).
 template <typename SY>
-__device__ int lb_cauchy(LbCtxT<SY>& c) {
+__device__ __noinline__ int lb_cauchy(LbCtxT<SY>& c) {
   LbState& S = *c.S;
   const ProbDesc& P = *c.P;
   const int m = c.m, n = c.n, col = S.col, col2 = 2 * col;
@@ -810,10 +802,8 @@ __device__ int lb_cauchy(LbCtxT<SY>& c) {
     int pj[SMILI_MAXM_DEV];
 #pragma unroll
     for (int j = 0; j < SMILI_MAXM_DEV; ++j) pj[j] = j < col ? lptr(S, m, j) : 0;
-    // acc: [0]=f1 [1..2col]=p [2col+1]=nbreak [2col+2]=nfree_nb [2col+3]=notbnded
-    //      [2col+4]=tmin [2col+5]=tmax; accumulated in scalars and the
-    //      guarded, unrolled column arrays py/ps, packed after the loop
-    const int K = col2 + 6;
+    // sums: [0..5] Y'd, [6..11] S'd (zero past col), [12] f1, [13] nbreak,
+    // [14] nfree_nb; maxima: notbnded, -tmin, tmax
     double f1a = 0.0, nbr = 0.0, nfr = 0.0, notb = 0.0, tmn = 1.0e308, tmx = 0.0;
     double py[SMILI_MAXM_DEV], ps[SMILI_MAXM_DEV];
 #pragma unroll
@@ -861,32 +851,29 @@ __device__ int lb_cauchy(LbCtxT<SY>& c) {
       }
       c.bkey[i] = key;
     }
-    double acc[2 * SMILI_MAXM_DEV + 6];
-    acc[0] = f1a;
+    double acc[16];
 #pragma unroll
     for (int j = 0; j < SMILI_MAXM_DEV; ++j) {
-      if (j < col) {
-        acc[1 + j] = py[j];
-        acc[1 + col + j] = ps[j];
-      }
+      acc[j] = py[j];
+      acc[SMILI_MAXM_DEV + j] = ps[j];
     }
-    acc[col2 + 1] = nbr;
-    acc[col2 + 2] = nfr;
-    acc[col2 + 3] = notb;
-    acc[col2 + 4] = tmn;
-    acc[col2 + 5] = tmx;
-    for (int k = threadIdx.x; k < K; k += blockDim.x)
-      c.ops[k] = (k == col2 + 3 || k == col2 + 5) ? RED_MAX : (k == col2 + 4 ? RED_MIN : RED_SUM);
-    __syncthreads();
-    if (!lb_reduce(c, acc, K)) return -2;
-    const double f1 = c.red[0];
+    acc[12] = f1a;
+    acc[13] = nbr;
+    acc[14] = nfr;
+    acc[15] = 0.0;
+    const double accx[3] = {notb, -tmn, tmx};
+    if (!lb_reduce(c, acc, accx)) return -2;
+    const double f1 = c.red[12];
     double p[2 * SMILI_MAXM_DEV];
-    for (int j = 0; j < col2; ++j) p[j] = c.red[1 + j];
-    const int nbreak = (int)c.red[col2 + 1];
-    const int nfree_nb = (int)c.red[col2 + 2];
-    const int bnded = c.red[col2 + 3] > 0.5 ? 0 : 1;
-    const unsigned long long kmin = (unsigned long long)__double_as_longlong(c.red[col2 + 4]);
-    const unsigned long long kmax = (unsigned long long)__double_as_longlong(c.red[col2 + 5]);
+    for (int j = 0; j < col; ++j) {
+      p[j] = c.red[j];
+      p[col + j] = c.red[SMILI_MAXM_DEV + j];
+    }
+    const int nbreak = (int)c.red[13];
+    const int nfree_nb = (int)c.red[14];
+    const int bnded = c.red[16] > 0.5 ? 0 : 1;
+    const unsigned long long kmin = (unsigned long long)__double_as_longlong(-c.red[17]);
+    const unsigned long long kmax = (unsigned long long)__double_as_longlong(c.red[18]);
     if (S.theta != 1.0)
       for (int j = 0; j < col; ++j) p[col + j] *= S.theta;
     __syncthreads();
@@ -953,7 +940,7 @@ __device__ int lb_cauchy(LbCtxT<SY>& c) {
   const int mode = (int)cr_s[CR_MODE];
   if (mode != CM_XCP_IS_X && cr_s[CR_INFO] != 0) return -1;
   // apply the GCP and run freev (lbfgsb.f:2241-2340)
-  double acc[3] = {0, 0, 0};  // nfree, nenter, nleave
+  double acc[4] = {0, 0, 0, 0};  // nfree, nenter, nleave
   const u128 bnd = ((u128)(unsigned long long)__double_as_longlong(cr_s[CR_BHI]) << 64) |
                    (u128)(unsigned long long)__double_as_longlong(cr_s[CR_BLO]);
   const double tsum = cr_s[CR_TSUM];
@@ -978,8 +965,8 @@ __device__ int lb_cauchy(LbCtxT<SY>& c) {
     c.freef[i] = (unsigned char)fnew;
     acc[0] += fnew;
   }
-  set_ops(c, 3, RED_SUM);
-  if (!lb_reduce(c, acc, 3)) return -2;
+  const double none[1] = {0.0};
+  if (!lb_reduce(c, acc, none)) return -2;
   if (threadIdx.x == 0) {
     if (mode != CM_XCP_IS_X) {
       S.nseg = (int)cr_s[CR_NSEG];
@@ -1008,7 +995,7 @@ __device__ __forceinline__ void dmma_884(double (&d)[2], double a, double b) {
 }
 
 template <typename SY>
-__device__ int lb_formk(LbCtxT<SY>& c) {
+__device__ __noinline__ int lb_formk(LbCtxT<SY>& c) {
   LbState& S = *c.S;
   const int m = c.m, n = c.n, col = S.col;
   // entries: Fyy (a<=b), Ass (a<=b), Fsy (a,b), Asy (a,b) over physical columns
@@ -1060,6 +1047,7 @@ __device__ int lb_formk(LbCtxT<SY>& c) {
     pw[193] = asy[1];
   }
   __syncthreads();
+  double* row = group_row(*c.g, c.red);
   for (int e = threadIdx.x; e < E; e += blockDim.x) {
     int t, a, b;
     if (e < 2 * nsym) {  // triangular index -> (a, b), a <= b
@@ -1080,11 +1068,9 @@ __device__ int lb_formk(LbCtxT<SY>& c) {
     }
     double sum = 0.0;
     for (int w = 0; w < nw; ++w) sum += part[(size_t)w * 256 + t * 64 + a * 8 + b];
-    c.red[e] = sum;
+    row[e] = sum;
   }
-  for (int k = threadIdx.x; k < E; k += blockDim.x) c.ops[k] = RED_SUM;
-  __syncthreads();
-  if (!group_reduce(*c.g, c.red, c.ops, E)) return -9;
+  if (!group_combine(*c.g, E, E, c.red, c.scratch)) return -9;
   int info = 0;
   if (threadIdx.x == 0) {
     auto sym = [&](int base, int a, int b) {  // symmetric block entry
@@ -1145,7 +1131,7 @@ __device__ int lb_formk(LbCtxT<SY>& c) {
 // cmprlb + subsm (lbfgsb.f:1720-1786, 2991-3346).  Returns 0 or an error.
 // ---------------------------------------------------------------------------
 template <typename SY>
-__device__ int lb_cmprlb_subsm(LbCtxT<SY>& c) {
+__device__ __noinline__ int lb_cmprlb_subsm(LbCtxT<SY>& c) {
   LbState& S = *c.S;
   const ProbDesc& P = *c.P;
   const int m = c.m, n = c.n, col = S.col, col2 = 2 * col;
@@ -1203,21 +1189,21 @@ __device__ int lb_cmprlb_subsm(LbCtxT<SY>& c) {
       }
     }
   }
-  double acc[2 * SMILI_MAXM_DEV];
+  double acc[16];
 #pragma unroll
   for (int j = 0; j < SMILI_MAXM_DEV; ++j) {
-    if (j < col) {
-      acc[j] = ay[j];
-      acc[col + j] = as[j];
-    }
+    acc[j] = ay[j];
+    acc[SMILI_MAXM_DEV + j] = as[j];
   }
-  set_ops(c, col2, RED_SUM);
-  if (!lb_reduce(c, acc, col2)) return -9;
+#pragma unroll
+  for (int j = 2 * SMILI_MAXM_DEV; j < 16; ++j) acc[j] = 0.0;
+  const double none[1] = {0.0};
+  if (!lb_reduce(c, acc, none)) return -9;
   if (threadIdx.x == 0) {
     double wv[2 * SMILI_MAXM_DEV];
     for (int j = 0; j < col; ++j) {
       wv[j] = c.red[j];
-      wv[col + j] = theta * c.red[col + j];
+      wv[col + j] = theta * c.red[SMILI_MAXM_DEV + j];
     }
     const int m2 = 2 * m;
     if (d_tri_solve(S.wn, m2, col2, wv, true)) {
@@ -1231,7 +1217,7 @@ __device__ int lb_cmprlb_subsm(LbCtxT<SY>& c) {
   __syncthreads();
   if (err_s) return err_s;
   // d := (d + W wv) / theta on the free set, then project z + d
-  double acc2[2] = {0.0, 0.0};  // iword (max), dd_p (sum)
+  double iwd[1] = {0.0}, ddp[1] = {0.0};  // iword (max), dd_p (sum)
   double wq[SMILI_MAXM_DEV], wr[SMILI_MAXM_DEV];
 #pragma unroll
   for (int j = 0; j < SMILI_MAXM_DEV; ++j) {
@@ -1265,54 +1251,48 @@ __device__ int lb_cmprlb_subsm(LbCtxT<SY>& c) {
       c.r[i] = ri;
       if (P.nonneg) {
         zn = fmax(0.0, zi + ri);
-        if (zn == 0.0) acc2[0] = 1.0;
+        if (zn == 0.0) iwd[0] = 1.0;
       } else {
         zn = zi + ri;
       }
       c.z[i] = zn;
     }
-    acc2[1] += (zn - xv) * gvi;
+    ddp[0] += (zn - xv) * gvi;
   }
-  if (threadIdx.x == 0) {
-    c.ops[0] = RED_MAX;
-    c.ops[1] = RED_SUM;
-  }
-  __syncthreads();
-  if (!lb_reduce(c, acc2, 2)) return -9;
-  const int iword = c.red[0] > 0.5;
-  const double dd_p = c.red[1];
+  if (!lb_reduce(c, ddp, iwd)) return -9;
+  const int iword = c.red[1] > 0.5;
+  const double dd_p = c.red[0];
   if (threadIdx.x == 0) S.iword = iword;
   __syncthreads();
   if (!iword || dd_p <= 0.0) return 0;
   // backtrack: z = xp, alpha = largest feasible step along d (lbfgsb.f:3270-3330)
-  double acc3[1] = {1.0};
+  double zero[1] = {0.0}, acc3[1] = {-1.0};  // minima as maxima of the negated values
   for (int i = c.lo + threadIdx.x; i < c.hi; i += blockDim.x) {
     c.z[i] = c.xp[i];
     if ((c.freef[i] || unc) && P.nonneg) {
       const double dk = c.r[i];
       if (dk < 0.0) {
         const double t2 = -c.z[i];
-        acc3[0] = fmin(acc3[0], t2 >= 0.0 ? 0.0 : t2 / dk);
+        acc3[0] = fmax(acc3[0], t2 >= 0.0 ? 0.0 : -(t2 / dk));
       }
     }
   }
-  set_ops(c, 1, RED_MIN);
-  if (!lb_reduce(c, acc3, 1)) return -9;
-  const double alpha = c.red[0];
+  if (!lb_reduce(c, zero, acc3)) return -9;
+  const double alpha = -c.red[1];
   __syncthreads();
-  double acc4[1] = {(double)n};
+  double acc4[1] = {-(double)n};
   if (alpha < 1.0) {
     for (int i = c.lo + threadIdx.x; i < c.hi; i += blockDim.x) {
       if ((c.freef[i] || unc) && P.nonneg && c.r[i] < 0.0) {
         const double t2 = -c.z[i];
         const double v = t2 >= 0.0 ? 0.0 : t2 / c.r[i];
-        if (v == alpha) acc4[0] = fmin(acc4[0], (double)i);
+        if (v == alpha) acc4[0] = fmax(acc4[0], -(double)i);
       }
     }
-    set_ops(c, 1, RED_MIN);
-    if (!lb_reduce(c, acc4, 1)) return -9;
+    zero[0] = 0.0;
+    if (!lb_reduce(c, zero, acc4)) return -9;
   }
-  const int ibd = alpha < 1.0 ? (int)c.red[0] : -1;
+  const int ibd = alpha < 1.0 ? -(int)c.red[1] : -1;
   __syncthreads();
   for (int i = c.lo + threadIdx.x; i < c.hi; i += blockDim.x) {
     if (c.freef[i] || unc) {
@@ -1388,10 +1368,10 @@ __device__ int lb_ls_fail(LbCtxT<SY>& c) {
 
 // label 555 + the first part of lnsrlb (lbfgsb.f:2480-2575)
 template <typename SY>
-__device__ int lb_lnsrch_start(LbCtxT<SY>& c) {
+__device__ __noinline__ int lb_lnsrch_start(LbCtxT<SY>& c) {
   LbState& S = *c.S;
   const bool bounded_steps = S.cnstnd && S.iter > 0;
-  double acc[3] = {0.0, 1.0e10, 0.0};  // dtd, stpmx (min), gd
+  double acc[2] = {0.0, 0.0}, stm[1] = {-1.0e10};  // dtd, gd; -stpmx (max)
   for (int i = c.lo + threadIdx.x; i < c.hi; i += blockDim.x) {
     const double di = c.z[i] - c.x[i];
     const double xi = c.x[i], gi = c.gv[i];
@@ -1399,31 +1379,25 @@ __device__ int lb_lnsrch_start(LbCtxT<SY>& c) {
     c.t[i] = xi;
     c.r[i] = gi;
     acc[0] += di * di;
-    acc[2] += gi * di;
+    acc[1] += gi * di;
     if (bounded_steps && c.P->nonneg && di < 0.0) {
       const double a2 = -xi;  // l - x with l = 0
-      acc[1] = fmin(acc[1], a2 >= 0.0 ? 0.0 : a2 / di);
+      stm[0] = fmax(stm[0], a2 >= 0.0 ? 0.0 : -(a2 / di));
     }
   }
-  if (threadIdx.x == 0) {
-    c.ops[0] = RED_SUM;
-    c.ops[1] = RED_MIN;
-    c.ops[2] = RED_SUM;
-  }
-  __syncthreads();
-  if (!lb_reduce(c, acc, 3)) return LB_RET_ABORT;
+  if (!lb_reduce(c, acc, stm)) return LB_RET_ABORT;
   __shared__ int act_s;
   if (threadIdx.x == 0) {
     S.dtd = c.red[0];
     S.dnorm = sqrt(S.dtd);
     S.stpmx = 1.0e10;
-    if (S.cnstnd) S.stpmx = (S.iter == 0) ? 1.0 : c.red[1];
+    if (S.cnstnd) S.stpmx = (S.iter == 0) ? 1.0 : -c.red[2];
     S.stp = (S.iter == 0 && !S.boxed) ? fmin(1.0 / S.dnorm, S.stpmx) : 1.0;
     S.fold = S.f;
     S.ifun = 0;
     S.iback = 0;
     S.csave = CS_START;
-    S.gd = c.red[2];
+    S.gd = c.red[1];
     S.gdold = S.gd;
     if (S.gd >= 0.0) {
       S.info = -4;  // ascent direction in projection
@@ -1452,7 +1426,7 @@ __device__ int lb_lnsrch_start(LbCtxT<SY>& c) {
 
 // label 222 onwards: Cauchy point, subspace minimisation, line-search start
 template <typename SY>
-__device__ int lb_iter(LbCtxT<SY>& c) {
+__device__ __noinline__ int lb_iter(LbCtxT<SY>& c) {
   LbState& S = *c.S;
   for (int guard = 0; guard < 4; ++guard) {
     if (threadIdx.x == 0) S.iword = -1;
@@ -1513,7 +1487,7 @@ __device__ int lb_iter(LbCtxT<SY>& c) {
 // f, g.d and projected-gradient norm.  Returns LB_RET_FG when x holds the next
 // point to evaluate, LB_RET_DONE when the solve is over.
 template <typename SY>
-__device__ int lb_after_fg(LbCtxT<SY>& c, double f, double gd_fg, double sbg) {
+__device__ __noinline__ int lb_after_fg(LbCtxT<SY>& c, double f, double gd_fg, double sbg) {
   LbState& S = *c.S;
   const ProbDesc& P = *c.P;
   const int m = c.m;
@@ -1616,7 +1590,6 @@ __device__ int lb_after_fg(LbCtxT<SY>& c, double f, double gd_fg, double sbg) {
     // matupd (lbfgsb.f:2584-2670) fused with r = g - r, d = stp d and rr
     const int n = c.n, itail = S.itail - 1;
     const double sc = (S.stp == 1.0) ? 1.0 : S.stp;
-    const int K = 1 + 2 * m;
     // per-column partial sums in registers: the column loops are unrolled
     // to the largest memory with a guard, so no array is indexed at run time
     double rr_acc = 0.0, ay[SMILI_MAXM_DEV], as[SMILI_MAXM_DEV];
@@ -1637,19 +1610,19 @@ __device__ int lb_after_fg(LbCtxT<SY>& c, double f, double gd_fg, double sbg) {
       c.r[i] = ri;
       c.d[i] = di;
     }
-    double acc[1 + 2 * SMILI_MAXM_DEV];
-    acc[0] = rr_acc;
+    double acc[16];
 #pragma unroll
     for (int j = 0; j < SMILI_MAXM_DEV; ++j) {
-      if (j < m) {
-        acc[1 + j] = ay[j];
-        acc[1 + m + j] = as[j];
-      }
+      acc[j] = ay[j];
+      acc[SMILI_MAXM_DEV + j] = as[j];
     }
-    set_ops(c, K, RED_SUM);
-    if (!lb_reduce(c, acc, K)) return lb_abort(c);
+    acc[12] = rr_acc;
+#pragma unroll
+    for (int j = 13; j < 16; ++j) acc[j] = 0.0;
+    const double none[1] = {0.0};
+    if (!lb_reduce(c, acc, none)) return lb_abort(c);
     if (threadIdx.x == 0) {
-      const double rr = c.red[0], dr = S.wa[0];
+      const double rr = c.red[12], dr = S.wa[0];
       const int col = S.col;
 #define SY(i, j) S.sy[((i)-1) + m * ((j)-1)]
 #define SS(i, j) S.ss[((i)-1) + m * ((j)-1)]
@@ -1662,8 +1635,8 @@ __device__ int lb_after_fg(LbCtxT<SY>& c, double f, double gd_fg, double sbg) {
       }
       int pointr = S.head;
       for (int j = 1; j <= col - 1; ++j) {
-        SY(col, j) = c.red[1 + (pointr - 1)];
-        SS(j, col) = c.red[1 + m + (pointr - 1)];
+        SY(col, j) = c.red[pointr - 1];
+        SS(j, col) = c.red[SMILI_MAXM_DEV + (pointr - 1)];
         pointr = pointr % m + 1;
       }
       SS(col, col) = (S.stp == 1.0) ? S.dtd : S.stp * S.stp * S.dtd;

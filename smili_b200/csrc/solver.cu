@@ -41,9 +41,9 @@ struct BatchArgs {
   const ProbDesc* descs;
   int nprob, G, mode;
   int* queue;
-  unsigned* bars;      // [ngroups][2]
-  double* red_part;    // [ngroups][G][SMILI_REDK]
-  double* red_out;     // [ngroups][SMILI_REDK]
+  unsigned* bars;      // [ngroups][8]: arrival counter of each group, one per 32-byte sector
+  double* red_part;    // [ngroups][2][G][redk]
+  int redk;
   int* grp_prob;       // [ngroups]
   int* abort_flag;
   ProbResult* results; // [nprob]
@@ -53,6 +53,15 @@ struct BatchArgs {
 // ---------------------------------------------------------------------------
 // one function/gradient evaluation by the group (stages F1..F8)
 // ---------------------------------------------------------------------------
+// group-wide sums of the ten image moments into red[0..10)
+__device__ bool reduce_moments(GroupCtx& g, const double (&mom)[10], double* red, double* scratch) {
+  double s[16];
+#pragma unroll
+  for (int k = 0; k < 16; ++k) s[k] = k < 10 ? mom[k] : 0.0;
+  const double none[1] = {0.0};
+  return group_reduce<16, 1>(g, s, none, red, scratch);
+}
+
 // Stages F1-F8 of one evaluation of a 2D problem by group g: per-thread
 // partial sums acc[0..3] = chi-square terms (weighted), acc[4..11] = the
 // per-pixel regularizers (l1, tv, tsv, kl, gs, -, -, -), acc[12] = g.d,
@@ -60,9 +69,8 @@ struct BatchArgs {
 // false leaves acc[12..13] alone (a movie frame).  A frame without data
 // (nuv == 0) only evaluates its regularizers.
 template <typename R>
-__device__ bool fg_stages(FgCtx<R>& fc, GroupCtx& g, int lo, int hi, double* red, unsigned char* ops,
-                          double* scratch, double (&acc)[16], RegMoments& rm, int mode, bool opt_terms,
-                          Prof& pf) {
+__device__ bool fg_stages(FgCtx<R>& fc, GroupCtx& g, int lo, int hi, double* red, double* scratch,
+                          double (&acc)[16], RegMoments& rm, int mode, bool opt_terms, Prof& pf) {
   const ProbDesc& P = *fc.P;
   memset(&rm, 0, sizeof(rm));
   double chi[4] = {0, 0, 0, 0};
@@ -71,10 +79,7 @@ __device__ bool fg_stages(FgCtx<R>& fc, GroupCtx& g, int lo, int hi, double* red
     for (int k = 0; k < 10; ++k) mom[k] = 0.0;
     fg_t2_rows(fc, g, mom);
     if (P.has_tfd || P.has_cen || P.has_sm) {
-      for (int k = threadIdx.x; k < 10; k += blockDim.x) ops[k] = RED_SUM;
-      __syncthreads();
-      block_reduce_arr(mom, ops, 10, red, scratch);
-      if (!group_reduce(g, red, ops, 10)) return false;
+      if (!reduce_moments(g, mom, red, scratch)) return false;
       double mm[10];
       for (int k = 0; k < 10; ++k) mm[k] = red[k];
       reg_moments(P, mm, rm);
@@ -108,10 +113,8 @@ __device__ bool fg_stages(FgCtx<R>& fc, GroupCtx& g, int lo, int hi, double* red
   } else if (P.has_tfd || P.has_sm) {
     double mom[10];
     for (int k = 0; k < 10; ++k) mom[k] = 0.0;
-    frame_moments(P, fc.base, mom);
-    for (int k = threadIdx.x; k < 10; k += blockDim.x) ops[k] = RED_SUM;
-    __syncthreads();
-    block_reduce_arr(mom, ops, 10, red, scratch);
+    frame_moments(P, fc.base, mom);  // a frame of a movie: one CTA
+    if (!reduce_moments(g, mom, red, scratch)) return false;
     double mm[10];
     for (int k = 0; k < 10; ++k) mm[k] = red[k];
     reg_moments(P, mm, rm);
@@ -141,23 +144,22 @@ __device__ __forceinline__ void global_regs(const ProbDesc& P, const RegMoments&
 // One evaluation of a 2D problem: f, g.d, projected-gradient norm and the
 // 15 cost terms (fftim2d.f90:387-607).
 template <typename R>
-__device__ bool group_fg(FgCtx<R>& fc, GroupCtx& g, LbCtxT<R>& lc, double* red, unsigned char* ops,
-                         double* scratch, double& f, double& gd, double& sbg, double* terms,
-                         int mode) {
+__device__ bool group_fg(FgCtx<R>& fc, GroupCtx& g, LbCtxT<R>& lc, double* red, double* scratch, double& f,
+                         double& gd, double& sbg, double* terms, int mode) {
   const ProbDesc& P = *fc.P;
   Prof& pf = *lc.prof;
   pf.mark(PR_OTHER);
   double acc[16];
   for (int k = 0; k < 16; ++k) acc[k] = 0.0;
   RegMoments rm;
-  if (!fg_stages(fc, g, lc.lo, lc.hi, red, ops, scratch, acc, rm, mode, true, pf)) return false;
+  if (!fg_stages(fc, g, lc.lo, lc.hi, red, scratch, acc, rm, mode, true, pf)) return false;
   if (mode == MODE_T1 || mode == MODE_T2) return true;
-  for (int k = threadIdx.x; k < 14; k += blockDim.x) ops[k] = (k == 13) ? RED_MAX : RED_SUM;
-  __syncthreads();
-  block_reduce_arr(acc, ops, 14, red, scratch);
-  if (!group_reduce(g, red, ops, 14)) return false;
+  const double mx[1] = {acc[13]};
+  acc[13] = 0.0;
+  if (!group_reduce<16, 1>(g, acc, mx, red, scratch)) return false;
   double r[14];
-  for (int k = 0; k < 14; ++k) r[k] = red[k];
+  for (int k = 0; k < 13; ++k) r[k] = red[k];
+  r[13] = red[16];
   __syncthreads();
   pf.mark(PR_F8);
   pf.count(PR_COUNT);
@@ -190,8 +192,8 @@ __device__ bool group_fg(FgCtx<R>& fc, GroupCtx& g, LbCtxT<R>& lc, double* red, 
 // iz < Nz as the reference does) and forms g.d and the projected gradient
 // over the whole vector.  terms[20] follow the fftim3d.imaging order.
 template <typename R>
-__device__ bool movie_fg(FgCtx<R>& fc, GroupCtx& g, LbCtxT<R>& lc, double* red, unsigned char* ops,
-                         double* scratch, double& f, double& gd, double& sbg, double* terms) {
+__device__ bool movie_fg(FgCtx<R>& fc, GroupCtx& g, LbCtxT<R>& lc, double* red, double* scratch, double& f,
+                         double& gd, double& sbg, double* terms) {
   const ProbDesc& M = *fc.P;
   char* base = fc.base;
   Prof& pf = *lc.prof;
@@ -206,7 +208,7 @@ __device__ bool movie_fg(FgCtx<R>& fc, GroupCtx& g, LbCtxT<R>& lc, double* red, 
     FgCtx<R> fz = fc;
     fz.P = &frames[z];
     RegMoments rm;
-    if (!fg_stages(fz, g1, 0, frames[z].npix, red, ops, scratch, acc, rm, MODE_FG, false, pf)) return false;
+    if (!fg_stages(fz, g1, 0, frames[z].npix, red, scratch, acc, rm, MODE_FG, false, pf)) return false;
     if (threadIdx.x == 0) {
       double tfd, cen, sm;
       global_regs(frames[z], rm, tfd, cen, sm);
@@ -255,12 +257,12 @@ __device__ bool movie_fg(FgCtx<R>& fc, GroupCtx& g, LbCtxT<R>& lc, double* red, 
     if (M.nonneg && gi >= 0.0) gi = fmin(x[idx], gi);
     acc[13] = fmax(acc[13], fabs(gi));
   }
-  for (int k = threadIdx.x; k < 16; k += blockDim.x) ops[k] = (k == 13) ? RED_MAX : RED_SUM;
-  __syncthreads();
-  block_reduce_arr(acc, ops, 16, red, scratch);
-  if (!group_reduce(g, red, ops, 16)) return false;
+  const double mx[1] = {acc[13]};
+  acc[13] = 0.0;
+  if (!group_reduce<16, 1>(g, acc, mx, red, scratch)) return false;
   double r[16];
   for (int k = 0; k < 16; ++k) r[k] = red[k];
+  r[13] = red[16];
   __syncthreads();
   pf.mark(PR_F8);
   pf.count(PR_COUNT);
@@ -301,8 +303,7 @@ __global__ void __launch_bounds__(Shape<R>::threads, Shape<R>::min_blocks) smili
   extern __shared__ __align__(16) char dyn[];
   __shared__ LbState S;
   __shared__ double red[SMILI_REDK];
-  __shared__ unsigned char ops[SMILI_REDK];
-  __shared__ double scratch[Shape<R>::warps * SMILI_REDK];
+  __shared__ double scratch[Shape<R>::threads];
   __shared__ int prob_s;
   const int grp = blockIdx.x / a.G, rank = blockIdx.x % a.G;
   Prof prof;
@@ -312,9 +313,11 @@ __global__ void __launch_bounds__(Shape<R>::threads, Shape<R>::min_blocks) smili
   GroupCtx g;
   g.rank = rank;
   g.G = a.G;
-  g.bar = a.bars + 2 * grp;
-  g.red_part = a.red_part + (size_t)grp * a.G * SMILI_REDK;
-  g.red_out = a.red_out + (size_t)grp * SMILI_REDK;
+  g.bar = a.bars + 8 * grp;
+  g.target = 0;
+  g.red_part = a.red_part + (size_t)grp * 2 * a.G * a.redk;
+  g.redk = a.redk;
+  g.parity = 0;
   g.abort_flag = a.abort_flag;
   g.spin_limit = SMILI_SPIN_LIMIT;
   if (a.mode == MODE_BARRIER) {  // cost of the group barrier: 1000 waits
@@ -375,7 +378,6 @@ __global__ void __launch_bounds__(Shape<R>::threads, Shape<R>::min_blocks) smili
     lc.lred = at<double>(base, P.o_lred);
     lc.trace = at<double>(base, P.o_trace);
     lc.red = red;
-    lc.ops = ops;
     lc.scratch = scratch;
     lc.dyn = dyn;
     lc.prof = &prof;
@@ -403,8 +405,8 @@ __global__ void __launch_bounds__(Shape<R>::threads, Shape<R>::min_blocks) smili
     prof.mark(PR_INIT);
     while (ok) {
       double f = 0, gd = 0, sbg = 0;
-      const bool okf = P.nframes > 0 ? movie_fg<R>(fc, g, lc, red, ops, scratch, f, gd, sbg, S.terms)
-                                     : group_fg<R>(fc, g, lc, red, ops, scratch, f, gd, sbg, S.terms, a.mode);
+      const bool okf = P.nframes > 0 ? movie_fg<R>(fc, g, lc, red, scratch, f, gd, sbg, S.terms)
+                                     : group_fg<R>(fc, g, lc, red, scratch, f, gd, sbg, S.terms, a.mode);
       if (!okf) {
         ok = false;
         break;
@@ -423,8 +425,8 @@ __global__ void __launch_bounds__(Shape<R>::threads, Shape<R>::min_blocks) smili
       // final summary evaluation at the returned image (fftim2d.f90:356-376)
       if (!group_sync(g)) ok = false;
       double f = 0, gd = 0, sbg = 0;
-      if (ok && !(P.nframes > 0 ? movie_fg<R>(fc, g, lc, red, ops, scratch, f, gd, sbg, S.terms)
-                                : group_fg<R>(fc, g, lc, red, ops, scratch, f, gd, sbg, S.terms, MODE_FG)))
+      if (ok && !(P.nframes > 0 ? movie_fg<R>(fc, g, lc, red, scratch, f, gd, sbg, S.terms)
+                                : group_fg<R>(fc, g, lc, red, scratch, f, gd, sbg, S.terms, MODE_FG)))
         ok = false;
       if (threadIdx.x == 0) S.nfg_total++;
     }
@@ -1069,7 +1071,7 @@ struct smili_batch {
   int* d_queue = nullptr;
   unsigned* d_bars = nullptr;
   double* d_red_part = nullptr;
-  double* d_red_out = nullptr;
+  int redk = SMILI_REDK;
   int* d_grp_prob = nullptr;
   int* d_abort = nullptr;
   unsigned long long* d_prof = nullptr;
@@ -1092,7 +1094,7 @@ int launch_batch(smili_batch* b, int mode, float* ms) {
   const size_t aux_reset = 0;
   (void)aux_reset;
   CUDA_TRY(cudaMemsetAsync(b->d_queue, 0, sizeof(int), b->stream));
-  CUDA_TRY(cudaMemsetAsync(b->d_bars, 0, sizeof(unsigned) * 2 * b->ngroups, b->stream));
+  CUDA_TRY(cudaMemsetAsync(b->d_bars, 0, sizeof(unsigned) * 8 * b->ngroups, b->stream));
   CUDA_TRY(cudaMemsetAsync(b->d_abort, 0, sizeof(int), b->stream));
   BatchArgs a;
   a.arena = b->d_arena;
@@ -1103,7 +1105,7 @@ int launch_batch(smili_batch* b, int mode, float* ms) {
   a.queue = b->d_queue;
   a.bars = b->d_bars;
   a.red_part = b->d_red_part;
-  a.red_out = b->d_red_out;
+  a.redk = b->redk;
   a.grp_prob = b->d_grp_prob;
   a.abort_flag = b->d_abort;
   a.results = b->d_results;
@@ -1256,9 +1258,8 @@ int finish_batch(smili_batch* b, std::vector<HostProb>& hps, int maxn, const smi
     return o;
   };
   const size_t o_desc = take(sizeof(ProbDesc) * nprob), o_res = take(sizeof(ProbResult) * nprob),
-               o_q = take(sizeof(int)), o_bar = take(sizeof(unsigned) * 2 * b->ngroups),
-               o_rp = take(sizeof(double) * (size_t)b->ngroups * G * SMILI_REDK),
-               o_ro = take(sizeof(double) * (size_t)b->ngroups * SMILI_REDK),
+               o_q = take(sizeof(int)), o_bar = take(sizeof(unsigned) * 8 * b->ngroups),
+               o_rp = take(sizeof(double) * (size_t)b->ngroups * 2 * G * b->redk),
                o_gp = take(sizeof(int) * b->ngroups), o_ab = take(sizeof(int)),
                o_pf = take(sizeof(unsigned long long) * PR_NSTAGE);
   if (cudaMalloc(&b->d_aux, aux) != cudaSuccess) return cleanup(fail(SMILI_ERR_CUDA, "cudaMalloc aux failed"));
@@ -1267,7 +1268,6 @@ int finish_batch(smili_batch* b, std::vector<HostProb>& hps, int maxn, const smi
   b->d_queue = reinterpret_cast<int*>(b->d_aux + o_q);
   b->d_bars = reinterpret_cast<unsigned*>(b->d_aux + o_bar);
   b->d_red_part = reinterpret_cast<double*>(b->d_aux + o_rp);
-  b->d_red_out = reinterpret_cast<double*>(b->d_aux + o_ro);
   b->d_grp_prob = reinterpret_cast<int*>(b->d_aux + o_gp);
   b->d_abort = reinterpret_cast<int*>(b->d_aux + o_ab);
   b->d_prof = reinterpret_cast<unsigned long long*>(b->d_aux + o_pf);
@@ -2249,6 +2249,7 @@ int calc_cost_noalloc(const smili_imaging_args* a, const double* x, const smili_
   G = std::min(G, maxres);
   b.G = G;
   b.ngroups = 1;
+  b.redk = SMILI_REDK_FG;
   // bookkeeping after the arena, laid out as in create_batch
   size_t off = arena_al;
   auto take = [&](size_t n) {
@@ -2257,8 +2258,8 @@ int calc_cost_noalloc(const smili_imaging_args* a, const double* x, const smili_
     return o;
   };
   const size_t o_desc = take(sizeof(ProbDesc)), o_res = take(sizeof(ProbResult)), o_q = take(sizeof(int)),
-               o_bar = take(sizeof(unsigned) * 2), o_rp = take(sizeof(double) * (size_t)G * SMILI_REDK),
-               o_ro = take(sizeof(double) * SMILI_REDK), o_gp = take(sizeof(int)), o_ab = take(sizeof(int)),
+               o_bar = take(sizeof(unsigned) * 8), o_rp = take(sizeof(double) * (size_t)2 * G * b.redk),
+               o_gp = take(sizeof(int)), o_ab = take(sizeof(int)),
                o_pf = take(sizeof(unsigned long long) * PR_NSTAGE);
   if (off > kNoAllocBytes)
     return fail(SMILI_ERR_ARG, "smili_calc_cost_noalloc: the problem needs " + std::to_string(off) +
@@ -2272,7 +2273,6 @@ int calc_cost_noalloc(const smili_imaging_args* a, const double* x, const smili_
   b.d_queue = reinterpret_cast<int*>(scratch + o_q);
   b.d_bars = reinterpret_cast<unsigned*>(scratch + o_bar);
   b.d_red_part = reinterpret_cast<double*>(scratch + o_rp);
-  b.d_red_out = reinterpret_cast<double*>(scratch + o_ro);
   b.d_grp_prob = reinterpret_cast<int*>(scratch + o_gp);
   b.d_abort = reinterpret_cast<int*>(scratch + o_ab);
   b.d_prof = reinterpret_cast<unsigned long long*>(scratch + o_pf);
