@@ -392,6 +392,29 @@ __device__ __noinline__ void fg_t2_cols(FgCtx<R>& c, const GroupCtx& g) {
   }
 }
 
+// The kernel weights of every uv point, taps[q][j] = psi at tap q < w of axis 1
+// and [w + q][j] of axis 2, once per launch (FP64; P.o_taps).  The points do
+// not move, and 2 w exponentials and roots per point and use cost more than
+// everything else interpolation and spreading do in FP64; read back, they
+// are 16 w coalesced bytes.  FP32 evaluates them with the hardware
+// exponential each time: the table would not stay in L2 beside a batch.
+template <typename R>
+__device__ __noinline__ void fg_taps(const ProbDesc& P, char* base, const GroupCtx& g) {
+  const R* xu = at<R>(base, P.o_u);
+  const R* xv = at<R>(base, P.o_v);
+  R* taps = at<R>(base, P.o_taps);
+  const int w = P.w, n = P.nuv;
+  const R beta = (R)P.beta, half = (R)0.5 * (R)w, inv = (R)1 / half;
+  for (int i = g.rank * blockDim.x + threadIdx.x; i < 2 * n; i += g.G * blockDim.x) {
+    const int j = i < n ? i : i - n;
+    const R x = i < n ? xu[j] : xv[j];
+    const int l = (int)ceil(x - half);
+    R* t = taps + (i < n ? (size_t)0 : (size_t)w * n) + j;
+#pragma unroll 4
+    for (int q = 0; q < w; ++q) t[(size_t)q * n] = es_kernel(((R)(l + q) - x) * inv, beta);
+  }
+}
+
 // Interpolation of the points j = j0, j0 + dj, ... < nuv from the band:
 // V_j = sum_b psi(v_j - l2 - b) sum_a psi(u_j - l1 - a) band[l2 + b][l1 + a].
 // The kernel width W is a template constant so both tap vectors stay in
@@ -399,17 +422,25 @@ __device__ __noinline__ void fg_t2_cols(FgCtx<R>& c, const GroupCtx& g) {
 template <int W, typename R>
 __device__ __noinline__ void interp_points(const ProbDesc& P, const R* __restrict__ xu, const R* __restrict__ xv,
                                               const cpx<R>* bandA, cpx<R>* V, cpx<R>* cacc, R beta, int j0,
-                                              int dj) {
+                                              int dj, const R* taps) {
   const R half = (R)0.5 * (R)W;
   const R inv = (R)1 / half;
   for (int j = j0; j < P.nuv; j += dj) {
     const R x1 = xu[j], x2 = xv[j];
     const int l1 = (int)ceil(x1 - half), l2 = (int)ceil(x2 - half);
     R k1[W], k2[W];
+    if (taps) {
 #pragma unroll
-    for (int a = 0; a < W; ++a) {
-      k1[a] = es_kernel(((R)(l1 + a) - x1) * inv, beta);
-      k2[a] = es_kernel(((R)(l2 + a) - x2) * inv, beta);
+      for (int a = 0; a < W; ++a) {
+        k1[a] = taps[(size_t)a * P.nuv + j];
+        k2[a] = taps[(size_t)(W + a) * P.nuv + j];
+      }
+    } else {
+#pragma unroll
+      for (int a = 0; a < W; ++a) {
+        k1[a] = es_kernel(((R)(l1 + a) - x1) * inv, beta);
+        k2[a] = es_kernel(((R)(l2 + a) - x2) * inv, beta);
+      }
     }
     const int c1 = imod(l1 - P.b1s, P.nf1), c2 = imod(l2 - P.b2s, P.nf2);
     R ar = 0, ai = 0;
@@ -447,6 +478,7 @@ __device__ void fg_interp(FgCtx<R>& c, const GroupCtx& g, bool zero_acc) {
   const cpx<R>* gband = at<cpx<R>>(c.base, P.o_bandA);
   cpx<R>* V = at<cpx<R>>(c.base, P.o_V);
   cpx<R>* cacc = zero_acc ? at<cpx<R>>(c.base, P.o_contrib) : nullptr;
+  const R* taps = P.o_taps ? at<R>(c.base, P.o_taps) : nullptr;
   const int w = P.w;
   const R beta = (R)P.beta;
   const int ncell = P.b1n * P.b2n;
@@ -464,11 +496,11 @@ __device__ void fg_interp(FgCtx<R>& c, const GroupCtx& g, bool zero_acc) {
   const int j0 = g.rank * blockDim.x + threadIdx.x, dj = g.G * blockDim.x;
   switch (w) {
 #define SMILI_INTERP_W(W) \
-  case W: interp_points<W>(P, xu, xv, bandA, V, cacc, beta, j0, dj); break;
+  case W: interp_points<W>(P, xu, xv, bandA, V, cacc, beta, j0, dj, taps); break;
     SMILI_INTERP_W(2) SMILI_INTERP_W(3) SMILI_INTERP_W(4) SMILI_INTERP_W(5) SMILI_INTERP_W(6)
     SMILI_INTERP_W(7) SMILI_INTERP_W(8) SMILI_INTERP_W(9) SMILI_INTERP_W(10) SMILI_INTERP_W(11)
     SMILI_INTERP_W(12) SMILI_INTERP_W(13) SMILI_INTERP_W(14) SMILI_INTERP_W(15)
-    default: interp_points<16>(P, xu, xv, bandA, V, cacc, beta, j0, dj); break;  // w <= SMILI_MAXW = 16
+    default: interp_points<16>(P, xu, xv, bandA, V, cacc, beta, j0, dj, taps); break;  // w <= SMILI_MAXW = 16
 #undef SMILI_INTERP_W
   }
   __syncthreads();
@@ -824,8 +856,147 @@ __device__ __noinline__ void fg_spread_tc(FgCtx<float>& c, const GroupCtx& g) {
   }
 }
 
+// ---------------------------------------------------------------------------
+// F5 in FP64 with the subgrid in registers (w <= 9, 8 x 8 tiles).  The warps
+// take equal contiguous ranges of the sorted points (at least 32), so that no
+// warp walks a 128-point item while others have none.  A warp holds its
+// tile's 16 x 16 subgrid as 8 rows of one column per lane; a point's weights
+// sit in a zero-padded 16-entry row per axis in shared memory at its offset
+// inside the tile, so a lane reads its column's weight, the 8 row weights
+// (the same address in half a warp) and does 16 independent FMAs: no tap
+// waits on the point before, as it does with a subgrid in shared memory.  The
+// tile is added to the band when the next point lies in another one.
+// 256 x 256 / 97 200 points, 64 CTAs, a solve's stage with its barrier: 126 us
+// with shared subgrids and the weights evaluated each time, 33 us with
+// this and fg_taps.
+// ---------------------------------------------------------------------------
+constexpr int SPREAD_ROW = 34;  // 16 axis-1 weights, 16 axis-2 weights, Re c, Im c
+template <int W>
+__device__ __noinline__ void fg_spread_reg(FgCtx<double>& c, const GroupCtx& g) {
+  const ProbDesc& P = *c.P;
+  const double* xu = at<double>(c.base, P.o_u);
+  const double* xv = at<double>(c.base, P.o_v);
+  const double* taps = P.o_taps ? at<double>(c.base, P.o_taps) : nullptr;
+  const int4* items = at<int4>(c.base, P.o_items);
+  const cpx<double>* cacc = at<cpx<double>>(c.base, P.o_contrib);
+  double* gband = at<double>(c.base, P.o_bandC);
+  const double beta = P.beta, half = 0.5 * W, inv = 1.0 / half;
+  const int nuv = P.nuv, nf1 = P.nf1, nf2 = P.nf2, b1s = P.b1s, b2s = P.b2s, b1n = P.b1n, b2n = P.b2n;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int col = lane & 15, r0 = (lane >> 4) * 8;
+  double* tab = reinterpret_cast<double*>(c.sbuf) + (size_t)warp * 32 * SPREAD_ROW;
+  const int nwt = g.G * nw, gw = g.rank * nw + warp;
+  const int share = max(32, (nuv + nwt - 1) / nwt);
+  const long first = (long)gw * share;
+  if (first >= nuv) return;
+  const int p0 = (int)first, p1 = min(nuv, p0 + share);
+  // the item that holds p0 (items cover the points in order)
+  int it = 0;
+  for (int hi = P.nitems; hi - it > 1;) {
+    const int mid = (it + hi) >> 1;
+    if (items[mid].x <= p0) it = mid;
+    else hi = mid;
+  }
+  double ar[8], ai[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) ar[i] = ai[i] = 0.0;
+  int trow = -1, tcol = -1;
+  auto flush = [&]() {
+    int cl = tcol + col;
+    if (cl >= nf1) cl -= nf1;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      int rw = trow + r0 + i;
+      if (rw >= nf2) rw -= nf2;
+      // outside the tile's 8 + W - 1 cells, or beyond the band, only zero taps land
+      if (r0 + i < 8 + W - 1 && col < 8 + W - 1 && rw < b2n && cl < b1n && (ar[i] != 0.0 || ai[i] != 0.0)) {
+        double* dst = gband + 2 * ((size_t)rw * b1n + cl);
+        atomicAdd(dst, ar[i]);
+        atomicAdd(dst + 1, ai[i]);
+      }
+      ar[i] = ai[i] = 0.0;
+    }
+  };
+  for (int jb = p0; jb < p1; ++it) {
+    const int4 item = items[it];
+    if (item.z != trow || item.w != tcol) {
+      if (trow >= 0) flush();
+      trow = item.z;
+      tcol = item.w;
+    }
+    const int je = min(p1, item.y);
+    for (; jb < je; jb += 32) {
+      const int np = min(32, je - jb);
+      if (lane < np) {
+        const int j = jb + lane;
+        double* row = tab + lane * SPREAD_ROW;
+        const cpx<double> cj = cacc[j];
+        const double x1 = xu[j], x2 = xv[j];
+        const int l1 = (int)ceil(x1 - half), l2 = (int)ceil(x2 - half);
+        double k1[W], k2[W];
+        if (taps) {
+#pragma unroll
+          for (int q = 0; q < W; ++q) {
+            k1[q] = taps[(size_t)q * nuv + j];
+            k2[q] = taps[(size_t)(W + q) * nuv + j];
+          }
+        } else {
+#pragma unroll
+          for (int q = 0; q < W; ++q) {
+            k1[q] = es_kernel(((double)(l1 + q) - x1) * inv, beta);
+            k2[q] = es_kernel(((double)(l2 + q) - x2) * inv, beta);
+          }
+        }
+        const int lc = imod(l1 - b1s, nf1) - tcol, lr = imod(l2 - b2s, nf2) - trow;  // in [0, 8)
+#pragma unroll
+        for (int q = 0; q < 16; ++q) reinterpret_cast<double2*>(row)[q] = make_double2(0.0, 0.0);
+        reinterpret_cast<double2*>(row)[16] = make_double2(cj.x, -cj.y);  // c = Vresre - i Vresim
+#pragma unroll
+        for (int q = 0; q < W; ++q) {
+          row[lc + q] = k1[q];
+          row[16 + lr + q] = k2[q];
+        }
+      }
+      __syncwarp();
+#pragma unroll 2
+      for (int p = 0; p < np; ++p) {
+        const double* row = tab + p * SPREAD_ROW;
+        const double2 cv = *reinterpret_cast<const double2*>(row + 32);
+        const double wx = row[col];
+        const double2* wy = reinterpret_cast<const double2*>(row + 16 + r0);
+        const double a = wx * cv.x, b = wx * cv.y;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const double2 y = wy[i];
+          ar[2 * i] += y.x * a;
+          ai[2 * i] += y.x * b;
+          ar[2 * i + 1] += y.y * a;
+          ai[2 * i + 1] += y.y * b;
+        }
+      }
+      __syncwarp();
+    }
+    jb = je;
+  }
+  flush();
+}
+
 template <typename R>
 __device__ __noinline__ void fg_spread(FgCtx<R>& c, const GroupCtx& g) {
+  if constexpr (std::is_same<R, double>::value) {
+    // 69 632 bytes of weight rows for 8 warps, of the 98 304 an FP64 CTA has
+    static_assert((size_t)Shape<double>::warps * 32 * SPREAD_ROW * 8 <= 6144 * sizeof(cpx<double>), "weight rows");
+    if (c.P->bin == 8) {
+      switch (c.P->w) {
+#define SMILI_SPREAD_W(W) \
+  case W: fg_spread_reg<W>(c, g); return;
+        SMILI_SPREAD_W(2) SMILI_SPREAD_W(3) SMILI_SPREAD_W(4) SMILI_SPREAD_W(5) SMILI_SPREAD_W(6)
+        SMILI_SPREAD_W(7) SMILI_SPREAD_W(8) SMILI_SPREAD_W(9)
+#undef SMILI_SPREAD_W
+        default: break;  // a subgrid wider than 16 cells
+      }
+    }
+  }
   if constexpr (std::is_same<R, float>::value) {
     if (c.P->w <= 9 && c.P->bin == 8) {
       fg_spread_tc(c, g);

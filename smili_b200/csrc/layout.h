@@ -71,6 +71,7 @@ struct ProbDesc {
   int64_t o_l1w, o_tvw, o_tsvw, o_klw, o_gsw;
   int64_t o_dc1, o_dc2, o_tw1, o_tw2;   // deconvolution factors, twiddle tables
   int64_t o_u, o_v;                     // fine-grid coordinates xi = u n / 2pi (R)
+  int64_t o_taps;                       // kernel weights [2 w][nuv] (R), written at the launch's start, or 0
   int64_t o_dre, o_dim, o_dvar;         // per datum: value(s) and variance (R)
   int64_t o_didx;                       // per slot: 0-based uv index (sorted order)
   int64_t o_dsgn;                       // per slot: sign (+1 / -1) as int8
@@ -92,7 +93,7 @@ struct ProbDesc {
 // every arena offset of ProbDesc, for code that moves a problem's region
 #define SMILI_PROB_OFFSETS(X)                                                                          \
   X(o_x0) X(o_xidx) X(o_yidx) X(o_inv) X(o_xg) X(o_ex) X(o_ey) X(o_l1w) X(o_tvw) X(o_tsvw) X(o_klw)  \
-  X(o_gsw) X(o_dc1) X(o_dc2) X(o_tw1) X(o_tw2) X(o_u) X(o_v) X(o_dre) X(o_dim) X(o_dvar) X(o_didx)   \
+  X(o_gsw) X(o_dc1) X(o_dc2) X(o_tw1) X(o_tw2) X(o_u) X(o_v) X(o_taps) X(o_dre) X(o_dim) X(o_dvar) X(o_didx)   \
   X(o_dsgn) X(o_items) X(o_tmpA) X(o_bandA) X(o_V) X(o_contrib) X(o_bandC) \
   X(o_tmpC) X(o_gchi) X(o_part) X(o_x) X(o_g) X(o_z) X(o_r) X(o_d) X(o_t) X(o_xp) X(o_ws) X(o_wy)     \
   X(o_iwh) X(o_free) X(o_bkey) X(o_sbk) X(o_sbi) X(o_hist) X(o_cand) X(o_lred) X(o_state) X(o_trace) \

@@ -401,6 +401,14 @@ __global__ void __launch_bounds__(Shape<R>::threads, Shape<R>::min_blocks) smili
       }
       __syncthreads();
     }
+    // the kernel weights of the launch's evaluations
+    if (P.o_taps) {
+      fg_taps<R>(P, base, g);
+    } else if (P.nframes > 0) {
+      const ProbDesc* frames = at<ProbDesc>(base, P.o_frames);
+      for (int z = 0; z < P.nframes; ++z)
+        if (frames[z].o_taps) fg_taps<R>(frames[z], base, g);
+    }
     bool ok = group_sync(g);
     prof.mark(PR_INIT);
     while (ok) {
@@ -544,6 +552,20 @@ size_t dyn_smem_bytes() {
   return b;
 }
 
+// PK_FRAME: one frame of a movie; PK_MODEL: one evaluation that also returns per-datum models
+enum { PK_SOLVE = 0, PK_FG = 1, PK_T2 = 2, PK_T1 = 3, PK_FRAME = 4, PK_MODEL = 5 };
+
+// Whether the problems of a launch keep their kernel weights (fg_taps): FP64
+// launches that use them at least twice (a bare transform uses them once),
+// unless the tables would take more than 16 GB of the device's memory.
+template <typename R>
+bool keep_taps(int kind, double eps, double nuv_total) {
+  int w;
+  double beta;
+  es_params(eps, w, beta);
+  return sizeof(R) == 8 && kind != PK_T1 && kind != PK_T2 && nuv_total * 2 * w * sizeof(R) <= 16e9;
+}
+
 struct Arena {
   size_t bytes = 0;
   int64_t take(size_t nbytes) {
@@ -574,9 +596,6 @@ struct HostProb {
     put(off, v.data(), v.size());
   }
 };
-
-// PK_FRAME: one frame of a movie; PK_MODEL: one evaluation that also returns per-datum models
-enum { PK_SOLVE = 0, PK_FG = 1, PK_T2 = 2, PK_T1 = 3, PK_FRAME = 4, PK_MODEL = 5 };
 
 // The order of [0, n) by key(i) in [0, nkey), ties in index order: a
 // counting sort, the same order as std::stable_sort by key in O(n + nkey).
@@ -612,7 +631,7 @@ template <typename R>
 int pack_problem(const smili_imaging_args& a, int kind, int niter, int nonneg, int m, double factr,
                  double pgtol, double eps, Arena& ar, HostProb& hp, const double* x_override,
                  const double* c_re, const double* c_im, double wtotal_override = 0.0, int bin = 8,
-                 int transform = 0) {
+                 int transform = 0, bool taps = false) {
   ProbDesc& d = hp.d;
   std::memset(&d, 0, sizeof(d));
   const int N = a.npix, nx = a.nx, ny = a.ny, nuv = a.nuv;
@@ -971,6 +990,7 @@ int pack_problem(const smili_imaging_args& a, int kind, int niter, int nonneg, i
   }
   d.o_u = ar.take(sizeof(R) * nuv);
   d.o_v = ar.take(sizeof(R) * nuv);
+  if (taps) d.o_taps = ar.take(sizeof(R) * 2 * w * (size_t)nuv);
   d.o_dre = ar.take(sizeof(R) * dre.size());
   d.o_dim = ar.take(sizeof(R) * dim.size());
   d.o_dvar = ar.take(sizeof(R) * dvar.size());
@@ -1159,6 +1179,9 @@ int create_batch(int nprob, const smili_imaging_args* const* probs, const int* n
   std::vector<HostProb> hps(nprob);
   std::vector<int> rcs(nprob, SMILI_OK);
   std::vector<std::string> errs(nprob);
+  double nuv_total = 0;
+  for (int p = 0; p < nprob; ++p) nuv_total += std::max(probs[p]->nuv, 0);
+  const bool taps = keep_taps<R>(kind, eps, nuv_total);
   std::atomic<int> next{0};
   auto work = [&]() {
     for (int p = next.fetch_add(1); p < nprob; p = next.fetch_add(1)) {
@@ -1166,7 +1189,7 @@ int create_batch(int nprob, const smili_imaging_args* const* probs, const int* n
         ars[p].take(256);
         rcs[p] = pack_problem<R>(*probs[p], kind, niter ? niter[p] : 0, nonneg, m, factr, pgtol, eps, ars[p],
                                  hps[p], x_over ? x_over[p] : nullptr, c_re, c_im, 0.0,
-                                 opt && opt->spread_bin ? opt->spread_bin : 8, opt ? opt->transform : 0);
+                                 opt && opt->spread_bin ? opt->spread_bin : 8, opt ? opt->transform : 0, taps);
         if (rcs[p] != SMILI_OK) errs[p] = g_err;
       } catch (const std::exception& ex) {
         rcs[p] = SMILI_ERR_ARG;
@@ -1533,7 +1556,7 @@ int pack_movie(const smili_imaging3d_args& a, int kind, int niter, int nonneg, i
     fa.wca = a.wca;
     fa.inormfactr = a.inormfactr;
     if ((rc = pack_problem<R>(fa, PK_FRAME, 0, nonneg, m, factr, pgtol, eps, ar, fh[z], nullptr, nullptr, nullptr,
-                              wtotal, spread_bin, transform)) != SMILI_OK)
+                              wtotal, spread_bin, transform, keep_taps<R>(PK_FRAME, eps, nuv))) != SMILI_OK)
       return rc;
     ProbDesc& F = fh[z].d;
     F.o_x = d.o_x + (int64_t)sizeof(double) * z * N;
@@ -1601,7 +1624,8 @@ int create_model(const smili_imaging_args& a, const double* x, const smili_optio
   Arena ar;
   std::vector<HostProb> hps(1);
   const int rc = pack_problem<R>(b0, PK_MODEL, 0, 0, 5, 1e1, 0.0, eps, ar, hps[0], x, nullptr, nullptr, w,
-                                 opt && opt->spread_bin ? opt->spread_bin : 8, opt ? opt->transform : 0);
+                                 opt && opt->spread_bin ? opt->spread_bin : 8, opt ? opt->transform : 0,
+                                 keep_taps<R>(PK_MODEL, eps, std::max(a.nuv, 0)));
   if (rc != SMILI_OK) {
     delete b;
     return rc;
