@@ -198,17 +198,21 @@ __device__ __noinline__ bool group_combine(GroupCtx& g, int K, int ns, double* o
   return true;
 }
 
+// doubles of shared scratch the reductions need with T threads: one per
+// thread, or up to 40 values per warp
+#define SMILI_SCRATCH(T) ((T) / 32 * 40)
+
 // the row this CTA writes before group_combine
 __device__ __forceinline__ double* group_row(GroupCtx& g, double* out) {
   return g.G == 1 ? out : g.red_part + ((size_t)g.parity * g.G + g.rank) * g.redk;
 }
 
-// Group-wide sums of s[0..NS) and maxima of x[0..NX) over all threads:
-// out[0..NS) and out[NS..NS+NX) (shared) in every CTA.  s is clobbered.
-// scratch: max(blockDim.x, warps * (NS + NX)) doubles of shared memory.
+// Sums of s[0..NS) and maxima of x[0..NX) over the block's threads into
+// row[0..NS) and row[NS..NS+NX).  s is clobbered.
 template <int NS, int NX>
-__device__ __noinline__ bool group_reduce(GroupCtx& g, double (&s)[NS], const double (&x)[NX], double* out, double* scratch) {
+__device__ __forceinline__ void block_partials(double (&s)[NS], const double (&x)[NX], double* row, double* scratch) {
   constexpr int K = NS + NX, L = 32 / NS;
+  static_assert(K <= 40, "scratch");
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const double v = warp_fold<NS>(s, lane);
   if (lane % L == 0) scratch[wid * K + lane / L] = v;
@@ -227,9 +231,18 @@ __device__ __noinline__ bool group_reduce(GroupCtx& g, double (&s)[NS], const do
       const double b = scratch[w * K + threadIdx.x];
       a = (int)threadIdx.x < NS ? a + b : fmax(a, b);
     }
-    group_row(g, out)[threadIdx.x] = a;
+    row[threadIdx.x] = a;
   }
-  return group_combine(g, K, NS, out, scratch);
+}
+
+// Group-wide sums of s[0..NS) and maxima of x[0..NX) over all threads:
+// out[0..NS) and out[NS..NS+NX) (shared) in every CTA.  s is clobbered.
+// scratch: SMILI_SCRATCH(blockDim.x) doubles of shared memory.
+template <int NS, int NX>
+__device__ __noinline__ bool group_reduce(GroupCtx& g, double (&s)[NS], const double (&x)[NX], double* out,
+                                          double* scratch) {
+  block_partials<NS, NX>(s, x, group_row(g, out), scratch);
+  return group_combine(g, NS + NX, NS, out, scratch);
 }
 
 // ---------------------------------------------------------------------------

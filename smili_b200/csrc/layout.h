@@ -82,7 +82,7 @@ struct ProbDesc {
   // optimiser (double precision)
   int64_t o_x, o_g, o_z, o_r, o_d, o_t, o_xp, o_ws, o_wy, o_iwh, o_free, o_bkey;
   int64_t o_sbk, o_sbi, o_hist;         // bucketed breakpoints, bucket counts/cursors
-  int64_t o_cand, o_lred, o_state;
+  int64_t o_cand, o_state;
   int64_t o_trace;                      // cost at each NEW_X (double[niter+2])
   int64_t o_model;                      // per datum: model re, im, residual re, im (double), or 0
   int64_t o_frames;                     // movie: ProbDesc[nframes]
@@ -96,7 +96,7 @@ struct ProbDesc {
   X(o_gsw) X(o_dc1) X(o_dc2) X(o_tw1) X(o_tw2) X(o_u) X(o_v) X(o_taps) X(o_dre) X(o_dim) X(o_dvar) X(o_didx)   \
   X(o_dsgn) X(o_items) X(o_tmpA) X(o_bandA) X(o_V) X(o_contrib) X(o_bandC) \
   X(o_tmpC) X(o_gchi) X(o_part) X(o_x) X(o_g) X(o_z) X(o_r) X(o_d) X(o_t) X(o_xp) X(o_ws) X(o_wy)     \
-  X(o_iwh) X(o_free) X(o_bkey) X(o_sbk) X(o_sbi) X(o_hist) X(o_cand) X(o_lred) X(o_state) X(o_trace) \
+  X(o_iwh) X(o_free) X(o_bkey) X(o_sbk) X(o_sbi) X(o_hist) X(o_cand) X(o_state) X(o_trace) \
   X(o_model) X(o_frames) X(o_rtw) X(o_riw) X(o_lcf) X(o_iavg) X(o_out)
 
 // Scalar L-BFGS-B state (setulb's isave/dsave/lsave plus the small matrices).

@@ -12,9 +12,9 @@
 //    active sets instead of updating it with entering / leaving variables
 //    (same matrix in exact arithmetic, lbfgsb.f:1848-2172);
 //  * the generalized Cauchy point (cauchy, lbfgsb.f:1222-1719) visits the
-//    breakpoints in increasing (t, index) order, taken in batches by radix
-//    selection, and evaluates the piecewise quadratic in closed form from
-//    prefix sums (D_k = sum d^2 over moving variables, P_k = W'd_k,
+//    breakpoints in increasing (t, index) order, bucketed and then sorted by
+//    the CTAs of the group, and evaluates the piecewise quadratic in closed
+//    form from prefix sums (D_k = sum d^2 over moving variables, P_k = W'd_k,
 //    Q_k = sum t_i d_i w_i), instead of popping a heap and updating f1, f2
 //    incrementally.  The f2 safeguard max(eps*f2_org, f2) is applied per
 //    segment.  Ties between equal breakpoints are visited in index order.
@@ -26,7 +26,7 @@
 #include "common.cuh"
 
 #define SMILI_MAXM_DEV 6  // largest L-BFGS-B memory the device solver accepts
-#define SMILI_KC 1024     // breakpoints per selection round of the Cauchy search
+#define SMILI_KC 1024     // breakpoints of one sorted batch of the Cauchy search
 
 typedef unsigned __int128 u128;
 
@@ -45,7 +45,6 @@ struct LbCtxT {
   signed char* iwh;
   unsigned char* freef;
   unsigned long long* bkey;
-  double* lred;   // global scratch for results of the group-leader scan
   double* trace;
   double* red;    // shared [SMILI_REDK]
   double* scratch;  // shared, blockDim.x doubles (group_reduce)
@@ -369,9 +368,9 @@ __device__ void lb_init(LbCtxT<SY>& c, const double* x0) {
 // ---------------------------------------------------------------------------
 // Cauchy point
 // ---------------------------------------------------------------------------
-// results written by the group leader to c.lred (global) for all CTAs
+// result of the search
 enum {
-  CR_INFO = 0, CR_MODE, CR_TSUM, CR_NSEG, CR_BHI, CR_BLO, CR_C  // CR_C.. 2m values of c
+  CR_INFO = 0, CR_MODE, CR_TSUM, CR_NSEG, CR_BHI, CR_BLO, CR_C  // CR_C.. 6 + 6 values of c (Y and S part)
 };
 enum { CM_NONE_FIXED = 0, CM_BOUNDARY = 1, CM_XCP_IS_X = 2 };
 
@@ -379,65 +378,61 @@ __device__ __forceinline__ u128 comp_key(unsigned long long key, int idx) {
   return ((u128)key << 32) | (u128)(unsigned)idx;
 }
 
-// Block-wide inclusive scan of V values per thread (vals in/out), V <= 32.
-__device__ void block_scan_incl(double* vals, int V, double* wtot /* shared [WARPS][32] */) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  for (int v = 0; v < V; ++v) {
-    double a = vals[v];
-    for (int s = 1; s < 32; s <<= 1) {
-      const double o = __shfl_up_sync(0xffffffffu, a, s);
-      if (lane >= s) a += o;
-    }
-    vals[v] = a;
-    if (lane == 31) wtot[wid * 32 + v] = a;
-  }
-  __syncthreads();
-  for (int v = 0; v < V; ++v) {
-    double pre = 0.0;
-    for (int w = 0; w < wid; ++w) pre += wtot[w * 32 + v];
-    vals[v] += pre;
-  }
-  __syncthreads();
-}
+// Breakpoint buckets.  Keys are the IEEE bits of the breakpoint times t > 0,
+// which order like the times; bucket = (key - kmin) >> shift, the outermost
+// buckets taking what lies outside.  2048 buckets, or 4096 for more than
+// 131 072 variables, so that the crowded ones stay near a CTA's sort.
+#define SMILI_NBUCKET_MAX 4096
+__device__ __forceinline__ int cauchy_buckets(int n) { return n > 131072 ? 4096 : 2048; }
 
-// Breakpoint bucketing (all CTAs of the group).  Keys are the IEEE bits of
-// the breakpoint times t > 0, which order like the times; bucket =
-// (key - kmin) >> shift, with the shift chosen so that the keys span at most
-// SMILI_NBUCKET buckets.  sbk/sbi receive the breakpoints grouped by bucket in
-// increasing bucket order (unordered inside a bucket); hist the bucket counts.
-#define SMILI_NBUCKET 2048
-
-__device__ __forceinline__ int bucket_of(unsigned long long k, unsigned long long kmin, int shift) {
+__device__ __forceinline__ int bucket_of(unsigned long long k, unsigned long long kmin, int shift, int nb) {
+  if (k <= kmin) return 0;
   const unsigned long long q = (k - kmin) >> shift;
-  return q < (unsigned long long)SMILI_NBUCKET ? (int)q : SMILI_NBUCKET - 1;
+  return q < (unsigned long long)nb ? (int)q : nb - 1;
 }
+
+// Shared memory of the search inside the dynamic region
+struct CauchySmem {
+  unsigned start[SMILI_NBUCKET_MAX + 4];                // first position of each bucket; [nb] = nbreak
+  u128 cand[SMILI_KC];                                  // one batch of (key, index)
+  unsigned hist2[256];                                  // digits of the oversized-bucket selection
+  double wtot[SMILI_MAX_WARPS][28];                     // warp totals of the scan
+  double a_s[SMILI_MAX_THREADS], b_s[SMILI_MAX_THREADS];
+  double Mm[144];                                       // dense middle matrix, 6 + 6 rows and columns
+  double st[3];                                         // D, t, dtm at the last element passed
+  double P[12], Q[12];                                  // p and sum t d w there
+  double cum[32];                                       // sums over the rounds done: d^2, d w, t d w, max t
+  double pre[32], tot[32];
+};
+// Bytes of dynamic shared memory; the launch gives every CTA at least this much.
+constexpr size_t SMILI_CAUCHY_SMEM = sizeof(CauchySmem);
 
 // Select the next batch (<= SMILI_KC elements, the smallest composites above
 // lo_key) from the unordered range [r0, r1) of the bucketed arrays into cand,
-// by radix selection on 12-bit digits of the 96-bit composite (key, index).
+// by radix selection on 8-bit digits of the 96-bit composite (key, index).
 // Used for a bucket that holds more than SMILI_KC breakpoints.
 template <typename SY>
 __device__ __noinline__ int select_from_range(LbCtxT<SY>& c, const unsigned long long* sbk, const int* sbi, int r0,
-                                 int r1, u128 lo_key, u128* cand, unsigned* hist) {
+                                              int r1, u128 lo_key, u128* cand, unsigned* hist) {
   __shared__ int cnt_s, vstar_s, cum_s;
   u128 prefix = 0;
   int level = 0, budget = SMILI_KC;
   u128 sel_hi = ~(u128)0;
   bool have_hi = false;
   while (true) {
-    const int shift = 96 - 12 * (level + 1);
-    for (int i = threadIdx.x; i < 4096; i += blockDim.x) hist[i] = 0;
+    const int shift = 96 - 8 * (level + 1);
+    for (int i = threadIdx.x; i < 256; i += blockDim.x) hist[i] = 0;
     __syncthreads();
     for (int i = r0 + threadIdx.x; i < r1; i += blockDim.x) {
       const u128 ck = comp_key(sbk[i], sbi[i]);
       if (ck <= lo_key) continue;
-      if (level > 0 && (ck >> (96 - 12 * level)) != prefix) continue;
-      atomicAdd(&hist[(unsigned)((ck >> shift) & 0xfffu)], 1u);
+      if (level > 0 && (ck >> (96 - 8 * level)) != prefix) continue;
+      atomicAdd(&hist[(unsigned)((ck >> shift) & 0xffu)], 1u);
     }
     __syncthreads();
     if (threadIdx.x == 0) {
       int cum = 0, vstar = -1;
-      for (int b = 0; b < 4096; ++b) {
+      for (int b = 0; b < 256; ++b) {
         if (cum + (int)hist[b] > budget) {
           vstar = b;
           break;
@@ -451,13 +446,13 @@ __device__ __noinline__ int select_from_range(LbCtxT<SY>& c, const unsigned long
     const int vstar = vstar_s, cum = cum_s;
     if (vstar < 0) {
       if (level > 0) {
-        sel_hi = (prefix + 1) << (96 - 12 * level);
+        sel_hi = (prefix + 1) << (96 - 8 * level);
         have_hi = true;
       }
       break;
     }
-    const u128 np = (prefix << 12) | (u128)vstar;
-    if (cum == budget || (cum > 0 && (4 * cum >= budget || level == 7))) {
+    const u128 np = (prefix << 8) | (u128)vstar;
+    if (cum == budget || (cum > 0 && (4 * cum >= budget || level == 11))) {
       sel_hi = np << shift;
       have_hi = true;
       break;
@@ -492,296 +487,452 @@ __device__ __noinline__ int select_from_range(LbCtxT<SY>& c, const unsigned long
   return cnt;
 }
 
-// Sequential-order scan of the bucketed breakpoints by one CTA (the group
-// leader): batches of whole buckets (<= SMILI_KC elements) are sorted by
-// (t, index) and swept with the closed-form piecewise quadratic.  Writes the
-// CR_* results.
-// Bytes of dynamic shared memory the scan lays out (cand, hist, hist2, wtot,
-// dtm_s, t_s, Mm, st); the launch gives every CTA at least this much.
-constexpr size_t SMILI_CAUCHY_SMEM =
-    16 * SMILI_KC + 4 * SMILI_NBUCKET + 4 * 4096 +
-    8 * (SMILI_MAX_WARPS * 32 + 2 * SMILI_MAX_THREADS + 4 * SMILI_MAXM_DEV * SMILI_MAXM_DEV + 5 + 4 * SMILI_MAXM_DEV);
-template <typename SY>
-__device__ __noinline__ void cauchy_scan(LbCtxT<SY>& c, double f1_0, const double* p0, int nbreak, int bnded,
-                            const unsigned long long* sbk, const int* sbi, const int* ghist) {
-  LbState& S = *c.S;
-  const int m = c.m, col = S.col, col2 = 2 * col, n = c.n;
-  const double theta = S.theta;
-  // shared layout inside dyn
-  u128* cand = reinterpret_cast<u128*>(c.dyn);                        // SMILI_KC
-  unsigned* hist = reinterpret_cast<unsigned*>(cand + SMILI_KC);      // NBUCKET (bucket counts)
-  unsigned* hist2 = hist + SMILI_NBUCKET;                             // 4096 (fallback)
-  double* wtot = reinterpret_cast<double*>(hist2 + 4096);             // MAX_WARPS*32
-  double* dtm_s = wtot + SMILI_MAX_WARPS * 32;                        // MAX_THREADS
-  double* t_s = dtm_s + SMILI_MAX_THREADS;                            // MAX_THREADS
-  double* Mm = t_s + SMILI_MAX_THREADS;                               // dense M (2col)^2
-  double* st = Mm + 4 * SMILI_MAXM_DEV * SMILI_MAXM_DEV;              // carried state
-  // st: [0]=D [1]=tprev [2]=dtm_cur [3..] unused [5..5+2m)=P [..+2m)=Q
-  __shared__ unsigned long long bnd_hi_s, bnd_lo_s;
-  __shared__ int e_star_s, info_s;
-  __shared__ double f2org_s;
-  double* Pst = st + 5;
-  double* Qst = Pst + 2 * SMILI_MAXM_DEV;
-  Prof& pf = *c.prof;
-  double* lr = c.lred;
+// Ascending bitonic sort of cand[0..cnt), cnt <= SMILI_KC.  Up to blockDim.x
+// elements it runs with one element per thread: strides below 32 by
+// shuffles, the others through shared memory (256 elements: 6 of 36 steps
+// need a block barrier).
+__device__ __noinline__ void sort_batch(u128* cand, int cnt) {
+  int np2 = 32;
+  while (np2 < cnt) np2 <<= 1;
+  for (int i = cnt + threadIdx.x; i < np2; i += blockDim.x) cand[i] = ~(u128)0;
+  __syncthreads();
+  if (np2 <= (int)blockDim.x) {
+    const int i = threadIdx.x;
+    const bool act = i < np2;  // whole warps: np2 is a multiple of 32
+    u128 v = act ? cand[i] : ~(u128)0;
+    for (int k2 = 2; k2 <= np2; k2 <<= 1) {
+      for (int j2 = k2 >> 1; j2 > 0; j2 >>= 1) {
+        u128 o;
+        if (j2 >= 32) {
+          if (act) cand[i] = v;
+          __syncthreads();
+          o = act ? cand[i ^ j2] : v;
+          __syncthreads();
+        } else {
+          const unsigned lo = __shfl_xor_sync(0xffffffffu, (unsigned)v, j2);
+          const unsigned mi = __shfl_xor_sync(0xffffffffu, (unsigned)(v >> 32), j2);
+          const unsigned hi = __shfl_xor_sync(0xffffffffu, (unsigned)(v >> 64), j2);
+          const unsigned pad = __shfl_xor_sync(0xffffffffu, (unsigned)(v >> 96), j2);
+          o = ((u128)pad << 96) | ((u128)hi << 64) | ((u128)mi << 32) | lo;
+        }
+        const bool up = (i & k2) == 0, lower = (i & j2) == 0;
+        if ((lower == up) == (o < v)) v = o;
+      }
+    }
+    if (act) cand[i] = v;
+    __syncthreads();
+    return;
+  }
+  for (int k2 = 2; k2 <= np2; k2 <<= 1) {
+    for (int j2 = k2 >> 1; j2 > 0; j2 >>= 1) {
+      for (int i = threadIdx.x; i < np2; i += blockDim.x) {
+        const int ixj = i ^ j2;
+        if (ixj > i) {
+          const u128 a = cand[i], b = cand[ixj];
+          const bool up = (i & k2) == 0;
+          if ((a > b) == up) {
+            cand[i] = b;
+            cand[ixj] = a;
+          }
+        }
+      }
+      __syncthreads();
+    }
+  }
+}
 
-  // dense middle matrix: column j = M e_j
+// f1 and f2 of the segment that starts at time t, from D, p and c = W'(z - x)
+// there (rows 0..5 the Y part, 6..11 the S part, zero past col), and its
+// minimiser's distance -f1 / f2
+__device__ __forceinline__ double segment_dtm(const double* Mm, double D, double t, const double (&Pk)[12],
+                                              const double (&ck)[12], double theta, double f2_floor) {
+  double cMp = 0.0, pMp = 0.0;
+#pragma unroll
+  for (int i = 0; i < 12; ++i) {
+    double mp = 0.0;
+#pragma unroll
+    for (int j = 0; j < 12; ++j) mp += Mm[i * 12 + j] * Pk[j];
+    cMp += ck[i] * mp;
+    pMp += Pk[i] * mp;
+  }
+  const double f1 = -D + theta * t * D - cMp;
+  const double f2 = fmax(f2_floor, theta * D - pMp);
+  return -f1 / f2;
+}
+
+// First breakpoint position of a CTA whose nominal start is p: bucket
+// boundaries at or after p.
+__device__ __forceinline__ int bucket_cut(int p, int nbreak, const unsigned long long* sbk, const unsigned* start,
+                                          unsigned long long kmin, int shift, int nb) {
+  if (p >= nbreak) return nbreak;
+  const int b = bucket_of(sbk[p], kmin, shift, nb);
+  return (int)start[b] == p ? p : (int)start[b + 1];
+}
+
+// The generalized Cauchy point over the bucketed breakpoints, all CTAs of the
+// group together.  Each round gives every CTA the buckets of about 256
+// breakpoints (later rounds 1024): the CTAs sum d^2, d w and t d w over their
+// buckets, exchange the sums, and so know the state of the piecewise
+// quadratic where their buckets begin; each then sorts its own breakpoints by
+// (t, index), scans them and tests every segment, and the first CTA in order
+// that stopped has the result.  The rounds are serial only in their number:
+// one CTA that walked all breakpoints, 1024 at a time, took 130 of a 64 x 64
+// solve's 387 us per evaluation, and 19 of 20 ms at 1024 x 1024, where a
+// minimiser lies some 190 000 breakpoints out.  A bucket of more than SMILI_KC
+// breakpoints (equal times, mostly) is taken in batches by radix selection.
+// cr[] (shared): the CR_* values.  Returns 0, -1 (singular middle matrix) or
+// -2 (a wait timed out).
+template <typename SY>
+__device__ __noinline__ int cauchy_search(LbCtxT<SY>& c, double f1_0, const double* p0, int nbreak, int bnded,
+                                          const unsigned long long* sbk, const int* sbi, unsigned long long kmin,
+                                          int shift, int nb, double* cr) {
+  LbState& S = *c.S;
+  GroupCtx& g = *c.g;
+  CauchySmem& sm = *reinterpret_cast<CauchySmem*>(c.dyn);
+  const int m = c.m, col = S.col, col2 = 2 * col, n = c.n;
+  const int T = blockDim.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = T >> 5;
+  const double theta = S.theta;
+  __shared__ unsigned long long bnd_hi_s, bnd_lo_s;
+  __shared__ int e_star_s, info_s, win_s;
+  __shared__ double f2org_s;
+  Prof& pf = *c.prof;
+  // dense middle matrix: column j = M e_j, at rows / columns a (Y) and 6 + a (S)
+  for (int i = threadIdx.x; i < 144; i += T) sm.Mm[i] = 0.0;
+  if (threadIdx.x < 32) sm.cum[threadIdx.x] = 0.0;
   if (threadIdx.x == 0) info_s = 0;
   __syncthreads();
   if (threadIdx.x < col2) {
     double e[2 * SMILI_MAXM_DEV], mc[2 * SMILI_MAXM_DEV];
     for (int k = 0; k < col2; ++k) e[k] = (k == (int)threadIdx.x) ? 1.0 : 0.0;
     if (d_bmv(S, m, col, e, mc)) info_s = -1;
-    for (int k = 0; k < col2; ++k) Mm[k * col2 + threadIdx.x] = mc[k];
+    const int jc = (int)threadIdx.x < col ? (int)threadIdx.x : 6 + (int)threadIdx.x - col;
+    for (int k = 0; k < col2; ++k) sm.Mm[(k < col ? k : 6 + k - col) * 12 + jc] = mc[k];
   }
-  for (int i = threadIdx.x; i < SMILI_NBUCKET; i += blockDim.x) hist[i] = (unsigned)ghist[i];
   __syncthreads();
-  if (info_s) {  // singular middle matrix (bmv failure)
-    if (threadIdx.x == 0) lr[CR_INFO] = -1;
-    __syncthreads();
-    return;
-  }
+  if (info_s) return -1;  // singular middle matrix (bmv failure)
   if (threadIdx.x == 0) {
     double f2 = -theta * f1_0;
-    const double f2_org = f2;
-    if (col > 0) {
-      double s = 0;
-      for (int i = 0; i < col2; ++i)
-        for (int j = 0; j < col2; ++j) s += p0[i] * Mm[i * col2 + j] * p0[j];
-      f2 -= s;
-    }
-    st[0] = -f1_0;
-    st[1] = 0.0;
-    st[2] = -f1_0 / f2;
-    for (int j = 0; j < col2; ++j) {
-      Pst[j] = p0[j];
-      Qst[j] = 0.0;
-    }
-    f2org_s = f2_org;
+    f2org_s = f2;
+    double s = 0;
+    for (int i = 0; i < 12; ++i)
+      for (int j = 0; j < 12; ++j) s += p0[i] * sm.Mm[i * 12 + j] * p0[j];
+    f2 -= s;
+    sm.st[0] = -f1_0;
+    sm.st[1] = 0.0;
+    sm.st[2] = -f1_0 / f2;
     bnd_hi_s = 0;
     bnd_lo_s = 0;
   }
+  if (threadIdx.x < 12) {
+    sm.P[threadIdx.x] = p0[threadIdx.x];
+    sm.Q[threadIdx.x] = 0.0;
+  }
   __syncthreads();
-  const double f2_org = f2org_s;
+  const double f2_floor = S.epsmch * f2org_s;
   if (nbreak == 0) {  // GCP in the first segment (lbfgsb.f:1433, label 888)
     if (threadIdx.x == 0) {
-      double dtm = st[2];
-      if (dtm <= 0.0) dtm = 0.0;
-      lr[CR_INFO] = 0;
-      lr[CR_MODE] = CM_NONE_FIXED;
-      lr[CR_TSUM] = dtm;
-      lr[CR_NSEG] = 1;
-      lr[CR_BHI] = 0.0;
-      lr[CR_BLO] = 0.0;
-      for (int j = 0; j < col2; ++j) lr[CR_C + j] = dtm * Pst[j];
+      const double dtm = fmax(sm.st[2], 0.0);
+      cr[CR_INFO] = 0;
+      cr[CR_MODE] = CM_NONE_FIXED;
+      cr[CR_TSUM] = dtm;
+      cr[CR_NSEG] = 1;
+      cr[CR_BHI] = 0.0;
+      cr[CR_BLO] = 0.0;
+      for (int j = 0; j < 12; ++j) cr[CR_C + j] = dtm * sm.P[j];
     }
     __syncthreads();
-    return;
+    return 0;
   }
   int pj[SMILI_MAXM_DEV];
-  for (int j = 0; j < col; ++j) pj[j] = lptr(S, m, j);
-  const int V = 1 + 2 * col2;
-  int kdone = 0, pos = 0, bucket = 0;
-  // state of an oversized bucket being consumed by radix selection
-  int big_r0 = -1, big_r1 = -1;
-  while (true) {
-    // ---------------- next batch ----------------
-    int cnt = 0;
-    const u128 lo_key = ((u128)bnd_hi_s << 64) | (u128)bnd_lo_s;
-    if (big_r0 < 0) {
-      while (bucket < SMILI_NBUCKET && hist[bucket] == 0) ++bucket;
-      if (bucket < SMILI_NBUCKET && (int)hist[bucket] > SMILI_KC) {
-        big_r0 = pos;
-        big_r1 = pos + (int)hist[bucket];
+#pragma unroll
+  for (int j = 0; j < SMILI_MAXM_DEV; ++j) pj[j] = j < col ? lptr(S, m, j) : 0;
+  int round0 = 0;  // first position of the round
+  for (int round = 0;; ++round) {
+    const int B = round == 0 ? 256 : 1024;
+    int r0 = 0, r1 = nbreak, rnext = nbreak;
+    if (g.G > 1) {
+      const long nom = (long)round0 + (long)g.rank * B;
+      r0 = g.rank == 0 ? round0 : bucket_cut((int)min(nom, (long)nbreak), nbreak, sbk, sm.start, kmin, shift, nb);
+      r1 = bucket_cut((int)min(nom + B, (long)nbreak), nbreak, sbk, sm.start, kmin, shift, nb);
+      rnext = bucket_cut((int)min((long)round0 + (long)g.G * B, (long)nbreak), nbreak, sbk, sm.start, kmin, shift, nb);
+      // ---- sums over this CTA's buckets, and what precedes them ----
+      double s[32], mx[1] = {0.0};
+#pragma unroll
+      for (int k = 0; k < 32; ++k) s[k] = 0.0;
+      for (int i = r0 + threadIdx.x; i < r1; i += T) {
+        const int idx = sbi[i];
+        const double te = __longlong_as_double((long long)sbk[i]);
+        const double d = c.d[idx];
+        s[0] += d * d;
+        mx[0] = fmax(mx[0], te);
+#pragma unroll
+        for (int j = 0; j < SMILI_MAXM_DEV; ++j) {
+          if (j < col) {
+            const double y = d * ld_wy(c, (size_t)pj[j] * n + idx);
+            const double w = d * (theta * ld_ws(c, (size_t)pj[j] * n + idx));
+            s[1 + j] += y;
+            s[7 + j] += w;
+            s[13 + j] += te * y;
+            s[19 + j] += te * w;
+          }
+        }
+      }
+      block_partials<32, 1>(s, mx, group_row(g, c.red), c.scratch);
+      const double* part = g.red_part + (size_t)g.parity * g.G * g.redk;
+      g.parity ^= 1;
+      if (!group_sync(g)) return -2;
+      {
+        const int k = threadIdx.x & 31, sl = threadIdx.x >> 5, S_ = T >> 5;
+        const bool sum = k < 31;
+        double pre = 0.0, tot = 0.0;
+#pragma unroll 4
+        for (int r = sl; r < g.G; r += S_) {
+          const double v = __ldcg(part + (size_t)r * g.redk + (sum ? k : 32));
+          tot = sum ? tot + v : fmax(tot, v);
+          if (r < g.rank) pre = sum ? pre + v : fmax(pre, v);
+        }
+        sm.a_s[threadIdx.x] = pre;
+        sm.b_s[threadIdx.x] = tot;
+        __syncthreads();
+        if (threadIdx.x < 32) {
+          double a = sm.a_s[k], b = sm.b_s[k];
+          for (int q = 1; q < S_; ++q) {
+            a = sum ? a + sm.a_s[q * 32 + k] : fmax(a, sm.a_s[q * 32 + k]);
+            b = sum ? b + sm.b_s[q * 32 + k] : fmax(b, sm.b_s[q * 32 + k]);
+          }
+          // sums and latest time over everything before this CTA's buckets
+          const double cu = sm.cum[k];
+          sm.pre[k] = sum ? cu + a : fmax(cu, a);
+          sm.cum[k] = sum ? cu + b : fmax(cu, b);
+        }
+        __syncthreads();
+      }
+      if (r0 > 0 && r0 < r1) {
+        if (threadIdx.x < 12) {
+          sm.P[threadIdx.x] = p0[threadIdx.x] - sm.pre[1 + threadIdx.x];
+          sm.Q[threadIdx.x] = sm.pre[13 + threadIdx.x];
+        }
+        if (threadIdx.x == 0) {
+          const double D = -f1_0 - sm.pre[0], t = sm.pre[31];
+          double Pk[12], ck[12];
+#pragma unroll
+          for (int j = 0; j < 12; ++j) {
+            Pk[j] = p0[j] - sm.pre[1 + j];
+            ck[j] = t * Pk[j] + sm.pre[13 + j];
+          }
+          sm.st[0] = D;
+          sm.st[1] = t;
+          sm.st[2] = segment_dtm(sm.Mm, D, t, Pk, ck, theta, f2_floor);
+          // every breakpoint before these buckets, whatever its index
+          const u128 ckk = comp_key((unsigned long long)__double_as_longlong(t), -1);
+          bnd_hi_s = (unsigned long long)(ckk >> 64);
+          bnd_lo_s = (unsigned long long)ckk;
+        }
+      }
+      pf.mark(PR_C_GATHER);
+    }
+    __syncthreads();
+    // ---- this CTA's breakpoints, a batch of whole buckets at a time ----
+    bool finished = false;
+    int pos = r0, kdone = r0;
+    int big_r0 = -1, big_r1 = -1;  // an oversized bucket being consumed by radix selection
+    while (pos < r1 && !finished) {
+      int cnt;
+      if (big_r0 < 0) {
+        int e = min(pos + T, r1);
+        if (e < r1) {
+          const int b = bucket_of(sbk[e], kmin, shift, nb);
+          e = (int)sm.start[b];                   // the batch ends where e's bucket begins,
+          if (e <= pos) e = (int)sm.start[b + 1];  // or is that one bucket
+        }
+        cnt = e - pos;
+        if (cnt > SMILI_KC) {
+          big_r0 = pos;
+          big_r1 = e;
+        } else {
+          for (int i = threadIdx.x; i < cnt; i += T) sm.cand[i] = comp_key(sbk[pos + i], sbi[pos + i]);
+        }
+      }
+      if (big_r0 >= 0) {
+        const u128 lo_key = ((u128)bnd_hi_s << 64) | (u128)bnd_lo_s;
+        cnt = select_from_range(c, sbk, sbi, big_r0, big_r1, lo_key, sm.cand, sm.hist2);
+      }
+      __syncthreads();
+      pf.count(PR_C_ROUNDS);
+      sort_batch(sm.cand, cnt);
+      pf.mark(PR_C_SORT);
+      // ---- scan in chunks of T ----
+      for (int base = 0; base < cnt; base += T) {
+        const int e = threadIdx.x, ge = base + e;
+        const bool valid = ge < cnt;
+        double vals[25];
+        double te = 0.0;
+        int idx = 0;
+#pragma unroll
+        for (int v = 0; v < 25; ++v) vals[v] = 0.0;
+        if (valid) {
+          const u128 ck = sm.cand[ge];
+          idx = (int)(unsigned)(ck & 0xffffffffu);
+          te = __longlong_as_double((long long)(unsigned long long)(ck >> 32));
+          const double dibp = c.d[idx];
+          vals[0] = dibp * dibp;
+#pragma unroll
+          for (int j = 0; j < SMILI_MAXM_DEV; ++j) {
+            if (j < col) {
+              const double y = dibp * ld_wy(c, (size_t)pj[j] * n + idx);
+              const double w = dibp * (theta * ld_ws(c, (size_t)pj[j] * n + idx));
+              vals[1 + j] = y;
+              vals[7 + j] = w;
+              vals[13 + j] = te * y;
+              vals[19 + j] = te * w;
+            }
+          }
+        }
+        // inclusive scan over the block: warps, then the warps' totals
+#pragma unroll
+        for (int v = 0; v < 25; ++v) {
+          double a = vals[v];
+#pragma unroll
+          for (int sft = 1; sft < 32; sft <<= 1) {
+            const double o = __shfl_up_sync(0xffffffffu, a, sft);
+            if (lane >= sft) a += o;
+          }
+          vals[v] = a;
+          if (lane == 31) sm.wtot[wid][v] = a;
+        }
+        if (threadIdx.x == 0) e_star_s = T;
+        __syncthreads();
+        if (threadIdx.x < 25) {
+          double run = 0.0;
+          for (int w = 0; w < nw; ++w) {
+            const double x = sm.wtot[w][threadIdx.x];
+            sm.wtot[w][threadIdx.x] = run;
+            run += x;
+          }
+        }
+        __syncthreads();
+        double dtm_e = 0.0, Dk = 0.0, Pk[12], ck_[12];
+        if (valid) {
+          Dk = sm.st[0] - (vals[0] + sm.wtot[wid][0]);
+#pragma unroll
+          for (int j = 0; j < 12; ++j) {
+            Pk[j] = sm.P[j] - (vals[1 + j] + sm.wtot[wid][1 + j]);
+            ck_[j] = te * Pk[j] + (sm.Q[j] + (vals[13 + j] + sm.wtot[wid][13 + j]));
+          }
+          dtm_e = segment_dtm(sm.Mm, Dk, te, Pk, ck_, theta, f2_floor);
+          sm.a_s[e] = dtm_e;
+          sm.b_s[e] = te;
+        }
+        __syncthreads();
+        // stop test for the segment ending at this element
+        if (valid) {
+          const double pd = (e == 0) ? sm.st[2] : sm.a_s[e - 1];
+          const double pt = (e == 0) ? sm.st[1] : sm.b_s[e - 1];
+          if (pd < (te - pt)) atomicMin(&e_star_s, e);
+        }
+        __syncthreads();
+        const int es = e_star_s;
+        const int nvalid = min(T, cnt - base);
+        if (es < T) {
+          // GCP inside the segment before element es: breakpoints up to es-1 fixed
+          if ((es == 0 && threadIdx.x == 0) || (es > 0 && e == es - 1)) {
+            double tsum, dtm;
+            if (es == 0) {
+              tsum = sm.st[1];
+              dtm = fmax(sm.st[2], 0.0);
+#pragma unroll
+              for (int j = 0; j < 12; ++j) cr[CR_C + j] = tsum * sm.P[j] + sm.Q[j] + dtm * sm.P[j];
+            } else {
+              tsum = te;
+              dtm = fmax(dtm_e, 0.0);
+#pragma unroll
+              for (int j = 0; j < 12; ++j) cr[CR_C + j] = ck_[j] + dtm * Pk[j];
+              const u128 ckk = comp_key(__double_as_longlong(te), idx);
+              bnd_hi_s = (unsigned long long)(ckk >> 64);
+              bnd_lo_s = (unsigned long long)ckk;
+            }
+            cr[CR_MODE] = (kdone + es == 0) ? CM_NONE_FIXED : CM_BOUNDARY;
+            cr[CR_TSUM] = tsum + dtm;
+            cr[CR_NSEG] = kdone + es + 1;
+          }
+          finished = true;
+          __syncthreads();
+          break;
+        }
+        // no stop in this chunk: carry the state of its last element
+        if (e == nvalid - 1) {
+          sm.st[0] = Dk;
+          sm.st[1] = te;
+          sm.st[2] = dtm_e;
+#pragma unroll
+          for (int j = 0; j < 12; ++j) {
+            sm.P[j] = Pk[j];
+            sm.Q[j] = ck_[j] - te * Pk[j];
+          }
+          const u128 ckk = comp_key(__double_as_longlong(te), idx);
+          bnd_hi_s = (unsigned long long)(ckk >> 64);
+          bnd_lo_s = (unsigned long long)ckk;
+        }
+        __syncthreads();
+        kdone += nvalid;
+        if (kdone == nbreak) {
+          // every breakpoint passed without a stop (lbfgsb.f:1640-1660)
+          if (threadIdx.x == 0) {
+            cr[CR_MODE] = CM_BOUNDARY;
+            cr[CR_NSEG] = kdone;
+            // all variables at their bounds: c = W'(xcp - x) = t_n P_n + Q_n
+            const double dtm = (nbreak == n || bnded) ? 0.0 : fmax(sm.st[2], 0.0);
+            cr[CR_TSUM] = sm.st[1] + dtm;
+            for (int j = 0; j < 12; ++j) cr[CR_C + j] = sm.st[1] * sm.P[j] + sm.Q[j] + dtm * sm.P[j];
+          }
+          finished = true;
+          __syncthreads();
+          break;
+        }
+      }
+      pf.mark(PR_C_SCAN);
+      if (big_r0 >= 0) {
+        if (kdone >= big_r1) {  // the oversized bucket is consumed
+          pos = big_r1;
+          big_r0 = big_r1 = -1;
+        }
+      } else {
+        pos += cnt;
       }
     }
-    if (big_r0 >= 0) {
-      cnt = select_from_range(c, sbk, sbi, big_r0, big_r1, lo_key, cand, hist2);
-    } else {
-      int b2 = bucket, tot = 0;
-      while (b2 < SMILI_NBUCKET && tot + (int)hist[b2] <= SMILI_KC) tot += hist[b2++];
-      for (int i = threadIdx.x; i < tot; i += blockDim.x) cand[i] = comp_key(sbk[pos + i], sbi[pos + i]);
-      cnt = tot;
-      pos += tot;
-      bucket = b2;
+    if (finished && threadIdx.x == 0) {
+      cr[CR_INFO] = 0;
+      cr[CR_BHI] = __longlong_as_double((long long)bnd_hi_s);
+      cr[CR_BLO] = __longlong_as_double((long long)bnd_lo_s);
     }
+    __syncthreads();
+    if (g.G == 1) return 0;  // one CTA has walked every breakpoint it needs
+    // ---- the first CTA in order that stopped ----
+    double* row = group_row(g, c.red);
+    if (threadIdx.x < CR_C + 12 && finished) row[1 + threadIdx.x] = cr[threadIdx.x];
+    if (threadIdx.x == 0) {
+      row[0] = finished ? 1.0 : 0.0;
+      win_s = g.G;
+    }
+    const double* part = g.red_part + (size_t)g.parity * g.G * g.redk;
+    g.parity ^= 1;
+    if (!group_sync(g)) return -2;
+    for (int r = threadIdx.x; r < g.G; r += T)
+      if (__ldcg(part + (size_t)r * g.redk) != 0.0) {
+        atomicMin(&win_s, r);
+        break;
+      }
+    __syncthreads();
+    const int win = win_s;
+    if (win < g.G) {
+      if (threadIdx.x < CR_C + 12) cr[threadIdx.x] = __ldcg(part + (size_t)win * g.redk + 1 + threadIdx.x);
+      __syncthreads();
+      return 0;
+    }
+    round0 = rnext;
     __syncthreads();
     pf.mark(PR_C_SEL);
-    pf.count(PR_C_ROUNDS);
-    int np2 = 1;
-    while (np2 < cnt) np2 <<= 1;
-    for (int i = cnt + threadIdx.x; i < np2; i += blockDim.x) cand[i] = ~(u128)0;
-    __syncthreads();
-    // ---------------- bitonic sort ----------------
-    for (int k2 = 2; k2 <= np2; k2 <<= 1) {
-      for (int j2 = k2 >> 1; j2 > 0; j2 >>= 1) {
-        for (int i = threadIdx.x; i < np2; i += blockDim.x) {
-          const int ixj = i ^ j2;
-          if (ixj > i) {
-            const u128 a = cand[i], b = cand[ixj];
-            const bool up = (i & k2) == 0;
-            if ((a > b) == up) {
-              cand[i] = b;
-              cand[ixj] = a;
-            }
-          }
-        }
-        __syncthreads();
-      }
-    }
-    pf.mark(PR_C_SORT);
-    // ---------------- scan in chunks of THREADS ----------------
-    bool finished = false;
-    const int T = blockDim.x;
-    for (int base = 0; base < cnt; base += T) {
-      const int e = threadIdx.x;
-      const int ge = base + e;
-      const bool valid = ge < cnt;
-      double vals[1 + 4 * SMILI_MAXM_DEV];
-      double te = 0.0;
-      int idx = 0;
-      for (int v = 0; v < V; ++v) vals[v] = 0.0;
-      if (valid) {
-        const u128 ck = cand[ge];
-        idx = (int)(unsigned)(ck & 0xffffffffu);
-        const unsigned long long kb = (unsigned long long)(ck >> 32);
-        te = __longlong_as_double((long long)kb);
-        const double dibp = c.d[idx];
-        vals[0] = dibp * dibp;
-        for (int j = 0; j < col; ++j) {
-          const double wy_ = ld_wy(c, (size_t)pj[j] * n + idx);
-          const double ws_ = theta * ld_ws(c, (size_t)pj[j] * n + idx);
-          vals[1 + j] = dibp * wy_;
-          vals[1 + col + j] = dibp * ws_;
-          vals[1 + col2 + j] = te * dibp * wy_;
-          vals[1 + col2 + col + j] = te * dibp * ws_;
-        }
-      }
-      block_scan_incl(vals, V, wtot);
-      double dtm_e = 0.0;
-      double Pk[2 * SMILI_MAXM_DEV], ck_[2 * SMILI_MAXM_DEV];
-      double Dk = 0.0;
-      if (valid) {
-        Dk = st[0] - vals[0];
-        for (int j = 0; j < col2; ++j) {
-          Pk[j] = Pst[j] - vals[1 + j];
-          ck_[j] = te * Pk[j] + (Qst[j] + vals[1 + col2 + j]);
-        }
-        double cMp = 0.0, pMp = 0.0;
-        for (int i = 0; i < col2; ++i) {
-          double mp = 0.0;
-          for (int j = 0; j < col2; ++j) mp += Mm[i * col2 + j] * Pk[j];
-          cMp += ck_[i] * mp;
-          pMp += Pk[i] * mp;
-        }
-        const double f1 = -Dk + theta * te * Dk - cMp;
-        double f2 = theta * Dk - pMp;
-        f2 = fmax(S.epsmch * f2_org, f2);
-        dtm_e = -f1 / f2;
-        dtm_s[e] = dtm_e;
-        t_s[e] = te;
-      }
-      __syncthreads();
-      // stop test for the segment ending at this element
-      int stop = 0;
-      if (valid) {
-        const double pd = (e == 0) ? st[2] : dtm_s[e - 1];
-        const double pt = (e == 0) ? st[1] : t_s[e - 1];
-        stop = pd < (te - pt);
-      }
-      if (threadIdx.x == 0) e_star_s = T;
-      __syncthreads();
-      if (stop) atomicMin(&e_star_s, e);
-      __syncthreads();
-      const int es = e_star_s;
-      const int nvalid = min(T, cnt - base);
-      if (es < T) {
-        // GCP inside the segment before element es: breakpoints up to es-1 fixed
-        if ((es == 0 && threadIdx.x == 0) || (es > 0 && e == es - 1)) {
-          double Pf[2 * SMILI_MAXM_DEV], Cf[2 * SMILI_MAXM_DEV];
-          double tsum, dtm;
-          if (es == 0) {
-            tsum = st[1];
-            dtm = st[2];
-            for (int j = 0; j < col2; ++j) {
-              Pf[j] = Pst[j];
-              Cf[j] = tsum * Pst[j] + Qst[j];
-            }
-          } else {
-            tsum = te;
-            dtm = dtm_e;
-            for (int j = 0; j < col2; ++j) {
-              Pf[j] = Pk[j];
-              Cf[j] = ck_[j];
-            }
-            const u128 ckk = comp_key(__double_as_longlong(te), idx);
-            bnd_hi_s = (unsigned long long)(ckk >> 64);
-            bnd_lo_s = (unsigned long long)ckk;
-          }
-          if (dtm <= 0.0) dtm = 0.0;
-          lr[CR_INFO] = 0;
-          lr[CR_MODE] = (kdone + es == 0) ? CM_NONE_FIXED : CM_BOUNDARY;
-          lr[CR_TSUM] = tsum + dtm;
-          lr[CR_NSEG] = kdone + es + 1;
-          for (int j = 0; j < col2; ++j) lr[CR_C + j] = Cf[j] + dtm * Pf[j];
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-          lr[CR_BHI] = __longlong_as_double((long long)bnd_hi_s);
-          lr[CR_BLO] = __longlong_as_double((long long)bnd_lo_s);
-        }
-        finished = true;
-        __syncthreads();
-        break;
-      }
-      // no stop in this chunk: carry the state of its last element
-      if (e == nvalid - 1) {
-        st[0] = Dk;
-        st[1] = te;
-        st[2] = dtm_e;
-        for (int j = 0; j < col2; ++j) {
-          Pst[j] = Pk[j];
-          Qst[j] = ck_[j] - te * Pk[j];
-        }
-        const u128 ckk = comp_key(__double_as_longlong(te), idx);
-        bnd_hi_s = (unsigned long long)(ckk >> 64);
-        bnd_lo_s = (unsigned long long)ckk;
-      }
-      __syncthreads();
-      kdone += nvalid;
-      if (kdone == nbreak) {
-        // every breakpoint passed without a stop (lbfgsb.f:1640-1660)
-        if (threadIdx.x == 0) {
-          lr[CR_INFO] = 0;
-          lr[CR_MODE] = CM_BOUNDARY;
-          lr[CR_NSEG] = kdone;
-          lr[CR_BHI] = __longlong_as_double((long long)bnd_hi_s);
-          lr[CR_BLO] = __longlong_as_double((long long)bnd_lo_s);
-          if (nbreak == n) {
-            // all variables at their bounds; c = W'(xcp - x) = t_n P_n + Q_n
-            lr[CR_TSUM] = st[1];
-            for (int j = 0; j < col2; ++j) lr[CR_C + j] = st[1] * Pst[j] + Qst[j];
-          } else {
-            double dtm = bnded ? 0.0 : st[2];
-            if (dtm <= 0.0) dtm = 0.0;
-            lr[CR_TSUM] = st[1] + dtm;
-            for (int j = 0; j < col2; ++j) lr[CR_C + j] = st[1] * Pst[j] + Qst[j] + dtm * Pst[j];
-          }
-        }
-        finished = true;
-        __syncthreads();
-        break;
-      }
-    }
-    pf.mark(PR_C_SCAN);
-    if (finished) break;
-    if (big_r0 >= 0 && kdone >= big_r1) {  // the oversized bucket is consumed
-      pos = big_r1;
-      ++bucket;
-      big_r0 = big_r1 = -1;
-    }
   }
-  __syncthreads();
 }
 
 // Returns 0 on success, -1 when bmv failed (info != 0).
@@ -793,22 +944,25 @@ __device__ __noinline__ int lb_cauchy(LbCtxT<SY>& c) {
   const bool nonneg = P.nonneg;
   unsigned long long* sbk = at<unsigned long long>(c.base, P.o_sbk);
   int* sbi = at<int>(c.base, P.o_sbi);
-  int* ghist = at<int>(c.base, P.o_hist);  // [NBUCKET] counts, [NBUCKET] cursors
+  int* ghist = at<int>(c.base, P.o_hist);  // [SMILI_NBUCKET_MAX] counts, [SMILI_NBUCKET_MAX] cursors
+  __shared__ double cr_s[CR_C + 12], p0_s[12];
   if (S.sbgnrm <= 0.0) {
     // GCP = X (lbfgsb.f:1318-1322): z = x, iwhere untouched
     for (int i = c.lo + threadIdx.x; i < c.hi; i += blockDim.x) c.z[i] = c.x[i];
-    if (threadIdx.x == 0) c.lred[CR_MODE] = CM_XCP_IS_X;
+    if (threadIdx.x == 0) cr_s[CR_MODE] = CM_XCP_IS_X;
   } else {
     int pj[SMILI_MAXM_DEV];
 #pragma unroll
     for (int j = 0; j < SMILI_MAXM_DEV; ++j) pj[j] = j < col ? lptr(S, m, j) : 0;
     // sums: [0..5] Y'd, [6..11] S'd (zero past col), [12] f1, [13] nbreak,
-    // [14] nfree_nb; maxima: notbnded, -tmin, tmax
-    double f1a = 0.0, nbr = 0.0, nfr = 0.0, notb = 0.0, tmn = 1.0e308, tmx = 0.0;
+    // [14] and [15] the first two moments of the keys' upper words (less
+    // 1.0's); maxima: notbnded, -tmin, tmax, any variable without a breakpoint
+    double f1a = 0.0, nbr = 0.0, k1 = 0.0, k2 = 0.0, nfr = 0.0, notb = 0.0, tmn = 1.0e308, tmx = 0.0;
     double py[SMILI_MAXM_DEV], ps[SMILI_MAXM_DEV];
 #pragma unroll
     for (int j = 0; j < SMILI_MAXM_DEV; ++j) py[j] = ps[j] = 0.0;
-    for (int i = c.g->rank * blockDim.x + threadIdx.x; i < 2 * SMILI_NBUCKET; i += c.g->G * blockDim.x)
+    const int nb = cauchy_buckets(n);
+    for (int i = c.g->rank * blockDim.x + threadIdx.x; i < 2 * SMILI_NBUCKET_MAX; i += c.g->G * blockDim.x)
       ghist[i] = 0;
     for (int i = c.lo + threadIdx.x; i < c.hi; i += blockDim.x) {
       const double neggi = -c.gv[i];
@@ -844,8 +998,11 @@ __device__ __noinline__ int lb_cauchy(LbCtxT<SY>& c) {
           tmn = fmin(tmn, tb);
           tmx = fmax(tmx, tb);
           key = (unsigned long long)__double_as_longlong(tb);
+          const double kh = (double)((int)(key >> 32) - 0x3ff00000);
+          k1 += kh;
+          k2 += kh * kh;
         } else {
-          nfr += 1.0;
+          nfr = 1.0;
           if (fabs(neggi) > 0.0) notb = 1.0;
         }
       }
@@ -859,86 +1016,98 @@ __device__ __noinline__ int lb_cauchy(LbCtxT<SY>& c) {
     }
     acc[12] = f1a;
     acc[13] = nbr;
-    acc[14] = nfr;
-    acc[15] = 0.0;
-    const double accx[3] = {notb, -tmn, tmx};
+    acc[14] = k1;
+    acc[15] = k2;
+    const double accx[4] = {notb, -tmn, tmx, nfr};
     if (!lb_reduce(c, acc, accx)) return -2;
     const double f1 = c.red[12];
-    double p[2 * SMILI_MAXM_DEV];
-    for (int j = 0; j < col; ++j) {
-      p[j] = c.red[j];
-      p[col + j] = c.red[SMILI_MAXM_DEV + j];
-    }
+    if (threadIdx.x < 12) p0_s[threadIdx.x] = (threadIdx.x < 6 ? 1.0 : S.theta) * c.red[threadIdx.x];
     const int nbreak = (int)c.red[13];
-    const int nfree_nb = (int)c.red[14];
     const int bnded = c.red[16] > 0.5 ? 0 : 1;
-    const unsigned long long kmin = (unsigned long long)__double_as_longlong(-c.red[17]);
-    const unsigned long long kmax = (unsigned long long)__double_as_longlong(c.red[18]);
-    if (S.theta != 1.0)
-      for (int j = 0; j < col; ++j) p[col + j] *= S.theta;
+    const bool any_free = c.red[19] > 0.5;
+    // key range of the buckets: all of it, but no more than three standard
+    // deviations of the keys' exponents around their mean (a few far
+    // breakpoints would otherwise leave the bulk in a few buckets)
+    unsigned long long kmin = (unsigned long long)__double_as_longlong(-c.red[17]);
+    unsigned long long kmax = (unsigned long long)__double_as_longlong(c.red[18]);
+    if (nbreak > 0) {
+      const double mu = c.red[14] / nbreak, var = c.red[15] / nbreak - mu * mu;
+      const double sd = sqrt(fmax(var, 0.0)) + 64.0;
+      const double lo = floor(mu - 3.0 * sd) + 0x3ff00000, hi = ceil(mu + 3.0 * sd) + 0x3ff00000;
+      if (lo > 0.0 && lo < 2147483647.0) kmin = max(kmin, (unsigned long long)lo << 32);
+      if (hi > 0.0 && hi < 2147483647.0) kmax = min(kmax, (unsigned long long)hi << 32);
+      if (kmax < kmin) kmax = kmin;
+    }
     __syncthreads();
-    if (nbreak == 0 && nfree_nb == 0) {
+    if (nbreak == 0 && !any_free) {
       for (int i = c.lo + threadIdx.x; i < c.hi; i += blockDim.x) c.z[i] = c.x[i];
-      if (threadIdx.x == 0 && c.g->rank == 0) c.lred[CR_MODE] = CM_XCP_IS_X;
+      if (threadIdx.x == 0) cr_s[CR_MODE] = CM_XCP_IS_X;
     } else {
+      CauchySmem& sm = *reinterpret_cast<CauchySmem*>(c.dyn);
+      int shift = 0;
       if (nbreak > 0) {
         // bucket the breakpoints: histogram, then scatter in bucket order
-        int shift = 0;
-        while (shift < 63 && ((kmax - kmin) >> shift) >= (unsigned long long)SMILI_NBUCKET) ++shift;
-        unsigned* lh = reinterpret_cast<unsigned*>(c.dyn);
-        for (int i = threadIdx.x; i < SMILI_NBUCKET; i += blockDim.x) lh[i] = 0;
-        __syncthreads();
+        while (shift < 63 && ((kmax - kmin) >> shift) >= (unsigned long long)nb) ++shift;
         for (int i = c.lo + threadIdx.x; i < c.hi; i += blockDim.x) {
           const unsigned long long k = c.bkey[i];
-          if (k != ~0ULL) atomicAdd(&lh[bucket_of(k, kmin, shift)], 1u);
+          if (k != ~0ULL) atomicAdd(&ghist[bucket_of(k, kmin, shift, nb)], 1);
         }
-        __syncthreads();
-        for (int i = threadIdx.x; i < SMILI_NBUCKET; i += blockDim.x)
-          if (lh[i]) atomicAdd(&ghist[i], (int)lh[i]);
         if (!group_sync(*c.g)) return -2;
-        // exclusive prefix of the bucket counts -> start offsets (in lh)
-        for (int i = threadIdx.x; i < SMILI_NBUCKET; i += blockDim.x) lh[i] = (unsigned)((volatile int*)ghist)[i];
-        __syncthreads();
-        if (threadIdx.x < 32) {
-          // warp 0: sequential chunks of 128 buckets per lane, then a warp scan
-          const int per = SMILI_NBUCKET / 32;
-          unsigned run = 0;
-          for (int q = 0; q < per; ++q) run += lh[threadIdx.x * per + q];
+        // exclusive prefix of the bucket counts -> start offsets, in every CTA
+        {
+          __shared__ unsigned wsum_s[SMILI_MAX_WARPS];
+          const int per = nb / blockDim.x;  // 4, 8 or 16 buckets per thread
+          const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+          unsigned cnt[SMILI_NBUCKET_MAX / 256], run = 0;
+#pragma unroll
+          for (int q = 0; q < SMILI_NBUCKET_MAX / 256; q += 4) {
+            if (q < per) {
+              const int4 v = __ldcg(reinterpret_cast<const int4*>(ghist + threadIdx.x * per + q));
+              cnt[q] = v.x;
+              cnt[q + 1] = v.y;
+              cnt[q + 2] = v.z;
+              cnt[q + 3] = v.w;
+              run += v.x + v.y + v.z + v.w;
+            }
+          }
           unsigned incl = run;
+#pragma unroll
           for (int s2 = 1; s2 < 32; s2 <<= 1) {
             const unsigned o = __shfl_up_sync(0xffffffffu, incl, s2);
-            if (threadIdx.x >= s2) incl += o;
+            if (lane >= s2) incl += o;
           }
-          unsigned acc2 = incl - run;
-          for (int q = 0; q < per; ++q) {
-            const unsigned v = lh[threadIdx.x * per + q];
-            lh[threadIdx.x * per + q] = acc2;
-            acc2 += v;
+          if (lane == 31) wsum_s[wid] = incl;
+          __syncthreads();
+          unsigned off = incl - run;
+          for (int w = 0; w < wid; ++w) off += wsum_s[w];
+#pragma unroll
+          for (int q = 0; q < SMILI_NBUCKET_MAX / 256; ++q) {
+            if (q < per) {
+              sm.start[threadIdx.x * per + q] = off;
+              off += cnt[q];
+            }
           }
+          if (threadIdx.x == 0) sm.start[nb] = (unsigned)nbreak;
         }
         __syncthreads();
         for (int i = c.lo + threadIdx.x; i < c.hi; i += blockDim.x) {
           const unsigned long long k = c.bkey[i];
           if (k != ~0ULL) {
-            const int b = bucket_of(k, kmin, shift);
-            const int q = (int)lh[b] + atomicAdd(&ghist[SMILI_NBUCKET + b], 1);
+            const int b = bucket_of(k, kmin, shift, nb);
+            const int q = (int)sm.start[b] + atomicAdd(&ghist[SMILI_NBUCKET_MAX + b], 1);
             sbk[q] = k;
             sbi[q] = i;
           }
         }
         if (!group_sync(*c.g)) return -2;
+        c.prof->mark(PR_C_SEL);
       }
-      if (c.g->rank == 0) cauchy_scan(c, f1, p, nbreak, bnded, sbk, sbi, ghist);
+      const int rc = cauchy_search(c, f1, p0_s, nbreak, bnded, sbk, sbi, kmin, shift, nb, cr_s);
+      if (rc != 0) return rc;
     }
   }
-  if (!group_sync(*c.g)) return -2;
-  // every CTA reads the leader's results
-  const double* lr = c.lred;
-  __shared__ double cr_s[CR_C + 2 * SMILI_MAXM_DEV];
-  for (int k = threadIdx.x; k < CR_C + col2; k += blockDim.x) cr_s[k] = ((const volatile double*)lr)[k];
   __syncthreads();
   const int mode = (int)cr_s[CR_MODE];
-  if (mode != CM_XCP_IS_X && cr_s[CR_INFO] != 0) return -1;
   // apply the GCP and run freev (lbfgsb.f:2241-2340)
   double acc[4] = {0, 0, 0, 0};  // nfree, nenter, nleave
   const u128 bnd = ((u128)(unsigned long long)__double_as_longlong(cr_s[CR_BHI]) << 64) |
@@ -970,7 +1139,10 @@ __device__ __noinline__ int lb_cauchy(LbCtxT<SY>& c) {
   if (threadIdx.x == 0) {
     if (mode != CM_XCP_IS_X) {
       S.nseg = (int)cr_s[CR_NSEG];
-      for (int j = 0; j < col2; ++j) S.wa[2 * m + j] = cr_s[CR_C + j];  // c
+      for (int j = 0; j < col; ++j) {  // c
+        S.wa[2 * m + j] = cr_s[CR_C + j];
+        S.wa[2 * m + col + j] = cr_s[CR_C + 6 + j];
+      }
     }
     S.nfree = (int)c.red[0];
     S.nenter = (int)c.red[1];

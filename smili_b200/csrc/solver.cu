@@ -303,7 +303,7 @@ __global__ void __launch_bounds__(Shape<R>::threads, Shape<R>::min_blocks) smili
   extern __shared__ __align__(16) char dyn[];
   __shared__ LbState S;
   __shared__ double red[SMILI_REDK];
-  __shared__ double scratch[Shape<R>::threads];
+  __shared__ double scratch[SMILI_SCRATCH(Shape<R>::threads)];
   __shared__ int prob_s;
   const int grp = blockIdx.x / a.G, rank = blockIdx.x % a.G;
   Prof prof;
@@ -375,7 +375,6 @@ __global__ void __launch_bounds__(Shape<R>::threads, Shape<R>::min_blocks) smili
     lc.iwh = at<signed char>(base, P.o_iwh);
     lc.freef = at<unsigned char>(base, P.o_free);
     lc.bkey = at<unsigned long long>(base, P.o_bkey);
-    lc.lred = at<double>(base, P.o_lred);
     lc.trace = at<double>(base, P.o_trace);
     lc.red = red;
     lc.scratch = scratch;
@@ -1021,8 +1020,7 @@ int pack_problem(const smili_imaging_args& a, int kind, int niter, int nonneg, i
     d.o_bkey = ar.take(sizeof(unsigned long long) * N);
     d.o_sbk = ar.take(sizeof(unsigned long long) * N);
     d.o_sbi = ar.take(sizeof(int) * N);
-    d.o_hist = ar.take(sizeof(int) * 2 * 4096);
-    d.o_lred = ar.take(sizeof(double) * 64);
+    d.o_hist = ar.take(sizeof(int) * 2 * SMILI_NBUCKET_MAX);
     d.o_trace = ar.take(sizeof(double) * (niter + 2));
   }
   if (kind == PK_SOLVE) {  // S and Y: R per element (FP32 storage in the FP32 mode)
@@ -1462,8 +1460,7 @@ int pack_movie(const smili_imaging3d_args& a, int kind, int niter, int nonneg, i
   d.o_bkey = ar.take(sizeof(unsigned long long) * n);
   d.o_sbk = ar.take(sizeof(unsigned long long) * n);
   d.o_sbi = ar.take(sizeof(int) * n);
-  d.o_hist = ar.take(sizeof(int) * 2 * 4096);
-  d.o_lred = ar.take(sizeof(double) * 64);
+  d.o_hist = ar.take(sizeof(int) * 2 * SMILI_NBUCKET_MAX);
   d.o_trace = ar.take(sizeof(double) * (niter + 2));
   if (kind == PK_SOLVE) {  // S and Y: R per element (FP32 storage in the FP32 mode)
     d.o_ws = ar.take(sizeof(R) * (size_t)n * m);
