@@ -393,11 +393,11 @@ __device__ __noinline__ void fg_t2_cols(FgCtx<R>& c, const GroupCtx& g) {
 }
 
 // The kernel weights of every uv point, taps[q][j] = psi at tap q < w of axis 1
-// and [w + q][j] of axis 2, once per launch (FP64; P.o_taps).  The points do
-// not move, and 2 w exponentials and roots per point and use cost more than
-// everything else interpolation and spreading do in FP64; read back, they
-// are 16 w coalesced bytes.  FP32 evaluates them with the hardware
-// exponential each time: the table would not stay in L2 beside a batch.
+// and [w + q][j] of axis 2, once per launch (P.o_taps).  The points do not
+// move, and 2 w exponentials and roots per point and use cost more than
+// everything else interpolation and spreading do (in FP32 some 280 of 500
+// instructions of an interpolated point); read back, they are 2 w coalesced
+// loads.
 template <typename R>
 __device__ __noinline__ void fg_taps(const ProbDesc& P, char* base, const GroupCtx& g) {
   const R* xu = at<R>(base, P.o_u);
@@ -705,155 +705,15 @@ __device__ __forceinline__ R warp_sum(R v) {
 // points are ordered by __syncwarp), so the inner loop needs no atomics.  The
 // finished subgrid is added to the CTA's band copy (shared atomics, only the
 // overlapping halos collide) and the CTA's band to the global band at the end.
-// ---------------------------------------------------------------------------
-// F5 on the tensor cores (FP32, w <= 9, 8 x 8 tiles).  A tile's subgrid is a
-// product of two thin matrices:
-//   D[r][c] = sum_p wy_p[r] (c_p wx_p[c]),   r, c < 8 + w - 1 <= 16,
-// with wy_p / wx_p the point's kernel weights placed at its offset inside
-// the subgrid (zero elsewhere) and c_p = Vres_re - i Vres_im of the point.
-// A warp accumulates the real and imaginary parts of one tile's 16 x 16
-// subgrid in mma.sync.m16n8k8 TF32 fragments (8 points per k step) with the
-// three-term split a b ~ ah bh + ah bl + al bh (a = ah + al in TF32), which
-// keeps the products within a few FP32 ulps; the subgrid never touches
-// shared memory and no tap waits on another.
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t to_tf32(float x) {
-  uint32_t r;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
-  return r;
-}
-
-__device__ __forceinline__ void split_tf32(float x, uint32_t& hi, uint32_t& lo) {
-  hi = to_tf32(x);
-  lo = to_tf32(x - __uint_as_float(hi));
-}
-
-__device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-      "{%0,%1,%2,%3};\n"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-
-__device__ __noinline__ void fg_spread_tc(FgCtx<float>& c, const GroupCtx& g) {
-  const ProbDesc& P = *c.P;
-  const float* xu = at<float>(c.base, P.o_u);
-  const float* xv = at<float>(c.base, P.o_v);
-  const int4* items = at<int4>(c.base, P.o_items);
-  const cpx<float>* cacc = at<cpx<float>>(c.base, P.o_contrib);
-  float* gband = at<float>(c.base, P.o_bandC);
-  const int w = P.w;
-  const int SG = 8 + w - 1;  // <= 16
-  const float beta = (float)P.beta;
-  const float half = 0.5f * (float)w, inv = 1.f / half;
-  const int ncell = P.b1n * P.b2n;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int gq = lane >> 2, t = lane & 3;
-  // shared memory: [nw][32 points][2w] kernel weights, then (if it fits) a
-  // private copy of the band
-  const size_t wt_b = ((size_t)nw * 32 * 2 * w * sizeof(float) + 15) / 16 * 16;
-  float* wtab = reinterpret_cast<float*>(c.sbuf) + (size_t)warp * 32 * 2 * w;
-  cpx<float>* sband = reinterpret_cast<cpx<float>*>(reinterpret_cast<char*>(c.sbuf) + wt_b);
-  const bool staged = wt_b + (size_t)ncell * sizeof(cpx<float>) <= (size_t)c.dyn_cpx * sizeof(cpx<float>);
-  float* band = staged ? reinterpret_cast<float*>(sband) : gband;
-  if (staged) {
-    for (int i = threadIdx.x; i < ncell; i += blockDim.x) sband[i] = cmk<float>(0, 0);
-    __syncthreads();
+// The work item that holds point p0 (items cover the points in order)
+__device__ __forceinline__ int item_of(const int4* items, int nitems, int p0) {
+  int it = 0;
+  for (int hi = nitems; hi - it > 1;) {
+    const int mid = (it + hi) >> 1;
+    if (items[mid].x <= p0) it = mid;
+    else hi = mid;
   }
-  const int gw = g.rank * nw + warp, nwt = g.G * nw;
-  for (int it = gw; it < P.nitems; it += nwt) {
-    const int4 item = items[it];
-    float dre[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}}, dim[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
-    for (int jb = item.x; jb < item.y; jb += 32) {
-      // phase 1: every lane prepares one point (zero weights past the item)
-      const int jl = jb + lane;
-      float cre_l = 0.f, cim_l = 0.f;
-      int lr_l = 0, lc_l = 0;
-      float* wr = wtab + lane * 2 * w;
-      if (jl < item.y) {
-        const cpx<float> cj = cacc[jl];
-        cre_l = cj.x;
-        cim_l = -cj.y;  // c = Vresre - i Vresim
-        const float xi1 = xu[jl], xi2 = xv[jl];
-        const int l1 = (int)ceilf(xi1 - half), l2 = (int)ceilf(xi2 - half);
-        for (int q = 0; q < w; ++q) {
-          wr[q] = es_kernel(((float)(l1 + q) - xi1) * inv, beta);
-          wr[w + q] = es_kernel(((float)(l2 + q) - xi2) * inv, beta);
-        }
-        lr_l = imod(l2 - P.b2s, P.nf2) - item.z;
-        lc_l = imod(l1 - P.b1s, P.nf1) - item.w;
-      } else {
-        for (int q = 0; q < 2 * w; ++q) wr[q] = 0.f;
-      }
-      __syncwarp();
-      // phase 2: 8 points per k step; lane (gq, t) feeds points t and t + 4
-      const int np = min(32, item.y - jb);
-      for (int kb = 0; kb < np; kb += 8) {
-        const int p0 = kb + t, p1 = kb + t + 4;
-        const int lr0 = __shfl_sync(0xffffffffu, lr_l, p0), lr1 = __shfl_sync(0xffffffffu, lr_l, p1);
-        const int lc0 = __shfl_sync(0xffffffffu, lc_l, p0), lc1 = __shfl_sync(0xffffffffu, lc_l, p1);
-        const float cr0 = __shfl_sync(0xffffffffu, cre_l, p0), cr1 = __shfl_sync(0xffffffffu, cre_l, p1);
-        const float ci0 = __shfl_sync(0xffffffffu, cim_l, p0), ci1 = __shfl_sync(0xffffffffu, cim_l, p1);
-        const float* w0 = wtab + p0 * 2 * w;
-        const float* w1 = wtab + p1 * 2 * w;
-        auto wy = [&](const float* wp, int d) { return (unsigned)d < (unsigned)w ? wp[w + d] : 0.f; };
-        auto wx = [&](const float* wp, int d) { return (unsigned)d < (unsigned)w ? wp[d] : 0.f; };
-        uint32_t ah[4], al[4];
-        split_tf32(wy(w0, gq - lr0), ah[0], al[0]);
-        split_tf32(wy(w0, gq + 8 - lr0), ah[1], al[1]);
-        split_tf32(wy(w1, gq - lr1), ah[2], al[2]);
-        split_tf32(wy(w1, gq + 8 - lr1), ah[3], al[3]);
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          const int col = 8 * j + gq;
-          const float x0 = wx(w0, col - lc0), x1 = wx(w1, col - lc1);
-          uint32_t rh0, rl0, rh1, rl1, ih0, il0, ih1, il1;
-          split_tf32(x0 * cr0, rh0, rl0);
-          split_tf32(x1 * cr1, rh1, rl1);
-          split_tf32(x0 * ci0, ih0, il0);
-          split_tf32(x1 * ci1, ih1, il1);
-          mma_tf32(dre[j], ah, rh0, rh1);
-          mma_tf32(dre[j], ah, rl0, rl1);
-          mma_tf32(dre[j], al, rh0, rh1);
-          mma_tf32(dim[j], ah, ih0, ih1);
-          mma_tf32(dim[j], ah, il0, il1);
-          mma_tf32(dim[j], al, ih0, ih1);
-        }
-      }
-      __syncwarp();
-    }
-    // add the subgrid to the band: fragment element e of n-tile j is
-    // (row gq + 8 (e >= 2), col 8 j + 2 t + (e & 1))
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int r = gq + (e >= 2 ? 8 : 0), cc = 8 * j + 2 * t + (e & 1);
-        const float vr = dre[j][e], vi = dim[j][e];
-        if (r >= SG || cc >= SG || (vr == 0.f && vi == 0.f)) continue;
-        int rw = item.z + r, cl = item.w + cc;
-        if (rw >= P.nf2) rw -= P.nf2;
-        if (cl >= P.nf1) cl -= P.nf1;
-        if (rw >= P.b2n || cl >= P.b1n) continue;  // beyond the band: only zero taps land here
-        float* dst = band + 2 * ((size_t)rw * P.b1n + cl);
-        if (staged) {
-          atomicAdd(dst, vr);
-          atomicAdd(dst + 1, vi);
-        } else {
-          atomicAdd(reinterpret_cast<float2*>(dst), make_float2(vr, vi));  // one 8-byte global reduction
-        }
-      }
-    }
-  }
-  if (staged) {
-    __syncthreads();
-    for (int i = threadIdx.x; i < 2 * ncell; i += blockDim.x) {
-      const float vv = band[i];
-      if (vv != 0.f) atomicAdd(gband + i, vv);
-    }
-    __syncthreads();
-  }
+  return it;
 }
 
 // ---------------------------------------------------------------------------
@@ -867,8 +727,8 @@ __device__ __noinline__ void fg_spread_tc(FgCtx<float>& c, const GroupCtx& g) {
 // waits on the point before, as it does with a subgrid in shared memory.  The
 // tile is added to the band when the next point lies in another one.
 // 256 x 256 / 97 200 points, 64 CTAs, a solve's stage with its barrier: 126 us
-// with shared subgrids and the weights evaluated each time, 33 us with
-// this and fg_taps.
+// with shared subgrids and the weights evaluated each time, 33 us with this
+// and fg_taps.
 // ---------------------------------------------------------------------------
 constexpr int SPREAD_ROW = 34;  // 16 axis-1 weights, 16 axis-2 weights, Re c, Im c
 template <int W>
@@ -890,13 +750,7 @@ __device__ __noinline__ void fg_spread_reg(FgCtx<double>& c, const GroupCtx& g) 
   const long first = (long)gw * share;
   if (first >= nuv) return;
   const int p0 = (int)first, p1 = min(nuv, p0 + share);
-  // the item that holds p0 (items cover the points in order)
-  int it = 0;
-  for (int hi = P.nitems; hi - it > 1;) {
-    const int mid = (it + hi) >> 1;
-    if (items[mid].x <= p0) it = mid;
-    else hi = mid;
-  }
+  int it = item_of(items, P.nitems, p0);
   double ar[8], ai[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) ar[i] = ai[i] = 0.0;
@@ -981,26 +835,186 @@ __device__ __noinline__ void fg_spread_reg(FgCtx<double>& c, const GroupCtx& g) 
   flush();
 }
 
-template <typename R>
-__device__ __noinline__ void fg_spread(FgCtx<R>& c, const GroupCtx& g) {
-  if constexpr (std::is_same<R, double>::value) {
-    // 69 632 bytes of weight rows for 8 warps, of the 98 304 an FP64 CTA has
-    static_assert((size_t)Shape<double>::warps * 32 * SPREAD_ROW * 8 <= 6144 * sizeof(cpx<double>), "weight rows");
-    if (c.P->bin == 8) {
-      switch (c.P->w) {
-#define SMILI_SPREAD_W(W) \
-  case W: fg_spread_reg<W>(c, g); return;
-        SMILI_SPREAD_W(2) SMILI_SPREAD_W(3) SMILI_SPREAD_W(4) SMILI_SPREAD_W(5) SMILI_SPREAD_W(6)
-        SMILI_SPREAD_W(7) SMILI_SPREAD_W(8) SMILI_SPREAD_W(9)
-#undef SMILI_SPREAD_W
-        default: break;  // a subgrid wider than 16 cells
+// ---------------------------------------------------------------------------
+// F5 in FP32 on the tensor cores (w <= 9, 8 x 8 tiles).  A tile's subgrid is
+// a product of two thin matrices:
+//   D[r][c] = sum_p wy_p[r] (c_p wx_p[c]),   r, c < 8 + w - 1 <= 16,
+// with wy_p / wx_p the point's kernel weights placed at its offset inside
+// the subgrid (zero elsewhere) and c_p = Vres_re - i Vres_im of the point.
+// A warp accumulates the real and imaginary parts of one tile's 16 x 16
+// subgrid in mma.sync.m16n8k8 TF32 fragments (8 points per k step) with the
+// three-term split a b ~ ah bh + ah bl + al bh (a = ah + al in TF32), which
+// keeps the products within a few FP32 ulps.  The operands of 16 points at a
+// time lie in shared memory already padded and multiplied, wx Re c | wx Im c |
+// wy, 56 floats apart (the 8 rows x 4 points a fragment reads are 32 banks),
+// so a fragment element is one load and its split, and the loads of the next
+// 16 points' taps are in flight meanwhile.  As in FP64 the warps take equal
+// contiguous ranges; a tile is added to the band at the end of its work item
+// (at most 128 points).
+// 74 problems of 97 200 points on groups of 4 CTAs, a solve's stage with its
+// barrier: 400 us with operands looked up and multiplied per fragment (520
+// instructions per 8 points) and the weights evaluated each time; with a
+// CUDA-core subgrid as in FP64 547 us (its row loads fill the shared-memory
+// pipe); 372 us with this and fg_taps.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ uint32_t to_tf32(float x) {
+  uint32_t r;
+  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
+  return r;
+}
+
+__device__ __forceinline__ void split_tf32(float x, uint32_t& hi, uint32_t& lo) {
+  hi = to_tf32(x);
+  lo = to_tf32(x - __uint_as_float(hi));
+}
+
+__device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+      "{%0,%1,%2,%3};\n"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+constexpr int SPREAD_TC_ROW = 56;     // floats per point: 16 wx Re c, 16 wx Im c, 16 wy, 8 unused
+constexpr int SPREAD_TC_POINTS = 16;  // points staged per warp
+template <int W>
+__device__ __noinline__ void fg_spread_tc(FgCtx<float>& c, const GroupCtx& g) {
+  const ProbDesc& P = *c.P;
+  const float* xu = at<float>(c.base, P.o_u);
+  const float* xv = at<float>(c.base, P.o_v);
+  const float* taps = P.o_taps ? at<float>(c.base, P.o_taps) : nullptr;
+  const int4* items = at<int4>(c.base, P.o_items);
+  const cpx<float>* cacc = at<cpx<float>>(c.base, P.o_contrib);
+  cpx<float>* gband = at<cpx<float>>(c.base, P.o_bandC);
+  const float beta = (float)P.beta, half = 0.5f * W, inv = 1.f / half;
+  const int nuv = P.nuv, nf1 = P.nf1, nf2 = P.nf2, b1n = P.b1n, b2n = P.b2n;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int gq = lane >> 2, t = lane & 3;
+  float* tab = reinterpret_cast<float*>(c.sbuf) + (size_t)warp * SPREAD_TC_POINTS * SPREAD_TC_ROW;
+  const int nwt = g.G * nw, gw = g.rank * nw + warp;
+  const int share = max(32, (nuv + nwt - 1) / nwt);
+  const long first = (long)gw * share;
+  if (first >= nuv) return;
+  const int p0 = (int)first, p1 = min(nuv, p0 + share);
+  int it = item_of(items, P.nitems, p0);
+  // lanes 0..15 prepare axis 1 (times c) of a point, lanes 16..31 axis 2
+  const int pt = lane & 15;
+  const bool ax1 = lane < 16;
+  const float* xs = ax1 ? xu : xv;
+  const float* tp = taps ? taps + (ax1 ? (size_t)0 : (size_t)W * nuv) : nullptr;
+  const int bs = ax1 ? P.b1s : P.b2s, nf = ax1 ? nf1 : nf2;
+  float k[W], x = 0.f;
+  cpx<float> cj = cmk<float>(0.f, 0.f);
+  auto fetch = [&](int j) {  // point j's coordinate, weights and value into registers
+    if (j < p1) {
+      x = xs[j];
+      if (tp) {
+#pragma unroll
+        for (int q = 0; q < W; ++q) k[q] = tp[(size_t)q * nuv + j];
+      }
+      if (ax1) cj = cacc[j];
+    }
+  };
+  fetch(p0 + pt);
+  for (int jb = p0; jb < p1; ++it) {
+    const int4 item = items[it];
+    const int origin = ax1 ? item.w : item.z;
+    const int je = min(p1, item.y);
+    float dre[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}}, dim[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
+    while (jb < je) {
+      const int np = min(SPREAD_TC_POINTS, je - jb);
+      {
+        float* row = tab + pt * SPREAD_TC_ROW + (ax1 ? 0 : 32);
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+        float4* r4 = reinterpret_cast<float4*>(row);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) r4[q] = zero;
+        if (ax1) {
+#pragma unroll
+          for (int q = 4; q < 8; ++q) r4[q] = zero;
+        }
+        if (pt < np) {
+          const int l = (int)ceilf(x - half);
+          if (!tp) {
+#pragma unroll
+            for (int q = 0; q < W; ++q) k[q] = es_kernel(((float)(l + q) - x) * inv, beta);
+          }
+          const int o = imod(l - bs, nf) - origin;  // in [0, 8)
+          if (ax1) {
+#pragma unroll
+            for (int q = 0; q < W; ++q) {
+              row[o + q] = k[q] * cj.x;
+              row[16 + o + q] = k[q] * -cj.y;  // c = Vresre - i Vresim
+            }
+          } else {
+#pragma unroll
+            for (int q = 0; q < W; ++q) row[o + q] = k[q];
+          }
+        }
+      }
+      jb += np;
+      fetch(jb + pt);
+      __syncwarp();
+      // 8 points per k step; lane (gq, t) feeds points t and t + 4
+#pragma unroll
+      for (int kb = 0; kb < SPREAD_TC_POINTS; kb += 8) {
+        if (kb >= np) break;
+        const float* w0 = tab + (kb + t) * SPREAD_TC_ROW + gq;
+        const float* w1 = w0 + 4 * SPREAD_TC_ROW;
+        uint32_t ah[4], al[4];
+        split_tf32(w0[32], ah[0], al[0]);
+        split_tf32(w0[40], ah[1], al[1]);
+        split_tf32(w1[32], ah[2], al[2]);
+        split_tf32(w1[40], ah[3], al[3]);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          uint32_t h0, l0, h1, l1;
+          split_tf32(w0[8 * j], h0, l0);
+          split_tf32(w1[8 * j], h1, l1);
+          mma_tf32(dre[j], ah, h0, h1);
+          mma_tf32(dre[j], ah, l0, l1);
+          mma_tf32(dre[j], al, h0, h1);
+          split_tf32(w0[16 + 8 * j], h0, l0);
+          split_tf32(w1[16 + 8 * j], h1, l1);
+          mma_tf32(dim[j], ah, h0, h1);
+          mma_tf32(dim[j], ah, l0, l1);
+          mma_tf32(dim[j], al, h0, h1);
+        }
+      }
+      __syncwarp();
+    }
+    // add the subgrid to the band: fragment element e of n-tile j is
+    // (row gq + 8 (e >= 2), col 8 j + 2 t + (e & 1))
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int r = gq + (e >= 2 ? 8 : 0), cc = 8 * j + 2 * t + (e & 1);
+        const float vr = dre[j][e], vi = dim[j][e];
+        if (r >= 8 + W - 1 || cc >= 8 + W - 1 || (vr == 0.f && vi == 0.f)) continue;
+        int rw = item.z + r, cl = item.w + cc;
+        if (rw >= nf2) rw -= nf2;
+        if (cl >= nf1) cl -= nf1;
+        if (rw < b2n && cl < b1n) acc_add(gband + ((size_t)rw * b1n + cl), cmk(vr, vi));  // else only zero taps land here
       }
     }
   }
-  if constexpr (std::is_same<R, float>::value) {
-    if (c.P->w <= 9 && c.P->bin == 8) {
-      fg_spread_tc(c, g);
-      return;
+}
+
+template <typename R>
+__device__ __noinline__ void fg_spread(FgCtx<R>& c, const GroupCtx& g) {
+  if (c.P->bin == 8) {
+    switch (c.P->w) {
+#define SMILI_SPREAD_W(W)                                                      \
+  case W:                                                                      \
+    if constexpr (std::is_same<R, double>::value) fg_spread_reg<W>(c, g);      \
+    else fg_spread_tc<W>(c, g);                                                \
+    return;
+      SMILI_SPREAD_W(2) SMILI_SPREAD_W(3) SMILI_SPREAD_W(4) SMILI_SPREAD_W(5) SMILI_SPREAD_W(6)
+      SMILI_SPREAD_W(7) SMILI_SPREAD_W(8) SMILI_SPREAD_W(9)
+#undef SMILI_SPREAD_W
+      default: break;  // a subgrid wider than 16 cells
     }
   }
   const ProbDesc& P = *c.P;

@@ -542,11 +542,15 @@ std::vector<double> deconv_factors(int N, int nf, int w, double beta) {
   return out;
 }
 
-// Dynamic shared memory per CTA: the FFT/spread staging buffers, at least
-// 48 KB, and never less than the Cauchy scan's layout.
+// Dynamic shared memory per CTA: the FFT staging buffers, and never less
+// than the spreading operands' or the Cauchy search's layout (96 KB in FP64,
+// 56 KB in FP32).
 template <typename R>
 size_t dyn_smem_bytes() {
-  size_t b = std::max((size_t)SMILI_DYN_CPX * sizeof(cpx<R>), (size_t)48 * 1024);
+  size_t b = (size_t)SMILI_DYN_CPX * sizeof(cpx<R>);
+  const size_t spread = sizeof(R) == 8 ? (size_t)Shape<R>::warps * 32 * SPREAD_ROW * 8
+                                       : (size_t)Shape<R>::warps * SPREAD_TC_POINTS * SPREAD_TC_ROW * 4;
+  b = std::max(b, (spread + 1023) / 1024 * 1024);
   b = std::max(b, (SMILI_CAUCHY_SMEM + 1023) / 1024 * 1024);
   return b;
 }
@@ -554,7 +558,7 @@ size_t dyn_smem_bytes() {
 // PK_FRAME: one frame of a movie; PK_MODEL: one evaluation that also returns per-datum models
 enum { PK_SOLVE = 0, PK_FG = 1, PK_T2 = 2, PK_T1 = 3, PK_FRAME = 4, PK_MODEL = 5 };
 
-// Whether the problems of a launch keep their kernel weights (fg_taps): FP64
+// Whether the problems of a launch keep their kernel weights (fg_taps):
 // launches that use them at least twice (a bare transform uses them once),
 // unless the tables would take more than 16 GB of the device's memory.
 template <typename R>
@@ -562,7 +566,7 @@ bool keep_taps(int kind, double eps, double nuv_total) {
   int w;
   double beta;
   es_params(eps, w, beta);
-  return sizeof(R) == 8 && kind != PK_T1 && kind != PK_T2 && nuv_total * 2 * w * sizeof(R) <= 16e9;
+  return kind != PK_T1 && kind != PK_T2 && nuv_total * 2 * w * sizeof(R) <= 16e9;
 }
 
 struct Arena {
@@ -819,15 +823,21 @@ int pack_problem(const smili_imaging_args& a, int kind, int niter, int nonneg, i
     return r < 0 ? r + n : r;
   };
   std::vector<long> bkey(nuv);
-  std::vector<int> bidx(nuv);
+  std::vector<int> bidx(nuv), cidx(nuv);
   const int nb1 = (d.nf1 + bin - 1) / bin, nb2 = (d.nf2 + bin - 1) / bin;
   for (int j = 0; j < nuv; ++j) {
     const long c1 = imodh((long)std::ceil(xu[j] - half) - d.b1s, d.nf1);
     const long c2 = imodh((long)std::ceil(xv[j] - half) - d.b2s, d.nf2);
     bkey[j] = ((c2 / bin) << 32) + (c1 / bin);
     bidx[j] = (int)(c2 / bin) * nb1 + (int)(c1 / bin);  // the same order as bkey
+    cidx[j] = (int)(c2 % bin) * bin + (int)(c1 % bin);
   }
-  const std::vector<int> perm = counting_order(nuv, nb1 * nb2, [&](int j) { return bidx[j]; });
+  // by tile, and inside a tile by cell: neighbouring threads of the
+  // interpolation then read the same band cells (a shared-memory broadcast
+  // instead of a bank conflict) wherever cells hold several points
+  const std::vector<int> by_cell = counting_order(nuv, bin * bin, [&](int j) { return cidx[j]; });
+  std::vector<int> perm = counting_order(nuv, nb1 * nb2, [&](int j) { return bidx[by_cell[j]]; });
+  for (int& j : perm) j = by_cell[j];
   // spreading work items: <= 128 consecutive points of one bin
   std::vector<int> items;
   for (int j = 0; j < nuv;) {
