@@ -41,6 +41,10 @@ int smili_unet_conv3x3_wgrad(const void* x, int ldx, const void* dy, int lddy, i
 /* db[c] (+)= sum over npix pixels of dy[p][c] */
 int smili_unet_bias_grad(const void* dy, int ld, long long npix, int C, float* db, int accumulate, void* stream);
 
+/* smili_unet_relu_mask, then smili_unet_bias_grad, in one pass over dy */
+int smili_unet_relu_bias_grad(const void* y, int ldy, void* dy, int lddy, long long npix, int C, float* db,
+                              int accumulate, void* stream);
+
 /* wt[ci][ky][kx][co] = w[co][2-ky][2-kx][ci]: the weights of the data-gradient
  * convolution (dx = conv3x3(dy, wt) with Cin and Cout exchanged). */
 int smili_unet_flip_weights(const void* w, void* wt, int Cout, int Cin, void* stream);

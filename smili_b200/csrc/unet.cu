@@ -21,11 +21,13 @@
 // and so do weight gradients whose channel counts and strides are multiples
 // of 8; the mma.sync kernels below take the rest (the one-channel input and
 // output layers).
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "../../include/smili_unet.h"
 #include "conv_tc.cuh"
@@ -171,6 +173,91 @@ __global__ void __launch_bounds__(256) conv3x3_kernel(ConvArgs a) {
 }
 
 // ---------------------------------------------------------------------------
+// conv3x3 of a one-channel input (the network's first layer), 8 NT output
+// channels per CTA.  The same mma.sync products in the same order as
+// conv3x3_kernel, of whose 16 input channels 15 are zero padding; here the
+// weights stay in registers, the fragments of the padding are the constant
+// zero, and only the input's own halo is staged.  32 x 128 x 128 pixels, 24
+// channels: 97 -> 21 us (25 MB to write).
+// ---------------------------------------------------------------------------
+constexpr int C1_H = 64;  // rows per CTA; a warp takes every eighth
+template <int NT>
+__global__ void __launch_bounds__(256) conv3x3_c1_kernel(ConvArgs a) {
+  __shared__ unsigned short halo[(C1_H + 2) * HALO_W];
+  const int tile = blockIdx.x;
+  const int tx = tile % a.tiles_x;
+  const int ty = (tile / a.tiles_x) % a.tiles_y;
+  const int n = tile / (a.tiles_x * a.tiles_y);
+  const int x0 = tx * TW, y0 = ty * C1_H;
+  const int co0 = blockIdx.y * NT * 8;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int g = lane >> 2, t = lane & 3;
+  const unsigned short* x = reinterpret_cast<const unsigned short*>(a.x);
+  const unsigned short* w = reinterpret_cast<const unsigned short*>(a.w);
+  uint32_t bf[9][NT];  // k = 0 sits in the low half of lane t = 0
+#pragma unroll
+  for (int tap = 0; tap < 9; ++tap)
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) {
+      const int co = co0 + nt * 8 + g;
+      bf[tap][nt] = (t == 0 && co < a.Cout) ? w[(size_t)co * 9 + tap] : 0u;
+    }
+  for (int q = threadIdx.x; q < (C1_H + 2) * HALO_W; q += blockDim.x) {
+    const int hy = q / HALO_W, hx = q - hy * HALO_W;
+    const int iy = y0 + hy - 1, ix = x0 + hx - 1;
+    halo[q] = (iy >= 0 && iy < a.H && ix >= 0 && ix < a.W) ? x[(((size_t)n * a.H + iy) * a.W + ix) * a.ldx] : 0;
+  }
+  float bias[NT][2];
+#pragma unroll
+  for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int co = co0 + nt * 8 + 2 * t + e;
+      bias[nt][e] = a.bias && co < a.Cout ? a.bias[co] : 0.f;
+    }
+  const bool pair = a.ldy % 2 == 0 && (reinterpret_cast<uintptr_t>(a.y) & 3) == 0;
+  __syncthreads();
+  for (int r = warp; r < C1_H && y0 + r < a.H; r += 8) {
+    float acc[NT][4];
+#pragma unroll
+    for (int i = 0; i < NT; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+#pragma unroll
+    for (int tap = 0; tap < 9; ++tap) {
+      const int ky = tap / 3, kx = tap - ky * 3;
+      const unsigned short* h = halo + (r + ky) * HALO_W + kx + g;
+      const uint32_t af[4] = {t == 0 ? (uint32_t)h[0] : 0u, t == 0 ? (uint32_t)h[8] : 0u, 0u, 0u};
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt) mma_bf16(acc[nt], af, bf[tap][nt], 0u);
+    }
+#pragma unroll
+    for (int hlf = 0; hlf < 2; ++hlf) {
+      const int ox = x0 + g + hlf * 8;
+      if (ox >= a.W) continue;
+      __nv_bfloat16* dst = a.y + (((size_t)n * a.H + y0 + r) * a.W + ox) * a.ldy;
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt) {
+        const int co = co0 + nt * 8 + 2 * t;
+        __nv_bfloat16 o[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          float v = acc[nt][hlf * 2 + e];
+          if (a.bias) v += bias[nt][e];
+          if (a.relu) v = fmaxf(v, 0.f);
+          if (a.accumulate && co + e < a.Cout) v += __bfloat162float(dst[co + e]);
+          o[e] = __float2bfloat16(v);
+        }
+        if (pair && co + 1 < a.Cout) {
+          *reinterpret_cast<uint32_t*>(dst + co) = pack2(o[0], o[1]);
+        } else {
+          if (co < a.Cout) dst[co] = o[0];
+          if (co + 1 < a.Cout) dst[co + 1] = o[1];
+        }
+      }
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
 // conv3x3 weight gradient: dW[co][tap][ci] = sum_p dY[p][co] X[p + s(tap)][ci]
 // A = dY^T (co x pixels), B = shifted X (pixels x ci); one k16 step is one
 // tile row of 16 pixels.  A CTA owns 64 output x 16 input channels for all 9
@@ -259,28 +346,214 @@ __global__ void __launch_bounds__(256) conv3x3_wgrad_kernel(WgradArgs a) {
   }
 }
 
-// sum the split partials in a fixed order: dw (+)= sum_s partial[s]
-__global__ void sum_partials_kernel(const float* partial, int nsplit, size_t count, float* dw, int accumulate) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < count; i += (size_t)gridDim.x * blockDim.x) {
-    float s = 0.f;
-    for (int k = 0; k < nsplit; ++k) s += partial[(size_t)k * count + i];
-    dw[i] = accumulate ? dw[i] + s : s;
+// ---------------------------------------------------------------------------
+// Weight gradient where one side has one channel (the network's first layer
+// and its head): 9 sums per channel of the wide side, a few multiply-adds per
+// byte, so memory bound and no matter for the tensor cores, whose tiles would
+// be padding.  A CTA owns 8 wide channels and the pixel tiles of its split; a
+// thread reads its pixel's 8 channels in one access and the thin side's 9
+// neighbours from shared memory.  THIN_X: x is the thin side, at p + s(tap);
+// otherwise dY, at p - s(tap) of x's pixel p.  32 x 128 x 128 pixels, 24
+// channels: 246 and 462 us on mma.sync, 40 us with this.
+// ---------------------------------------------------------------------------
+template <bool THIN_X>
+__global__ void __launch_bounds__(256) wgrad_thin_kernel(WgradArgs a) {
+  constexpr int HS = 18;
+  __shared__ float halo[HS * HS];
+  __shared__ float red[8][72];
+  const int split = blockIdx.x, c0 = blockIdx.y * 8, C = THIN_X ? a.Cout : a.Cin;
+  const __nv_bfloat16* wide = THIN_X ? a.dy : a.x;
+  const __nv_bfloat16* thin = THIN_X ? a.x : a.dy;
+  const int ldw = THIN_X ? a.lddy : a.ldx, ldt = THIN_X ? a.ldx : a.lddy;
+  const int tiles_x = (a.W + 15) / 16, tiles_y = (a.H + 15) / 16, ntiles = tiles_x * tiles_y * a.N;
+  const int r = threadIdx.x >> 4, cx = threadIdx.x & 15;
+  float acc[9][8];
+#pragma unroll
+  for (int t = 0; t < 9; ++t)
+#pragma unroll
+    for (int e = 0; e < 8; ++e) acc[t][e] = 0.f;
+  for (int tile = split; tile < ntiles; tile += a.nsplit) {
+    const int tx = tile % tiles_x, ty = (tile / tiles_x) % tiles_y, n = tile / (tiles_x * tiles_y);
+    const int x0 = tx * 16, y0 = ty * 16, iy = y0 + r, ix = x0 + cx;
+    const bool in = iy < a.H && ix < a.W;
+    uint4 v = make_uint4(0, 0, 0, 0);
+    if (in) v = *reinterpret_cast<const uint4*>(wide + (((size_t)n * a.H + iy) * a.W + ix) * ldw + c0);
+    __syncthreads();
+    for (int q = threadIdx.x; q < HS * HS; q += 256) {
+      const int hy = y0 + q / HS - 1, hx = x0 + q % HS - 1;
+      halo[q] = (hy >= 0 && hy < a.H && hx >= 0 && hx < a.W)
+                    ? __bfloat162float(thin[(((size_t)n * a.H + hy) * a.W + hx) * ldt])
+                    : 0.f;
+    }
+    __syncthreads();
+    const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int t = 0; t < 9; ++t) {
+      const int ky = t / 3, kx = t - ky * 3;
+      const float h = THIN_X ? halo[(r + ky) * HS + cx + kx] : halo[(r + 2 - ky) * HS + cx + 2 - kx];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        acc[t][2 * e] += __uint_as_float(u[e] << 16) * h;
+        acc[t][2 * e + 1] += __uint_as_float(u[e] & 0xffff0000u) * h;
+      }
+    }
+  }
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+  for (int t = 0; t < 9; ++t)
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      float s = acc[t][e];
+#pragma unroll
+      for (int b = 16; b >= 1; b >>= 1) s += __shfl_xor_sync(0xffffffffu, s, b);
+      if (lane == 0) red[warp][t * 8 + e] = s;
+    }
+  __syncthreads();
+  if (threadIdx.x < 72) {
+    float s = red[0][threadIdx.x];
+#pragma unroll
+    for (int w = 1; w < 8; ++w) s += red[w][threadIdx.x];
+    const int t = threadIdx.x >> 3, c = c0 + (threadIdx.x & 7);
+    // [split][co][tap][ci] with one of co, ci zero
+    a.partial[((size_t)split * 9) * C + (THIN_X ? (size_t)c * 9 + t : (size_t)t * C + c)] = s;
   }
 }
 
-// bias gradient: db[c] (+)= sum over pixels of dy[p][c] (fixed order per channel)
-__global__ void bias_grad_kernel(const __nv_bfloat16* dy, int ld, size_t npix, int C, float* db, int accumulate) {
-  __shared__ float red[256];
-  const int c = blockIdx.x;
+// Sum the split partials in their order: dw (+)= sum_s partial[s], the loads of
+// 32 splits in flight before their additions (148 splits of 5184 values: 18
+// us with a load per addition, 7 with 32).
+__global__ void __launch_bounds__(128) sum_partials_kernel(const float* partial, int nsplit, size_t count, float* dw,
+                                                           int accumulate) {
+  const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  if (i >= count) return;
+  const float* p = partial + i;
   float s = 0.f;
-  for (size_t p = threadIdx.x; p < npix; p += blockDim.x) s += __bfloat162float(dy[p * ld + c]);
-  red[threadIdx.x] = s;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
+  int k = 0;
+  for (; k + 32 <= nsplit; k += 32, p += 32 * count) {
+    float v[32];
+#pragma unroll
+    for (int q = 0; q < 32; ++q) v[q] = p[(size_t)q * count];
+#pragma unroll
+    for (int q = 0; q < 32; ++q) s += v[q];
+  }
+#pragma unroll 8
+  for (; k < nsplit; ++k, p += count) s += *p;
+  dw[i] = accumulate ? dw[i] + s : s;
+}
+
+// ---------------------------------------------------------------------------
+// Eight bf16 channels as one 16-byte access: the elementwise kernels below take
+// it where every channel count and stride is a multiple of 8 and the bases
+// are 16-byte aligned, and single elements elsewhere.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void unpack8(const uint4& v, float (&f)[8]) {
+  const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    f[2 * i] = __uint_as_float(u[i] << 16);
+    f[2 * i + 1] = __uint_as_float(u[i] & 0xffff0000u);
+  }
+}
+__device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
+  uint4 v;
+  v.x = pack2(__float2bfloat16(f[0]), __float2bfloat16(f[1]));
+  v.y = pack2(__float2bfloat16(f[2]), __float2bfloat16(f[3]));
+  v.z = pack2(__float2bfloat16(f[4]), __float2bfloat16(f[5]));
+  v.w = pack2(__float2bfloat16(f[6]), __float2bfloat16(f[7]));
+  return v;
+}
+__device__ __forceinline__ uint4 ld8(const __nv_bfloat16* p) { return *reinterpret_cast<const uint4*>(p); }
+__device__ __forceinline__ void st8(__nv_bfloat16* p, const uint4& v) { *reinterpret_cast<uint4*>(p) = v; }
+
+// dy where y > 0, else 0 (also where y is NaN)
+__device__ __forceinline__ uint32_t mask2(uint32_t y, uint32_t dy) {
+  const __nv_bfloat162 zero = __floats2bfloat162_rn(0.f, 0.f);
+  return dy & __hgt2_mask(*reinterpret_cast<const __nv_bfloat162*>(&y), zero);
+}
+__device__ __forceinline__ uint4 mask8(const uint4& y, const uint4& d) {
+  return make_uint4(mask2(y.x, d.x), mask2(y.y, d.y), mask2(y.z, d.z), mask2(y.w, d.w));
+}
+
+// Bias gradient db[c] (+)= sum over pixels of dy[p][c], with MASK after dy *=
+// (y > 0) in place.  The order of the sum is fixed: 256 chains, chain t over the
+// pixels t, t + 256, ... one after another, then a tree over the chains.  A
+// cluster of 16 CTAs sums one group of 8 channels (one channel where 16-byte
+// access does not apply): each CTA owns 16 chains, all its threads bring
+// their pixels into shared memory (eight 16-byte loads in flight each, the
+// next ones while this batch is added), one thread per chain and channel
+// adds, and rank 0 gathers the chains over distributed shared memory.
+// 24 channels of 32 x 128 x 128 pixels took 400 to 930 us with one CTA per
+// channel and 2-byte loads a row apart, 43 us with this and the mask.
+constexpr int BG_CTAS = 16, BG_THREADS = 512, BG_U = 8, BG_CHAINS = 256 / BG_CTAS;
+constexpr int BG_STEPS = BG_U * BG_THREADS / BG_CHAINS;  // additions per chain and batch: 256
+template <int E>
+constexpr int bg_smem() { return BG_STEPS * BG_CHAINS * E * 2; }
+template <bool VEC, bool MASK>
+__global__ void __launch_bounds__(BG_THREADS) bias_grad_kernel(const __nv_bfloat16* y, int ldy, __nv_bfloat16* dy,
+                                                               int lddy, size_t npix, float* db, int accumulate) {
+  constexpr int E = VEC ? 8 : 1;
+  typedef typename std::conditional<VEC, uint4, unsigned short>::type V;
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  extern __shared__ __align__(16) unsigned char bg_dyn[];  // [step][chain][E] bf16
+  __shared__ float red[256 * E];
+  V* buf = reinterpret_cast<V*>(bg_dyn);
+  const unsigned short* buf1 = reinterpret_cast<const unsigned short*>(bg_dyn);
+  const int c0 = (int)(blockIdx.x / BG_CTAS) * E, rank = blockIdx.x % BG_CTAS;
+  // loader: pixel (step, chain); adder: chain tid / E, channel tid % E
+  const int lt = threadIdx.x % BG_CHAINS, lk = threadIdx.x / BG_CHAINS;
+  const size_t steps = (npix + 255) / 256;
+  V v[BG_U], a[BG_U];
+  memset(a, 0, sizeof(a));
+  auto pixel = [&](size_t k0, int u) { return (k0 + u * (BG_THREADS / BG_CHAINS) + lk) * 256 + rank * BG_CHAINS + lt; };
+  auto load = [&](size_t k0) {
+#pragma unroll
+    for (int u = 0; u < BG_U; ++u) {
+      const size_t p = pixel(k0, u);
+      memset(&v[u], 0, sizeof(V));
+      if (p < npix) {
+        v[u] = *reinterpret_cast<const V*>(dy + p * lddy + c0);
+        if (MASK) a[u] = *reinterpret_cast<const V*>(y + p * ldy + c0);
+      }
+    }
+  };
+  auto store = [&](size_t k0) {
+#pragma unroll
+    for (int u = 0; u < BG_U; ++u) {
+      if (MASK) {
+        if constexpr (VEC) {
+          v[u] = mask8(a[u], v[u]);
+        } else {
+          v[u] = __bfloat162float(__ushort_as_bfloat16(a[u])) > 0.f ? v[u] : (unsigned short)0;
+        }
+        const size_t p = pixel(k0, u);
+        if (p < npix) *reinterpret_cast<V*>(dy + p * lddy + c0) = v[u];
+      }
+      buf[(u * (BG_THREADS / BG_CHAINS) + lk) * BG_CHAINS + lt] = v[u];
+    }
+  };
+  float s = 0.f;
+  load(0);
+  for (size_t k0 = 0; k0 < steps; k0 += BG_STEPS) {
+    store(k0);
+    __syncthreads();
+    if (k0 + BG_STEPS < steps) load(k0 + BG_STEPS);
+    if (threadIdx.x < BG_CHAINS * E) {
+#pragma unroll 32
+      for (int k = 0; k < BG_STEPS; ++k)
+        s += __uint_as_float((uint32_t)buf1[k * BG_CHAINS * E + threadIdx.x] << 16);
+    }
     __syncthreads();
   }
-  if (threadIdx.x == 0) db[c] = accumulate ? db[c] + red[0] : red[0];
+  if (threadIdx.x < BG_CHAINS * E)
+    cluster.map_shared_rank(red, 0)[rank * BG_CHAINS * E + threadIdx.x] = s;
+  cluster.sync();
+  if (rank != 0) return;
+  for (int w = 128; w > 0; w >>= 1) {
+    for (int i = threadIdx.x; i < w * E; i += BG_THREADS) red[i] += red[i + w * E];
+    __syncthreads();
+  }
+  if (threadIdx.x < E) db[c0 + threadIdx.x] = accumulate ? db[c0 + threadIdx.x] + red[threadIdx.x] : red[threadIdx.x];
 }
 
 // wt[ci][ky][kx][co] = w[co][2-ky][2-kx][ci]
@@ -304,7 +577,103 @@ __global__ void relu_mask_kernel(const __nv_bfloat16* y, int ldy, __nv_bfloat16*
   }
 }
 
-// 2x2 average pooling (H, W even) and its gradient
+// The 16-byte forms: chunk i of 8 channels of pixel p, with 32-bit indices
+// (the launch takes them where N H W C fits).  One thread reads or writes a
+// whole 2 x 2 block, in the scalar kernels' order of additions.
+struct Pool8 {
+  unsigned total, nch, Wh, Hh;  // chunks in all, chunks per pixel, coarse width and height
+};
+__device__ __forceinline__ void pool_index(const Pool8& q, unsigned i, unsigned& c, size_t& coarse, size_t& fine) {
+  const unsigned p = i / q.nch;
+  c = (i - p * q.nch) * 8;
+  const unsigned r = p / q.Wh, x = p - r * q.Wh, n = r / q.Hh, y = r - n * q.Hh;
+  coarse = p;
+  fine = ((size_t)n * 2 * q.Hh + 2 * y) * 2 * q.Wh + 2 * x;
+}
+__global__ void relu_mask8_kernel(const __nv_bfloat16* y, int ldy, __nv_bfloat16* dy, int lddy, unsigned total,
+                                  unsigned nch) {
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    const unsigned p = i / nch, c = (i - p * nch) * 8;
+    __nv_bfloat16* d = dy + (size_t)p * lddy + c;
+    st8(d, mask8(ld8(y + (size_t)p * ldy + c), ld8(d)));
+  }
+}
+__global__ void avgpool2x8_kernel(const __nv_bfloat16* x, int ldx, __nv_bfloat16* y, int ldy, Pool8 q) {
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < q.total; i += gridDim.x * blockDim.x) {
+    unsigned c;
+    size_t o, b;
+    pool_index(q, i, c, o, b);
+    const size_t W = 2 * q.Wh;
+    const uint4 v[4] = {ld8(x + b * ldx + c), ld8(x + (b + 1) * ldx + c), ld8(x + (b + W) * ldx + c),
+                        ld8(x + (b + W + 1) * ldx + c)};
+    float f[4][8], r[8];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) unpack8(v[k], f[k]);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) r[e] = 0.25f * (f[0][e] + f[1][e] + f[2][e] + f[3][e]);
+    st8(y + o * ldy + c, pack8(r));
+  }
+}
+__global__ void avgpool2x8_bwd_kernel(const __nv_bfloat16* dy, int lddy, __nv_bfloat16* dx, int lddx, Pool8 q,
+                                      int accumulate) {
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < q.total; i += gridDim.x * blockDim.x) {
+    unsigned c;
+    size_t o, b;
+    pool_index(q, i, c, o, b);
+    const size_t W = 2 * q.Wh, px[4] = {b, b + 1, b + W, b + W + 1};
+    const uint4 g = ld8(dy + o * lddy + c);
+    uint4 old[4];
+    if (accumulate) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) old[k] = ld8(dx + px[k] * lddx + c);
+    }
+    float f[8];
+    unpack8(g, f);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      float r[8], a[8];
+      if (accumulate) unpack8(old[k], a);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) r[e] = accumulate ? 0.25f * f[e] + a[e] : 0.25f * f[e];
+      st8(dx + px[k] * lddx + c, pack8(r));
+    }
+  }
+}
+__global__ void upsample2x8_kernel(const __nv_bfloat16* x, int ldx, __nv_bfloat16* y, int ldy, Pool8 q) {
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < q.total; i += gridDim.x * blockDim.x) {
+    unsigned c;
+    size_t o, b;
+    pool_index(q, i, c, o, b);
+    const size_t W = 2 * q.Wh;
+    const uint4 v = ld8(x + o * ldx + c);
+    st8(y + b * ldy + c, v);
+    st8(y + (b + 1) * ldy + c, v);
+    st8(y + (b + W) * ldy + c, v);
+    st8(y + (b + W + 1) * ldy + c, v);
+  }
+}
+__global__ void upsample2x8_bwd_kernel(const __nv_bfloat16* dy, int lddy, __nv_bfloat16* dx, int lddx, Pool8 q,
+                                       int accumulate) {
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < q.total; i += gridDim.x * blockDim.x) {
+    unsigned c;
+    size_t o, b;
+    pool_index(q, i, c, o, b);
+    const size_t W = 2 * q.Wh;
+    const uint4 v[4] = {ld8(dy + b * lddy + c), ld8(dy + (b + 1) * lddy + c), ld8(dy + (b + W) * lddy + c),
+                        ld8(dy + (b + W + 1) * lddy + c)};
+    float f[4][8], r[8], a[8];
+    if (accumulate) unpack8(ld8(dx + o * lddx + c), a);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) unpack8(v[k], f[k]);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      r[e] = f[0][e] + f[1][e] + f[2][e] + f[3][e];
+      if (accumulate) r[e] += a[e];
+    }
+    st8(dx + o * lddx + c, pack8(r));
+  }
+}
+
 __global__ void avgpool2_kernel(const __nv_bfloat16* x, int ldx, __nv_bfloat16* y, int ldy, int N, int H, int W,
                                 int C) {
   const int Ho = H / 2, Wo = W / 2;
@@ -428,9 +797,58 @@ int grid_for(size_t n, int block = 256) {
   return (int)(g < 1 ? 1 : g);
 }
 
+// whether two tensors' channels can be taken eight at a time
+bool vec8(const void* a, int lda, const void* b, int ldb, int C) {
+  return C % 8 == 0 && lda % 8 == 0 && ldb % 8 == 0 && (reinterpret_cast<uintptr_t>(a) & 15) == 0 &&
+         (reinterpret_cast<uintptr_t>(b) & 15) == 0;
+}
+
+// the 2 x 2 blocks of an N x 2 Hh x 2 Wh image with C channels; false when
+// the 32-bit indices of the 16-byte kernels do not reach
+bool pool8(Pool8& q, int N, int Hh, int Wh, int C) {
+  const size_t total = (size_t)N * Hh * Wh * (C / 8);
+  q.total = (unsigned)total;
+  q.nch = C / 8;
+  q.Wh = Wh;
+  q.Hh = Hh;
+  return total <= 0x7fffffffull;
+}
+
 int check_launch() {
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : SMILI_UNET_ERR_CUDA;
+}
+
+// bias gradient, after masking dy by y > 0 where y is given
+int launch_bias_grad(const void* y, int ldy, void* dy, int lddy, long long npix, int C, float* db, int accumulate,
+                     void* stream) {
+  const bool vec = vec8(dy, lddy, y ? y : dy, y ? ldy : lddy, C);
+  const void* fn = vec ? (y ? (const void*)bias_grad_kernel<true, true> : (const void*)bias_grad_kernel<true, false>)
+                       : (y ? (const void*)bias_grad_kernel<false, true> : (const void*)bias_grad_kernel<false, false>);
+  // 16 CTAs of a cluster, beyond the portable 8, and 64 KB of shared memory:
+  // both opted into, per device
+  const int smem = vec ? bg_smem<8>() : bg_smem<1>();
+  if (cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+      cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+    return SMILI_UNET_ERR_CUDA;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = BG_CTAS;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.gridDim = dim3((unsigned)BG_CTAS * (vec ? C / 8 : C));
+  cfg.blockDim = dim3(BG_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = static_cast<cudaStream_t>(stream);
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  const __nv_bfloat16* yp = static_cast<const __nv_bfloat16*>(y);
+  __nv_bfloat16* dp = static_cast<__nv_bfloat16*>(dy);
+  size_t n = (size_t)npix;
+  void* args[] = {&yp, &ldy, &dp, &lddy, &n, &db, &accumulate};
+  if (cudaLaunchKernelExC(&cfg, fn, args) != cudaSuccess) return SMILI_UNET_ERR_CUDA;
+  return check_launch();
 }
 
 }  // namespace
@@ -465,6 +883,15 @@ int smili_unet_conv3x3(const void* x, int N, int H, int W, int Cin, int ldx, con
                       g_conv_path == 2 ? 1 : 2) == 0
                ? 0
                : SMILI_UNET_ERR_CUDA;
+  if (g_conv_path != 1 && Cin == 1) {
+    a.tiles_y = (H + C1_H - 1) / C1_H;
+    const unsigned t1 = (unsigned)((long long)a.tiles_x * a.tiles_y * N);
+    if (Cout <= 8) conv3x3_c1_kernel<1><<<t1, 256, 0, s>>>(a);
+    else if (Cout <= 16) conv3x3_c1_kernel<2><<<t1, 256, 0, s>>>(a);
+    else if (Cout <= 24) conv3x3_c1_kernel<3><<<t1, 256, 0, s>>>(a);
+    else conv3x3_c1_kernel<4><<<dim3(t1, (Cout + 31) / 32), 256, 0, s>>>(a);
+    return check_launch();
+  }
   if (Cout <= 8) {
     conv3x3_kernel<1><<<dim3((unsigned)tiles, 1), 256, 0, s>>>(a);
   } else if (Cout <= 16) {
@@ -501,19 +928,27 @@ int smili_unet_conv3x3_wgrad(const void* x, int ldx, const void* dy, int lddy, i
   if (g_conv_path != 1 && tc::wgrad_eligible(x, ldx, dy, lddy, Cin, Cout)) {
     if (tc::launch_wgrad(a.x, ldx, a.dy, lddy, N, H, W, Cin, Cout, partial, nsplit, s) != 0)
       return SMILI_UNET_ERR_CUDA;
+  } else if (g_conv_path != 1 && Cin == 1 && vec8(dy, lddy, dy, lddy, Cout) && Cout / 8 <= 65535) {
+    wgrad_thin_kernel<true><<<dim3(nsplit, Cout / 8), 256, 0, s>>>(a);
+  } else if (g_conv_path != 1 && Cout == 1 && vec8(x, ldx, x, ldx, Cin) && Cin / 8 <= 65535) {
+    wgrad_thin_kernel<false><<<dim3(nsplit, Cin / 8), 256, 0, s>>>(a);
   } else {
     conv3x3_wgrad_kernel<<<dim3(nsplit, (Cout + 63) / 64, (Cin + KC - 1) / KC), 256, 0, s>>>(a);
   }
   const size_t count = (size_t)Cout * 9 * Cin;
-  sum_partials_kernel<<<grid_for(count), 256, 0, s>>>(partial, nsplit, count, dw, accumulate);
+  sum_partials_kernel<<<(unsigned)((count + 127) / 128), 128, 0, s>>>(partial, nsplit, count, dw, accumulate);
   return check_launch();
 }
 
 int smili_unet_bias_grad(const void* dy, int ld, long long npix, int C, float* db, int accumulate, void* stream) {
   if (!dy || !db || npix < 1 || C < 1 || ld < C) return SMILI_UNET_ERR_ARG;
-  bias_grad_kernel<<<C, 256, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const __nv_bfloat16*>(dy), ld,
-                                                                      (size_t)npix, C, db, accumulate);
-  return check_launch();
+  return launch_bias_grad(nullptr, C, const_cast<void*>(dy), ld, npix, C, db, accumulate, stream);
+}
+
+int smili_unet_relu_bias_grad(const void* y, int ldy, void* dy, int lddy, long long npix, int C, float* db,
+                              int accumulate, void* stream) {
+  if (!y || !dy || !db || npix < 1 || C < 1 || ldy < C || lddy < C) return SMILI_UNET_ERR_ARG;
+  return launch_bias_grad(y, ldy, dy, lddy, npix, C, db, accumulate, stream);
 }
 
 int smili_unet_flip_weights(const void* w, void* wt, int Cout, int Cin, void* stream) {
@@ -525,6 +960,12 @@ int smili_unet_flip_weights(const void* w, void* wt, int Cout, int Cin, void* st
 
 int smili_unet_relu_mask(const void* y, int ldy, void* dy, int lddy, long long npix, int C, void* stream) {
   if (!y || !dy || npix < 1 || C < 1 || ldy < C || lddy < C) return SMILI_UNET_ERR_ARG;
+  const size_t chunks = (size_t)npix * (C / 8);
+  if (vec8(y, ldy, dy, lddy, C) && chunks <= 0x7fffffffull) {
+    relu_mask8_kernel<<<grid_for(chunks), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+        static_cast<const __nv_bfloat16*>(y), ldy, static_cast<__nv_bfloat16*>(dy), lddy, (unsigned)chunks, C / 8);
+    return check_launch();
+  }
   relu_mask_kernel<<<grid_for((size_t)npix * C), 256, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const __nv_bfloat16*>(y), ldy, static_cast<__nv_bfloat16*>(dy), lddy, (size_t)npix, C);
   return check_launch();
@@ -533,6 +974,12 @@ int smili_unet_relu_mask(const void* y, int ldy, void* dy, int lddy, long long n
 int smili_unet_avgpool2(const void* x, int ldx, void* y, int ldy, int N, int H, int W, int C, void* stream) {
   if (!x || !y || N < 1 || H < 2 || W < 2 || (H & 1) || (W & 1) || C < 1 || ldx < C || ldy < C)
     return SMILI_UNET_ERR_ARG;
+  Pool8 q;
+  if (vec8(x, ldx, y, ldy, C) && pool8(q, N, H / 2, W / 2, C)) {
+    avgpool2x8_kernel<<<grid_for(q.total), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+        static_cast<const __nv_bfloat16*>(x), ldx, static_cast<__nv_bfloat16*>(y), ldy, q);
+    return check_launch();
+  }
   avgpool2_kernel<<<grid_for((size_t)N * H * W * C / 4), 256, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const __nv_bfloat16*>(x), ldx, static_cast<__nv_bfloat16*>(y), ldy, N, H, W, C);
   return check_launch();
@@ -542,6 +989,12 @@ int smili_unet_avgpool2_bwd(const void* dy, int lddy, void* dx, int lddx, int N,
                             int accumulate, void* stream) {
   if (!dy || !dx || N < 1 || H < 2 || W < 2 || (H & 1) || (W & 1) || C < 1 || lddx < C || lddy < C)
     return SMILI_UNET_ERR_ARG;
+  Pool8 q;
+  if (vec8(dy, lddy, dx, lddx, C) && pool8(q, N, H / 2, W / 2, C)) {
+    avgpool2x8_bwd_kernel<<<grid_for(q.total), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+        static_cast<const __nv_bfloat16*>(dy), lddy, static_cast<__nv_bfloat16*>(dx), lddx, q, accumulate);
+    return check_launch();
+  }
   avgpool2_bwd_kernel<<<grid_for((size_t)N * H * W * C), 256, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const __nv_bfloat16*>(dy), lddy, static_cast<__nv_bfloat16*>(dx), lddx, N, H, W, C, accumulate);
   return check_launch();
@@ -549,6 +1002,12 @@ int smili_unet_avgpool2_bwd(const void* dy, int lddy, void* dx, int lddx, int N,
 
 int smili_unet_upsample2(const void* x, int ldx, void* y, int ldy, int N, int H, int W, int C, void* stream) {
   if (!x || !y || N < 1 || H < 1 || W < 1 || C < 1 || ldx < C || ldy < C) return SMILI_UNET_ERR_ARG;
+  Pool8 q;
+  if (vec8(x, ldx, y, ldy, C) && pool8(q, N, H, W, C)) {
+    upsample2x8_kernel<<<grid_for(q.total), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+        static_cast<const __nv_bfloat16*>(x), ldx, static_cast<__nv_bfloat16*>(y), ldy, q);
+    return check_launch();
+  }
   upsample2_kernel<<<grid_for((size_t)N * H * W * C * 4), 256, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const __nv_bfloat16*>(x), ldx, static_cast<__nv_bfloat16*>(y), ldy, N, H, W, C);
   return check_launch();
@@ -557,6 +1016,12 @@ int smili_unet_upsample2(const void* x, int ldx, void* y, int ldy, int N, int H,
 int smili_unet_upsample2_bwd(const void* dy, int lddy, void* dx, int lddx, int N, int H, int W, int C,
                              int accumulate, void* stream) {
   if (!dy || !dx || N < 1 || H < 1 || W < 1 || C < 1 || lddx < C || lddy < C) return SMILI_UNET_ERR_ARG;
+  Pool8 q;
+  if (vec8(dy, lddy, dx, lddx, C) && pool8(q, N, H, W, C)) {
+    upsample2x8_bwd_kernel<<<grid_for(q.total), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+        static_cast<const __nv_bfloat16*>(dy), lddy, static_cast<__nv_bfloat16*>(dx), lddx, q, accumulate);
+    return check_launch();
+  }
   upsample2_bwd_kernel<<<grid_for((size_t)N * H * W * C), 256, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const __nv_bfloat16*>(dy), lddy, static_cast<__nv_bfloat16*>(dx), lddx, N, H, W, C, accumulate);
   return check_launch();

@@ -15,7 +15,7 @@ LIB_PATH = os.path.join(HERE, "libsmili_unet.so")
 EXPORTS = ["smili_unet_conv3x3", "smili_unet_conv3x3_wgrad", "smili_unet_bias_grad", "smili_unet_flip_weights",
            "smili_unet_relu_mask", "smili_unet_avgpool2", "smili_unet_avgpool2_bwd", "smili_unet_upsample2",
            "smili_unet_upsample2_bwd", "smili_unet_mse", "smili_unet_adam", "smili_unet_f32_to_bf16",
-           "smili_unet_set_conv_path", "smili_unet_tc_status", "smili_unet_last_error"]
+           "smili_unet_set_conv_path", "smili_unet_tc_status", "smili_unet_last_error", "smili_unet_relu_bias_grad"]
 
 _lib = None
 
@@ -31,6 +31,7 @@ def lib():
             "smili_unet_conv3x3": [vp, i, i, i, i, i, vp, vp, vp, i, i, i, i, vp],
             "smili_unet_conv3x3_wgrad": [vp, i, vp, i, i, i, i, i, i, vp, i, vp, i, vp],
             "smili_unet_bias_grad": [vp, i, ll, i, vp, i, vp],
+            "smili_unet_relu_bias_grad": [vp, i, vp, i, ll, i, vp, i, vp],
             "smili_unet_flip_weights": [vp, vp, i, i, vp],
             "smili_unet_relu_mask": [vp, i, vp, i, ll, i, vp],
             "smili_unet_avgpool2": [vp, i, vp, i, i, i, i, i, vp],
@@ -86,6 +87,12 @@ def conv3x3_wgrad(x, ldx, dy, lddy, N, H, W, Cin, Cout, partial, nsplit, dw, acc
 
 def bias_grad(dy, ld, npix, C_, db, accumulate=False):
     _check(lib().smili_unet_bias_grad(_p(dy), ld, npix, C_, _p(db), int(accumulate), _stream()), "bias_grad")
+
+
+def relu_bias_grad(y, ldy, dy, lddy, npix, C_, db, accumulate=False):
+    """relu_mask, then bias_grad, in one pass over dy."""
+    _check(lib().smili_unet_relu_bias_grad(_p(y), ldy, _p(dy), lddy, npix, C_, _p(db), int(accumulate), _stream()),
+           "relu_bias_grad")
 
 
 def flip_weights(w, wt, Cout, Cin):

@@ -225,9 +225,10 @@ class UNet:
         h, w = self.hw[name]
         npix = B * h * w
         if L.relu:
-            K.relu_mask(yout, ldyout, dy, lddy, npix, L.cout)
+            K.relu_bias_grad(yout, ldyout, dy, lddy, npix, L.cout, L.db)
+        else:
+            K.bias_grad(dy, lddy, npix, L.cout, L.db)
         K.conv3x3_wgrad(x, ldx, dy, lddy, B, h, w, L.cin, L.cout, self.partial, self.nsplit[name], L.dw)
-        K.bias_grad(dy, lddy, npix, L.cout, L.db)
         if need_dx:
             K.conv3x3(dy, B, h, w, L.cout, lddy, L.wt, None, dx, lddx, L.cin, False)
 
