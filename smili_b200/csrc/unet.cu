@@ -54,6 +54,39 @@ __device__ __forceinline__ uint32_t pack2(__nv_bfloat16 lo, __nv_bfloat16 hi) {
 }
 
 // ---------------------------------------------------------------------------
+// Eight bf16 channels as one 16-byte access: the elementwise kernels below take
+// it where every channel count and stride is a multiple of 8 and the bases
+// are 16-byte aligned, and single elements elsewhere.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void unpack8(const uint4& v, float (&f)[8]) {
+  const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    f[2 * i] = __uint_as_float(u[i] << 16);
+    f[2 * i + 1] = __uint_as_float(u[i] & 0xffff0000u);
+  }
+}
+__device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
+  uint4 v;
+  v.x = pack2(__float2bfloat16(f[0]), __float2bfloat16(f[1]));
+  v.y = pack2(__float2bfloat16(f[2]), __float2bfloat16(f[3]));
+  v.z = pack2(__float2bfloat16(f[4]), __float2bfloat16(f[5]));
+  v.w = pack2(__float2bfloat16(f[6]), __float2bfloat16(f[7]));
+  return v;
+}
+__device__ __forceinline__ uint4 ld8(const __nv_bfloat16* p) { return *reinterpret_cast<const uint4*>(p); }
+__device__ __forceinline__ void st8(__nv_bfloat16* p, const uint4& v) { *reinterpret_cast<uint4*>(p) = v; }
+
+// dy where y > 0, else 0 (also where y is NaN)
+__device__ __forceinline__ uint32_t mask2(uint32_t y, uint32_t dy) {
+  const __nv_bfloat162 zero = __floats2bfloat162_rn(0.f, 0.f);
+  return dy & __hgt2_mask(*reinterpret_cast<const __nv_bfloat162*>(&y), zero);
+}
+__device__ __forceinline__ uint4 mask8(const uint4& y, const uint4& d) {
+  return make_uint4(mask2(y.x, d.x), mask2(y.y, d.y), mask2(y.z, d.z), mask2(y.w, d.w));
+}
+
+// ---------------------------------------------------------------------------
 // conv3x3 forward / data-gradient
 // ---------------------------------------------------------------------------
 struct ConvArgs {
@@ -348,74 +381,111 @@ __global__ void __launch_bounds__(256) conv3x3_wgrad_kernel(WgradArgs a) {
 
 // ---------------------------------------------------------------------------
 // Weight gradient where one side has one channel (the network's first layer
-// and its head): 9 sums per channel of the wide side, a few multiply-adds per
-// byte, so memory bound and no matter for the tensor cores, whose tiles would
-// be padding.  A CTA owns 8 wide channels and the pixel tiles of its split; a
-// thread reads its pixel's 8 channels in one access and the thin side's 9
-// neighbours from shared memory.  THIN_X: x is the thin side, at p + s(tap);
-// otherwise dY, at p - s(tap) of x's pixel p.  32 x 128 x 128 pixels, 24
-// channels: 246 and 462 us on mma.sync, 40 us with this.
+// and its head): the products of conv3x3_wgrad_kernel in its order (per split the
+// tiles in turn, per tile its eight 16-pixel rows), without its staging of 64 x
+// 16 channels of which one side is padding.  A CTA owns 32 channels of the wide
+// side, one warp each tap; the wide side's tile lies in shared memory as it
+// lies in global memory and its fragments come transposed by ldmatrix, the
+// thin side's are a few of its pixels; the next tile's loads are in flight
+// meanwhile.  THIN_X: x is the thin side (its halo is staged) and dY the A
+// operand; otherwise dY is thin and x (its halo) the B operand.  32 x 128 x 128
+// pixels, 24 channels: 246 and 462 us with the padding, 25 and 36 without.
 // ---------------------------------------------------------------------------
+constexpr int THIN_CH = 32, THIN_ROW = THIN_CH + 8, THIN_THREADS = 9 * 32;
 template <bool THIN_X>
-__global__ void __launch_bounds__(256) wgrad_thin_kernel(WgradArgs a) {
-  constexpr int HS = 18;
-  __shared__ float halo[HS * HS];
-  __shared__ float red[8][72];
-  const int split = blockIdx.x, c0 = blockIdx.y * 8, C = THIN_X ? a.Cout : a.Cin;
+__global__ void __launch_bounds__(THIN_THREADS) wgrad_thin_kernel(WgradArgs a) {
+  constexpr int WPX = THIN_X ? TH * TW : HALO_H * HALO_W;  // staged pixels of the wide side
+  constexpr int TPX = THIN_X ? HALO_H * HALO_W : TH * TW;  // and of the thin side
+  constexpr int NV = (WPX * (THIN_CH / 8) + THIN_THREADS - 1) / THIN_THREADS;
+  __shared__ __align__(16) __nv_bfloat16 ws[2][WPX * THIN_ROW];
+  __shared__ __align__(4) unsigned short ts[2][TPX + 1];
+  const int split = blockIdx.x, c0 = blockIdx.y * THIN_CH, C = THIN_X ? a.Cout : a.Cin;
   const __nv_bfloat16* wide = THIN_X ? a.dy : a.x;
-  const __nv_bfloat16* thin = THIN_X ? a.x : a.dy;
+  const unsigned short* thin = reinterpret_cast<const unsigned short*>(THIN_X ? a.x : a.dy);
   const int ldw = THIN_X ? a.lddy : a.ldx, ldt = THIN_X ? a.ldx : a.lddy;
-  const int tiles_x = (a.W + 15) / 16, tiles_y = (a.H + 15) / 16, ntiles = tiles_x * tiles_y * a.N;
-  const int r = threadIdx.x >> 4, cx = threadIdx.x & 15;
-  float acc[9][8];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int tap = warp, ky = tap / 3, kx = tap - ky * 3;
+  uint4 v[NV];
+  unsigned short tv = 0;
+  auto fetch = [&](int tile) {  // a tile's pixels into registers (zeros outside the image)
+    const int tx = tile % a.tiles_x, ty = (tile / a.tiles_x) % a.tiles_y, n = tile / (a.tiles_x * a.tiles_y);
+    const int x0 = tx * TW, y0 = ty * TH;
 #pragma unroll
-  for (int t = 0; t < 9; ++t)
-#pragma unroll
-    for (int e = 0; e < 8; ++e) acc[t][e] = 0.f;
-  for (int tile = split; tile < ntiles; tile += a.nsplit) {
-    const int tx = tile % tiles_x, ty = (tile / tiles_x) % tiles_y, n = tile / (tiles_x * tiles_y);
-    const int x0 = tx * 16, y0 = ty * 16, iy = y0 + r, ix = x0 + cx;
-    const bool in = iy < a.H && ix < a.W;
-    uint4 v = make_uint4(0, 0, 0, 0);
-    if (in) v = *reinterpret_cast<const uint4*>(wide + (((size_t)n * a.H + iy) * a.W + ix) * ldw + c0);
-    __syncthreads();
-    for (int q = threadIdx.x; q < HS * HS; q += 256) {
-      const int hy = y0 + q / HS - 1, hx = x0 + q % HS - 1;
-      halo[q] = (hy >= 0 && hy < a.H && hx >= 0 && hx < a.W)
-                    ? __bfloat162float(thin[(((size_t)n * a.H + hy) * a.W + hx) * ldt])
-                    : 0.f;
+    for (int q = 0; q < NV; ++q) {
+      const int i = threadIdx.x + q * THIN_THREADS, px = i / (THIN_CH / 8), ch = c0 + (i % (THIN_CH / 8)) * 8;
+      const int iy = THIN_X ? y0 + px / TW : y0 + px / HALO_W - 1, ix = THIN_X ? x0 + px % TW : x0 + px % HALO_W - 1;
+      v[q] = make_uint4(0, 0, 0, 0);
+      if (px < WPX && ch < C && iy >= 0 && iy < a.H && ix >= 0 && ix < a.W)
+        v[q] = ld8(wide + (((size_t)n * a.H + iy) * a.W + ix) * ldw + ch);
     }
+    if (threadIdx.x < TPX) {
+      const int px = threadIdx.x;
+      const int iy = THIN_X ? y0 + px / HALO_W - 1 : y0 + px / TW, ix = THIN_X ? x0 + px % HALO_W - 1 : x0 + px % TW;
+      tv = (iy >= 0 && iy < a.H && ix >= 0 && ix < a.W) ? thin[(((size_t)n * a.H + iy) * a.W + ix) * ldt] : 0;
+    }
+  };
+  auto stage = [&](int b) {
+#pragma unroll
+    for (int q = 0; q < NV; ++q) {
+      const int i = threadIdx.x + q * THIN_THREADS, px = i / (THIN_CH / 8);
+      if (px < WPX) st8(ws[b] + px * THIN_ROW + (i % (THIN_CH / 8)) * 8, v[q]);
+    }
+    if (threadIdx.x < TPX) ts[b][threadIdx.x] = tv;
+  };
+  // fragments of 16 output channels (THIN_X) or 8 input channels
+  constexpr int NF = THIN_X ? THIN_CH / 16 : THIN_CH / 8;
+  float acc[NF][4];
+#pragma unroll
+  for (int f = 0; f < NF; ++f) acc[f][0] = acc[f][1] = acc[f][2] = acc[f][3] = 0.f;
+  if (split < a.ntiles) fetch(split);
+  int b = 0;
+  for (int tile = split; tile < a.ntiles; tile += a.nsplit, b ^= 1) {
+    stage(b);
     __syncthreads();
-    const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+    if (tile + a.nsplit < a.ntiles) fetch(tile + a.nsplit);
 #pragma unroll
-    for (int t = 0; t < 9; ++t) {
-      const int ky = t / 3, kx = t - ky * 3;
-      const float h = THIN_X ? halo[(r + ky) * HS + cx + kx] : halo[(r + 2 - ky) * HS + cx + 2 - kx];
+    for (int r = 0; r < TH; ++r) {
+      // the thin side's 16 pixels: lanes of its one channel hold two pairs
+      const unsigned short* h = THIN_X ? &ts[b][(r + ky) * HALO_W + kx + 2 * t] : &ts[b][r * TW + 2 * t];
+      const uint32_t t0 = g == 0 ? (uint32_t)h[0] | ((uint32_t)h[1] << 16) : 0u;
+      const uint32_t t1 = g == 0 ? (uint32_t)h[8] | ((uint32_t)h[9] << 16) : 0u;
+      const __nv_bfloat16* row = ws[b] + (THIN_X ? r * TW : (r + ky) * HALO_W + kx) * THIN_ROW;
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        acc[t][2 * e] += __uint_as_float(u[e] << 16) * h;
-        acc[t][2 * e + 1] += __uint_as_float(u[e] & 0xffff0000u) * h;
+      for (int f = 0; f < NF; ++f) {
+        if constexpr (THIN_X) {  // A = dY^T: (channels 0-7 | 8-15) x (pixels 0-7 | 8-15)
+          uint32_t af[4];
+          const __nv_bfloat16* src = row + ((lane & 7) + (lane & 16 ? 8 : 0)) * THIN_ROW + 16 * f + (lane & 8 ? 8 : 0);
+          asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                       : "=r"(af[0]), "=r"(af[1]), "=r"(af[2]), "=r"(af[3])
+                       : "r"((uint32_t)__cvta_generic_to_shared(src))
+                       : "memory");
+          mma_bf16(acc[f], af, t0, t1);
+        } else {  // B = x: pixels (0-7 | 8-15) x 8 channels
+          uint32_t b0, b1;
+          const __nv_bfloat16* src = row + (lane & 15) * THIN_ROW + 8 * f;
+          asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0, %1}, [%2];"
+                       : "=r"(b0), "=r"(b1)
+                       : "r"((uint32_t)__cvta_generic_to_shared(src))
+                       : "memory");
+          const uint32_t af[4] = {t0, 0u, t1, 0u};
+          mma_bf16(acc[f], af, b0, b1);
+        }
       }
     }
   }
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // partial[split][co][tap][ci], one of co and ci zero
+  float* out = a.partial + (size_t)split * 9 * C;
 #pragma unroll
-  for (int t = 0; t < 9; ++t)
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      float s = acc[t][e];
-#pragma unroll
-      for (int b = 16; b >= 1; b >>= 1) s += __shfl_xor_sync(0xffffffffu, s, b);
-      if (lane == 0) red[warp][t * 8 + e] = s;
+  for (int f = 0; f < NF; ++f) {
+    if constexpr (THIN_X) {  // column 0: rows g and g + 8
+      const int c = c0 + 16 * f + g;
+      if (t == 0 && c < C) out[(size_t)c * 9 + tap] = acc[f][0];
+      if (t == 0 && c + 8 < C) out[(size_t)(c + 8) * 9 + tap] = acc[f][2];
+    } else {  // row 0: columns 2 t and 2 t + 1
+      const int c = c0 + 8 * f + 2 * t;
+      if (g == 0 && c < C) out[(size_t)tap * C + c] = acc[f][0];
+      if (g == 0 && c + 1 < C) out[(size_t)tap * C + c + 1] = acc[f][1];
     }
-  __syncthreads();
-  if (threadIdx.x < 72) {
-    float s = red[0][threadIdx.x];
-#pragma unroll
-    for (int w = 1; w < 8; ++w) s += red[w][threadIdx.x];
-    const int t = threadIdx.x >> 3, c = c0 + (threadIdx.x & 7);
-    // [split][co][tap][ci] with one of co, ci zero
-    a.partial[((size_t)split * 9) * C + (THIN_X ? (size_t)c * 9 + t : (size_t)t * C + c)] = s;
   }
 }
 
@@ -439,39 +509,6 @@ __global__ void __launch_bounds__(128) sum_partials_kernel(const float* partial,
 #pragma unroll 8
   for (; k < nsplit; ++k, p += count) s += *p;
   dw[i] = accumulate ? dw[i] + s : s;
-}
-
-// ---------------------------------------------------------------------------
-// Eight bf16 channels as one 16-byte access: the elementwise kernels below take
-// it where every channel count and stride is a multiple of 8 and the bases
-// are 16-byte aligned, and single elements elsewhere.
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ void unpack8(const uint4& v, float (&f)[8]) {
-  const uint32_t u[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    f[2 * i] = __uint_as_float(u[i] << 16);
-    f[2 * i + 1] = __uint_as_float(u[i] & 0xffff0000u);
-  }
-}
-__device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
-  uint4 v;
-  v.x = pack2(__float2bfloat16(f[0]), __float2bfloat16(f[1]));
-  v.y = pack2(__float2bfloat16(f[2]), __float2bfloat16(f[3]));
-  v.z = pack2(__float2bfloat16(f[4]), __float2bfloat16(f[5]));
-  v.w = pack2(__float2bfloat16(f[6]), __float2bfloat16(f[7]));
-  return v;
-}
-__device__ __forceinline__ uint4 ld8(const __nv_bfloat16* p) { return *reinterpret_cast<const uint4*>(p); }
-__device__ __forceinline__ void st8(__nv_bfloat16* p, const uint4& v) { *reinterpret_cast<uint4*>(p) = v; }
-
-// dy where y > 0, else 0 (also where y is NaN)
-__device__ __forceinline__ uint32_t mask2(uint32_t y, uint32_t dy) {
-  const __nv_bfloat162 zero = __floats2bfloat162_rn(0.f, 0.f);
-  return dy & __hgt2_mask(*reinterpret_cast<const __nv_bfloat162*>(&y), zero);
-}
-__device__ __forceinline__ uint4 mask8(const uint4& y, const uint4& d) {
-  return make_uint4(mask2(y.x, d.x), mask2(y.y, d.y), mask2(y.z, d.z), mask2(y.w, d.w));
 }
 
 // Bias gradient db[c] (+)= sum over pixels of dy[p][c], with MASK after dy *=
@@ -928,10 +965,10 @@ int smili_unet_conv3x3_wgrad(const void* x, int ldx, const void* dy, int lddy, i
   if (g_conv_path != 1 && tc::wgrad_eligible(x, ldx, dy, lddy, Cin, Cout)) {
     if (tc::launch_wgrad(a.x, ldx, a.dy, lddy, N, H, W, Cin, Cout, partial, nsplit, s) != 0)
       return SMILI_UNET_ERR_CUDA;
-  } else if (g_conv_path != 1 && Cin == 1 && vec8(dy, lddy, dy, lddy, Cout) && Cout / 8 <= 65535) {
-    wgrad_thin_kernel<true><<<dim3(nsplit, Cout / 8), 256, 0, s>>>(a);
-  } else if (g_conv_path != 1 && Cout == 1 && vec8(x, ldx, x, ldx, Cin) && Cin / 8 <= 65535) {
-    wgrad_thin_kernel<false><<<dim3(nsplit, Cin / 8), 256, 0, s>>>(a);
+  } else if (g_conv_path != 1 && Cin == 1 && vec8(dy, lddy, dy, lddy, Cout) && Cout <= 65535 * THIN_CH) {
+    wgrad_thin_kernel<true><<<dim3(nsplit, (Cout + THIN_CH - 1) / THIN_CH), THIN_THREADS, 0, s>>>(a);
+  } else if (g_conv_path != 1 && Cout == 1 && vec8(x, ldx, x, ldx, Cin) && Cin <= 65535 * THIN_CH) {
+    wgrad_thin_kernel<false><<<dim3(nsplit, (Cin + THIN_CH - 1) / THIN_CH), THIN_THREADS, 0, s>>>(a);
   } else {
     conv3x3_wgrad_kernel<<<dim3(nsplit, (Cout + 63) / 64, (Cin + KC - 1) / KC), 256, 0, s>>>(a);
   }
