@@ -825,7 +825,7 @@ __global__ void f32_to_bf16_kernel(const float* x, __nv_bfloat16* y, size_t n) {
 }
 
 // 0: tensor-core (tcgen05) path where it applies, else mma.sync; 1: always
-// mma.sync; 2: tcgen05 with one 128-pixel tile per CTA (for comparisons)
+// mma.sync; 2: tcgen05 with one 128-pixel tile per group (for comparisons)
 int g_conv_path = 0;
 
 int grid_for(size_t n, int block = 256) {
@@ -917,7 +917,7 @@ int smili_unet_conv3x3(const void* x, int N, int H, int W, int Cin, int ldx, con
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (g_conv_path != 1 && tc::eligible(x, Cin, ldx, w, Cout))
     return tc::launch(a.x, N, H, W, Cin, ldx, a.w, bias, a.y, ldy, Cout, relu, accumulate, s,
-                      g_conv_path == 2 ? 1 : 2) == 0
+                      g_conv_path == 2 ? 1 : tc::MAX_SUB) == 0
                ? 0
                : SMILI_UNET_ERR_CUDA;
   if (g_conv_path != 1 && Cin == 1) {

@@ -111,3 +111,32 @@ def test_one_channel_weight_gradient(thin_x, C, H, W, nsplit):
         mag[:, t] += np.einsum("nhwo,nhwi->oi", np.abs(d), np.abs(s))
     # products exact in FP32; additions on the tensor cores may truncate (2^-23 each)
     assert (np.abs(dw.double().cpu().numpy() - ref) <= (N * H * W + nsplit) * 2.0 ** -23 * mag).all()
+
+
+# (N, H, W, Cin, Cout, ldx, ldy): tiles and groups with remainders, 32- and
+# 64-channel planes, resident and streamed weights, one to four tiles per
+# group, several output-channel and input-channel blocks
+CONV = [(2, 5, 3, 8, 1, 8, 1), (3, 17, 9, 24, 24, 72, 40), (150, 20, 12, 24, 24, 24, 24), (40, 33, 20, 72, 24, 72, 24),
+        (2, 16, 16, 48, 48, 48, 48), (3, 32, 32, 144, 48, 144, 48), (2, 16, 24, 96, 192, 96, 192),
+        (40, 32, 32, 192, 192, 192, 288), (1, 16, 16, 192, 272, 192, 272), (1, 20, 12, 640, 40, 640, 40)]
+
+
+@pytest.mark.parametrize("N,H,W,Cin,Cout,ldx,ldy", CONV)
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_tensor_core_convolution(N, H, W, Cin, Cout, ldx, ldy, accumulate):
+    import torch
+    from smili_b200.warmstart import kernels as K
+    x, w = _rand((N, H, W, ldx), 11), _rand((Cout, 3, 3, Cin), 12, 1 / (3 * Cin ** 0.5))
+    b = torch.randn(Cout, device="cuda")
+    y = _rand((N, H, W, ldy), 13)
+    old = y.clone()
+    K.conv3x3(x, N, H, W, Cin, ldx, w, b, y, ldy, Cout, True, accumulate)
+    assert K.tc_status() == 0
+    xd, wd = x[..., :Cin].double().permute(0, 3, 1, 2), w.double().permute(0, 3, 1, 2)
+    add = old[..., :Cout].double() if accumulate else 0.0
+    ref = torch.relu(torch.nn.functional.conv2d(xd, wd, b.double(), padding=1)).permute(0, 2, 3, 1) + add
+    mag = torch.nn.functional.conv2d(xd.abs(), wd.abs(), b.double().abs(), padding=1).permute(0, 2, 3, 1) + abs(add)
+    # FP32 sums of 9 Cin products and the bf16 rounding of the result
+    bound = (9 * Cin + 2) * 2.0 ** -23 * mag + 2.0 ** -8 * ref.abs()
+    assert ((y[..., :Cout].double() - ref).abs() <= bound).all()
+    assert torch.equal(y[..., Cout:], old[..., Cout:])
