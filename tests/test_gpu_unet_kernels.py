@@ -140,3 +140,31 @@ def test_tensor_core_convolution(N, H, W, Cin, Cout, ldx, ldy, accumulate):
     bound = (9 * Cin + 2) * 2.0 ** -23 * mag + 2.0 ** -8 * ref.abs()
     assert ((y[..., :Cout].double() - ref).abs() <= bound).all()
     assert torch.equal(y[..., Cout:], old[..., Cout:])
+
+
+# (N, H, W, Cin, Cout, nsplit): one, three and nine taps per CTA, either side
+# on M, several M and N tiles, splits with and without pixels
+WGRAD = [(1, 8, 16, 8, 16, 1), (3, 17, 9, 24, 24, 4), (2, 32, 32, 72, 24, 7), (64, 16, 32, 24, 24, 128),
+         (2, 20, 40, 96, 96, 5), (2, 16, 16, 288, 96, 3), (4, 32, 32, 192, 192, 8), (1, 16, 16, 16, 272, 2),
+         (1, 9, 9, 24, 24, 30)]
+
+
+@pytest.mark.parametrize("N,H,W,Cin,Cout,nsplit", WGRAD)
+def test_tensor_core_weight_gradient(N, H, W, Cin, Cout, nsplit):
+    import torch
+    from smili_b200.warmstart import kernels as K
+    ldx, ldd = Cin + 8, Cout + 16
+    x, dy = _rand((N, H, W, ldx), 14), _rand((N, H, W, ldd), 15)
+    part = torch.full((nsplit, Cout, 9, Cin), float("nan"), device="cuda")
+    dw = torch.ones(Cout, 3, 3, Cin, device="cuda")
+    K.conv3x3_wgrad(x, ldx, dy, ldd, N, H, W, Cin, Cout, part, nsplit, dw, accumulate=True)
+    assert K.tc_status() == 0
+
+    def grad(a, d):
+        w = torch.zeros(Cout, Cin, 3, 3, dtype=torch.float64, device="cuda", requires_grad=True)
+        y = torch.nn.functional.conv2d(a.double().permute(0, 3, 1, 2), w, padding=1)
+        y.backward(d.double().permute(0, 3, 1, 2))
+        return w.grad.permute(0, 2, 3, 1) + 1.0
+    xs, ds = x[..., :Cin], dy[..., :Cout]
+    bound = (N * H * W + nsplit) * 2.0 ** -23 * grad(xs.abs(), ds.abs())
+    assert ((dw.double() - grad(xs, ds)).abs() <= bound).all()
