@@ -49,6 +49,15 @@ __device__ __forceinline__ int fft_batch(int n) {
   return s < 1 ? 1 : s;
 }
 
+// global atomic addition of a complex value: one vector reduction in FP32, two in FP64
+__device__ __forceinline__ void acc_add(cpx<float>* p, cpx<float> v) {
+  atomicAdd(reinterpret_cast<float2*>(p), make_float2(v.x, v.y));
+}
+__device__ __forceinline__ void acc_add(cpx<double>* p, cpx<double> v) {
+  atomicAdd(&p->x, v.x);
+  atomicAdd(&p->y, v.y);
+}
+
 // Working context of one problem inside a kernel
 template <typename R>
 struct FgCtx {
@@ -92,20 +101,42 @@ struct KSumF {
 //   F6  tmpC[r][ix]  = sum_b  bandC[r][b] Ex[b][ix]
 //   F7  gchi[iy][ix] = Re sum_r Ey[r][iy] tmpC[r][ix]  * dc1[ix] dc2[iy]
 // (the same twiddles the radix passes apply, exp periodic in nf).  Used
-// for bands of at most 64 x 64 cells, where each pass is a few million
-// multiply-adds that run as register-tiled loops.
+// for bands of at most 64 x 64 cells, 2048 in all, where each pass is a few
+// million multiply-adds.  F1 and F2 are one stage: a CTA takes its share of the
+// image rows through both and adds its part of the band to bandA (zeroed by the
+// spreading stage before); so are F6 and F7, a CTA taking its share of the
+// image columns.  As four stages of register tiles, each stage had work for 4 to
+// 16 CTAs only: 256 x 256, 44 x 21 cells, FP64 on 64 CTAs, 70 + 40 + 24 + 14 us
+// per evaluation, 23 + 21 as two; FP32 on groups of 4 CTAs (74 problems), 100 +
+// 40 + 44 + 141 and 131 + 96.
 // ---------------------------------------------------------------------------
-constexpr int DFT_NB = 64;  // largest band side on this path
-constexpr int DFT_KC = 32;  // image columns per staged chunk in F1
+constexpr int DFT_NB = 64;  // largest band side on this path (and 2048 cells in all)
 
-// F1 on the DFT path; also writes the dense image grid and the moments.
-// Threads: 16 column lanes x (T/16) row lanes; each thread accumulates 2 rows
-// x 4 band columns (b = lane, lane + 16, ...).  Row blocks of 2 T/16 rows go
-// to the group's CTAs in turn; per block the image and Ex are staged in
-// chunks of DFT_KC columns (rows padded by one element against bank
-// conflicts).
-template <typename R>
-__device__ __noinline__ void dft_t2_rows(FgCtx<R>& c, const GroupCtx& g, double (&mom)[10]) {
+// Sum of each of v[0..N) over the warp (N a power of two up to 32): lane l
+// returns the sum of value l / (32 / N), as warp_fold in the compute type.
+template <int N, typename R>
+__device__ __forceinline__ R warp_fold_r(R (&v)[N], int lane) {
+  int b = 16;
+#pragma unroll
+  for (int h = N / 2; h >= 1; h >>= 1, b >>= 1) {
+    const bool up = (lane & b) != 0;
+#pragma unroll
+    for (int i = 0; i < h; ++i) {
+      const R send = up ? v[i] : v[i + h], keep = up ? v[i + h] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, b);
+    }
+  }
+#pragma unroll
+  for (int q = 16 / N; q >= 1; q >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], q);
+  return v[0];
+}
+
+// F1 + F2.  Up to 32 image rows at a time in shared memory; a warp takes RB of
+// them and two band columns, its lanes the image columns (coalesced in Ex,
+// conflict free in the rows); then every thread adds the rows' parts of its
+// band cells.  Also writes the dense image grid and accumulates the moments.
+template <int RB, typename R>
+__device__ __noinline__ void dft_forward(FgCtx<R>& c, const GroupCtx& g, double (&mom)[10]) {
   const ProbDesc& P = *c.P;
   const double* x = at<double>(c.base, P.o_x);
   const int* inv = at<int>(c.base, P.o_inv);
@@ -113,186 +144,151 @@ __device__ __noinline__ void dft_t2_rows(FgCtx<R>& c, const GroupCtx& g, double 
   const double* dc1 = at<double>(c.base, P.o_dc1);
   const double* dc2 = at<double>(c.base, P.o_dc2);
   const cpx<R>* Ex = at<cpx<R>>(c.base, P.o_ex);
-  cpx<R>* tmpA = at<cpx<R>>(c.base, P.o_tmpA);
+  const cpx<R>* Ey = at<cpx<R>>(c.base, P.o_ey);
+  cpx<R>* bandA = at<cpx<R>>(c.base, P.o_bandA);
   cpx<R>* bandC = at<cpx<R>>(c.base, P.o_bandC);
-  const int nx = P.nx, ny = P.ny, nb = P.b1n;
-  const int T = blockDim.x, tc = threadIdx.x & 15, tr = threadIdx.x >> 4;
-  const int RB = 2 * (T >> 4);  // rows per block
-  const int KP = DFT_KC + 1;
-  R* Us = reinterpret_cast<R*>(c.sbuf);                                             // [RB][KP]
-  cpx<R>* Es = reinterpret_cast<cpx<R>*>(c.sbuf) + ((size_t)RB * KP * sizeof(R) + sizeof(cpx<R>) - 1) / sizeof(cpx<R>);  // [64][KP]
-  for (int i = g.rank * T + threadIdx.x; i < P.b2n * P.b1n; i += g.G * T) bandC[i] = cmk<R>(0, 0);
-  const bool need_mom = P.has_tfd || P.has_cen || P.has_sm;
-  for (int y0 = g.rank * RB; y0 < ny; y0 += g.G * RB) {
-    cpx<R> acc[2][4];
-#pragma unroll
-    for (int a = 0; a < 2; ++a)
-#pragma unroll
-      for (int q = 0; q < 4; ++q) acc[a][q] = cmk<R>(0, 0);
-    for (int k0 = 0; k0 < nx; k0 += DFT_KC) {
-      for (int i = threadIdx.x; i < RB * DFT_KC; i += T) {
-        const int rr = i / DFT_KC, kk = i - rr * DFT_KC, iy = y0 + rr, ix = k0 + kk;
-        R u = 0;
-        if (iy < ny && ix < nx) {
-          const int pv = P.ident ? iy * nx + ix : inv[iy * nx + ix];
-          const double val = pv >= 0 ? x[pv] : 0.0;
-          if (!P.ident) xg[(size_t)iy * nx + ix] = val;
-          u = (R)(val * dc1[ix] * dc2[iy]);
-          if (need_mom && pv >= 0) {
-            const double fx = ix + 1, fy = iy + 1;  // 1-based pixel numbers as the reference
-            mom[0] += val;
-            mom[1] += fabs(val);
-            mom[2] += val * fx;
-            mom[3] += val * fy;
-            mom[4] += val * fx * fx;
-            mom[5] += val * fy * fy;
-            mom[6] += val * fx * fy;
-            if (P.has_cen) {
-              const double Ip = fabs(P.cen_alpha - 1) < 1e-10 ? smabs(val) : pow(smabs(val), P.cen_alpha);
-              mom[7] += Ip * (fx - P.nxref);
-              mom[8] += Ip * (fy - P.nyref);
-              mom[9] += Ip;
-            }
+  const int nx = P.nx, ny = P.ny, nb = P.b1n, ncell = P.b1n * P.b2n;
+  const int T = blockDim.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = T >> 5;
+  const int share = (ny + g.G - 1) / g.G, y1 = min(ny, (g.rank + 1) * share);
+  const int nxe = (nx + 1) & ~1;
+  int RS = (min(share, 32) + RB - 1) / RB * RB;  // staged rows (nx <= 1024: at least 8 fit)
+  while (RS > RB && (size_t)RS * (nxe * sizeof(R) + nb * sizeof(cpx<R>)) > (size_t)c.dyn_cpx * sizeof(cpx<R>)) RS -= RB;
+  R* Us = reinterpret_cast<R*>(c.sbuf);                    // [RS][nx]
+  cpx<R>* ts = reinterpret_cast<cpx<R>*>(Us + RS * nxe);   // [RS][nb]
+  for (int i = g.rank * T + threadIdx.x; i < ncell; i += g.G * T) bandC[i] = cmk<R>(0, 0);
+  const bool need_mom = P.has_tfd || P.has_cen || P.has_sm, ident = P.ident;
+  const int npair = (nb + 1) >> 1;
+  for (int y0 = g.rank * share; y0 < y1; y0 += RS) {
+    const int rows = min(RS, y1 - y0), nsub = (rows + RB - 1) / RB;
+    for (int i = threadIdx.x; i < nsub * RB * nx; i += T) {
+      const int rr = i / nx, ix = i - rr * nx, iy = y0 + rr;
+      R u = 0;
+      if (iy < y1) {
+        const int pv = ident ? iy * nx + ix : inv[iy * nx + ix];
+        const double val = pv >= 0 ? x[pv] : 0.0;
+        if (!ident) xg[(size_t)iy * nx + ix] = val;
+        u = (R)(val * dc1[ix] * dc2[iy]);
+        if (need_mom && pv >= 0) {
+          const double fx = ix + 1, fy = iy + 1;  // 1-based pixel numbers as the reference
+          mom[0] += val;
+          mom[1] += fabs(val);
+          mom[2] += val * fx;
+          mom[3] += val * fy;
+          mom[4] += val * fx * fx;
+          mom[5] += val * fy * fy;
+          mom[6] += val * fx * fy;
+          if (P.has_cen) {
+            const double Ip = fabs(P.cen_alpha - 1) < 1e-10 ? smabs(val) : pow(smabs(val), P.cen_alpha);
+            mom[7] += Ip * (fx - P.nxref);
+            mom[8] += Ip * (fy - P.nyref);
+            mom[9] += Ip;
           }
         }
-        Us[rr * KP + kk] = u;
       }
-      for (int i = threadIdx.x; i < DFT_NB * DFT_KC; i += T) {
-        const int b = i / DFT_KC, kk = i - b * DFT_KC, ix = k0 + kk;
-        Es[b * KP + kk] = (b < nb && ix < nx) ? Ex[(size_t)b * nx + ix] : cmk<R>(0, 0);
-      }
-      __syncthreads();
-      const R* u0 = Us + (2 * tr) * KP;
-#pragma unroll 4
-      for (int kk = 0; kk < DFT_KC; ++kk) {
-        const R ua = u0[kk], ub = u0[KP + kk];
+      Us[i] = u;
+    }
+    __syncthreads();
+    for (int task = warp; task < nsub * npair; task += nw) {
+      const int sb = task / npair, b0 = 2 * (task - sb * npair);
+      const R* us = Us + sb * RB * nx;
+      const cpx<R>* e0 = Ex + (size_t)b0 * nx;
+      const cpx<R>* e1 = Ex + (size_t)min(b0 + 1, nb - 1) * nx;
+      R v[4 * RB];  // [row][column][re, im]
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const cpx<R> e = Es[(tc + 16 * q) * KP + kk];
-          acc[0][q].x += ua * e.x;
-          acc[0][q].y += ua * e.y;
-          acc[1][q].x += ub * e.x;
-          acc[1][q].y += ub * e.y;
+      for (int q = 0; q < 4 * RB; ++q) v[q] = 0;
+#pragma unroll 2
+      for (int ix = lane; ix < nx; ix += 32) {
+        const cpx<R> ea = e0[ix], eb = e1[ix];
+#pragma unroll
+        for (int r = 0; r < RB; ++r) {
+          const R u = us[r * nx + ix];
+          v[4 * r] += u * ea.x;
+          v[4 * r + 1] += u * ea.y;
+          v[4 * r + 2] += u * eb.x;
+          v[4 * r + 3] += u * eb.y;
         }
       }
-      __syncthreads();
+      const R sum = warp_fold_r<4 * RB>(v, lane);
+      const int q = lane / (32 / (4 * RB)), r = sb * RB + (q >> 2), b = b0 + ((q >> 1) & 1);
+      if (lane % (32 / (4 * RB)) == 0 && b < nb) (q & 1 ? ts[r * nb + b].y : ts[r * nb + b].x) = sum;
     }
-#pragma unroll
-    for (int a = 0; a < 2; ++a) {
-      const int iy = y0 + 2 * tr + a;
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int b = tc + 16 * q;
-        if (iy < ny && b < nb) tmpA[(size_t)iy * nb + b] = acc[a][q];
+    __syncthreads();
+    for (int o = threadIdx.x; o < ncell; o += T) {
+      const int r = o / nb, b = o - r * nb;
+      const cpx<R>* ey = Ey + (size_t)r * ny + y0;
+      cpx<R> acc = cmk<R>(0, 0);
+#pragma unroll 4
+      for (int i = 0; i < rows; ++i) {
+        const cpx<R> e = ey[i], t = ts[i * nb + b];
+        acc.x += e.x * t.x - e.y * t.y;
+        acc.y += e.x * t.y + e.y * t.x;
       }
+      acc_add(bandA + o, acc);
     }
+    __syncthreads();
   }
 }
 
-// F2 on the DFT path: one band cell per thread and pass; tmpA and Ey staged
-// in chunks of DFT_KC rows.
-template <typename R>
-__device__ __noinline__ void dft_t2_cols(FgCtx<R>& c, const GroupCtx& g) {
-  const ProbDesc& P = *c.P;
-  const cpx<R>* Ey = at<cpx<R>>(c.base, P.o_ey);
-  const cpx<R>* tmpA = at<cpx<R>>(c.base, P.o_tmpA);
-  cpx<R>* bandA = at<cpx<R>>(c.base, P.o_bandA);
-  const int ny = P.ny, nb = P.b1n, nr = P.b2n, ncell = nb * nr;
-  const int T = blockDim.x, KP = DFT_KC + 1;
-  cpx<R>* As = c.sbuf;                   // [DFT_KC][nb]
-  cpx<R>* Ys = c.sbuf + DFT_KC * DFT_NB;  // [nr][KP]
-  for (int o0 = g.rank * T; o0 < ncell; o0 += g.G * T) {
-    const int o = o0 + threadIdx.x, r = o / nb, b = o - r * nb;
-    cpx<R> acc = cmk<R>(0, 0);
-    for (int k0 = 0; k0 < ny; k0 += DFT_KC) {
-      for (int i = threadIdx.x; i < DFT_KC * nb; i += T) {
-        const int kk = i / nb, bb = i - kk * nb;
-        As[i] = k0 + kk < ny ? tmpA[(size_t)(k0 + kk) * nb + bb] : cmk<R>(0, 0);
-      }
-      for (int i = threadIdx.x; i < nr * DFT_KC; i += T) {
-        const int rr = i / DFT_KC, kk = i - rr * DFT_KC;
-        Ys[rr * KP + kk] = k0 + kk < ny ? Ey[(size_t)rr * ny + k0 + kk] : cmk<R>(0, 0);
-      }
-      __syncthreads();
-      if (o < ncell) {
-#pragma unroll 4
-        for (int kk = 0; kk < DFT_KC; ++kk) {
-          const cpx<R> e = Ys[r * KP + kk], t = As[kk * nb + b];
-          acc.x += e.x * t.x - e.y * t.y;
-          acc.y += e.x * t.y + e.y * t.x;
-        }
-      }
-      __syncthreads();
-    }
-    if (o < ncell) bandA[o] = acc;
-  }
-}
-
-// F6 on the DFT path: bandC staged whole; a thread takes one image column
-// and up to 8 band rows, streaming its column of Ex.
-template <typename R>
-__device__ __noinline__ void dft_t1_rows(FgCtx<R>& c, const GroupCtx& g) {
+// F6 + F7.  CB image columns at a time: their tmpC in shared memory beside
+// bandC, then a thread takes one image row and JC of the columns (wide shares
+// take 16, so that a twiddle from L2 serves 32 multiply-adds).
+template <int CB, int JC, typename R>
+__device__ __noinline__ void dft_adjoint(FgCtx<R>& c, const GroupCtx& g) {
   const ProbDesc& P = *c.P;
   const cpx<R>* Ex = at<cpx<R>>(c.base, P.o_ex);
-  const cpx<R>* bandC = at<cpx<R>>(c.base, P.o_bandC);
-  cpx<R>* tmpC = at<cpx<R>>(c.base, P.o_tmpC);
-  const int nx = P.nx, nb = P.b1n, nr = P.b2n;
-  const int T = blockDim.x;
-  cpx<R>* Bs = c.sbuf;  // [nr][nb]
-  for (int i = threadIdx.x; i < nr * nb; i += T) Bs[i] = bandC[i];
-  __syncthreads();
-  const int ngrp = (nr + 7) >> 3, items = nx * ngrp;
-  for (int it = g.rank * T + threadIdx.x; it < items; it += g.G * T) {
-    const int rg = it / nx, ix = it - rg * nx, r0 = 8 * rg;
-    cpx<R> acc[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) acc[j] = cmk<R>(0, 0);
-    for (int b = 0; b < nb; ++b) {
-      const cpx<R> e = Ex[(size_t)b * nx + ix];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        if (r0 + j < nr) {
-          const cpx<R> v = Bs[(r0 + j) * nb + b];
-          acc[j].x += v.x * e.x - v.y * e.y;
-          acc[j].y += v.x * e.y + v.y * e.x;
-        }
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-      if (r0 + j < nr) tmpC[(size_t)(r0 + j) * nx + ix] = acc[j];
-  }
-  __syncthreads();
-}
-
-// F7 on the DFT path: a thread takes one image column and 4 image rows.
-template <typename R>
-__device__ __noinline__ void dft_t1_cols(FgCtx<R>& c, const GroupCtx& g) {
-  const ProbDesc& P = *c.P;
   const cpx<R>* Ey = at<cpx<R>>(c.base, P.o_ey);
-  const cpx<R>* tmpC = at<cpx<R>>(c.base, P.o_tmpC);
+  const cpx<R>* bandC = at<cpx<R>>(c.base, P.o_bandC);
   const double* dc1 = at<double>(c.base, P.o_dc1);
   const double* dc2 = at<double>(c.base, P.o_dc2);
   double* gchi = at<double>(c.base, P.o_gchi);
-  const int nx = P.nx, ny = P.ny, nr = P.b2n;
-  const int T = blockDim.x, ngrp = (ny + 3) >> 2, items = nx * ngrp;
-  for (int it = g.rank * T + threadIdx.x; it < items; it += g.G * T) {
-    const int yg = it / nx, ix = it - yg * nx, y0 = 4 * yg;
-    R acc[4] = {0, 0, 0, 0};
-    for (int r = 0; r < nr; ++r) {
-      const cpx<R> t = tmpC[(size_t)r * nx + ix];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        if (y0 + j < ny) {
-          const cpx<R> e = Ey[(size_t)r * ny + y0 + j];
-          acc[j] += e.x * t.x - e.y * t.y;
+  const int nx = P.nx, ny = P.ny, nb = P.b1n, nr = P.b2n;
+  const int T = blockDim.x;
+  cpx<R>* Cs = c.sbuf;                    // [nr][CB]
+  cpx<R>* Bs = c.sbuf + DFT_NB * CB;      // [nr][nb]
+  const int share = (nx + g.G - 1) / g.G, x1 = min(nx, (g.rank + 1) * share);
+  if (g.rank * share >= x1) return;
+  for (int i = threadIdx.x; i < nr * nb; i += T) Bs[i] = bandC[i];
+  for (int x0 = g.rank * share; x0 < x1; x0 += CB) {
+    const int cols = min(CB, x1 - x0), cj = (cols + JC - 1) / JC;
+    __syncthreads();
+    for (int i = threadIdx.x; i < nr * JC * cj; i += T) {
+      const int r = i / (JC * cj), cc = i - r * JC * cj;
+      cpx<R> t = cmk<R>(0, 0);
+      if (cc < cols) {
+        const cpx<R>* ex = Ex + x0 + cc;
+        const cpx<R>* v = Bs + r * nb;
+#pragma unroll 8
+        for (int b = 0; b < nb; ++b) {
+          const cpx<R> e = ex[(size_t)b * nx], w = v[b];
+          t.x += w.x * e.x - w.y * e.y;
+          t.y += w.x * e.y + w.y * e.x;
         }
       }
+      Cs[r * CB + cc] = t;
     }
+    __syncthreads();
+    for (int it = threadIdx.x; it < ny * cj; it += T) {
+      const int cq = it / ny, iy = it - cq * ny;
+      const cpx<R>* ey = Ey + iy;
+      const cpx<R>* t = Cs + JC * cq;
+      R acc[JC];
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-      if (y0 + j < ny) gchi[(size_t)(y0 + j) * nx + ix] = (double)acc[j] * dc1[ix] * dc2[y0 + j];
+      for (int j = 0; j < JC; ++j) acc[j] = 0;
+#pragma unroll 4
+      for (int r = 0; r < nr; ++r) {
+        const cpx<R> e = ey[(size_t)r * ny];
+#pragma unroll
+        for (int j = 0; j < JC; ++j) acc[j] += e.x * t[r * CB + j].x - e.y * t[r * CB + j].y;
+      }
+      const double d2 = dc2[iy];
+#pragma unroll
+      for (int j = 0; j < JC; ++j) {
+        const int ix = x0 + JC * cq + j;
+        if (ix < x1) gchi[(size_t)iy * nx + ix] = (double)acc[j] * dc1[ix] * d2;
+      }
+    }
   }
+  __syncthreads();
 }
 
 // ---------------------------------------------------------------------------
@@ -303,7 +299,8 @@ __device__ __noinline__ void dft_t1_cols(FgCtx<R>& c, const GroupCtx& g) {
 template <typename R>
 __device__ __noinline__ void fg_t2_rows(FgCtx<R>& c, const GroupCtx& g, double (&mom)[10]) {
   if (c.P->dft) {
-    dft_t2_rows(c, g, mom);
+    if ((c.P->ny + g.G - 1) / g.G <= 4) dft_forward<4>(c, g, mom);
+    else dft_forward<8>(c, g, mom);
     return;
   }
   const ProbDesc& P = *c.P;
@@ -363,10 +360,6 @@ __device__ __noinline__ void fg_t2_rows(FgCtx<R>& c, const GroupCtx& g, double (
 // ---------------------------------------------------------------------------
 template <typename R>
 __device__ __noinline__ void fg_t2_cols(FgCtx<R>& c, const GroupCtx& g) {
-  if (c.P->dft) {
-    dft_t2_cols(c, g);
-    return;
-  }
   const ProbDesc& P = *c.P;
   const cpx<R>* tw2 = at<cpx<R>>(c.base, P.o_tw2);
   const cpx<R>* tmpA = at<cpx<R>>(c.base, P.o_tmpA);
@@ -515,14 +508,6 @@ __device__ void fg_interp(FgCtx<R>& c, const GroupCtx& g, bool zero_acc) {
 // its own point order.
 // chi[0..3] = fcv, amp, cp, ca (weighted by the normalised data weights).
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void acc_add(cpx<float>* p, cpx<float> v) {
-  atomicAdd(reinterpret_cast<float2*>(p), make_float2(v.x, v.y));
-}
-__device__ __forceinline__ void acc_add(cpx<double>* p, cpx<double> v) {
-  atomicAdd(&p->x, v.x);
-  atomicAdd(&p->y, v.y);
-}
-
 template <typename R>
 __device__ __noinline__ void fg_chisq(FgCtx<R>& c, const GroupCtx& g, double (&chi)[4]) {
   const ProbDesc& P = *c.P;
@@ -1004,6 +989,11 @@ __device__ __noinline__ void fg_spread_tc(FgCtx<float>& c, const GroupCtx& g) {
 
 template <typename R>
 __device__ __noinline__ void fg_spread(FgCtx<R>& c, const GroupCtx& g) {
+  if (c.P->dft) {  // interpolation has read the band: clear it for the next F1
+    cpx<R>* bandA = at<cpx<R>>(c.base, c.P->o_bandA);
+    for (int i = g.rank * blockDim.x + threadIdx.x; i < c.P->b1n * c.P->b2n; i += g.G * blockDim.x)
+      bandA[i] = cmk<R>(0, 0);
+  }
   if (c.P->bin == 8) {
     switch (c.P->w) {
 #define SMILI_SPREAD_W(W)                                                      \
@@ -1129,10 +1119,6 @@ __device__ __noinline__ void fg_spread(FgCtx<R>& c, const GroupCtx& g) {
 // ---------------------------------------------------------------------------
 template <typename R>
 __device__ __noinline__ void fg_t1_rows(FgCtx<R>& c, const GroupCtx& g) {
-  if (c.P->dft) {
-    dft_t1_rows(c, g);
-    return;
-  }
   const ProbDesc& P = *c.P;
   const cpx<R>* tw1 = at<cpx<R>>(c.base, P.o_tw1);
   const cpx<R>* bandC = at<cpx<R>>(c.base, P.o_bandC);
@@ -1164,7 +1150,8 @@ __device__ __noinline__ void fg_t1_rows(FgCtx<R>& c, const GroupCtx& g) {
 template <typename R>
 __device__ __noinline__ void fg_t1_cols(FgCtx<R>& c, const GroupCtx& g) {
   if (c.P->dft) {
-    dft_t1_cols(c, g);
+    if ((c.P->nx + g.G - 1) / g.G <= 16) dft_adjoint<16, 4>(c, g);
+    else dft_adjoint<64, 16>(c, g);
     return;
   }
   const ProbDesc& P = *c.P;

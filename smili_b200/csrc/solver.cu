@@ -88,8 +88,10 @@ __device__ bool fg_stages(FgCtx<R>& fc, GroupCtx& g, int lo, int hi, double* red
       return false;
     }
     pf.mark(PR_F1);
-    fg_t2_cols(fc, g);
-    if (!group_sync(g)) return false;
+    if (!P.dft) {  // else part of F1
+      fg_t2_cols(fc, g);
+      if (!group_sync(g)) return false;
+    }
     pf.mark(PR_F2);
     fg_interp(fc, g, mode != MODE_T1);
     if (!group_sync(g)) return false;
@@ -103,8 +105,10 @@ __device__ bool fg_stages(FgCtx<R>& fc, GroupCtx& g, int lo, int hi, double* red
     fg_spread(fc, g);
     if (!group_sync(g)) return false;
     pf.mark(PR_F5);
-    fg_t1_rows(fc, g);
-    if (!group_sync(g)) return false;
+    if (!P.dft) {  // else part of F7
+      fg_t1_rows(fc, g);
+      if (!group_sync(g)) return false;
+    }
     pf.mark(PR_F6);
     fg_t1_cols(fc, g);
     if (!group_sync(g)) return false;
@@ -399,6 +403,17 @@ __global__ void __launch_bounds__(Shape<R>::threads, Shape<R>::min_blocks) smili
         S.nfg_total = 0;
       }
       __syncthreads();
+    }
+    // an empty band for the first evaluation (dense band passes add into it)
+    auto clear_band = [&](const ProbDesc& D) {
+      if (!D.dft) return;
+      cpx<R>* bandA = at<cpx<R>>(base, D.o_bandA);
+      for (int i = rank * blockDim.x + threadIdx.x; i < D.b1n * D.b2n; i += a.G * blockDim.x) bandA[i] = cmk<R>(0, 0);
+    };
+    clear_band(P);
+    if (P.nframes > 0) {
+      const ProbDesc* frames = at<ProbDesc>(base, P.o_frames);
+      for (int z = 0; z < P.nframes; ++z) clear_band(frames[z]);
     }
     // the kernel weights of the launch's evaluations
     if (P.o_taps) {
