@@ -102,15 +102,49 @@ struct KSumF {
 //   F7  gchi[iy][ix] = Re sum_r Ey[r][iy] tmpC[r][ix]  * dc1[ix] dc2[iy]
 // (the same twiddles the radix passes apply, exp periodic in nf).  Used
 // for bands of at most 64 x 64 cells, 2048 in all, where each pass is a few
-// million multiply-adds.  F1 and F2 are one stage: a CTA takes its share of the
-// image rows through both and adds its part of the band to bandA (zeroed by the
-// spreading stage before); so are F6 and F7, a CTA taking its share of the
-// image columns.  As four stages of register tiles, each stage had work for 4 to
-// 16 CTAs only: 256 x 256, 44 x 21 cells, FP64 on 64 CTAs, 70 + 40 + 24 + 14 us
-// per evaluation, 23 + 21 as two; FP32 on groups of 4 CTAs (74 problems), 100 +
-// 40 + 44 + 141 and 131 + 96.
+// million multiply-adds.  F1 splits the image rows over the CTAs, F2 the band
+// cells; F6 and F7 are one stage, a CTA taking its share of the image columns
+// through both.  In FP64 the lanes of a warp share the sums of F1 and F2; in
+// FP32 every sum runs along its row or column in one thread, in the order of
+// the radix-free definition: a solve amplifies the last bit of an FP32
+// visibility by up to 1e4, and sums in another order move its image by more
+// than the spreading's atomics do.  (F1 and F2 as one stage that adds each
+// CTA's part of the band with atomics is no faster, and an FP64 solve with
+// near-null baselines then changes from run to run by 4e-9 instead of 1e-11.)
+// As register tiles of 64 rows, 512 cells, 8 band rows and 4 image rows the
+// stages had work for 4 to 16 CTAs only: 256 x 256, 44 x 21 cells, FP64 on 64
+// CTAs, 70 + 40 + 24 + 14 us per evaluation, 18 + 7 + 21 on 96 now; FP32 on
+// groups of 2 CTAs (148 problems) 100 + 40 + 44 + 141, now 112 + 42 + 96.
 // ---------------------------------------------------------------------------
 constexpr int DFT_NB = 64;  // largest band side on this path (and 2048 cells in all)
+constexpr int DFT_KC = 32;  // image columns per staged chunk of the FP32 F1
+
+// One pixel of the dense image grid: its value into xg, its moments, and the
+// deconvolved value that the transform takes.
+template <typename R>
+__device__ __forceinline__ R dense_pixel(const ProbDesc& P, const double* x, const int* inv, double* xg, double d1,
+                                         double d2, int iy, int ix, bool need_mom, double (&mom)[10]) {
+  const int cell = iy * P.nx + ix, pv = P.ident ? cell : inv[cell];
+  const double val = pv >= 0 ? x[pv] : 0.0;
+  if (!P.ident) xg[cell] = val;
+  if (need_mom && pv >= 0) {
+    const double fx = ix + 1, fy = iy + 1;  // 1-based pixel numbers as the reference
+    mom[0] += val;
+    mom[1] += fabs(val);
+    mom[2] += val * fx;
+    mom[3] += val * fy;
+    mom[4] += val * fx * fx;
+    mom[5] += val * fy * fy;
+    mom[6] += val * fx * fy;
+    if (P.has_cen) {
+      const double Ip = fabs(P.cen_alpha - 1) < 1e-10 ? smabs(val) : pow(smabs(val), P.cen_alpha);
+      mom[7] += Ip * (fx - P.nxref);
+      mom[8] += Ip * (fy - P.nyref);
+      mom[9] += Ip;
+    }
+  }
+  return (R)(val * d1 * d2);
+}
 
 // Sum of each of v[0..N) over the warp (N a power of two up to 32): lane l
 // returns the sum of value l / (32 / N), as warp_fold in the compute type.
@@ -131,12 +165,13 @@ __device__ __forceinline__ R warp_fold_r(R (&v)[N], int lane) {
   return v[0];
 }
 
-// F1 + F2.  Up to 32 image rows at a time in shared memory; a warp takes RB of
+// F1 in FP64.  Up to 32 image rows at a time in shared memory; a warp takes RB of
 // them and two band columns, its lanes the image columns (coalesced in Ex,
-// conflict free in the rows); then every thread adds the rows' parts of its
-// band cells.  Also writes the dense image grid and accumulates the moments.
-template <int RB, typename R>
-__device__ __noinline__ void dft_forward(FgCtx<R>& c, const GroupCtx& g, double (&mom)[10]) {
+// conflict free in the rows).  Also writes the dense image grid and
+// accumulates the moments.
+template <int RB>
+__device__ __noinline__ void dft_rows(FgCtx<double>& c, const GroupCtx& g, double (&mom)[10]) {
+  using R = double;
   const ProbDesc& P = *c.P;
   const double* x = at<double>(c.base, P.o_x);
   const int* inv = at<int>(c.base, P.o_inv);
@@ -144,47 +179,23 @@ __device__ __noinline__ void dft_forward(FgCtx<R>& c, const GroupCtx& g, double 
   const double* dc1 = at<double>(c.base, P.o_dc1);
   const double* dc2 = at<double>(c.base, P.o_dc2);
   const cpx<R>* Ex = at<cpx<R>>(c.base, P.o_ex);
-  const cpx<R>* Ey = at<cpx<R>>(c.base, P.o_ey);
-  cpx<R>* bandA = at<cpx<R>>(c.base, P.o_bandA);
+  cpx<R>* tmpA = at<cpx<R>>(c.base, P.o_tmpA);  // [nb][ny]
   cpx<R>* bandC = at<cpx<R>>(c.base, P.o_bandC);
   const int nx = P.nx, ny = P.ny, nb = P.b1n, ncell = P.b1n * P.b2n;
   const int T = blockDim.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = T >> 5;
   const int share = (ny + g.G - 1) / g.G, y1 = min(ny, (g.rank + 1) * share);
-  const int nxe = (nx + 1) & ~1;
   int RS = (min(share, 32) + RB - 1) / RB * RB;  // staged rows (nx <= 1024: at least 8 fit)
-  while (RS > RB && (size_t)RS * (nxe * sizeof(R) + nb * sizeof(cpx<R>)) > (size_t)c.dyn_cpx * sizeof(cpx<R>)) RS -= RB;
-  R* Us = reinterpret_cast<R*>(c.sbuf);                    // [RS][nx]
-  cpx<R>* ts = reinterpret_cast<cpx<R>*>(Us + RS * nxe);   // [RS][nb]
+  while (RS > RB && (size_t)RS * nx > (size_t)c.dyn_cpx * 2) RS -= RB;
+  R* Us = reinterpret_cast<R*>(c.sbuf);  // [RS][nx]
   for (int i = g.rank * T + threadIdx.x; i < ncell; i += g.G * T) bandC[i] = cmk<R>(0, 0);
-  const bool need_mom = P.has_tfd || P.has_cen || P.has_sm, ident = P.ident;
+  const bool need_mom = P.has_tfd || P.has_cen || P.has_sm;
   const int npair = (nb + 1) >> 1;
   for (int y0 = g.rank * share; y0 < y1; y0 += RS) {
     const int rows = min(RS, y1 - y0), nsub = (rows + RB - 1) / RB;
     for (int i = threadIdx.x; i < nsub * RB * nx; i += T) {
       const int rr = i / nx, ix = i - rr * nx, iy = y0 + rr;
       R u = 0;
-      if (iy < y1) {
-        const int pv = ident ? iy * nx + ix : inv[iy * nx + ix];
-        const double val = pv >= 0 ? x[pv] : 0.0;
-        if (!ident) xg[(size_t)iy * nx + ix] = val;
-        u = (R)(val * dc1[ix] * dc2[iy]);
-        if (need_mom && pv >= 0) {
-          const double fx = ix + 1, fy = iy + 1;  // 1-based pixel numbers as the reference
-          mom[0] += val;
-          mom[1] += fabs(val);
-          mom[2] += val * fx;
-          mom[3] += val * fy;
-          mom[4] += val * fx * fx;
-          mom[5] += val * fy * fy;
-          mom[6] += val * fx * fy;
-          if (P.has_cen) {
-            const double Ip = fabs(P.cen_alpha - 1) < 1e-10 ? smabs(val) : pow(smabs(val), P.cen_alpha);
-            mom[7] += Ip * (fx - P.nxref);
-            mom[8] += Ip * (fy - P.nyref);
-            mom[9] += Ip;
-          }
-        }
-      }
+      if (iy < y1) u = dense_pixel<R>(P, x, inv, xg, dc1[ix], dc2[iy], iy, ix, need_mom, mom);
       Us[i] = u;
     }
     __syncthreads();
@@ -209,23 +220,157 @@ __device__ __noinline__ void dft_forward(FgCtx<R>& c, const GroupCtx& g, double 
         }
       }
       const R sum = warp_fold_r<4 * RB>(v, lane);
-      const int q = lane / (32 / (4 * RB)), r = sb * RB + (q >> 2), b = b0 + ((q >> 1) & 1);
-      if (lane % (32 / (4 * RB)) == 0 && b < nb) (q & 1 ? ts[r * nb + b].y : ts[r * nb + b].x) = sum;
+      const int q = lane / (32 / (4 * RB)), iy = y0 + sb * RB + (q >> 2), b = b0 + ((q >> 1) & 1);
+      if (lane % (32 / (4 * RB)) == 0 && b < nb && iy < y1)
+        (q & 1 ? tmpA[(size_t)b * ny + iy].y : tmpA[(size_t)b * ny + iy].x) = sum;
     }
     __syncthreads();
-    for (int o = threadIdx.x; o < ncell; o += T) {
-      const int r = o / nb, b = o - r * nb;
-      const cpx<R>* ey = Ey + (size_t)r * ny + y0;
-      cpx<R> acc = cmk<R>(0, 0);
-#pragma unroll 4
-      for (int i = 0; i < rows; ++i) {
-        const cpx<R> e = ey[i], t = ts[i * nb + b];
-        acc.x += e.x * t.x - e.y * t.y;
-        acc.y += e.x * t.y + e.y * t.x;
+  }
+}
+
+// F2 in FP64.  A warp takes NR band rows of one or two band columns, its lanes iy
+// (coalesced in Ey and tmpA).  Tiles of 4 x 2 cells where every warp has
+// several (5 loads of L2 serve 8 products), single cells where the group has
+// warps to spare and the latency of one product counts.
+template <int NR, int NC>
+__device__ __noinline__ void dft_cols(FgCtx<double>& c, const GroupCtx& g) {
+  using R = double;
+  const ProbDesc& P = *c.P;
+  const cpx<R>* Ey = at<cpx<R>>(c.base, P.o_ey);
+  const cpx<R>* tmpA = at<cpx<R>>(c.base, P.o_tmpA);  // [nb][ny]
+  cpx<R>* bandA = at<cpx<R>>(c.base, P.o_bandA);
+  const int ny = P.ny, nb = P.b1n, nr = P.b2n;
+  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5, tc = (nb + NC - 1) / NC, tr = (nr + NR - 1) / NR;
+  for (int task = g.rank * nw + (threadIdx.x >> 5); task < tc * tr; task += g.G * nw) {
+    const int r0 = task / tc * NR, b0 = task % tc * NC;
+    R v[2 * NR * NC];
+#pragma unroll
+    for (int q = 0; q < 2 * NR * NC; ++q) v[q] = 0;
+#pragma unroll 2
+    for (int iy = lane; iy < ny; iy += 32) {
+      cpx<R> t[NC];
+#pragma unroll
+      for (int k = 0; k < NC; ++k) t[k] = tmpA[(size_t)min(b0 + k, nb - 1) * ny + iy];
+#pragma unroll
+      for (int r = 0; r < NR; ++r) {
+        const cpx<R> e = Ey[(size_t)min(r0 + r, nr - 1) * ny + iy];
+#pragma unroll
+        for (int k = 0; k < NC; ++k) {
+          v[2 * (r * NC + k)] += e.x * t[k].x - e.y * t[k].y;
+          v[2 * (r * NC + k) + 1] += e.x * t[k].y + e.y * t[k].x;
+        }
       }
-      acc_add(bandA + o, acc);
     }
-    __syncthreads();
+    const R sum = warp_fold_r<2 * NR * NC>(v, lane);
+    constexpr int L = 32 / (2 * NR * NC);
+    const int q = lane / L, r = r0 + (q >> 1) / NC, b = b0 + (q >> 1) % NC;
+    if (lane % L == 0 && r < nr && b < nb) (q & 1 ? bandA[r * nb + b].y : bandA[r * nb + b].x) = sum;
+  }
+}
+
+// F1 in FP32.  Up to 128 rows at a time, the image and Ex staged in chunks of
+// DFT_KC columns; a thread takes TR rows and TC band columns (4 x 4: three
+// 16-byte shared loads per 32 multiply-adds; single sums for narrow shares).
+template <int TR, int TC>
+__device__ __noinline__ void dft_rows_seq(FgCtx<float>& c, const GroupCtx& g, double (&mom)[10]) {
+  const ProbDesc& P = *c.P;
+  const double* x = at<double>(c.base, P.o_x);
+  const int* inv = at<int>(c.base, P.o_inv);
+  double* xg = at<double>(c.base, P.o_xg);
+  const double* dc1 = at<double>(c.base, P.o_dc1);
+  const double* dc2 = at<double>(c.base, P.o_dc2);
+  const float2* Ex = at<float2>(c.base, P.o_ex);
+  float2* tmpA = at<float2>(c.base, P.o_tmpA);  // [ny][nb]
+  float2* bandC = at<float2>(c.base, P.o_bandC);
+  const int nx = P.nx, ny = P.ny, nb = P.b1n, ncell = P.b1n * P.b2n, T = blockDim.x;
+  constexpr int RM = 128, US = RM + 4;
+  const int share = (ny + g.G - 1) / g.G, y1 = min(ny, (g.rank + 1) * share);
+  float* Us = reinterpret_cast<float*>(c.sbuf);              // [DFT_KC][US]
+  float2* Es = reinterpret_cast<float2*>(Us + DFT_KC * US);  // [DFT_KC][DFT_NB + 2]
+  constexpr int ES = DFT_NB + 2;
+  for (int i = g.rank * T + threadIdx.x; i < ncell; i += g.G * T) bandC[i] = make_float2(0.f, 0.f);
+  const bool need_mom = P.has_tfd || P.has_cen || P.has_sm;
+  const int tcn = (nb + TC - 1) / TC;
+  for (int y0 = g.rank * share; y0 < y1; y0 += RM) {
+    const int rows = min(RM, y1 - y0), rpad = (rows + TR - 1) / TR * TR, ntask = rpad / TR * tcn;
+    for (int t0 = 0; t0 < ntask; t0 += T) {  // one pass of the threads over the tiles
+      const int task = t0 + (int)threadIdx.x, r0 = task / tcn * TR, b0 = task % tcn * TC;
+      float2 acc[TR][TC];
+#pragma unroll
+      for (int a = 0; a < TR; ++a)
+#pragma unroll
+        for (int q = 0; q < TC; ++q) acc[a][q] = make_float2(0.f, 0.f);
+      for (int k0 = 0; k0 < nx; k0 += DFT_KC) {
+        for (int i = threadIdx.x; i < rpad * DFT_KC; i += T) {
+          const int rr = i / DFT_KC, kk = i % DFT_KC, iy = y0 + rr, ix = k0 + kk;
+          float u = 0.f;
+          if (iy < y1 && ix < nx)
+            u = dense_pixel<float>(P, x, inv, xg, dc1[ix], dc2[iy], iy, ix, need_mom && t0 == 0, mom);
+          Us[kk * US + rr] = u;
+        }
+        for (int i = threadIdx.x; i < tcn * TC * DFT_KC; i += T) {
+          const int b = i / DFT_KC, kk = i % DFT_KC, ix = k0 + kk;
+          Es[kk * ES + b] = (b < nb && ix < nx) ? Ex[(size_t)b * nx + ix] : make_float2(0.f, 0.f);
+        }
+        __syncthreads();
+        if (task < ntask) {
+#pragma unroll 4
+          for (int kk = 0; kk < DFT_KC; ++kk) {
+            float u[TR];
+            float2 e[TC];
+            if constexpr (TR == 4 && TC == 4) {
+              *reinterpret_cast<float4*>(u) = *reinterpret_cast<const float4*>(Us + kk * US + r0);
+              *reinterpret_cast<float4*>(e) = *reinterpret_cast<const float4*>(Es + kk * ES + b0);
+              *reinterpret_cast<float4*>(e + 2) = *reinterpret_cast<const float4*>(Es + kk * ES + b0 + 2);
+            } else {
+#pragma unroll
+              for (int a = 0; a < TR; ++a) u[a] = Us[kk * US + r0 + a];
+#pragma unroll
+              for (int q = 0; q < TC; ++q) e[q] = Es[kk * ES + b0 + q];
+            }
+#pragma unroll
+            for (int a = 0; a < TR; ++a)
+#pragma unroll
+              for (int q = 0; q < TC; ++q) {
+                acc[a][q].x += u[a] * e[q].x;
+                acc[a][q].y += u[a] * e[q].y;
+              }
+          }
+        }
+        __syncthreads();
+      }
+      if (task < ntask) {
+#pragma unroll
+        for (int a = 0; a < TR; ++a)
+#pragma unroll
+          for (int q = 0; q < TC; ++q)
+            if (y0 + r0 + a < y1 && b0 + q < nb) tmpA[(size_t)(y0 + r0 + a) * nb + b0 + q] = acc[a][q];
+      }
+    }
+  }
+}
+
+// F2 in FP32.  A thread takes a band cell; consecutive threads read
+// consecutive tmpA and the same Ey.
+__device__ __noinline__ void dft_cols_seq(FgCtx<float>& c, const GroupCtx& g) {
+  const ProbDesc& P = *c.P;
+  const float2* Ey = at<float2>(c.base, P.o_ey);
+  const float2* tmpA = at<float2>(c.base, P.o_tmpA);  // [ny][nb]
+  float2* bandA = at<float2>(c.base, P.o_bandA);
+  const int ny = P.ny, nb = P.b1n, ncell = nb * P.b2n, share = (ncell + g.G - 1) / g.G;
+  const int o1 = min(ncell, (g.rank + 1) * share);
+  for (int o = g.rank * share + threadIdx.x; o < o1; o += blockDim.x) {
+    const int r = o / nb;
+    const float2* ey = Ey + (size_t)r * ny;
+    const float2* t = tmpA + (o - r * nb);
+    float2 acc = make_float2(0.f, 0.f);
+#pragma unroll 8
+    for (int iy = 0; iy < ny; ++iy) {
+      const float2 e = ey[iy], v = t[(size_t)iy * nb];
+      acc.x += e.x * v.x - e.y * v.y;
+      acc.y += e.x * v.y + e.y * v.x;
+    }
+    bandA[o] = acc;
   }
 }
 
@@ -299,8 +444,14 @@ __device__ __noinline__ void dft_adjoint(FgCtx<R>& c, const GroupCtx& g) {
 template <typename R>
 __device__ __noinline__ void fg_t2_rows(FgCtx<R>& c, const GroupCtx& g, double (&mom)[10]) {
   if (c.P->dft) {
-    if ((c.P->ny + g.G - 1) / g.G <= 4) dft_forward<4>(c, g, mom);
-    else dft_forward<8>(c, g, mom);
+    const int share = (c.P->ny + g.G - 1) / g.G;
+    if constexpr (sizeof(R) == 8) {
+      if (share <= 4) dft_rows<4>(c, g, mom);
+      else dft_rows<8>(c, g, mom);
+    } else {
+      if (share <= 16) dft_rows_seq<1, 1>(c, g, mom);
+      else dft_rows_seq<4, 4>(c, g, mom);
+    }
     return;
   }
   const ProbDesc& P = *c.P;
@@ -360,6 +511,15 @@ __device__ __noinline__ void fg_t2_rows(FgCtx<R>& c, const GroupCtx& g, double (
 // ---------------------------------------------------------------------------
 template <typename R>
 __device__ __noinline__ void fg_t2_cols(FgCtx<R>& c, const GroupCtx& g) {
+  if (c.P->dft) {
+    if constexpr (sizeof(R) == 8) {
+      if (c.P->b1n * c.P->b2n > g.G * (int)(blockDim.x >> 5) * 8) dft_cols<4, 2>(c, g);
+      else dft_cols<1, 1>(c, g);
+    } else {
+      dft_cols_seq(c, g);
+    }
+    return;
+  }
   const ProbDesc& P = *c.P;
   const cpx<R>* tw2 = at<cpx<R>>(c.base, P.o_tw2);
   const cpx<R>* tmpA = at<cpx<R>>(c.base, P.o_tmpA);
@@ -989,11 +1149,6 @@ __device__ __noinline__ void fg_spread_tc(FgCtx<float>& c, const GroupCtx& g) {
 
 template <typename R>
 __device__ __noinline__ void fg_spread(FgCtx<R>& c, const GroupCtx& g) {
-  if (c.P->dft) {  // interpolation has read the band: clear it for the next F1
-    cpx<R>* bandA = at<cpx<R>>(c.base, c.P->o_bandA);
-    for (int i = g.rank * blockDim.x + threadIdx.x; i < c.P->b1n * c.P->b2n; i += g.G * blockDim.x)
-      bandA[i] = cmk<R>(0, 0);
-  }
   if (c.P->bin == 8) {
     switch (c.P->w) {
 #define SMILI_SPREAD_W(W)                                                      \
@@ -1266,12 +1421,13 @@ __device__ void reg_moments(const ProbDesc& P, const double (&m)[10], RegMoments
 }
 
 // image moments of a movie frame that has no data (the row pass of F1
-// accumulates the same sums for frames with data); one CTA, per-thread partials
-__device__ void frame_moments(const ProbDesc& P, char* base, double (&mom)[10]) {
+// accumulates the same sums for frames with data): per-thread partials over
+// this CTA's pixels lo..hi
+__device__ void frame_moments(const ProbDesc& P, char* base, int lo, int hi, double (&mom)[10]) {
   const double* x = at<double>(base, P.o_x);
   const int* xi = at<int>(base, P.o_xidx);
   const int* yi = at<int>(base, P.o_yidx);
-  for (int p = threadIdx.x; p < P.npix; p += blockDim.x) {
+  for (int p = lo + threadIdx.x; p < hi; p += blockDim.x) {
     const double val = x[p], fx = xi[p] + 1, fy = yi[p] + 1;
     mom[0] += val;
     mom[1] += fabs(val);

@@ -39,11 +39,14 @@ enum { MODE_SOLVE = 0, MODE_FG = 1, MODE_T2 = 2, MODE_T1 = 3, MODE_BARRIER = 4, 
 struct BatchArgs {
   char* arena;
   const ProbDesc* descs;
-  int nprob, G, mode;
+  int nprob, ngroups, mode;
+  const int4* ctas;    // [grid]: group, first CTA and CTA count of each CTA's group
   int* queue;
   unsigned* bars;      // [ngroups][8]: arrival counter of each group, one per 32-byte sector
-  double* red_part;    // [ngroups][2][G][redk]
+  double* red_part;    // [2][G][redk] of each group, one group after the other
   int redk;
+  unsigned* sub_bars;  // [grid][8] and [grid][2][SMILI_REDK_FG]: the same for the sub-groups
+  double* sub_red;     // of a movie's frames, at each sub-group's first CTA (null: no movie)
   int* grp_prob;       // [ngroups]
   int* abort_flag;
   ProbResult* results; // [nprob]
@@ -88,10 +91,8 @@ __device__ bool fg_stages(FgCtx<R>& fc, GroupCtx& g, int lo, int hi, double* red
       return false;
     }
     pf.mark(PR_F1);
-    if (!P.dft) {  // else part of F1
-      fg_t2_cols(fc, g);
-      if (!group_sync(g)) return false;
-    }
+    fg_t2_cols(fc, g);
+    if (!group_sync(g)) return false;
     pf.mark(PR_F2);
     fg_interp(fc, g, mode != MODE_T1);
     if (!group_sync(g)) return false;
@@ -117,7 +118,7 @@ __device__ bool fg_stages(FgCtx<R>& fc, GroupCtx& g, int lo, int hi, double* red
   } else if (P.has_tfd || P.has_sm) {
     double mom[10];
     for (int k = 0; k < 10; ++k) mom[k] = 0.0;
-    frame_moments(P, fc.base, mom);  // a frame of a movie: one CTA
+    frame_moments(P, fc.base, lo, hi, mom);
     if (!reduce_moments(g, mom, red, scratch)) return false;
     double mm[10];
     for (int k = 0; k < 10; ++k) mm[k] = red[k];
@@ -189,14 +190,16 @@ __device__ bool group_fg(FgCtx<R>& fc, GroupCtx& g, LbCtxT<R>& lc, double* red, 
 }
 
 // One evaluation of a movie (fftim3d.f90:473-614, fftlib3d.f90:14-205,
-// image3d.f90:15-425).  Every frame is a complete 2D evaluation run by one
-// CTA (frames z = rank, rank + G, ...) with the frame's regularizer weights
-// already divided by the frame count; after a group barrier the movie pass
+// image3d.f90:15-425).  Every frame is a complete 2D evaluation run by a
+// sub-group gs of the CTAs (sub-group `sub` of nsub takes the frames z = sub,
+// sub + nsub, ...; CTAs left over have sub >= nsub) with the frame's
+// regularizer weights already divided by the frame count; after a group
+// barrier the movie pass
 // adds the Rt / Ri gradients (image3d.f90:280-392, Rt only for frames
 // iz < Nz as the reference does) and forms g.d and the projected gradient
 // over the whole vector.  terms[20] follow the fftim3d.imaging order.
 template <typename R>
-__device__ bool movie_fg(FgCtx<R>& fc, GroupCtx& g, LbCtxT<R>& lc, double* red, double* scratch, double& f,
+__device__ bool movie_fg(FgCtx<R>& fc, GroupCtx& g, GroupCtx& gs, int sub, int nsub, LbCtxT<R>& lc, double* red, double* scratch, double& f,
                          double& gd, double& sbg, double* terms) {
   const ProbDesc& M = *fc.P;
   char* base = fc.base;
@@ -205,15 +208,13 @@ __device__ bool movie_fg(FgCtx<R>& fc, GroupCtx& g, LbCtxT<R>& lc, double* red, 
   const ProbDesc* frames = at<ProbDesc>(base, M.o_frames);
   double acc[16];
   for (int k = 0; k < 16; ++k) acc[k] = 0.0;
-  GroupCtx g1 = g;  // one CTA per frame: G == 1 barriers are block barriers
-  g1.rank = 0;
-  g1.G = 1;
-  for (int z = g.rank; z < M.nframes; z += g.G) {
+  for (int z = sub; z < M.nframes; z = sub < nsub ? z + nsub : M.nframes) {
     FgCtx<R> fz = fc;
     fz.P = &frames[z];
     RegMoments rm;
-    if (!fg_stages(fz, g1, 0, frames[z].npix, red, scratch, acc, rm, MODE_FG, false, pf)) return false;
-    if (threadIdx.x == 0) {
+    const int share = ((frames[z].npix + gs.G - 1) / gs.G + 31) / 32 * 32, lo = min(frames[z].npix, gs.rank * share);
+    if (!fg_stages(fz, gs, lo, min(frames[z].npix, lo + share), red, scratch, acc, rm, MODE_FG, false, pf)) return false;
+    if (gs.rank == 0 && threadIdx.x == 0) {
       double tfd, cen, sm;
       global_regs(frames[z], rm, tfd, cen, sm);
       acc[4 + 5] += tfd;  // the light-curve term when M.has_lc
@@ -309,17 +310,18 @@ __global__ void __launch_bounds__(Shape<R>::threads, Shape<R>::min_blocks) smili
   __shared__ double red[SMILI_REDK];
   __shared__ double scratch[SMILI_SCRATCH(Shape<R>::threads)];
   __shared__ int prob_s;
-  const int grp = blockIdx.x / a.G, rank = blockIdx.x % a.G;
+  const int4 cta = a.ctas[blockIdx.x];
+  const int grp = cta.x, rank = (int)blockIdx.x - cta.y, G = cta.z;
   Prof prof;
   prof.acc = (blockIdx.x == 0 && threadIdx.x == 0) ? a.prof : nullptr;
   prof.t = 0;
   prof.start();
   GroupCtx g;
   g.rank = rank;
-  g.G = a.G;
+  g.G = G;
   g.bar = a.bars + 8 * grp;
   g.target = 0;
-  g.red_part = a.red_part + (size_t)grp * 2 * a.G * a.redk;
+  g.red_part = a.red_part + (size_t)cta.y * 2 * a.redk;
   g.redk = a.redk;
   g.parity = 0;
   g.abort_flag = a.abort_flag;
@@ -337,17 +339,8 @@ __global__ void __launch_bounds__(Shape<R>::threads, Shape<R>::min_blocks) smili
     if (rank != 0) group_sync(g);
     return;
   }
-  while (true) {
-    if (rank == 0 && threadIdx.x == 0) {
-      const int p = atomicAdd(a.queue, 1);
-      a.grp_prob[grp] = p;
-      __threadfence();
-    }
-    if (!group_sync(g)) return;
-    if (threadIdx.x == 0) prob_s = ((volatile int*)a.grp_prob)[grp];
-    __syncthreads();
-    const int p = prob_s;
-    if (p >= a.nprob) return;
+  // the group's size was chosen for problem grp, which it takes first
+  for (int p = grp; p < a.nprob;) {
     const ProbDesc& P = a.descs[p];
     char* base = a.arena;
     FgCtx<R> fc;
@@ -364,7 +357,7 @@ __global__ void __launch_bounds__(Shape<R>::threads, Shape<R>::min_blocks) smili
     lc.S = &S;
     lc.n = P.npix;
     lc.m = P.m;
-    const int chunk = ((P.npix + a.G - 1) / a.G + 31) / 32 * 32;
+    const int chunk = ((P.npix + G - 1) / G + 31) / 32 * 32;
     lc.lo = min(P.npix, rank * chunk);
     lc.hi = min(P.npix, lc.lo + chunk);
     lc.x = at<double>(base, P.o_x);
@@ -404,17 +397,6 @@ __global__ void __launch_bounds__(Shape<R>::threads, Shape<R>::min_blocks) smili
       }
       __syncthreads();
     }
-    // an empty band for the first evaluation (dense band passes add into it)
-    auto clear_band = [&](const ProbDesc& D) {
-      if (!D.dft) return;
-      cpx<R>* bandA = at<cpx<R>>(base, D.o_bandA);
-      for (int i = rank * blockDim.x + threadIdx.x; i < D.b1n * D.b2n; i += a.G * blockDim.x) bandA[i] = cmk<R>(0, 0);
-    };
-    clear_band(P);
-    if (P.nframes > 0) {
-      const ProbDesc* frames = at<ProbDesc>(base, P.o_frames);
-      for (int z = 0; z < P.nframes; ++z) clear_band(frames[z]);
-    }
     // the kernel weights of the launch's evaluations
     if (P.o_taps) {
       fg_taps<R>(P, base, g);
@@ -423,11 +405,28 @@ __global__ void __launch_bounds__(Shape<R>::threads, Shape<R>::min_blocks) smili
       for (int z = 0; z < P.nframes; ++z)
         if (frames[z].o_taps) fg_taps<R>(frames[z], base, g);
     }
+    // A movie's frames are shared out to sub-groups of G / nframes CTAs.  The
+    // arrival count of a sub-group is read before the group barrier, so before
+    // any of its CTAs can arrive again.
+    GroupCtx gs = g;
+    int sub = 0, nsub = 1;
+    if (P.nframes > 0) {
+      gs.G = max(1, G / P.nframes);
+      sub = rank / gs.G;
+      nsub = G / gs.G;
+      gs.rank = rank % gs.G;
+      const int lead = (int)blockIdx.x - gs.rank;
+      gs.bar = a.sub_bars + 8 * (size_t)lead;
+      gs.target = ld_relaxed(gs.bar);
+      gs.red_part = a.sub_red + (size_t)lead * 2 * SMILI_REDK_FG;
+      gs.redk = SMILI_REDK_FG;
+      gs.parity = 0;
+    }
     bool ok = group_sync(g);
     prof.mark(PR_INIT);
     while (ok) {
       double f = 0, gd = 0, sbg = 0;
-      const bool okf = P.nframes > 0 ? movie_fg<R>(fc, g, lc, red, scratch, f, gd, sbg, S.terms)
+      const bool okf = P.nframes > 0 ? movie_fg<R>(fc, g, gs, sub, nsub, lc, red, scratch, f, gd, sbg, S.terms)
                                      : group_fg<R>(fc, g, lc, red, scratch, f, gd, sbg, S.terms, a.mode);
       if (!okf) {
         ok = false;
@@ -447,7 +446,7 @@ __global__ void __launch_bounds__(Shape<R>::threads, Shape<R>::min_blocks) smili
       // final summary evaluation at the returned image (fftim2d.f90:356-376)
       if (!group_sync(g)) ok = false;
       double f = 0, gd = 0, sbg = 0;
-      if (ok && !(P.nframes > 0 ? movie_fg<R>(fc, g, lc, red, scratch, f, gd, sbg, S.terms)
+      if (ok && !(P.nframes > 0 ? movie_fg<R>(fc, g, gs, sub, nsub, lc, red, scratch, f, gd, sbg, S.terms)
                                 : group_fg<R>(fc, g, lc, red, scratch, f, gd, sbg, S.terms, MODE_FG)))
         ok = false;
       if (threadIdx.x == 0) S.nfg_total++;
@@ -462,7 +461,15 @@ __global__ void __launch_bounds__(Shape<R>::threads, Shape<R>::min_blocks) smili
       res.error = ok ? S.error : 1;
     }
     if (!ok) return;
+    if (a.nprob == a.ngroups) return;  // a group for every problem: no queue
+    if (rank == 0 && threadIdx.x == 0) {
+      a.grp_prob[grp] = a.ngroups + atomicAdd(a.queue, 1);
+      __threadfence();
+    }
     if (!group_sync(g)) return;
+    if (threadIdx.x == 0) prob_s = ((volatile int*)a.grp_prob)[grp];
+    __syncthreads();
+    p = prob_s;
   }
 }
 
@@ -1102,7 +1109,7 @@ int pack_problem(const smili_imaging_args& a, int kind, int niter, int nonneg, i
 }  // namespace
 
 struct smili_batch {
-  int nprob = 0, prec64 = 1, G = 1, ngroups = 1, device = 0;
+  int nprob = 0, prec64 = 1, grid = 1, ngroups = 1, device = 0;
   int kind = PK_SOLVE;
   std::vector<ProbDesc> descs;
   std::vector<std::vector<int>> perms;
@@ -1115,6 +1122,9 @@ struct smili_batch {
   unsigned* d_bars = nullptr;
   double* d_red_part = nullptr;
   int redk = SMILI_REDK;
+  int4* d_ctas = nullptr;
+  unsigned* d_sub_bars = nullptr;
+  double* d_sub_red = nullptr;
   int* d_grp_prob = nullptr;
   int* d_abort = nullptr;
   unsigned long long* d_prof = nullptr;
@@ -1131,19 +1141,86 @@ struct smili_batch {
 
 namespace {
 
+// CTAs that one problem is worth when the device has it to itself.  Per CTA a
+// pixel or a uv point costs little against a stage's fixed latency, so a group
+// grows until its barriers and group sums cost what a larger one saves.  Ten
+// iterations on a B200 in FP64 (the FP32 optima are close), kernel ms at four
+// pixels per thread / at this rule: 64^2 px, 2.0 k points 3.58 at 4 CTAs /
+// 2.65 at 19; 7.6 k px, 4.2 k points 4.16 at 8 / 3.00 at 35; 64^2 px, 50 k
+// points 8.85 at 4 / 3.18 at 66; 128^2 px, 50 k points 4.71 at 16 / 3.28 at
+// 72; 256^2 px 5.21 at 64 / 4.91 at 96; 512^2 px 4.3 at 256 / 3.85 at 148.
+// Two CTAs on an SM only pay from about 2^19 pixels (1024^2: 148 8.9, 296 8.4).
+int group_size(double npix, double nuv, int nsm, int maxres) {
+  double G = std::min(npix / 256 + nuv / 800, 64 + npix / 2048);
+  if (npix <= 1 << 19) G = std::min(G, (double)nsm);
+  return std::max(1, std::min(maxres, (int)G));
+}
+
+// Groups of a launch: (group, first CTA, CTA count) of every CTA.  A fixed
+// size (or more problems than the device holds CTAs) gives equal groups and a
+// queue.  Otherwise every problem gets a group, and the CTAs are dealt out so
+// that the largest share of work per CTA is as small as it can be: the launch
+// ends with its slowest problem.  Work counts 19 per pixel and 8.4 per uv
+// point, the optimiser's and the data side's measured ratio.  Sizes that do
+// not lower the largest share are taken back, so equal problems get equal
+// groups.
+std::vector<int4> group_table(const std::vector<ProbDesc>& descs, int fixed, int nsm, int maxres) {
+  const int nprob = (int)descs.size();
+  std::vector<int> size;
+  if (fixed > 0 || nprob > maxres) {
+    const int G = std::max(1, std::min(fixed, maxres));
+    size.assign(std::max(1, std::min(nprob, maxres / G)), G);
+  } else {
+    std::vector<int> cap(nprob);
+    std::vector<double> work(nprob);
+    for (int p = 0; p < nprob; ++p) {
+      cap[p] = group_size(descs[p].npix, descs[p].nuv, nsm, maxres);
+      work[p] = 19.0 * descs[p].npix + 8.4 * descs[p].nuv;
+    }
+    size.assign(nprob, 1);
+    std::vector<std::pair<double, int>> heap;
+    for (int p = 0; p < nprob; ++p)
+      if (cap[p] > 1) heap.emplace_back(work[p], p);
+    std::make_heap(heap.begin(), heap.end());
+    for (int left = maxres - nprob; left > 0 && !heap.empty(); --left) {
+      std::pop_heap(heap.begin(), heap.end());
+      const int p = heap.back().second;
+      if (++size[p] < cap[p]) {
+        heap.back().first = work[p] / size[p];
+        std::push_heap(heap.begin(), heap.end());
+      } else {
+        heap.pop_back();
+      }
+    }
+    if (!heap.empty()) {  // the CTAs ran out: what the largest share needs
+      const double share = heap.front().first * (1 + 1e-12);
+      for (int p = 0; p < nprob; ++p)
+        size[p] = std::max(1, std::min(size[p], (int)std::ceil(work[p] / share)));
+    }
+  }
+  std::vector<int4> ctas;
+  for (int g = 0; g < (int)size.size(); ++g) {
+    const int first = (int)ctas.size();
+    ctas.insert(ctas.end(), size[g], int4{g, first, size[g], 0});
+  }
+  return ctas;
+}
+
 template <typename R>
 int launch_batch(smili_batch* b, int mode, float* ms) {
   const void* fn = (const void*)smili_batch_kernel<R>;
-  const size_t aux_reset = 0;
-  (void)aux_reset;
   CUDA_TRY(cudaMemsetAsync(b->d_queue, 0, sizeof(int), b->stream));
   CUDA_TRY(cudaMemsetAsync(b->d_bars, 0, sizeof(unsigned) * 8 * b->ngroups, b->stream));
+  if (b->d_sub_bars) CUDA_TRY(cudaMemsetAsync(b->d_sub_bars, 0, sizeof(unsigned) * 8 * b->grid, b->stream));
   CUDA_TRY(cudaMemsetAsync(b->d_abort, 0, sizeof(int), b->stream));
   BatchArgs a;
   a.arena = b->d_arena;
   a.descs = b->d_descs;
   a.nprob = b->nprob;
-  a.G = b->G;
+  a.ngroups = b->ngroups;
+  a.ctas = b->d_ctas;
+  a.sub_bars = b->d_sub_bars;
+  a.sub_red = b->d_sub_red;
   a.mode = mode;
   a.queue = b->d_queue;
   a.bars = b->d_bars;
@@ -1161,7 +1238,7 @@ int launch_batch(smili_batch* b, int mode, float* ms) {
     CUDA_TRY(cudaEventCreate(&e1));
     CUDA_TRY(cudaEventRecord(e0, b->stream));
   }
-  CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(b->G * b->ngroups), dim3(Shape<R>::threads), args,
+  CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(b->grid), dim3(Shape<R>::threads), args,
                                        b->dyn_bytes, b->stream));
   if (ms) {
     CUDA_TRY(cudaEventRecord(e1, b->stream));
@@ -1178,8 +1255,7 @@ int launch_batch(smili_batch* b, int mode, float* ms) {
 }
 
 template <typename R>
-int finish_batch(smili_batch* b, std::vector<HostProb>& hps, int maxn, const smili_options* opt,
-                 smili_batch** out);
+int finish_batch(smili_batch* b, std::vector<HostProb>& hps, const smili_options* opt, smili_batch** out);
 
 template <typename R>
 int create_batch(int nprob, const smili_imaging_args* const* probs, const int* niter, int nonneg,
@@ -1230,7 +1306,6 @@ int create_batch(int nprob, const smili_imaging_args* const* probs, const int* n
       delete b;
       return fail(rcs[p], errs[p]);
     }
-  int maxn = 1;
   size_t base = 0;
   for (int p = 0; p < nprob; ++p) {
     ProbDesc& d = hps[p].d;
@@ -1242,17 +1317,15 @@ int create_batch(int nprob, const smili_imaging_args* const* probs, const int* n
       if (bl.first >= 0) bl.first += (int64_t)base;
     base += ars[p].bytes;
     b->descs.push_back(d);
-    maxn = std::max(maxn, d.npix);
   }
   b->arena_bytes = base;
-  return finish_batch<R>(b, hps, maxn, opt, out);
+  return finish_batch<R>(b, hps, opt, out);
 }
 
 // Device side of a batch whose problems are packed (descs, arena size, host
 // blobs): launch geometry, buffers, upload.  Takes ownership of b.
 template <typename R>
-int finish_batch(smili_batch* b, std::vector<HostProb>& hps, int maxn, const smili_options* opt,
-                 smili_batch** out) {
+int finish_batch(smili_batch* b, std::vector<HostProb>& hps, const smili_options* opt, smili_batch** out) {
   const int device = b->device;
   const int nprob = b->nprob;
   b->niter_cap.clear();
@@ -1285,15 +1358,10 @@ int finish_batch(smili_batch* b, std::vector<HostProb>& hps, int maxn, const smi
   CUDA_TRY(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device));
   if (!coop || occ < 1) return cleanup(fail(SMILI_ERR_CUDA, "cooperative launch unavailable"));
   const int maxres = occ * nsm;
-  int G = opt && opt->ctas_per_problem > 0 ? opt->ctas_per_problem : 0;
-  if (G <= 0) {
-    const int per_cta = 4 * Shape<R>::threads;  // about four pixels per thread
-    G = std::max(1, std::min(maxres, (maxn + per_cta - 1) / per_cta));
-    if (nprob > 1) G = std::max(1, std::min(G, maxres / nprob));
-  }
-  G = std::min(G, maxres);
-  b->G = G;
-  b->ngroups = std::max(1, std::min(nprob, maxres / G));
+  const std::vector<int4> ctas = group_table(b->descs, opt ? opt->ctas_per_problem : 0, nsm, maxres);
+  b->grid = (int)ctas.size();
+  b->ngroups = ctas.back().x + 1;
+  const bool movie = b->descs[0].nframes > 0;
   // device buffers
   if (cudaMalloc(&b->d_arena, std::max<size_t>(b->arena_bytes, 256)) != cudaSuccess)
     return cleanup(fail(SMILI_ERR_CUDA, "cudaMalloc of the problem arena failed"));
@@ -1305,7 +1373,9 @@ int finish_batch(smili_batch* b, std::vector<HostProb>& hps, int maxn, const smi
   };
   const size_t o_desc = take(sizeof(ProbDesc) * nprob), o_res = take(sizeof(ProbResult) * nprob),
                o_q = take(sizeof(int)), o_bar = take(sizeof(unsigned) * 8 * b->ngroups),
-               o_rp = take(sizeof(double) * (size_t)b->ngroups * 2 * G * b->redk),
+               o_rp = take(sizeof(double) * (size_t)b->grid * 2 * b->redk),
+               o_ct = take(sizeof(int4) * b->grid), o_sb = take(movie ? sizeof(unsigned) * 8 * b->grid : 0),
+               o_sr = take(movie ? sizeof(double) * 2 * SMILI_REDK_FG * (size_t)b->grid : 0),
                o_gp = take(sizeof(int) * b->ngroups), o_ab = take(sizeof(int)),
                o_pf = take(sizeof(unsigned long long) * PR_NSTAGE);
   if (cudaMalloc(&b->d_aux, aux) != cudaSuccess) return cleanup(fail(SMILI_ERR_CUDA, "cudaMalloc aux failed"));
@@ -1314,6 +1384,11 @@ int finish_batch(smili_batch* b, std::vector<HostProb>& hps, int maxn, const smi
   b->d_queue = reinterpret_cast<int*>(b->d_aux + o_q);
   b->d_bars = reinterpret_cast<unsigned*>(b->d_aux + o_bar);
   b->d_red_part = reinterpret_cast<double*>(b->d_aux + o_rp);
+  b->d_ctas = reinterpret_cast<int4*>(b->d_aux + o_ct);
+  if (movie) {
+    b->d_sub_bars = reinterpret_cast<unsigned*>(b->d_aux + o_sb);
+    b->d_sub_red = reinterpret_cast<double*>(b->d_aux + o_sr);
+  }
   b->d_grp_prob = reinterpret_cast<int*>(b->d_aux + o_gp);
   b->d_abort = reinterpret_cast<int*>(b->d_aux + o_ab);
   b->d_prof = reinterpret_cast<unsigned long long*>(b->d_aux + o_pf);
@@ -1338,6 +1413,7 @@ int finish_batch(smili_batch* b, std::vector<HostProb>& hps, int maxn, const smi
   }
   CUDA_TRY(cudaMemcpyAsync(b->d_descs, b->descs.data(), sizeof(ProbDesc) * nprob, cudaMemcpyHostToDevice,
                            b->stream));
+  CUDA_TRY(cudaMemcpyAsync(b->d_ctas, ctas.data(), sizeof(int4) * ctas.size(), cudaMemcpyHostToDevice, b->stream));
   CUDA_TRY(cudaStreamSynchronize(b->stream));
   *out = b;
   return SMILI_OK;
@@ -1622,7 +1698,7 @@ int create_movie(const smili_imaging3d_args* a, int kind, int niter, int nonneg,
   }
   b->descs.push_back(hps[0].d);
   b->arena_bytes = ar.bytes;
-  return finish_batch<R>(b, hps, hps[0].d.npix, opt, out);
+  return finish_batch<R>(b, hps, opt, out);
 }
 
 // One evaluation of a single data term with unit weight and no
@@ -1654,7 +1730,7 @@ int create_model(const smili_imaging_args& a, const double* x, const smili_optio
   }
   b->descs.push_back(hps[0].d);
   b->arena_bytes = ar.bytes;
-  return finish_batch<R>(b, hps, hps[0].d.npix, opt, out);
+  return finish_batch<R>(b, hps, opt, out);
 }
 
 int create_movie_any(const smili_imaging3d_args* a, int kind, int niter, int nonneg, int m, double factr,
@@ -2288,14 +2364,15 @@ int calc_cost_noalloc(const smili_imaging_args* a, const double* x, const smili_
   if (!coop || occ < 1) return fail(SMILI_ERR_CUDA, "cooperative launch unavailable");
   const int maxres = occ * nsm;
   int G = opt && opt->ctas_per_problem > 0 ? opt->ctas_per_problem : 0;
-  if (G <= 0) {  // finish_batch's rule for one problem: about four pixels per thread
-    const int per_cta = 4 * Shape<R>::threads;
-    G = std::max(1, std::min(maxres, (hp.d.npix + per_cta - 1) / per_cta));
-  }
-  G = std::min(G, maxres);
-  b.G = G;
   b.ngroups = 1;
   b.redk = SMILI_REDK_FG;
+  if (G <= 0) {  // group_size, as far as the scratch has room for the partial sums
+    const size_t per_cta = sizeof(double) * 2 * b.redk + sizeof(int4);
+    const size_t room = kNoAllocBytes - arena_al, rest = sizeof(ProbDesc) + sizeof(ProbResult) + (8 << 10);
+    G = group_size(hp.d.npix, hp.d.nuv, nsm, room > rest ? (int)std::min<size_t>(maxres, (room - rest) / per_cta) : 1);
+  }
+  G = std::min(G, maxres);
+  b.grid = G;
   // bookkeeping after the arena, laid out as in create_batch
   size_t off = arena_al;
   auto take = [&](size_t n) {
@@ -2303,8 +2380,9 @@ int calc_cost_noalloc(const smili_imaging_args* a, const double* x, const smili_
     off += round256(n);
     return o;
   };
+  const std::vector<int4> ctas(G, int4{0, 0, G, 0});
   const size_t o_desc = take(sizeof(ProbDesc)), o_res = take(sizeof(ProbResult)), o_q = take(sizeof(int)),
-               o_bar = take(sizeof(unsigned) * 8), o_rp = take(sizeof(double) * (size_t)2 * G * b.redk),
+               o_bar = take(sizeof(unsigned) * 8), o_ct = take(sizeof(int4) * G), o_rp = take(sizeof(double) * (size_t)2 * G * b.redk),
                o_gp = take(sizeof(int)), o_ab = take(sizeof(int)),
                o_pf = take(sizeof(unsigned long long) * PR_NSTAGE);
   if (off > kNoAllocBytes)
@@ -2319,6 +2397,7 @@ int calc_cost_noalloc(const smili_imaging_args* a, const double* x, const smili_
   b.d_queue = reinterpret_cast<int*>(scratch + o_q);
   b.d_bars = reinterpret_cast<unsigned*>(scratch + o_bar);
   b.d_red_part = reinterpret_cast<double*>(scratch + o_rp);
+  b.d_ctas = reinterpret_cast<int4*>(scratch + o_ct);
   b.d_grp_prob = reinterpret_cast<int*>(scratch + o_gp);
   b.d_abort = reinterpret_cast<int*>(scratch + o_ab);
   b.d_prof = reinterpret_cast<unsigned long long*>(scratch + o_pf);
@@ -2333,6 +2412,7 @@ int calc_cost_noalloc(const smili_imaging_args* a, const double* x, const smili_
                              b.stream));
   }
   CUDA_TRY(cudaMemcpyAsync(b.d_descs, b.descs.data(), sizeof(ProbDesc), cudaMemcpyHostToDevice, b.stream));
+  CUDA_TRY(cudaMemcpyAsync(b.d_ctas, ctas.data(), sizeof(int4) * G, cudaMemcpyHostToDevice, b.stream));
   rc = launch_batch<R>(&b, MODE_FG, nullptr);
   if (rc != SMILI_OK) return rc;
   return smili_batch_fetch(&b, 0, nullptr, terms, grad, nullptr);
