@@ -13,6 +13,8 @@
 #include <complex>
 #include <cstdio>
 #include <cstring>
+#include <memory>
+#include <mutex>
 #include <numeric>
 #include <stdexcept>
 #include <string>
@@ -546,22 +548,119 @@ void gl_positive(int q, std::vector<double>& x, std::vector<double>& wt) {
   }
 }
 
-// 1 / psi_hat(k) for the N modes k = -N/2..(N-1)/2 on a fine grid of nf cells
-std::vector<double> deconv_factors(int N, int nf, int w, double beta) {
-  std::vector<double> gx, gw;
-  gl_positive(80, gx, gw);
-  std::vector<double> out(N);
-  for (int i = 0; i < N; ++i) {
-    const int k = i - N / 2;
-    double acc = 0;
-    for (size_t q = 0; q < gx.size(); ++q) {
-      const double z = gx[q], s = 1.0 - z * z;
-      const double phi = s > 0 ? std::exp(beta * (std::sqrt(s) - 1.0)) : 0.0;
-      acc += gw[q] * phi * std::cos(M_PI * k * w * z / nf);
+// A batch's two device buffers come from a memory pool of this library, one
+// per device, that keeps up to kPoolKeep bytes of freed buffers for the next
+// batch and returns the rest to the device when a batch is destroyed.  A
+// one-shot call (fftim2d.imaging, calc_cost, the bare transforms) spent 0.9 to
+// 1.3 ms, and now and then 14, in cudaMalloc and cudaFree.  Stream ordered and
+// safe from several threads (the driver's pool).  Null where the device has no
+// pools: plain cudaMalloc then.
+constexpr unsigned long long kPoolKeep = 256ull << 20;
+constexpr int kPoolMaxDev = 64;
+
+cudaMemPool_t device_pool(int device) {
+  static std::mutex mu;
+  static cudaMemPool_t pools[kPoolMaxDev] = {};
+  static bool tried[kPoolMaxDev] = {};
+  if (device < 0 || device >= kPoolMaxDev) return nullptr;
+  std::lock_guard<std::mutex> lock(mu);
+  if (!tried[device]) {
+    tried[device] = true;
+    int have = 0;
+    cudaMemPool_t p = nullptr;
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    unsigned long long keep = kPoolKeep;
+    if (cudaDeviceGetAttribute(&have, cudaDevAttrMemoryPoolsSupported, device) == cudaSuccess && have &&
+        cudaMemPoolCreate(&p, &props) == cudaSuccess &&
+        cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess)
+      pools[device] = p;
+    else
+      cudaGetLastError();
+  }
+  return pools[device];
+}
+
+// Calls pack(0), ..., pack(n - 1) on the host cores; the first (by index)
+// error code with its message, or SMILI_OK.
+template <class F>
+int pack_parallel(int n, F pack) {
+  std::vector<int> rcs(n, SMILI_OK);
+  std::vector<std::string> errs(n);
+  std::atomic<int> next{0};
+  auto work = [&]() {
+    for (int p = next.fetch_add(1); p < n; p = next.fetch_add(1)) {
+      try {  // an exception must not leave a worker thread (std::terminate)
+        rcs[p] = pack(p);
+        if (rcs[p] != SMILI_OK) errs[p] = g_err;
+      } catch (const std::exception& ex) {
+        rcs[p] = SMILI_ERR_ARG;
+        errs[p] = std::string("host packing of a problem failed: ") + ex.what();
+      }
     }
-    out[i] = 1.0 / (w * acc);
+  };
+  const int nth = std::max(1, std::min(n, (int)std::thread::hardware_concurrency()));
+  std::vector<std::thread> pool;
+  for (int t = 1; t < nth; ++t) pool.emplace_back(work);
+  work();
+  for (auto& th : pool) th.join();
+  for (int p = 0; p < n; ++p)
+    if (rcs[p] != SMILI_OK) return fail(rcs[p], errs[p]);
+  return SMILI_OK;
+}
+
+// 1 / psi_hat(k) for the N modes k = -N/2..(N-1)/2 on a fine grid of nf
+// cells, by a Gauss-Legendre rule (gx, gw); even in k
+std::vector<double> deconv_factors(int N, int nf, int w, double beta, const std::vector<double>& gx,
+                                   const std::vector<double>& gw) {
+  std::vector<double> gp(gx.size());
+  for (size_t q = 0; q < gx.size(); ++q) {
+    const double z = gx[q], s = 1.0 - z * z;
+    gp[q] = gw[q] * (s > 0 ? std::exp(beta * (std::sqrt(s) - 1.0)) : 0.0);
+  }
+  std::vector<double> out(N);
+  for (int k = 0; k <= N / 2; ++k) {
+    double acc = 0;
+    for (size_t q = 0; q < gx.size(); ++q) acc += gp[q] * std::cos(M_PI * k * w * gx[q] / nf);
+    const double f = 1.0 / (w * acc);
+    out[N / 2 - k] = f;
+    if (N / 2 + k < N) out[N / 2 + k] = f;
   }
   return out;
+}
+
+// The tables of a transform that depend on the image and fine-grid sizes
+// only: deconvolution factors and twiddles of both axes.  The frames of a
+// movie share one set.
+template <typename R>
+struct NufftTables {
+  std::vector<double> dc1, dc2;
+  std::vector<cpx<R>> tw1, tw2;
+  NufftTables(int nx, int ny, int nf1, int nf2, int w, double beta) {
+    std::vector<double> gx, gw;
+    gl_positive(80, gx, gw);
+    dc1 = deconv_factors(nx, nf1, w, beta, gx, gw);
+    dc2 = deconv_factors(ny, nf2, w, beta, gx, gw);
+    tw1 = twiddles(nf1);
+    tw2 = nf2 == nf1 ? tw1 : twiddles(nf2);
+  }
+  static std::vector<cpx<R>> twiddles(int n) {
+    std::vector<cpx<R>> t(n);
+    for (int k = 0; k < n; ++k) {
+      const long double ang = 2.0L * 3.14159265358979323846264338327950288L * k / n;
+      t[k].x = (R)std::cos(ang);
+      t[k].y = (R)std::sin(ang);
+    }
+    return t;
+  }
+};
+
+// fine grid of the NUFFT of an nx x ny image with kernel width w
+inline void fine_grid(int nx, int ny, int w, int& nf1, int& nf2) {
+  nf1 = next235even(std::max(2 * nx, 2 * w));
+  nf2 = next235even(std::max(2 * ny, 2 * w));
 }
 
 // Dynamic shared memory per CTA: the FFT staging buffers, and never less
@@ -622,6 +721,16 @@ struct HostProb {
   }
 };
 
+// Moves a packed problem's region to arena offset base.
+void move_region(ProbDesc& d, HostProb& hp, int64_t base) {
+#define SMILI_MOVE(f) \
+  if (d.f) d.f += base;
+  SMILI_PROB_OFFSETS(SMILI_MOVE)
+#undef SMILI_MOVE
+  for (auto& bl : hp.blobs)
+    if (bl.first >= 0) bl.first += base;
+}
+
 // The order of [0, n) by key(i) in [0, nkey), ties in index order: a
 // counting sort, the same order as std::stable_sort by key in O(n + nkey).
 template <class K>
@@ -656,7 +765,7 @@ template <typename R>
 int pack_problem(const smili_imaging_args& a, int kind, int niter, int nonneg, int m, double factr,
                  double pgtol, double eps, Arena& ar, HostProb& hp, const double* x_override,
                  const double* c_re, const double* c_im, double wtotal_override = 0.0, int bin = 8,
-                 int transform = 0, bool taps = false) {
+                 int transform = 0, bool taps = false, const NufftTables<R>* tables = nullptr) {
   ProbDesc& d = hp.d;
   std::memset(&d, 0, sizeof(d));
   const int N = a.npix, nx = a.nx, ny = a.ny, nuv = a.nuv;
@@ -684,8 +793,7 @@ int pack_problem(const smili_imaging_args& a, int kind, int niter, int nonneg, i
   es_params(eps, w, beta);
   d.w = w;
   d.beta = beta;
-  d.nf1 = next235even(std::max(2 * nx, 2 * w));
-  d.nf2 = next235even(std::max(2 * ny, 2 * w));
+  fine_grid(nx, ny, w, d.nf1, d.nf2);
   if (d.nf1 > SMILI_SMEM_CPX || d.nf2 > SMILI_SMEM_CPX)
     return fail(SMILI_ERR_UNSUPPORTED, "fine grid larger than 2048 cells per axis");
   d.npix = N;
@@ -841,40 +949,47 @@ int pack_problem(const smili_imaging_args& a, int kind, int niter, int nonneg, i
   // and locality); remap indices.  Band-relative cells are computed exactly as the
   // kernels do: imod(ceil(xi - w/2) - start, nf).
   auto imodh = [](long a, long n) {
-    long r = a % n;
+    if ((unsigned long)a < (unsigned long)n) return a;  // the common case
+    const long r = a % n;
     return r < 0 ? r + n : r;
   };
-  std::vector<long> bkey(nuv);
-  std::vector<int> bidx(nuv), cidx(nuv);
-  const int nb1 = (d.nf1 + bin - 1) / bin, nb2 = (d.nf2 + bin - 1) / bin;
-  for (int j = 0; j < nuv; ++j) {
-    const long c1 = imodh((long)std::ceil(xu[j] - half) - d.b1s, d.nf1);
-    const long c2 = imodh((long)std::ceil(xv[j] - half) - d.b2s, d.nf2);
-    bkey[j] = ((c2 / bin) << 32) + (c1 / bin);
-    bidx[j] = (int)(c2 / bin) * nb1 + (int)(c1 / bin);  // the same order as bkey
-    cidx[j] = (int)(c2 % bin) * bin + (int)(c1 % bin);
-  }
   // by tile, and inside a tile by cell: neighbouring threads of the
   // interpolation then read the same band cells (a shared-memory broadcast
-  // instead of a bank conflict) wherever cells hold several points
-  const std::vector<int> by_cell = counting_order(nuv, bin * bin, [&](int j) { return cidx[j]; });
-  std::vector<int> perm = counting_order(nuv, nb1 * nb2, [&](int j) { return bidx[by_cell[j]]; });
-  for (int& j : perm) j = by_cell[j];
+  // instead of a bank conflict) wherever cells hold several points.  One
+  // counting sort where its counters are few beside the points, else two.
+  const int nb1 = (d.nf1 + bin - 1) / bin, nb2 = (d.nf2 + bin - 1) / bin, ncell = bin * bin;
+  std::vector<int> tile(nuv), cidx(nuv);
+  for (int j = 0; j < nuv; ++j) {
+    const int c1 = (int)imodh((long)std::ceil(xu[j] - half) - d.b1s, d.nf1);
+    const int c2 = (int)imodh((long)std::ceil(xv[j] - half) - d.b2s, d.nf2);
+    const int t1 = c1 / bin, t2 = c2 / bin;
+    tile[j] = t2 * nb1 + t1;
+    cidx[j] = (c2 - t2 * bin) * bin + (c1 - t1 * bin);
+  }
+  std::vector<int> perm;
+  if ((long)nb1 * nb2 * ncell <= 4L * nuv) {
+    perm = counting_order(nuv, nb1 * nb2 * ncell, [&](int j) { return tile[j] * ncell + cidx[j]; });
+  } else {
+    const std::vector<int> by_cell = counting_order(nuv, ncell, [&](int j) { return cidx[j]; });
+    perm = counting_order(nuv, nb1 * nb2, [&](int j) { return tile[by_cell[j]]; });
+    for (int& j : perm) j = by_cell[j];
+  }
   // spreading work items: <= 128 consecutive points of one bin
   std::vector<int> items;
   for (int j = 0; j < nuv;) {
-    const long k = bkey[perm[j]];
+    const int k = tile[perm[j]];
     int e = j;
-    while (e < nuv && bkey[perm[e]] == k && e - j < 128) ++e;
+    while (e < nuv && e - j < 128 && tile[perm[e]] == k) ++e;
     items.push_back(j);
     items.push_back(e);
-    items.push_back((int)((k >> 32) * bin));
-    items.push_back((int)((k & 0xffffffffL) * bin));
+    items.push_back(k / nb1 * bin);
+    items.push_back(k % nb1 * bin);
     j = e;
   }
   d.nitems = (int)items.size() / 4;
-  std::vector<int> newpos(nuv);
-  for (int j = 0; j < nuv; ++j) newpos[perm[j]] = j;
+  std::vector<int> newpos(nslot && kind != PK_T1 ? nuv : 0);
+  if (!newpos.empty())
+    for (int j = 0; j < nuv; ++j) newpos[perm[j]] = j;
   std::vector<R> su(nuv), sv(nuv);
   for (int j = 0; j < nuv; ++j) {
     su[j] = xu[perm[j]];
@@ -990,16 +1105,11 @@ int pack_problem(const smili_imaging_args& a, int kind, int niter, int nonneg, i
     }
   }
   // deconvolution factors and twiddles
-  const std::vector<double> dc1 = deconv_factors(nx, d.nf1, w, beta), dc2 = deconv_factors(ny, d.nf2, w, beta);
-  auto twiddles = [](int n) {
-    std::vector<cpx<R>> t(n);
-    for (int k = 0; k < n; ++k) {
-      const long double ang = 2.0L * 3.14159265358979323846264338327950288L * k / n;
-      t[k].x = (R)std::cos(ang);
-      t[k].y = (R)std::sin(ang);
-    }
-    return t;
-  };
+  std::unique_ptr<NufftTables<R>> own_tables;
+  if (!tables) {
+    own_tables.reset(new NufftTables<R>(nx, ny, d.nf1, d.nf2, w, beta));
+    tables = own_tables.get();
+  }
   // ---- arena layout ----
   const size_t C = sizeof(cpx<R>);
   if (!frame) d.o_x0 = ar.take(sizeof(double) * N);
@@ -1021,13 +1131,14 @@ int pack_problem(const smili_imaging_args& a, int kind, int niter, int nonneg, i
   }
   d.o_u = ar.take(sizeof(R) * nuv);
   d.o_v = ar.take(sizeof(R) * nuv);
-  if (taps) d.o_taps = ar.take(sizeof(R) * 2 * w * (size_t)nuv);
   d.o_dre = ar.take(sizeof(R) * dre.size());
   d.o_dim = ar.take(sizeof(R) * dim.size());
   d.o_dvar = ar.take(sizeof(R) * dvar.size());
   d.o_didx = ar.take(sizeof(int) * didx.size());
   d.o_dsgn = ar.take(dsgn.size());
   d.o_items = ar.take(sizeof(int) * items.size());
+  // workspace: everything the host uploads lies before it in one run
+  if (taps) d.o_taps = ar.take(sizeof(R) * 2 * w * (size_t)nuv);
   d.o_tmpA = ar.take(C * (size_t)ny * d.b1n);
   d.o_bandA = ar.take(C * (size_t)d.b2n * d.b1n);
   d.o_V = ar.take(C * nuv);
@@ -1070,34 +1181,39 @@ int pack_problem(const smili_imaging_args& a, int kind, int niter, int nonneg, i
   if (d.has_kl) hp.put(d.o_klw, a.kl_wgt, (size_t)N);
   if (d.has_gs) hp.put(d.o_gsw, a.gs_wgt, (size_t)N);
   set_uniform_weights(d, a, N);
-  hp.put(d.o_dc1, dc1);
-  hp.put(d.o_dc2, dc2);
-  hp.put(d.o_tw1, twiddles(d.nf1));
-  hp.put(d.o_tw2, twiddles(d.nf2));
+  hp.put(d.o_dc1, tables->dc1);
+  hp.put(d.o_dc2, tables->dc2);
+  hp.put(d.o_tw1, tables->tw1);
+  hp.put(d.o_tw2, tables->tw2);
   if (d.dft) {
     // E[b][i] = tw[((i - n_img / 2) (bs + b)) mod nf]: the twiddle each FFT
     // pass applies between image index i and band index b
-    auto emat = [&](int nb, int bs, int nimg, int nf) {
-      const std::vector<cpx<R>> tw = twiddles(nf);
+    auto emat = [&](int nb, int bs, int nimg, int nf, const std::vector<cpx<R>>& tw) {
       std::vector<cpx<R>> e((size_t)nb * nimg);
       for (int b = 0; b < nb; ++b)
+      {
+        const int step = (int)(((long)(bs + b) % nf + nf) % nf);
+        int k = (int)((-(long)(nimg / 2) * step % nf + nf) % nf);
         for (int i = 0; i < nimg; ++i) {
-          long k = ((long)(i - nimg / 2) * (long)(bs + b)) % nf;
-          if (k < 0) k += nf;
           e[(size_t)b * nimg + i] = tw[k];
+          k += step;
+          if (k >= nf) k -= nf;
         }
+      }
       return e;
     };
-    hp.put(d.o_ex, emat(d.b1n, d.b1s, nx, d.nf1));
-    hp.put(d.o_ey, emat(d.b2n, d.b2s, ny, d.nf2));
+    hp.put(d.o_ex, emat(d.b1n, d.b1s, nx, d.nf1, tables->tw1));
+    hp.put(d.o_ey, emat(d.b2n, d.b2s, ny, d.nf2, tables->tw2));
   }
   hp.put(d.o_u, su);
   hp.put(d.o_v, sv);
   hp.put(d.o_dre, dre);
   hp.put(d.o_dim, dim);
   hp.put(d.o_dvar, dvar);
-  hp.put(d.o_didx, didx);
-  hp.put(d.o_dsgn, dsgn);
+  if (use_data) {  // a bare transform's are zeros, as the cleared arena is
+    hp.put(d.o_didx, didx);
+    hp.put(d.o_dsgn, dsgn);
+  }
   hp.put(d.o_items, items);
   if (kind == PK_T1) hp.put(d.o_contrib, contrib0);
   // the original -> sorted uv permutation is needed to return visibilities
@@ -1130,6 +1246,7 @@ struct smili_batch {
   unsigned long long* d_prof = nullptr;
   cudaStream_t stream = nullptr;
   bool own_stream = false;
+  bool pooled = false;  // d_arena and d_aux come from the device's pool
   size_t dyn_bytes = 0;
   int profile = 0;
   std::vector<int> niter_cap;  // iteration caps at packing (trace buffers are sized for them)
@@ -1276,47 +1393,24 @@ int create_batch(int nprob, const smili_imaging_args* const* probs, const int* n
   // to end and every offset moved by its region's start.
   std::vector<Arena> ars(nprob);
   std::vector<HostProb> hps(nprob);
-  std::vector<int> rcs(nprob, SMILI_OK);
-  std::vector<std::string> errs(nprob);
   double nuv_total = 0;
   for (int p = 0; p < nprob; ++p) nuv_total += std::max(probs[p]->nuv, 0);
   const bool taps = keep_taps<R>(kind, eps, nuv_total);
-  std::atomic<int> next{0};
-  auto work = [&]() {
-    for (int p = next.fetch_add(1); p < nprob; p = next.fetch_add(1)) {
-      try {  // an exception must not leave a worker thread (std::terminate)
-        ars[p].take(256);
-        rcs[p] = pack_problem<R>(*probs[p], kind, niter ? niter[p] : 0, nonneg, m, factr, pgtol, eps, ars[p],
-                                 hps[p], x_over ? x_over[p] : nullptr, c_re, c_im, 0.0,
-                                 opt && opt->spread_bin ? opt->spread_bin : 8, opt ? opt->transform : 0, taps);
-        if (rcs[p] != SMILI_OK) errs[p] = g_err;
-      } catch (const std::exception& ex) {
-        rcs[p] = SMILI_ERR_ARG;
-        errs[p] = std::string("host packing of a problem failed: ") + ex.what();
-      }
-    }
-  };
-  const int nth = std::max(1, std::min(nprob, (int)std::thread::hardware_concurrency()));
-  std::vector<std::thread> pool;
-  for (int t = 1; t < nth; ++t) pool.emplace_back(work);
-  work();
-  for (auto& th : pool) th.join();
-  for (int p = 0; p < nprob; ++p)
-    if (rcs[p] != SMILI_OK) {
-      delete b;
-      return fail(rcs[p], errs[p]);
-    }
+  const int rc = pack_parallel(nprob, [&](int p) -> int {
+    ars[p].take(256);
+    return pack_problem<R>(*probs[p], kind, niter ? niter[p] : 0, nonneg, m, factr, pgtol, eps, ars[p], hps[p],
+                           x_over ? x_over[p] : nullptr, c_re, c_im, 0.0,
+                           opt && opt->spread_bin ? opt->spread_bin : 8, opt ? opt->transform : 0, taps);
+  });
+  if (rc != SMILI_OK) {
+    delete b;
+    return rc;
+  }
   size_t base = 0;
   for (int p = 0; p < nprob; ++p) {
-    ProbDesc& d = hps[p].d;
-#define SMILI_MOVE(f) \
-  if (d.f) d.f += (int64_t)base;
-    SMILI_PROB_OFFSETS(SMILI_MOVE)
-#undef SMILI_MOVE
-    for (auto& bl : hps[p].blobs)
-      if (bl.first >= 0) bl.first += (int64_t)base;
+    move_region(hps[p].d, hps[p], (int64_t)base);
     base += ars[p].bytes;
-    b->descs.push_back(d);
+    b->descs.push_back(hps[p].d);
   }
   b->arena_bytes = base;
   return finish_batch<R>(b, hps, opt, out);
@@ -1362,23 +1456,40 @@ int finish_batch(smili_batch* b, std::vector<HostProb>& hps, const smili_options
   b->grid = (int)ctas.size();
   b->ngroups = ctas.back().x + 1;
   const bool movie = b->descs[0].nframes > 0;
-  // device buffers
-  if (cudaMalloc(&b->d_arena, std::max<size_t>(b->arena_bytes, 256)) != cudaSuccess)
-    return cleanup(fail(SMILI_ERR_CUDA, "cudaMalloc of the problem arena failed"));
   size_t aux = 0;
   auto take = [&](size_t n) {
     const size_t o = aux;
     aux += (n + 255) / 256 * 256;
     return o;
   };
-  const size_t o_desc = take(sizeof(ProbDesc) * nprob), o_res = take(sizeof(ProbResult) * nprob),
-               o_q = take(sizeof(int)), o_bar = take(sizeof(unsigned) * 8 * b->ngroups),
+  const size_t o_desc = take(sizeof(ProbDesc) * nprob), o_ct = take(sizeof(int4) * b->grid), host_aux = aux,
+               o_res = take(sizeof(ProbResult) * nprob), o_q = take(sizeof(int)),
+               o_bar = take(sizeof(unsigned) * 8 * b->ngroups),
                o_rp = take(sizeof(double) * (size_t)b->grid * 2 * b->redk),
-               o_ct = take(sizeof(int4) * b->grid), o_sb = take(movie ? sizeof(unsigned) * 8 * b->grid : 0),
+               o_sb = take(movie ? sizeof(unsigned) * 8 * b->grid : 0),
                o_sr = take(movie ? sizeof(double) * 2 * SMILI_REDK_FG * (size_t)b->grid : 0),
                o_gp = take(sizeof(int) * b->ngroups), o_ab = take(sizeof(int)),
                o_pf = take(sizeof(unsigned long long) * PR_NSTAGE);
-  if (cudaMalloc(&b->d_aux, aux) != cudaSuccess) return cleanup(fail(SMILI_ERR_CUDA, "cudaMalloc aux failed"));
+  if (opt && opt->stream) {
+    b->stream = (cudaStream_t)opt->stream;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(b->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+      b->stream = nullptr;  // not to be waited for
+      return cleanup(fail(SMILI_ERR_CUDA, "a batch cannot be created while its stream is being captured"));
+    }
+  } else {
+    if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess)
+      return cleanup(fail(SMILI_ERR_CUDA, "cudaStreamCreate failed"));
+    b->own_stream = true;
+  }
+  const cudaMemPool_t pool = device_pool(device);
+  b->pooled = pool != nullptr;
+  auto alloc = [&](void** p, size_t n) {
+    return (pool ? cudaMallocFromPoolAsync(p, n, pool, b->stream) : cudaMalloc(p, n)) == cudaSuccess;
+  };
+  if (!alloc((void**)&b->d_arena, std::max<size_t>(b->arena_bytes, 256)))
+    return cleanup(fail(SMILI_ERR_CUDA, "allocation of the problem arena failed"));
+  if (!alloc((void**)&b->d_aux, aux)) return cleanup(fail(SMILI_ERR_CUDA, "allocation of the launch's buffers failed"));
   b->d_descs = reinterpret_cast<ProbDesc*>(b->d_aux + o_desc);
   b->d_results = reinterpret_cast<ProbResult*>(b->d_aux + o_res);
   b->d_queue = reinterpret_cast<int*>(b->d_aux + o_q);
@@ -1392,28 +1503,46 @@ int finish_batch(smili_batch* b, std::vector<HostProb>& hps, const smili_options
   b->d_grp_prob = reinterpret_cast<int*>(b->d_aux + o_gp);
   b->d_abort = reinterpret_cast<int*>(b->d_aux + o_ab);
   b->d_prof = reinterpret_cast<unsigned long long*>(b->d_aux + o_pf);
-  if (opt && opt->stream) {
-    b->stream = (cudaStream_t)opt->stream;
-  } else {
-    CUDA_TRY(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
-    b->own_stream = true;
-  }
-  // upload: zero the arena, then every blob
+  // upload: zero the arena, then the arrays.  Those that lie end to end (a
+  // problem's all do) go in one copy, through a host buffer; only large ones
+  // are worth a copy of their own.  (One copy each, some 20 per problem and
+  // frame, cost about 8 us apiece.)
   CUDA_TRY(cudaMemsetAsync(b->d_arena, 0, b->arena_bytes, b->stream));
+  std::vector<char> stage;
+  int64_t start = 0;
+  auto flush = [&]() -> int {
+    if (!stage.empty())
+      CUDA_TRY(cudaMemcpyAsync(b->d_arena + start, stage.data(), stage.size(), cudaMemcpyHostToDevice, b->stream));
+    stage.clear();
+    return SMILI_OK;
+  };
+  constexpr size_t kLarge = 256 << 10, kStage = 4 << 20;
+  constexpr int64_t kGap = 255;  // between neighbours: the arena's rounding
   for (int p = 0; p < nprob; ++p) {
     for (auto& bl : hps[p].blobs) {
-      if (bl.first < 0) {
-        b->perms.emplace_back((const int*)bl.second.data(), (const int*)(bl.second.data() + bl.second.size()));
+      const int64_t off = bl.first, end = start + (int64_t)stage.size();
+      const size_t n = bl.second.size();
+      if (off < 0) {
+        b->perms.emplace_back((const int*)bl.second.data(), (const int*)(bl.second.data() + n));
         continue;
       }
-      if (!bl.second.empty())
-        CUDA_TRY(cudaMemcpyAsync(b->d_arena + bl.first, bl.second.data(), bl.second.size(),
-                                 cudaMemcpyHostToDevice, b->stream));
+      if (n == 0) continue;
+      if (!stage.empty() && (off < end || off > end + kGap || n >= kLarge || stage.size() + n > kStage))
+        if (const int rc = flush()) return rc;
+      if (n >= kLarge) {
+        CUDA_TRY(cudaMemcpyAsync(b->d_arena + off, bl.second.data(), n, cudaMemcpyHostToDevice, b->stream));
+        continue;
+      }
+      if (stage.empty()) start = off;
+      stage.resize((size_t)(off - start), 0);
+      stage.insert(stage.end(), bl.second.begin(), bl.second.end());
     }
   }
-  CUDA_TRY(cudaMemcpyAsync(b->d_descs, b->descs.data(), sizeof(ProbDesc) * nprob, cudaMemcpyHostToDevice,
-                           b->stream));
-  CUDA_TRY(cudaMemcpyAsync(b->d_ctas, ctas.data(), sizeof(int4) * ctas.size(), cudaMemcpyHostToDevice, b->stream));
+  if (const int rc = flush()) return rc;
+  stage.assign(host_aux, 0);
+  std::memcpy(stage.data() + o_desc, b->descs.data(), sizeof(ProbDesc) * nprob);
+  std::memcpy(stage.data() + o_ct, ctas.data(), sizeof(int4) * ctas.size());
+  CUDA_TRY(cudaMemcpyAsync(b->d_aux, stage.data(), host_aux, cudaMemcpyHostToDevice, b->stream));
   CUDA_TRY(cudaStreamSynchronize(b->stream));
   *out = b;
   return SMILI_OK;
@@ -1574,10 +1703,18 @@ int pack_movie(const smili_imaging3d_args& a, int kind, int niter, int nonneg, i
     d.o_riw = ar.take(sizeof(double) * N);
     d.o_iavg = ar.take(sizeof(double) * N);
   }
-  // frames
+  // frames, packed in parallel as the problems of a batch are, each into its
+  // own region after the movie's
   std::vector<HostProb> fh(Nz);
-  std::vector<double> w1, wtv, wtsv, wkl, wgs;
-  for (int z = 0; z < Nz; ++z) {
+  std::vector<Arena> fa_ar(Nz);
+  int w, nf1, nf2;
+  double beta;
+  es_params(eps, w, beta);
+  fine_grid(a.nx, a.ny, w, nf1, nf2);
+  const NufftTables<R> tables(a.nx, a.ny, nf1, nf2, w, beta);
+  auto pack_frame = [&](int z) -> int {
+    std::vector<double> w1, wtv, wtsv, wkl, wgs;
+    fa_ar[z].take(256);  // no present field at offset 0, the mark of an absent one
     const FrameData& f = fd[z];
     smili_imaging_args fa;
     std::memset(&fa, 0, sizeof(fa));
@@ -1653,10 +1790,13 @@ int pack_movie(const smili_imaging3d_args& a, int kind, int niter, int nonneg, i
     fa.varca = f.cavar.data();
     fa.wca = a.wca;
     fa.inormfactr = a.inormfactr;
-    if ((rc = pack_problem<R>(fa, PK_FRAME, 0, nonneg, m, factr, pgtol, eps, ar, fh[z], nullptr, nullptr, nullptr,
-                              wtotal, spread_bin, transform, keep_taps<R>(PK_FRAME, eps, nuv))) != SMILI_OK)
-      return rc;
+    return pack_problem<R>(fa, PK_FRAME, 0, nonneg, m, factr, pgtol, eps, fa_ar[z], fh[z], nullptr, nullptr, nullptr,
+                           wtotal, spread_bin, transform, keep_taps<R>(PK_FRAME, eps, nuv), &tables);
+  };
+  if ((rc = pack_parallel(Nz, pack_frame)) != SMILI_OK) return rc;
+  for (int z = 0; z < Nz; ++z) {
     ProbDesc& F = fh[z].d;
+    move_region(F, fh[z], ar.take(fa_ar[z].bytes));
     F.o_x = d.o_x + (int64_t)sizeof(double) * z * N;
     F.o_g = d.o_g + (int64_t)sizeof(double) * z * N;
     F.o_d = d.o_d + (int64_t)sizeof(double) * z * N;
@@ -2053,8 +2193,12 @@ void smili_batch_destroy(smili_batch* b) {
   if (!b) return;
   cudaSetDevice(b->device);
   if (b->stream) cudaStreamSynchronize(b->stream);
-  if (b->d_arena) cudaFree(b->d_arena);
-  if (b->d_aux) cudaFree(b->d_aux);
+  for (char* p : {b->d_arena, b->d_aux})
+    if (p) {
+      if (!b->pooled || cudaFreeAsync(p, b->stream) != cudaSuccess) cudaFree(p);
+    }
+  // what the pool does not keep goes back to the device with this wait
+  if (b->pooled && b->stream) cudaStreamSynchronize(b->stream);
   if (b->d_x0_saved) cudaFree(b->d_x0_saved);
   if (b->d_keep) cudaFree(b->d_keep);
   if (b->own_stream && b->stream) cudaStreamDestroy(b->stream);

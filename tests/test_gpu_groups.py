@@ -130,3 +130,47 @@ def test_movie_solves_agree_over_group_sizes():
     kw["niter"] = 5
     out = [fftim3d.imaging(nufft_eps=1e-12, ctas_per_problem=g, **kw)[20] for g in (1, 3, 50, 0)]
     assert np.max(np.abs(np.array(out) - out[0])) <= 1e-9 * abs(out[0])
+
+
+def test_batches_from_threads(lib):
+    """Batches made, run and freed by several threads at once, on the
+    library's streams and on the caller's, share the pooled device memory."""
+    import threading
+    import torch
+    kw = _obs(24, niter=3)
+    prob = lib.Problem(kw)
+
+    def solve(stream=None):
+        b = lib.Batch([prob], niter=3, options=lib.make_options(64, 1e-12, 2, stream=stream))
+        b.run()
+        c = b.fetch(0)[1]["cost"]
+        b.close()
+        return c
+
+    want, got = solve(), []
+
+    def work(own):
+        s = torch.cuda.Stream() if own else None
+        for _ in range(10):
+            got.append(solve(s.cuda_stream if own else None))
+
+    ts = [threading.Thread(target=work, args=(k % 2 == 0,)) for k in range(6)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert len(got) == 60 and np.max(np.abs(np.array(got) - want)) <= 1e-9 * abs(want)
+
+
+def test_batch_refuses_a_capturing_stream(lib):
+    import torch
+    prob = lib.Problem(_obs(24, niter=3))
+    s, g = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    x = torch.zeros(1, device="cuda")
+    with torch.cuda.graph(g, stream=s, capture_error_mode="relaxed"):
+        with pytest.raises(Exception):
+            lib.Batch([prob], niter=3, options=lib.make_options(64, 1e-12, 1, stream=s.cuda_stream))
+        x += 1
+    g.replay()
+    torch.cuda.synchronize()
+    assert float(x) == 1.0
