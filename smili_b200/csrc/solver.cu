@@ -27,6 +27,7 @@
 #include "fg.cuh"
 #include "layout.h"
 #include "lbfgsb.cuh"
+#include "uvsort.cuh"
 
 #define SMILI_VERSION 1
 #define SMILI_SMEM_CPX 2048   // complex elements per FFT buffer
@@ -700,15 +701,44 @@ struct Arena {
 };
 
 bool finite_all(const double* p, int n) {
-  for (int i = 0; i < n; ++i)
-    if (!std::isfinite(p[i])) return false;
-  return true;
+  double s[8] = {};  // 0 * x is NaN for NaN and infinities; no branch per value
+  int i = 0;
+  for (; i + 8 <= n; i += 8)
+    for (int k = 0; k < 8; ++k) s[k] += 0.0 * p[i + k];
+  for (; i < n; ++i) s[0] += 0.0 * p[i];
+  return s[0] + s[1] + s[2] + s[3] + s[4] + s[5] + s[6] + s[7] == 0.0;
+}
+
+// least and largest of n finite values
+void range_of(const double* p, int n, double& lo, double& hi) {
+  double l[8], h[8];
+  for (int k = 0; k < 8; ++k) l[k] = h[k] = p[0];
+  int i = 0;
+  for (; i + 8 <= n; i += 8)
+    for (int k = 0; k < 8; ++k) {
+      l[k] = std::min(l[k], p[i + k]);
+      h[k] = std::max(h[k], p[i + k]);
+    }
+  for (; i < n; ++i) {
+    l[0] = std::min(l[0], p[i]);
+    h[0] = std::max(h[0], p[i]);
+  }
+  lo = *std::min_element(l, l + 8);
+  hi = *std::max_element(h, h + 8);
 }
 
 // Host image of one problem: descriptor + the byte blobs to upload
 struct HostProb {
   ProbDesc d;
   std::vector<std::pair<int64_t, std::vector<char>>> blobs;
+  // arrays of the caller that are uploaded as they are
+  struct Direct {
+    int64_t off;
+    const void* p;
+    size_t bytes;
+  };
+  std::vector<Direct> direct;
+  UvSort sort;  // of a bare transform
   // one copy of the bytes (no zero fill first)
   template <typename T>
   void put(int64_t off, const T* p, size_t n) {
@@ -728,7 +758,11 @@ void move_region(ProbDesc& d, HostProb& hp, int64_t base) {
   SMILI_PROB_OFFSETS(SMILI_MOVE)
 #undef SMILI_MOVE
   for (auto& bl : hp.blobs)
-    if (bl.first >= 0) bl.first += base;
+    bl.first += base;
+  for (auto& t : hp.direct) t.off += base;
+  UvSort& q = hp.sort;
+  for (int64_t* o : {&q.o_u, &q.o_v, &q.o_cre, &q.o_cim, &q.o_key, &q.o_perm, &q.o_hist, &q.o_sums})
+    if (*o) *o += base;
 }
 
 // The order of [0, n) by key(i) in [0, nkey), ties in index order: a
@@ -824,7 +858,7 @@ int pack_problem(const smili_imaging_args& a, int kind, int niter, int nonneg, i
   d.ncp = ncp;
   d.nca = nca;
   d.ndata = nfcv + namp + ncp + nca;
-  const int nslot = (kind == PK_T1) ? nuv : nfcv + namp + 3 * ncp + 4 * nca;
+  const int nslot = nfcv + namp + 3 * ncp + 4 * nca;
   d.nslot = nslot;
   // normalised data weights (fftim2d.f90:178-213)
   double wtotal = 0;
@@ -896,19 +930,20 @@ int pack_problem(const smili_imaging_args& a, int kind, int niter, int nonneg, i
     return SMILI_OK;
   }
 
-  // fine-grid coordinates in the kernel precision, band of touched cells
-  std::vector<R> xu(nuv), xv(nuv);
+  // band of touched cells: the grid coordinate, its rounding to the kernel
+  // precision and ceil are monotone, so it follows from the extreme points
+  const bool bare = kind == PK_T1 || kind == PK_T2;  // points sorted on the device
   const R half = (R)0.5 * (R)w;
-  long mn1 = 1L << 40, mx1 = -(1L << 40), mn2 = 1L << 40, mx2 = -(1L << 40);
-  for (int j = 0; j < nuv; ++j) {
-    xu[j] = (R)(a.u[j] * d.nf1 / (2.0 * M_PI));
-    xv[j] = (R)(a.v[j] * d.nf2 / (2.0 * M_PI));
-    const long l1 = (long)std::ceil(xu[j] - half), l2 = (long)std::ceil(xv[j] - half);
-    mn1 = std::min(mn1, l1);
-    mx1 = std::max(mx1, l1 + w - 1);
-    mn2 = std::min(mn2, l2);
-    mx2 = std::max(mx2, l2 + w - 1);
-  }
+  auto coord = [](double u, int nf) { return (R)(u * nf / (2.0 * M_PI)); };
+  auto band = [&](const double* u, int nf, long& mn, long& mx) {
+    double lo, hi;
+    range_of(u, nuv, lo, hi);
+    mn = (long)std::ceil(coord(lo, nf) - half);
+    mx = (long)std::ceil(coord(hi, nf) - half) + w - 1;
+  };
+  long mn1, mx1, mn2, mx2;
+  band(a.u, d.nf1, mn1, mx1);
+  band(a.v, d.nf2, mn2, mx2);
   if (mx1 - mn1 + 1 >= d.nf1) {
     d.b1s = 0;
     d.b1n = d.nf1;
@@ -958,8 +993,12 @@ int pack_problem(const smili_imaging_args& a, int kind, int niter, int nonneg, i
   // instead of a bank conflict) wherever cells hold several points.  One
   // counting sort where its counters are few beside the points, else two.
   const int nb1 = (d.nf1 + bin - 1) / bin, nb2 = (d.nf2 + bin - 1) / bin, ncell = bin * bin;
-  std::vector<int> tile(nuv), cidx(nuv);
-  for (int j = 0; j < nuv; ++j) {
+  const int npt = bare ? 0 : nuv;  // points sorted here
+  std::vector<R> xu(npt), xv(npt);
+  std::vector<int> tile(npt), cidx(npt);
+  for (int j = 0; j < npt; ++j) {
+    xu[j] = coord(a.u[j], d.nf1);
+    xv[j] = coord(a.v[j], d.nf2);
     const int c1 = (int)imodh((long)std::ceil(xu[j] - half) - d.b1s, d.nf1);
     const int c2 = (int)imodh((long)std::ceil(xv[j] - half) - d.b2s, d.nf2);
     const int t1 = c1 / bin, t2 = c2 / bin;
@@ -967,19 +1006,19 @@ int pack_problem(const smili_imaging_args& a, int kind, int niter, int nonneg, i
     cidx[j] = (c2 - t2 * bin) * bin + (c1 - t1 * bin);
   }
   std::vector<int> perm;
-  if ((long)nb1 * nb2 * ncell <= 4L * nuv) {
-    perm = counting_order(nuv, nb1 * nb2 * ncell, [&](int j) { return tile[j] * ncell + cidx[j]; });
+  if ((long)nb1 * nb2 * ncell <= 4L * npt) {
+    perm = counting_order(npt, nb1 * nb2 * ncell, [&](int j) { return tile[j] * ncell + cidx[j]; });
   } else {
-    const std::vector<int> by_cell = counting_order(nuv, ncell, [&](int j) { return cidx[j]; });
-    perm = counting_order(nuv, nb1 * nb2, [&](int j) { return tile[by_cell[j]]; });
+    const std::vector<int> by_cell = counting_order(npt, ncell, [&](int j) { return cidx[j]; });
+    perm = counting_order(npt, nb1 * nb2, [&](int j) { return tile[by_cell[j]]; });
     for (int& j : perm) j = by_cell[j];
   }
   // spreading work items: <= 128 consecutive points of one bin
   std::vector<int> items;
-  for (int j = 0; j < nuv;) {
+  for (int j = 0; j < npt;) {
     const int k = tile[perm[j]];
     int e = j;
-    while (e < nuv && e - j < 128 && tile[perm[e]] == k) ++e;
+    while (e < npt && e - j < 128 && tile[perm[e]] == k) ++e;
     items.push_back(j);
     items.push_back(e);
     items.push_back(k / nb1 * bin);
@@ -987,11 +1026,10 @@ int pack_problem(const smili_imaging_args& a, int kind, int niter, int nonneg, i
     j = e;
   }
   d.nitems = (int)items.size() / 4;
-  std::vector<int> newpos(nslot && kind != PK_T1 ? nuv : 0);
-  if (!newpos.empty())
-    for (int j = 0; j < nuv; ++j) newpos[perm[j]] = j;
-  std::vector<R> su(nuv), sv(nuv);
-  for (int j = 0; j < nuv; ++j) {
+  std::vector<int> newpos(npt);
+  std::vector<R> su(npt), sv(npt);
+  for (int j = 0; j < npt; ++j) {
+    newpos[perm[j]] = j;
     su[j] = xu[perm[j]];
     sv[j] = xv[perm[j]];
   }
@@ -1092,18 +1130,6 @@ int pack_problem(const smili_imaging_args& a, int kind, int niter, int nonneg, i
     reorder(nfcv + namp, ncp, nfcv + namp, 3);
     reorder(nfcv + namp + ncp, nca, nfcv + namp + 3 * ncp, 4);
   }
-  // per-uv-point derivative accumulators: set here only for the bare type-1
-  // mode (c = (Re c, -Im c) in sorted order); otherwise F3 zeroes them and F4
-  // adds into them every evaluation
-  std::vector<cpx<R>> contrib0;
-  if (kind == PK_T1) {
-    contrib0.resize(nuv);
-    for (int j = 0; j < nuv; ++j) {
-      const int o = perm[j];
-      contrib0[j].x = (R)c_re[o];
-      contrib0[j].y = (R)(-c_im[o]);
-    }
-  }
   // deconvolution factors and twiddles
   std::unique_ptr<NufftTables<R>> own_tables;
   if (!tables) {
@@ -1136,7 +1162,25 @@ int pack_problem(const smili_imaging_args& a, int kind, int niter, int nonneg, i
   d.o_dvar = ar.take(sizeof(R) * dvar.size());
   d.o_didx = ar.take(sizeof(int) * didx.size());
   d.o_dsgn = ar.take(dsgn.size());
-  d.o_items = ar.take(sizeof(int) * items.size());
+  if (bare) {
+    UvSort& q = hp.sort;
+    q.nb1 = (d.b1n + bin - 1) / bin;
+    q.ntile = q.nb1 * ((d.b2n + bin - 1) / bin);
+    q.nkey = q.ntile * ncell;
+    d.o_items = ar.take(sizeof(int) * 4 * ((size_t)nuv / 128 + std::min(q.ntile, nuv)));
+    q.o_u = ar.take(sizeof(double) * nuv);
+    q.o_v = ar.take(sizeof(double) * nuv);
+    if (kind == PK_T1) {
+      q.o_cre = ar.take(sizeof(double) * nuv);
+      q.o_cim = ar.take(sizeof(double) * nuv);
+    }
+    q.o_key = ar.take(sizeof(int) * nuv);
+    q.o_perm = ar.take(sizeof(int) * nuv);
+    q.o_hist = ar.take(sizeof(int) * q.nkey);
+    q.o_sums = ar.take(sizeof(int) * ((q.nkey + UVSORT_CHUNK - 1) / UVSORT_CHUNK));
+  } else {
+    d.o_items = ar.take(sizeof(int) * items.size());
+  }
   // workspace: everything the host uploads lies before it in one run
   if (taps) d.o_taps = ar.take(sizeof(R) * 2 * w * (size_t)nuv);
   d.o_tmpA = ar.take(C * (size_t)ny * d.b1n);
@@ -1205,6 +1249,14 @@ int pack_problem(const smili_imaging_args& a, int kind, int niter, int nonneg, i
     hp.put(d.o_ex, emat(d.b1n, d.b1s, nx, d.nf1, tables->tw1));
     hp.put(d.o_ey, emat(d.b2n, d.b2s, ny, d.nf2, tables->tw2));
   }
+  if (bare) {
+    hp.direct.push_back({hp.sort.o_u, a.u, sizeof(double) * nuv});
+    hp.direct.push_back({hp.sort.o_v, a.v, sizeof(double) * nuv});
+    if (kind == PK_T1) {
+      hp.direct.push_back({hp.sort.o_cre, c_re, sizeof(double) * nuv});
+      hp.direct.push_back({hp.sort.o_cim, c_im, sizeof(double) * nuv});
+    }
+  }
   hp.put(d.o_u, su);
   hp.put(d.o_v, sv);
   hp.put(d.o_dre, dre);
@@ -1215,10 +1267,6 @@ int pack_problem(const smili_imaging_args& a, int kind, int niter, int nonneg, i
     hp.put(d.o_dsgn, dsgn);
   }
   hp.put(d.o_items, items);
-  if (kind == PK_T1) hp.put(d.o_contrib, contrib0);
-  // the original -> sorted uv permutation is needed to return visibilities
-  if (!frame)
-    hp.blobs.emplace_back(-1, std::vector<char>((const char*)perm.data(), (const char*)perm.data() + sizeof(int) * nuv));
   return SMILI_OK;
 }
 
@@ -1228,7 +1276,7 @@ struct smili_batch {
   int nprob = 0, prec64 = 1, grid = 1, ngroups = 1, device = 0;
   int kind = PK_SOLVE;
   std::vector<ProbDesc> descs;
-  std::vector<std::vector<int>> perms;
+  UvSort sort;  // of a bare transform
   char* d_arena = nullptr;
   size_t arena_bytes = 0;
   ProbDesc* d_descs = nullptr;
@@ -1522,10 +1570,6 @@ int finish_batch(smili_batch* b, std::vector<HostProb>& hps, const smili_options
     for (auto& bl : hps[p].blobs) {
       const int64_t off = bl.first, end = start + (int64_t)stage.size();
       const size_t n = bl.second.size();
-      if (off < 0) {
-        b->perms.emplace_back((const int*)bl.second.data(), (const int*)(bl.second.data() + n));
-        continue;
-      }
       if (n == 0) continue;
       if (!stage.empty() && (off < end || off > end + kGap || n >= kLarge || stage.size() + n > kStage))
         if (const int rc = flush()) return rc;
@@ -1539,6 +1583,9 @@ int finish_batch(smili_batch* b, std::vector<HostProb>& hps, const smili_options
     }
   }
   if (const int rc = flush()) return rc;
+  for (auto& t : hps[0].direct)
+    CUDA_TRY(cudaMemcpyAsync(b->d_arena + t.off, t.p, t.bytes, cudaMemcpyHostToDevice, b->stream));
+  b->sort = hps[0].sort;
   stage.assign(host_aux, 0);
   std::memcpy(stage.data() + o_desc, b->descs.data(), sizeof(ProbDesc) * nprob);
   std::memcpy(stage.data() + o_ct, ctas.data(), sizeof(int4) * ctas.size());
@@ -1811,7 +1858,7 @@ int pack_movie(const smili_imaging3d_args& a, int kind, int niter, int nonneg, i
   for (int z = 0; z < Nz; ++z) {
     fdesc[z] = fh[z].d;
     for (auto& bl : fh[z].blobs)
-      if (bl.first >= 0) hp.blobs.emplace_back(bl.first, std::move(bl.second));
+      hp.blobs.emplace_back(bl.first, std::move(bl.second));
   }
   hp.put(d.o_frames, fdesc);
   return SMILI_OK;
@@ -1885,6 +1932,31 @@ int create_movie_any(const smili_imaging3d_args* a, int kind, int niter, int non
 int run(smili_batch* b, int mode, float* ms) {
   CUDA_TRY(cudaSetDevice(b->device));
   return b->prec64 ? launch_batch<double>(b, mode, ms) : launch_batch<float>(b, mode, ms);
+}
+
+// A bare transform: sort the points, transform, and (forward) put the
+// visibilities into the caller's order.
+template <typename R>
+int launch_bare(smili_batch* b, int mode) {
+  const UvSort& q = b->sort;
+  const int nb = std::min(4 * 148, (b->descs[0].nuv + 255) / 256), nchunk = (q.nkey + UVSORT_CHUNK - 1) / UVSORT_CHUNK;
+  uvsort_count<R><<<nb, 256, 0, b->stream>>>(b->d_descs, b->d_arena, q);
+  uvsort_sums<<<nchunk, UVSORT_T, 0, b->stream>>>(b->d_arena, q);
+  uvsort_scan<<<nchunk, UVSORT_T, 0, b->stream>>>(b->d_arena, q);
+  uvsort_scatter<R><<<nb, 256, 0, b->stream>>>(b->d_descs, b->d_arena, q);
+  if (mode == MODE_T1) uvsort_items<<<1, UVSORT_T, 0, b->stream>>>(b->d_descs, b->d_arena, q);
+  CUDA_TRY(cudaGetLastError());
+  const int rc = launch_batch<R>(b, mode, nullptr);
+  if (rc != SMILI_OK || mode != MODE_T2) return rc;
+  uvsort_result<R><<<nb, 256, 0, b->stream>>>(b->d_descs, b->d_arena, q);
+  CUDA_TRY(cudaGetLastError());
+  CUDA_TRY(cudaStreamSynchronize(b->stream));
+  return SMILI_OK;
+}
+
+int run_bare(smili_batch* b, int mode) {
+  CUDA_TRY(cudaSetDevice(b->device));
+  return b->prec64 ? launch_bare<double>(b, mode) : launch_bare<float>(b, mode);
 }
 
 int create_any(int nprob, const smili_imaging_args* const* probs, const int* niter, int nonneg, int m,
@@ -2356,27 +2428,12 @@ int smili_nufft_fwd_real(int nuv, const double* u, const double* v, int nx, int 
     const smili_imaging_args* probs[1] = {&a};
     int rc = create_any(1, probs, nullptr, 0, 5, 1e1, 0.0, opt, PK_T2, nullptr, nullptr, nullptr, &b);
     if (rc != SMILI_OK) return rc;
-    // x = image in evaluation mode
-    rc = run(b, MODE_T2, nullptr);
+    rc = run_bare(b, MODE_T2);  // x = image in evaluation mode
     if (rc == SMILI_OK) {
-      const ProbDesc& d = b->descs[0];
-      const size_t C = b->prec64 ? 16 : 8;
-      std::vector<char> buf(C * nuv);
-      cudaError_t e = cudaMemcpy(buf.data(), b->d_arena + d.o_V, C * nuv, cudaMemcpyDeviceToHost);
+      cudaError_t e = cudaMemcpy(vreal, b->d_arena + b->sort.o_u, sizeof(double) * nuv, cudaMemcpyDeviceToHost);
+      if (e == cudaSuccess)
+        e = cudaMemcpy(vimag, b->d_arena + b->sort.o_v, sizeof(double) * nuv, cudaMemcpyDeviceToHost);
       if (e != cudaSuccess) rc = fail(SMILI_ERR_CUDA, cudaGetErrorString(e));
-      const std::vector<int>& perm = b->perms[0];
-      for (int j = 0; j < nuv && rc == SMILI_OK; ++j) {
-        double re, im_;
-        if (b->prec64) {
-          re = reinterpret_cast<double*>(buf.data())[2 * j];
-          im_ = reinterpret_cast<double*>(buf.data())[2 * j + 1];
-        } else {
-          re = reinterpret_cast<float*>(buf.data())[2 * j];
-          im_ = reinterpret_cast<float*>(buf.data())[2 * j + 1];
-        }
-        vreal[perm[j]] = re;
-        vimag[perm[j]] = im_;
-      }
     }
     smili_batch_destroy(b);
     return rc;
@@ -2395,7 +2452,7 @@ int smili_nufft_adj_real1d(int nuv, const double* u, const double* v, const doub
     const smili_imaging_args* probs[1] = {&a};
     int rc = create_any(1, probs, nullptr, 0, 5, 1e1, 0.0, opt, PK_T1, nullptr, vreal, vimag, &b);
     if (rc != SMILI_OK) return rc;
-    rc = run(b, MODE_T1, nullptr);
+    rc = run_bare(b, MODE_T1);
     if (rc == SMILI_OK) {
       const ProbDesc& d = b->descs[0];
       cudaError_t e = cudaMemcpy(img, b->d_arena + d.o_gchi, sizeof(double) * nx * ny, cudaMemcpyDeviceToHost);
@@ -2551,7 +2608,7 @@ int calc_cost_noalloc(const smili_imaging_args* a, const double* x, const smili_
   // the queue, barrier counters and abort flag are cleared by launch_batch
   CUDA_TRY(cudaMemsetAsync(b.d_arena, 0, arena_al, b.stream));
   for (auto& bl : hp.blobs) {
-    if (bl.first < 0 || bl.second.empty()) continue;  // host-side permutation; not needed for calc_cost
+    if (bl.second.empty()) continue;
     CUDA_TRY(cudaMemcpyAsync(b.d_arena + bl.first, bl.second.data(), bl.second.size(), cudaMemcpyHostToDevice,
                              b.stream));
   }
