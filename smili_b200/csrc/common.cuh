@@ -135,24 +135,24 @@ __device__ bool group_sync(GroupCtx& g) {
 // ---------------------------------------------------------------------------
 // Reductions over the group (deterministic, the same value in every CTA)
 // ---------------------------------------------------------------------------
-// Sums of N values (N a power of two up to 32) over a warp: every butterfly
-// step halves the values a lane carries, so N = 16 takes 16 exchanges instead
-// of 80.  Lane l returns the total of value l / (32 / N).
-template <int N>
-__device__ __forceinline__ double warp_fold(double (&v)[N], int lane) {
-  int b = 16;
-#pragma unroll
-  for (int h = N / 2; h >= 1; h >>= 1, b >>= 1) {
-    const bool up = (lane & b) != 0;
-#pragma unroll
-    for (int i = 0; i < h; ++i) {
-      const double send = up ? v[i] : v[i + h], keep = up ? v[i + h] : v[i];
-      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, b);
-    }
-  }
-#pragma unroll
-  for (int q = 16 / N; q >= 1; q >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], q);
-  return v[0];
+// One FP64 tensor-core product D = A B + D of an 8x4 by 4x8 tile
+// (mma.sync m8n8k4 f64).  Lane l holds A[l/4][l%4], B[l%4][l/4] and
+// D[l/4][2(l%4) + {0,1}].
+__device__ __forceinline__ void dmma_884(double (&d)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
+               : "+d"(d[0]), "+d"(d[1])
+               : "d"(a), "d"(b));
+}
+
+// Maximum over the warp (as fmax: a NaN only where all are): the doubles as
+// unsigned integers of the same order, their words one after the other.
+__device__ __forceinline__ double warp_max(double a) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(a), top = 1ULL << 63;
+  const unsigned long long k = a != a ? 0 : ((b & top) ? ~b : (b | top));
+  const unsigned hi = (unsigned)(k >> 32), mh = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? (unsigned)k : 0u);
+  const unsigned long long m = ((unsigned long long)mh << 32) | ml;
+  return __longlong_as_double((long long)((m & top) ? (m & ~top) : ~m));
 }
 
 // Second half of a group reduction: every CTA has its partials (ns sums,
@@ -207,42 +207,56 @@ __device__ __forceinline__ double* group_row(GroupCtx& g, double* out) {
   return g.G == 1 ? out : g.red_part + ((size_t)g.parity * g.G + g.rank) * g.redk;
 }
 
-// Sums of s[0..NS) and maxima of x[0..NX) over the block's threads into
-// row[0..NS) and row[NS..NS+NX).  s is clobbered.
-template <int NS, int NX>
-__device__ __forceinline__ void block_partials(double (&s)[NS], const double (&x)[NX], double* row, double* scratch) {
-  constexpr int K = NS + NX, L = 32 / NS;
-  static_assert(K <= 40, "scratch");
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const double v = warp_fold<NS>(s, lane);
-  if (lane % L == 0) scratch[wid * K + lane / L] = v;
-#pragma unroll
-  for (int q = 0; q < NX; ++q) {
-    double a = x[q];
-#pragma unroll
-    for (int b = 16; b >= 1; b >>= 1) a = fmax(a, __shfl_xor_sync(0xffffffffu, a, b));
-    if (lane == 0) scratch[wid * K + NS + q] = a;
+// Sums of each thread's s[0..ns) and maxima of its x[0..nx) over the block,
+// into row[0..ns) and row[ns..ns+nx); ns + nx <= 40.  A warp sums a value with
+// a tensor-core product by ones: 8 lanes per product, two exchanges for eight
+// values.  One routine with rolled loops for every reduction of the kernel:
+// each size unrolled (31 exchanges of two words for 16 values) spent most of
+// its time on fetching its instructions, 6.6 us per group sum of 16 values and
+// 4 maxima where the barrier in it takes 2 (B200).
+__device__ __noinline__ void block_partials(const double* s, int ns, const double* x, int nx, double* row,
+                                            double* scratch) {
+  const int K = ns + nx, lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5, q = lane >> 2;
+  double* w = scratch + wid * K;
+#pragma unroll 1
+  for (int v0 = 0; v0 < ns; v0 += 8) {
+    const int nv = min(8, ns - v0);
+    double r = 0.0;
+#pragma unroll 4
+    for (int i = 0; i < nv; ++i) {
+      double d[2] = {0.0, 0.0};
+      dmma_884(d, 1.0, s[v0 + i]);
+      const double t = d[0] + d[1];
+      r = q == i ? t : r;
+    }
+    r += __shfl_xor_sync(0xffffffffu, r, 1);
+    r += __shfl_xor_sync(0xffffffffu, r, 2);
+    if ((lane & 3) == 0 && q < nv) w[v0 + q] = r;
+  }
+#pragma unroll 1
+  for (int k = 0; k < nx; ++k) {
+    const double a = warp_max(x[k]);
+    if (lane == 0) w[ns + k] = a;
   }
   __syncthreads();
   if (threadIdx.x < K) {
     double a = scratch[threadIdx.x];
 #pragma unroll 4
-    for (int w = 1; w < nw; ++w) {
-      const double b = scratch[w * K + threadIdx.x];
-      a = (int)threadIdx.x < NS ? a + b : fmax(a, b);
+    for (int v = 1; v < nw; ++v) {
+      const double b = scratch[v * K + threadIdx.x];
+      a = (int)threadIdx.x < ns ? a + b : fmax(a, b);
     }
     row[threadIdx.x] = a;
   }
 }
 
-// Group-wide sums of s[0..NS) and maxima of x[0..NX) over all threads:
-// out[0..NS) and out[NS..NS+NX) (shared) in every CTA.  s is clobbered.
+// Group-wide sums of s[0..ns) and maxima of x[0..nx) over all threads:
+// out[0..ns) and out[ns..ns+nx) (shared) in every CTA.
 // scratch: SMILI_SCRATCH(blockDim.x) doubles of shared memory.
-template <int NS, int NX>
-__device__ __noinline__ bool group_reduce(GroupCtx& g, double (&s)[NS], const double (&x)[NX], double* out,
+__device__ __noinline__ bool group_reduce(GroupCtx& g, const double* s, int ns, const double* x, int nx, double* out,
                                           double* scratch) {
-  block_partials<NS, NX>(s, x, group_row(g, out), scratch);
-  return group_combine(g, NS + NX, NS, out, scratch);
+  block_partials(s, ns, x, nx, group_row(g, out), scratch);
+  return group_combine(g, ns + nx, ns, out, scratch);
 }
 
 // ---------------------------------------------------------------------------

@@ -111,7 +111,10 @@ struct LbState {
   double ginit, gtest, gx, gy, finit, fx, fy, stx, sty, stmin, stmax, width, width1;
   double terms[SMILI_NTERMS3D];
   double sy[SMILI_MAXM * SMILI_MAXM], ss[SMILI_MAXM * SMILI_MAXM], wt[SMILI_MAXM * SMILI_MAXM];
-  double wn[4 * SMILI_MAXM * SMILI_MAXM], wn1[4 * SMILI_MAXM * SMILI_MAXM];
+  double wn[4 * SMILI_MAXM * SMILI_MAXM];
+  // derived when the matrices change: sy(i,k) / sy(k,k); sqrt(sy(k,k)); and the
+  // reciprocals (0: divide instead) of those roots and of the diagonals of wt and wn
+  double lt[SMILI_MAXM * SMILI_MAXM], sq[SMILI_MAXM], rsq[SMILI_MAXM], rwt[SMILI_MAXM], rwn[2 * SMILI_MAXM];
   double wa[8 * SMILI_MAXM];
 };
 

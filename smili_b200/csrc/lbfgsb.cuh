@@ -64,84 +64,141 @@ __device__ __forceinline__ void st_sy(const LbCtxT<SY>& c, size_t i, double s, d
 }
 
 // ---------------------------------------------------------------------------
-// small dense algebra (thread 0)
+// small dense algebra, by one warp: an element or a row per lane, loops kept
+// rolled.  Bound by latency: of dependent FP64 operations, of the divisions
+// (avoided where the divisor is a known diagonal) and of fetching instructions,
+// as this code runs once per iteration and the stages between push it out of
+// the instruction cache.  Per call at m = 5, one thread in the reference's
+// loops / a column per lane, unrolled / as here: formk 22 / 13 / 8 us, the
+// two solves of subsm 9 / 7 / 2.8, an update 9 / 6 / 5 (B200).
 // ---------------------------------------------------------------------------
-__device__ int d_chol_upper(double* a, int lda, int nn) {  // linpack dpofa
-  for (int j = 0; j < nn; ++j) {
-    double s = 0.0;
-    for (int k = 0; k < j; ++k) {
-      double t = a[k + j * lda];
-      for (int i = 0; i < k; ++i) t -= a[i + k * lda] * a[i + j * lda];
-      t /= a[k + k * lda];
-      a[k + j * lda] = t;
-      s += t * t;
+// 1 / t for div_by, or 0 near the ends of the exponent range
+__device__ __forceinline__ double rcp_of(double t) {
+  const double a = fabs(t);
+  return a > 1e-280 && a < 1e280 ? 1.0 / t : 0.0;
+}
+
+// b / t from r = rcp_of(t): the product and one residual step, as accurate as
+// the division and a third of its latency
+__device__ __forceinline__ double div_by(double b, double t, double r) {
+  if (r == 0.0) return b / t;
+  const double q = b * r, c = fma(fma(-q, t, b), r, q);
+  return fabs(q) <= DBL_MAX ? c : q;
+}
+
+// Cholesky factor of the symmetric matrix in the upper triangle of a (shared,
+// column major, leading dimension ld).  The first n1 columns eliminate with
+// the opposite sign beyond row n1: [A B; B' C] becomes the factors of A and of
+// C + B' A^-1 B (formk's LEL' with E = diag(-I, I)); n1 = nn is the plain
+// factor.  The square roots are taken at the end, off the chain of pivots.
+// rdiag receives the reciprocals of the factor's diagonal.  One warp; returns
+// 0, -1 or -2 (a pivot of the first or second block is not positive), in every
+// lane.
+__device__ __noinline__ int warp_factor(double* a, int ld, int nn, int n1, double* rdiag) {
+  const int lane = threadIdx.x & 31;
+  // lanes 0..15 and 16..31: two halves of the rows of column lane & 15
+  const int j = lane & 15, half = lane >> 4;
+#pragma unroll 1
+  for (int k = 0; k < nn; ++k) {
+    const double d = a[k + ld * k];
+    if (d <= 0.0) return k < n1 ? -1 : -2;
+    const double u = j > k && j < nn ? a[k + ld * j] / d : 0.0;
+    if (j < nn) {
+#pragma unroll 1
+      for (int i = k + 1 + half; i <= j; i += 2) {
+        const double p = a[k + ld * i] * u;
+        a[i + ld * j] += k < n1 && i >= n1 ? p : -p;
+      }
     }
-    s = a[j + j * lda] - s;
-    if (s <= 0.0) return j + 1;
-    a[j + j * lda] = sqrt(s);
+    __syncwarp();
   }
+  const double sq = lane < nn ? sqrt(a[lane + ld * lane]) : 1.0, r = rcp_of(sq);
+  __syncwarp();
+#pragma unroll 1
+  for (int k = 0; k < nn; ++k) {
+    const double sk = __shfl_sync(0xffffffffu, sq, k), rk = __shfl_sync(0xffffffffu, r, k);
+    if (lane >= k && lane < nn) a[k + ld * lane] = lane == k ? sq : div_by(a[k + ld * lane], sk, rk);
+  }
+  if (lane < nn) rdiag[lane] = r;
+  __syncwarp();
   return 0;
 }
 
-__device__ int d_tri_solve(const double* t, int ldt, int nn, double* b, bool trans) {  // dtrsl 11/01
-  for (int i = 0; i < nn; ++i)
-    if (t[i + i * ldt] == 0.0) return i + 1;
-  if (trans) {
-    for (int j = 0; j < nn; ++j) {
-      double s = b[j];
-      for (int i = 0; i < j; ++i) s -= t[i + j * ldt] * b[i];
-      b[j] = s / t[j + j * ldt];
-    }
-  } else {
-    for (int j = nn - 1; j >= 0; --j) {
-      b[j] /= t[j + j * ldt];
-      const double bj = b[j];
-      for (int i = 0; i < j; ++i) b[i] -= bj * t[i + j * ldt];
-    }
+// x of R' x = b (trans) or R x = b, R the upper triangle of a as warp_factor
+// leaves it: lane i holds b_i and returns x_i.  ok: false in every lane when a
+// diagonal element is zero.
+__device__ __forceinline__ double warp_tri_solve(const double* a, int ld, int nn, const double* rdiag, double b,
+                                                 bool trans, bool& ok) {
+  const int lane = threadIdx.x & 31;
+  const bool in = lane < nn;
+  const double dg = in ? a[lane + ld * lane] : 1.0, rd = in ? rdiag[lane] : 1.0;
+  ok = !__any_sync(0xffffffffu, dg == 0.0);
+#pragma unroll 1
+  for (int s = 0; s < nn; ++s) {
+    const int j = trans ? s : nn - 1 - s;
+    if (lane == j) b = div_by(b, dg, rd);
+    const double xj = __shfl_sync(0xffffffffu, b, j);
+    if (in && (trans ? lane > j : lane < j)) b -= a[trans ? j + ld * lane : lane + ld * j] * xj;
   }
-  return 0;
+  return b;
 }
 
-// product with the 2col x 2col middle matrix (bmv, lbfgsb.f:1106-1220)
-__device__ int d_bmv(const LbState& S, int m, int col, const double* v, double* p) {
-  if (col == 0) return 0;
-#define SY(i, j) S.sy[((i)-1) + m * ((j)-1)]
-  p[col] = v[col];
-  for (int i = 2; i <= col; ++i) {
-    double s = 0.0;
-    for (int k = 1; k <= i - 1; ++k) s += SY(i, k) * v[k - 1] / SY(k, k);
-    p[col + i - 1] = v[col + i - 1] + s;
+// Product with the 2col x 2col middle matrix (bmv, lbfgsb.f:1106-1220): lane i
+// < col holds (vy_i, vs_i) and gets (M v)_i and (M v)_{col + i} there.  One
+// warp; false for a singular factor.
+__device__ __noinline__ bool warp_bmv(const LbState& S, int m, int col, double& vy, double& vs) {
+  const int lane = threadIdx.x & 31;
+  const bool in = lane < col;
+  double p = vs;
+#pragma unroll 1
+  for (int k = 0; k < col - 1; ++k) {
+    const double vk = __shfl_sync(0xffffffffu, vy, k);
+    if (in && lane > k) p += S.lt[lane + m * k] * vk;
   }
-  if (d_tri_solve(S.wt, m, col, p + col, true)) return -1;
-  for (int i = 1; i <= col; ++i) p[i - 1] = v[i - 1] / sqrt(SY(i, i));
-  if (d_tri_solve(S.wt, m, col, p + col, false)) return -1;
-  for (int i = 1; i <= col; ++i) p[i - 1] = -p[i - 1] / sqrt(SY(i, i));
-  for (int i = 1; i <= col; ++i) {
-    double s = 0.0;
-    for (int k = i + 1; k <= col; ++k) s += SY(k, i) * p[col + k - 1] / SY(i, i);
-    p[i - 1] += s;
+  bool ok, ok2;
+  p = warp_tri_solve(S.wt, m, col, S.rwt, p, true, ok);
+  p = warp_tri_solve(S.wt, m, col, S.rwt, p, false, ok2);
+  const double sq = in ? S.sq[lane] : 1.0, rsq = in ? S.rsq[lane] : 1.0;
+  double q = -div_by(div_by(vy, sq, rsq), sq, rsq);
+#pragma unroll 1
+  for (int k = 1; k < col; ++k) {
+    const double pk = __shfl_sync(0xffffffffu, p, k);
+    if (lane < k) q += S.lt[k + m * lane] * pk;
+  }
+  vy = q;
+  vs = p;
+  return ok;
+}
+
+// T = theta S'S + L D^-1 L' and its factor (formt, lbfgsb.f:2173-2240), with
+// the quotients and roots that warp_bmv reads.  One warp; returns nonzero in
+// every lane when T is not positive definite.
+__device__ __noinline__ int warp_formt(LbState& S, int m) {
+  const int col = S.col, lane = threadIdx.x & 31;
+#define SY(i, j) S.sy[(i) + m * (j)]
+#pragma unroll 1
+  for (int e = lane; e < col * col; e += 32) {
+    const int i = e % col, k = e / col;
+    if (i > k) S.lt[i + m * k] = SY(i, k) / SY(k, k);
+  }
+  if (lane < col) {
+    const double sq = sqrt(SY(lane, lane));
+    S.sq[lane] = sq;
+    S.rsq[lane] = rcp_of(sq);
+  }
+  __syncwarp();
+#pragma unroll 1
+  for (int e = lane; e < col * col; e += 32) {
+    const int i = e % col, j = e / col;
+    if (i > j) continue;
+    double dd = 0.0;
+#pragma unroll 1
+    for (int k = 0; k < i; ++k) dd += SY(i, k) * S.lt[j + m * k];
+    S.wt[i + m * j] = dd + S.theta * S.ss[i + m * j];
   }
 #undef SY
-  return 0;
-}
-
-__device__ int d_formt(LbState& S, int m) {  // lbfgsb.f:2173-2240
-  const int col = S.col;
-#define SY(i, j) S.sy[((i)-1) + m * ((j)-1)]
-#define SS(i, j) S.ss[((i)-1) + m * ((j)-1)]
-#define WT(i, j) S.wt[((i)-1) + m * ((j)-1)]
-  for (int j = 1; j <= col; ++j) WT(1, j) = S.theta * SS(1, j);
-  for (int i = 2; i <= col; ++i)
-    for (int j = i; j <= col; ++j) {
-      const int k1 = min(i, j) - 1;
-      double dd = 0.0;
-      for (int k = 1; k <= k1; ++k) dd += SY(i, k) * SY(j, k) / SY(k, k);
-      WT(i, j) = dd + S.theta * SS(i, j);
-    }
-#undef SY
-#undef SS
-#undef WT
-  return d_chol_upper(S.wt, m, col) ? -3 : 0;
+  __syncwarp();
+  return warp_factor(S.wt, m, col, col, S.rwt);
 }
 
 __device__ void d_dcstep(double& stx, double& fx, double& dx, double& sty, double& fy, double& dy,
@@ -306,7 +363,7 @@ __device__ __forceinline__ void reset_memory(LbState& S) {
 // Group-wide sums of s and maxima of x into c.red (sums first).
 template <int NS, int NX, typename SY>
 __device__ __forceinline__ bool lb_reduce(LbCtxT<SY>& c, double (&s)[NS], const double (&x)[NX]) {
-  return group_reduce<NS, NX>(*c.g, s, x, c.red, c.scratch);
+  return group_reduce(*c.g, s, NS, x, NX, c.red, c.scratch);
 }
 
 // ---------------------------------------------------------------------------
@@ -601,27 +658,36 @@ __device__ __noinline__ int cauchy_search(LbCtxT<SY>& c, double f1_0, const doub
   if (threadIdx.x < 32) sm.cum[threadIdx.x] = 0.0;
   if (threadIdx.x == 0) info_s = 0;
   __syncthreads();
-  if (threadIdx.x < col2) {
-    double e[2 * SMILI_MAXM_DEV], mc[2 * SMILI_MAXM_DEV];
-    for (int k = 0; k < col2; ++k) e[k] = (k == (int)threadIdx.x) ? 1.0 : 0.0;
-    if (d_bmv(S, m, col, e, mc)) info_s = -1;
-    const int jc = (int)threadIdx.x < col ? (int)threadIdx.x : 6 + (int)threadIdx.x - col;
-    for (int k = 0; k < col2; ++k) sm.Mm[(k < col ? k : 6 + k - col) * 12 + jc] = mc[k];
+  for (int j = wid; j < col2; j += nw) {  // column j of M, a warp each
+    double y = lane == j ? 1.0 : 0.0, s = lane == j - col ? 1.0 : 0.0;
+    if (!warp_bmv(S, m, col, y, s) && lane == 0) info_s = -1;
+    const int jc = j < col ? j : 6 + j - col;
+    if (lane < col) {
+      sm.Mm[lane * 12 + jc] = y;
+      sm.Mm[(6 + lane) * 12 + jc] = s;
+    }
   }
   __syncthreads();
   if (info_s) return -1;  // singular middle matrix (bmv failure)
-  if (threadIdx.x == 0) {
-    double f2 = -theta * f1_0;
-    f2org_s = f2;
+  if (threadIdx.x < 32) {
     double s = 0;
-    for (int i = 0; i < 12; ++i)
-      for (int j = 0; j < 12; ++j) s += p0[i] * sm.Mm[i * 12 + j] * p0[j];
-    f2 -= s;
-    sm.st[0] = -f1_0;
-    sm.st[1] = 0.0;
-    sm.st[2] = -f1_0 / f2;
-    bnd_hi_s = 0;
-    bnd_lo_s = 0;
+    if (lane < 12) {
+#pragma unroll
+      for (int j = 0; j < 12; ++j) s += sm.Mm[lane * 12 + j] * p0[j];
+      s *= p0[lane];
+    }
+#pragma unroll
+    for (int q = 8; q >= 1; q >>= 1) s += __shfl_xor_sync(0xffffffffu, s, q);
+    if (lane == 0) {
+      double f2 = -theta * f1_0;
+      f2org_s = f2;
+      f2 -= s;
+      sm.st[0] = -f1_0;
+      sm.st[1] = 0.0;
+      sm.st[2] = -f1_0 / f2;
+      bnd_hi_s = 0;
+      bnd_lo_s = 0;
+    }
   }
   if (threadIdx.x < 12) {
     sm.P[threadIdx.x] = p0[threadIdx.x];
@@ -677,7 +743,7 @@ __device__ __noinline__ int cauchy_search(LbCtxT<SY>& c, double f1_0, const doub
           }
         }
       }
-      block_partials<32, 1>(s, mx, group_row(g, c.red), c.scratch);
+      block_partials(s, 32, mx, 1, group_row(g, c.red), c.scratch);
       const double* part = g.red_part + (size_t)g.parity * g.G * g.redk;
       g.parity ^= 1;
       if (!group_sync(g)) return -2;
@@ -1157,15 +1223,6 @@ __device__ __noinline__ int lb_cauchy(LbCtxT<SY>& c) {
 // ---------------------------------------------------------------------------
 // formk (lbfgsb.f:1848-2172) from Gram sums over the free/active sets
 // ---------------------------------------------------------------------------
-// One FP64 tensor-core product D = A B + D of an 8x4 by 4x8 tile
-// (mma.sync m8n8k4 f64).  Lane l holds A[l/4][l%4], B[l%4][l/4] and
-// D[l/4][2(l%4) + {0,1}].
-__device__ __forceinline__ void dmma_884(double (&d)[2], double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
-               : "+d"(d[0]), "+d"(d[1])
-               : "d"(a), "d"(b));
-}
-
 template <typename SY>
 __device__ __noinline__ int lb_formk(LbCtxT<SY>& c) {
   LbState& S = *c.S;
@@ -1244,53 +1301,34 @@ __device__ __noinline__ int lb_formk(LbCtxT<SY>& c) {
   }
   if (!group_combine(*c.g, E, E, c.red, c.scratch)) return -9;
   int info = 0;
-  if (threadIdx.x == 0) {
-    auto sym = [&](int base, int a, int b) {  // symmetric block entry
-      if (a > b) {
-        const int t = a;
-        a = b;
-        b = t;
-      }
-      int e = 0;
-      for (int q = 0; q < a; ++q) e += m - q;
-      return c.red[base + e + (b - a)];
+  if (threadIdx.x < 32) {
+    // lane j < col: column j of the Y block; lane col + j: of the S block
+    const int col2 = 2 * col, jl = lane < col ? lane : lane - col;
+    const int pj = lane < col2 ? lptr(S, m, jl) : 0;
+    auto sym = [&](int base, int a, int b) {  // entry of a symmetric block
+      const int lo = min(a, b), hi = max(a, b);
+      return c.red[base + lo * m - lo * (lo - 1) / 2 + (hi - lo)];
     };
-    auto fyy = [&](int a, int b) { return sym(0, a, b); };
-    auto ass = [&](int a, int b) { return sym(nsym, a, b); };
-    auto fsy = [&](int a, int b) { return c.red[2 * nsym + a * m + b]; };
-    auto asy = [&](int a, int b) { return c.red[2 * nsym + m * m + a * m + b]; };
-    const int m2 = 2 * m;
-#define WN(i, j) S.wn[((i)-1) + m2 * ((j)-1)]
-#define SY(i, j) S.sy[((i)-1) + m * ((j)-1)]
-    for (int iy = 1; iy <= col; ++iy) {
-      const int is = col + iy;
-      const int pi = lptr(S, m, iy - 1);
-      for (int jy = 1; jy <= iy; ++jy) {
-        const int js = col + jy;
-        const int pjj = lptr(S, m, jy - 1);
-        WN(jy, iy) = fyy(pi, pjj) / S.theta;
-        WN(js, is) = ass(pi, pjj) * S.theta;
+#pragma unroll 1
+    for (int i = 0; i <= lane && lane < col2; ++i) {
+      const int pi = lptr(S, m, i < col ? i : i - col);
+      double v;
+      if (lane < col) {
+        v = sym(0, pj, pi) / S.theta;
+        if (i == lane) v += S.sy[i + m * i];
+      } else if (i < col) {
+        // wn1(m + j, i): minus the active sum before j, the free sum from there
+        v = i < jl ? -c.red[2 * nsym + m * m + pj * m + pi] : c.red[2 * nsym + pj * m + pi];
+      } else {
+        v = sym(nsym, pj, pi) * S.theta;
       }
-      // wn1(m+iy, jy): active sum for iy > jy, free sum for iy <= jy
-      for (int jy = 1; jy <= iy - 1; ++jy) WN(jy, is) = -asy(pi, lptr(S, m, jy - 1));
-      for (int jy = iy; jy <= col; ++jy) WN(jy, is) = fsy(pi, lptr(S, m, jy - 1));
-      WN(iy, iy) = WN(iy, iy) + SY(iy, iy);
+      S.wn[i + 2 * m * lane] = v;
     }
-    if (d_chol_upper(S.wn, m2, col)) {
-      info = -1;
-    } else {
-      const int col2 = 2 * col;
-      for (int js = col + 1; js <= col2; ++js) d_tri_solve(S.wn, m2, col, &WN(1, js), true);
-      for (int is = col + 1; is <= col2; ++is)
-        for (int js = is; js <= col2; ++js) {
-          double s = 0;
-          for (int k = 1; k <= col; ++k) s += WN(k, is) * WN(k, js);
-          WN(is, js) = WN(is, js) + s;
-        }
-      if (d_chol_upper(&WN(col + 1, col + 1), m2, col)) info = -2;
-    }
-#undef WN
-#undef SY
+    __syncwarp();
+    info = warp_factor(S.wn, 2 * m, col2, col, S.rwn);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
     c.red[0] = info;
   }
   __syncthreads();
@@ -1313,12 +1351,16 @@ __device__ __noinline__ int lb_cmprlb_subsm(LbCtxT<SY>& c) {
   __shared__ double a_s[2 * SMILI_MAXM_DEV], wv_s[2 * SMILI_MAXM_DEV];
   __shared__ int err_s;
   const bool unc = !S.cnstnd && col > 0;
-  if (threadIdx.x == 0) {
-    err_s = 0;
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x;
+    if (lane == 0) err_s = 0;
     if (!unc) {
-      double a[2 * SMILI_MAXM_DEV];
-      if (d_bmv(S, m, col, S.wa + 2 * m, a)) err_s = -8;
-      for (int j = 0; j < col2; ++j) a_s[j] = a[j];
+      double y = lane < col ? S.wa[2 * m + lane] : 0.0, s = lane < col ? S.wa[2 * m + col + lane] : 0.0;
+      if (!warp_bmv(S, m, col, y, s) && lane == 0) err_s = -8;
+      if (lane < col) {
+        a_s[lane] = y;
+        a_s[col + lane] = s;
+      }
     }
   }
   __syncthreads();
@@ -1371,20 +1413,15 @@ __device__ __noinline__ int lb_cmprlb_subsm(LbCtxT<SY>& c) {
   for (int j = 2 * SMILI_MAXM_DEV; j < 16; ++j) acc[j] = 0.0;
   const double none[1] = {0.0};
   if (!lb_reduce(c, acc, none)) return -9;
-  if (threadIdx.x == 0) {
-    double wv[2 * SMILI_MAXM_DEV];
-    for (int j = 0; j < col; ++j) {
-      wv[j] = c.red[j];
-      wv[col + j] = theta * c.red[SMILI_MAXM_DEV + j];
-    }
-    const int m2 = 2 * m;
-    if (d_tri_solve(S.wn, m2, col2, wv, true)) {
-      err_s = -1;
-    } else {
-      for (int j = 0; j < col; ++j) wv[j] = -wv[j];
-      if (d_tri_solve(S.wn, m2, col2, wv, false)) err_s = -1;
-    }
-    for (int j = 0; j < col2; ++j) wv_s[j] = wv[j];
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x;
+    bool ok, ok2;
+    double w = 0.0;
+    if (lane < col2) w = lane < col ? c.red[lane] : theta * c.red[SMILI_MAXM_DEV + lane - col];
+    w = warp_tri_solve(S.wn, 2 * m, col2, S.rwn, w, true, ok);
+    w = warp_tri_solve(S.wn, 2 * m, col2, S.rwn, lane < col ? -w : w, false, ok2);
+    if (!ok && lane == 0) err_s = -1;
+    if (lane < col2) wv_s[lane] = w;
   }
   __syncthreads();
   if (err_s) return err_s;
@@ -1793,29 +1830,37 @@ __device__ __noinline__ int lb_after_fg(LbCtxT<SY>& c, double f, double gd_fg, d
     for (int j = 13; j < 16; ++j) acc[j] = 0.0;
     const double none[1] = {0.0};
     if (!lb_reduce(c, acc, none)) return lb_abort(c);
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < 32) {
       const double rr = c.red[12], dr = S.wa[0];
-      const int col = S.col;
-#define SY(i, j) S.sy[((i)-1) + m * ((j)-1)]
-#define SS(i, j) S.ss[((i)-1) + m * ((j)-1)]
-      S.theta = rr / dr;
-      if (S.iupdat > m) {
-        for (int j = 1; j <= col - 1; ++j) {
-          for (int k = 0; k < j; ++k) SS(1 + k, j) = SS(2 + k, j + 1);
-          for (int k = 0; k < col - j; ++k) SY(j + k, j) = SY(j + 1 + k, j + 1);
+      const int col = S.col, lane = threadIdx.x;
+      // shift the matrices when the oldest pair leaves, then the new row and column
+      constexpr int NE = (SMILI_MAXM_DEV * SMILI_MAXM_DEV + 31) / 32;
+      double ns[NE], ny[NE];
+#pragma unroll
+      for (int q = 0; q < NE; ++q) {
+        const int e = lane + 32 * q, i = e % col, j = e / col;
+        if (e >= col * col) continue;
+        const int sh = (S.iupdat > m && i < col - 1 && j < col - 1) ? 1 + m : 0;
+        ns[q] = S.ss[i + m * j + sh];
+        ny[q] = S.sy[i + m * j + sh];
+        if (j == col - 1 && i < col - 1) ns[q] = c.red[SMILI_MAXM_DEV + (S.head - 1 + i) % m];
+        if (i == col - 1 && j < col - 1) ny[q] = c.red[(S.head - 1 + j) % m];
+        if (i == col - 1 && j == col - 1) {
+          ns[q] = (S.stp == 1.0) ? S.dtd : S.stp * S.stp * S.dtd;
+          ny[q] = dr;
         }
       }
-      int pointr = S.head;
-      for (int j = 1; j <= col - 1; ++j) {
-        SY(col, j) = c.red[pointr - 1];
-        SS(j, col) = c.red[SMILI_MAXM_DEV + (pointr - 1)];
-        pointr = pointr % m + 1;
+      __syncwarp();
+#pragma unroll
+      for (int q = 0; q < NE; ++q) {
+        const int e = lane + 32 * q, i = e % col, j = e / col;
+        if (e >= col * col) continue;
+        if (i <= j) S.ss[i + m * j] = ns[q];
+        if (i >= j) S.sy[i + m * j] = ny[q];
       }
-      SS(col, col) = (S.stp == 1.0) ? S.dtd : S.stp * S.stp * S.dtd;
-      SY(col, col) = dr;
-#undef SY
-#undef SS
-      if (d_formt(S, m) != 0) reset_memory(S);
+      if (lane == 0) S.theta = rr / dr;
+      __syncwarp();
+      if (warp_formt(S, m) != 0 && lane == 0) reset_memory(S);
     }
     __syncthreads();
   }

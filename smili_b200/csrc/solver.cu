@@ -61,11 +61,8 @@ struct BatchArgs {
 // ---------------------------------------------------------------------------
 // group-wide sums of the ten image moments into red[0..10)
 __device__ bool reduce_moments(GroupCtx& g, const double (&mom)[10], double* red, double* scratch) {
-  double s[16];
-#pragma unroll
-  for (int k = 0; k < 16; ++k) s[k] = k < 10 ? mom[k] : 0.0;
   const double none[1] = {0.0};
-  return group_reduce<16, 1>(g, s, none, red, scratch);
+  return group_reduce(g, mom, 10, none, 1, red, scratch);
 }
 
 // Stages F1-F8 of one evaluation of a 2D problem by group g: per-thread
@@ -164,7 +161,7 @@ __device__ bool group_fg(FgCtx<R>& fc, GroupCtx& g, LbCtxT<R>& lc, double* red, 
   if (mode == MODE_T1 || mode == MODE_T2) return true;
   const double mx[1] = {acc[13]};
   acc[13] = 0.0;
-  if (!group_reduce<16, 1>(g, acc, mx, red, scratch)) return false;
+  if (!group_reduce(g, acc, 16, mx, 1, red, scratch)) return false;
   double r[14];
   for (int k = 0; k < 13; ++k) r[k] = red[k];
   r[13] = red[16];
@@ -267,7 +264,7 @@ __device__ bool movie_fg(FgCtx<R>& fc, GroupCtx& g, GroupCtx& gs, int sub, int n
   }
   const double mx[1] = {acc[13]};
   acc[13] = 0.0;
-  if (!group_reduce<16, 1>(g, acc, mx, red, scratch)) return false;
+  if (!group_reduce(g, acc, 16, mx, 1, red, scratch)) return false;
   double r[16];
   for (int k = 0; k < 16; ++k) r[k] = red[k];
   r[13] = red[16];
