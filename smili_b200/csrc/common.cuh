@@ -155,6 +155,23 @@ __device__ __forceinline__ double warp_max(double a) {
   return __longlong_as_double((long long)((m & top) ? (m & ~top) : ~m));
 }
 
+// Sum (or maximum) of one value over the rows r0, r0 + step, ... < G, D loads
+// in flight.
+template <int D>
+__device__ __forceinline__ double fold_rows(const double* col, int r0, int step, int G, int redk, bool sum) {
+  const double none = sum ? 0.0 : -INFINITY;
+  double a = none;
+#pragma unroll 1
+  for (int r = r0; r < G; r += D * step) {
+    double v[D];
+#pragma unroll
+    for (int q = 0; q < D; ++q) v[q] = r + q * step < G ? __ldcg(col + (size_t)(r + q * step) * redk) : none;
+#pragma unroll
+    for (int q = 0; q < D; ++q) a = sum ? a + v[q] : fmax(a, v[q]);
+  }
+  return a;
+}
+
 // Second half of a group reduction: every CTA has its partials (ns sums,
 // then maxima, K in all) in its row of the current half of red_part, or in
 // out when G == 1.  After the barrier each CTA combines all rows itself, in
@@ -176,11 +193,9 @@ __device__ __noinline__ bool group_combine(GroupCtx& g, int K, int ns, double* o
   const bool sum = k < ns;
   double a = sum ? 0.0 : -INFINITY;
   if (k < K) {
-#pragma unroll 4
-    for (int r = sl; r < g.G; r += S) {
-      const double v = __ldcg(part + (size_t)r * g.redk + k);
-      a = sum ? a + v : fmax(a, v);
-    }
+    const double* col = part + k;
+    if (g.G <= 4 * S) a = fold_rows<4>(col, sl, S, g.G, g.redk, sum);  // one trip, little code
+    else a = fold_rows<8>(col, sl, S, g.G, g.redk, sum);
   }
   scratch[threadIdx.x] = a;
   __syncthreads();

@@ -751,11 +751,18 @@ __device__ __noinline__ int cauchy_search(LbCtxT<SY>& c, double f1_0, const doub
         const int k = threadIdx.x & 31, sl = threadIdx.x >> 5, S_ = T >> 5;
         const bool sum = k < 31;
         double pre = 0.0, tot = 0.0;
-#pragma unroll 4
-        for (int r = sl; r < g.G; r += S_) {
-          const double v = __ldcg(part + (size_t)r * g.redk + (sum ? k : 32));
-          tot = sum ? tot + v : fmax(tot, v);
-          if (r < g.rank) pre = sum ? pre + v : fmax(pre, v);
+        constexpr int D = 4;  // rows in flight
+        for (int r = sl; r < g.G; r += D * S_) {
+          double v[D];
+#pragma unroll
+          for (int q = 0; q < D; ++q)
+            v[q] = r + q * S_ < g.G ? __ldcg(part + (size_t)(r + q * S_) * g.redk + (sum ? k : 32)) : 0.0;
+#pragma unroll
+          for (int q = 0; q < D; ++q) {
+            const double b = r + q * S_ < g.rank ? v[q] : 0.0;
+            tot = sum ? tot + v[q] : fmax(tot, v[q]);
+            pre = sum ? pre + b : fmax(pre, b);
+          }
         }
         sm.a_s[threadIdx.x] = pre;
         sm.b_s[threadIdx.x] = tot;
@@ -774,25 +781,35 @@ __device__ __noinline__ int cauchy_search(LbCtxT<SY>& c, double f1_0, const doub
         __syncthreads();
       }
       if (r0 > 0 && r0 < r1) {
-        if (threadIdx.x < 12) {
-          sm.P[threadIdx.x] = p0[threadIdx.x] - sm.pre[1 + threadIdx.x];
-          sm.Q[threadIdx.x] = sm.pre[13 + threadIdx.x];
-        }
-        if (threadIdx.x == 0) {
+        if (threadIdx.x < 32) {  // segment_dtm, a row of M per lane
           const double D = -f1_0 - sm.pre[0], t = sm.pre[31];
-          double Pk[12], ck[12];
-#pragma unroll
-          for (int j = 0; j < 12; ++j) {
-            Pk[j] = p0[j] - sm.pre[1 + j];
-            ck[j] = t * Pk[j] + sm.pre[13 + j];
+          double Pl = 0.0, cl = 0.0, mp = 0.0;
+          if (lane < 12) {
+            Pl = p0[lane] - sm.pre[1 + lane];
+            cl = t * Pl + sm.pre[13 + lane];
+            sm.P[lane] = Pl;
+            sm.Q[lane] = sm.pre[13 + lane];
           }
-          sm.st[0] = D;
-          sm.st[1] = t;
-          sm.st[2] = segment_dtm(sm.Mm, D, t, Pk, ck, theta, f2_floor);
-          // every breakpoint before these buckets, whatever its index
-          const u128 ckk = comp_key((unsigned long long)__double_as_longlong(t), -1);
-          bnd_hi_s = (unsigned long long)(ckk >> 64);
-          bnd_lo_s = (unsigned long long)ckk;
+#pragma unroll 1
+          for (int j = 0; j < 12; ++j) {
+            const double pj_ = __shfl_sync(0xffffffffu, Pl, j);
+            if (lane < 12) mp += sm.Mm[lane * 12 + j] * pj_;
+          }
+          double cMp = cl * mp, pMp = Pl * mp;
+#pragma unroll
+          for (int q = 8; q >= 1; q >>= 1) {
+            cMp += __shfl_xor_sync(0xffffffffu, cMp, q);
+            pMp += __shfl_xor_sync(0xffffffffu, pMp, q);
+          }
+          if (lane == 0) {
+            sm.st[0] = D;
+            sm.st[1] = t;
+            sm.st[2] = (D - theta * t * D + cMp) / fmax(f2_floor, theta * D - pMp);
+            // every breakpoint before these buckets, whatever its index
+            const u128 ckk = comp_key((unsigned long long)__double_as_longlong(t), -1);
+            bnd_hi_s = (unsigned long long)(ckk >> 64);
+            bnd_lo_s = (unsigned long long)ckk;
+          }
         }
       }
       pf.mark(PR_C_GATHER);
@@ -1030,49 +1047,74 @@ __device__ __noinline__ int lb_cauchy(LbCtxT<SY>& c) {
     const int nb = cauchy_buckets(n);
     for (int i = c.g->rank * blockDim.x + threadIdx.x; i < 2 * SMILI_NBUCKET_MAX; i += c.g->G * blockDim.x)
       ghist[i] = 0;
-    for (int i = c.lo + threadIdx.x; i < c.hi; i += blockDim.x) {
-      const double neggi = -c.gv[i];
-      int iw = c.iwh[i];
-      double tl = 0.0;
-      if (iw != 3 && iw != -1) {
-        tl = c.x[i];  // x - l with l = 0 (nbd = 1)
-        const bool xlower = tl <= 0.0;
-        iw = 0;
-        if (xlower) {
-          if (neggi <= 0.0) iw = 1;
-        } else {
-          if (fabs(neggi) <= 0.0) iw = -3;
-        }
-        c.iwh[i] = (signed char)iw;
+    // U elements of a thread at a time, all loads of a step before its stores
+    // (which may alias them for the compiler): the pass is bound by the latency
+    // of its two dependent loads per step
+    constexpr int U = sizeof(SY) == 8 ? 2 : 1;
+    const int bd = blockDim.x;
+    for (int i0 = c.lo + threadIdx.x; i0 < c.hi; i0 += U * bd) {
+      double ng[U], xv[U];
+      int iw[U];
+      bool in[U], mv[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int i = i0 + u * bd;
+        in[u] = i < c.hi;
+        ng[u] = in[u] ? -c.gv[i] : 0.0;
+        xv[u] = in[u] ? c.x[i] : 0.0;
+        iw[u] = in[u] ? c.iwh[i] : 3;
       }
-      unsigned long long key = ~0ULL;
-      if (iw != 0 && iw != -1) {
-        c.d[i] = 0.0;
-      } else {
-        c.d[i] = neggi;
-        f1a -= neggi * neggi;
+      bool set[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        set[u] = in[u] && iw[u] != 3 && iw[u] != -1;
+        if (set[u]) {
+          // x - l with l = 0 (nbd = 1)
+          iw[u] = xv[u] <= 0.0 ? (ng[u] <= 0.0 ? 1 : 0) : (fabs(ng[u]) <= 0.0 ? -3 : 0);
+        }
+        mv[u] = in[u] && (iw[u] == 0 || iw[u] == -1);
+      }
+      SY wy[U][SMILI_MAXM_DEV], ws[U][SMILI_MAXM_DEV];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
 #pragma unroll
         for (int j = 0; j < SMILI_MAXM_DEV; ++j) {
-          if (j < col) {
-            py[j] += ld_wy(c, (size_t)pj[j] * n + i) * neggi;
-            ps[j] += ld_ws(c, (size_t)pj[j] * n + i) * neggi;
+          const bool l = mv[u] && j < col;
+          wy[u][j] = l ? c.wy[(size_t)pj[j] * n + i0 + u * bd] : (SY)0;
+          ws[u][j] = l ? c.ws[(size_t)pj[j] * n + i0 + u * bd] : (SY)0;
+        }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (!in[u]) continue;
+        const int i = i0 + u * bd;
+        unsigned long long key = ~0ULL;
+        if (mv[u]) {
+          f1a -= ng[u] * ng[u];
+#pragma unroll
+          for (int j = 0; j < SMILI_MAXM_DEV; ++j) {
+            if (j < col) {
+              py[j] += (double)wy[u][j] * ng[u];
+              ps[j] += (double)ws[u][j] * ng[u];
+            }
+          }
+          if (nonneg && ng[u] < 0.0) {
+            const double tb = (set[u] ? xv[u] : 0.0) / (-ng[u]);
+            nbr += 1.0;
+            tmn = fmin(tmn, tb);
+            tmx = fmax(tmx, tb);
+            key = (unsigned long long)__double_as_longlong(tb);
+            const double kh = (double)((int)(key >> 32) - 0x3ff00000);
+            k1 += kh;
+            k2 += kh * kh;
+          } else {
+            nfr = 1.0;
+            if (fabs(ng[u]) > 0.0) notb = 1.0;
           }
         }
-        if (nonneg && neggi < 0.0) {
-          const double tb = tl / (-neggi);
-          nbr += 1.0;
-          tmn = fmin(tmn, tb);
-          tmx = fmax(tmx, tb);
-          key = (unsigned long long)__double_as_longlong(tb);
-          const double kh = (double)((int)(key >> 32) - 0x3ff00000);
-          k1 += kh;
-          k2 += kh * kh;
-        } else {
-          nfr = 1.0;
-          if (fabs(neggi) > 0.0) notb = 1.0;
-        }
+        if (set[u]) c.iwh[i] = (signed char)iw[u];
+        c.d[i] = mv[u] ? ng[u] : 0.0;
+        c.bkey[i] = key;
       }
-      c.bkey[i] = key;
     }
     double acc[16];
 #pragma unroll
@@ -1113,7 +1155,7 @@ __device__ __noinline__ int lb_cauchy(LbCtxT<SY>& c) {
       int shift = 0;
       if (nbreak > 0) {
         // bucket the breakpoints: histogram, then scatter in bucket order
-        while (shift < 63 && ((kmax - kmin) >> shift) >= (unsigned long long)nb) ++shift;
+        shift = max(0, 32 + __clz(nb) - __clzll((long long)(kmax - kmin)) + 1);  // (kmax - kmin) >> shift < nb
         for (int i = c.lo + threadIdx.x; i < c.hi; i += blockDim.x) {
           const unsigned long long k = c.bkey[i];
           if (k != ~0ULL) atomicAdd(&ghist[bucket_of(k, kmin, shift, nb)], 1);
@@ -1180,25 +1222,43 @@ __device__ __noinline__ int lb_cauchy(LbCtxT<SY>& c) {
                    (u128)(unsigned long long)__double_as_longlong(cr_s[CR_BLO]);
   const double tsum = cr_s[CR_TSUM];
   const bool count_moves = S.iter > 0 && S.cnstnd;
-  for (int i = c.lo + threadIdx.x; i < c.hi; i += blockDim.x) {
-    if (mode == CM_BOUNDARY || mode == CM_NONE_FIXED) {
-      const unsigned long long k = c.bkey[i];
-      if (mode == CM_BOUNDARY && k != ~0ULL && comp_key(k, i) <= bnd) {
+  constexpr int UA = 2;  // elements in flight per thread
+  const int bda = blockDim.x;
+  const bool apply = mode == CM_BOUNDARY || mode == CM_NONE_FIXED;
+  for (int i0 = c.lo + threadIdx.x; i0 < c.hi; i0 += UA * bda) {
+    unsigned long long k[UA];
+    double xv[UA], dv[UA];
+    int iw[UA], fo[UA];
+#pragma unroll
+    for (int u = 0; u < UA; ++u) {
+      const int i = i0 + u * bda;
+      const bool in = i < c.hi;
+      k[u] = in && mode == CM_BOUNDARY ? c.bkey[i] : ~0ULL;
+      xv[u] = in && apply ? c.x[i] : 0.0;
+      dv[u] = in && apply ? c.d[i] : 0.0;
+      iw[u] = in ? c.iwh[i] : 1;
+      fo[u] = in ? c.freef[i] : 0;
+    }
+#pragma unroll
+    for (int u = 0; u < UA; ++u) {
+      const int i = i0 + u * bda;
+      if (i >= c.hi) continue;
+      if (k[u] != ~0ULL && comp_key(k[u], i) <= bnd) {
         c.z[i] = 0.0;  // lower bound (d < 0 at every breakpoint)
         c.iwh[i] = 1;
+        iw[u] = 1;
         c.d[i] = 0.0;
-      } else {
-        c.z[i] = c.x[i] + tsum * c.d[i];
+      } else if (apply) {
+        c.z[i] = xv[u] + tsum * dv[u];
       }
+      const int fnew = iw[u] <= 0;
+      if (count_moves) {
+        if (fo[u] && !fnew) acc[2] += 1;
+        if (!fo[u] && fnew) acc[1] += 1;
+      }
+      c.freef[i] = (unsigned char)fnew;
+      acc[0] += fnew;
     }
-    const int fnew = c.iwh[i] <= 0;
-    const int fold_ = c.freef[i];
-    if (count_moves) {
-      if (fold_ && !fnew) acc[2] += 1;
-      if (!fold_ && fnew) acc[1] += 1;
-    }
-    c.freef[i] = (unsigned char)fnew;
-    acc[0] += fnew;
   }
   const double none[1] = {0.0};
   if (!lb_reduce(c, acc, none)) return -2;
@@ -1338,10 +1398,12 @@ __device__ __noinline__ int lb_formk(LbCtxT<SY>& c) {
 }
 
 // ---------------------------------------------------------------------------
-// cmprlb + subsm (lbfgsb.f:1720-1786, 2991-3346).  Returns 0 or an error.
+// cmprlb + subsm (lbfgsb.f:1720-1786, 2991-3346).  Returns 0 or an error;
+// ls_ready: d, t and the sums of lb_lnsrch_start are made (c.red: g.d, d.d,
+// iword, -stpmx).
 // ---------------------------------------------------------------------------
 template <typename SY>
-__device__ __noinline__ int lb_cmprlb_subsm(LbCtxT<SY>& c) {
+__device__ __noinline__ int lb_cmprlb_subsm(LbCtxT<SY>& c, bool& ls_ready) {
   LbState& S = *c.S;
   const ProbDesc& P = *c.P;
   const int m = c.m, n = c.n, col = S.col, col2 = 2 * col;
@@ -1425,8 +1487,11 @@ __device__ __noinline__ int lb_cmprlb_subsm(LbCtxT<SY>& c) {
   }
   __syncthreads();
   if (err_s) return err_s;
-  // d := (d + W wv) / theta on the free set, then project z + d
-  double iwd[1] = {0.0}, ddp[1] = {0.0};  // iword (max), dd_p (sum)
+  // d := (d + W wv) / theta on the free set, then project z + d.  The pass also
+  // makes the line search's first step out of the result, which stands unless
+  // a backtrack follows: d = z - x, t = x, their sums and the largest step
+  const bool bounded_steps = S.cnstnd && S.iter > 0 && P.nonneg;
+  double mx2[2] = {0.0, -1.0e10}, sm2[2] = {0.0, 0.0};  // iword, -stpmx (maxima); g.d = dd_p, d.d (sums)
   double wq[SMILI_MAXM_DEV], wr[SMILI_MAXM_DEV];
 #pragma unroll
   for (int j = 0; j < SMILI_MAXM_DEV; ++j) {
@@ -1460,20 +1525,31 @@ __device__ __noinline__ int lb_cmprlb_subsm(LbCtxT<SY>& c) {
       c.r[i] = ri;
       if (P.nonneg) {
         zn = fmax(0.0, zi + ri);
-        if (zn == 0.0) iwd[0] = 1.0;
+        if (zn == 0.0) mx2[0] = 1.0;
       } else {
         zn = zi + ri;
       }
       c.z[i] = zn;
     }
-    ddp[0] += (zn - xv) * gvi;
+    const double di = zn - xv;
+    c.d[i] = di;
+    c.t[i] = xv;
+    sm2[0] += di * gvi;
+    sm2[1] += di * di;
+    if (bounded_steps && di < 0.0) {
+      const double a2 = -xv;  // l - x with l = 0
+      mx2[1] = fmax(mx2[1], a2 >= 0.0 ? 0.0 : -(a2 / di));
+    }
   }
-  if (!lb_reduce(c, ddp, iwd)) return -9;
-  const int iword = c.red[1] > 0.5;
+  if (!lb_reduce(c, sm2, mx2)) return -9;
+  const int iword = c.red[2] > 0.5;
   const double dd_p = c.red[0];
   if (threadIdx.x == 0) S.iword = iword;
   __syncthreads();
-  if (!iword || dd_p <= 0.0) return 0;
+  if (!iword || dd_p <= 0.0) {
+    ls_ready = true;
+    return 0;
+  }
   // backtrack: z = xp, alpha = largest feasible step along d (lbfgsb.f:3270-3330)
   double zero[1] = {0.0}, acc3[1] = {-1.0};  // minima as maxima of the negated values
   for (int i = c.lo + threadIdx.x; i < c.hi; i += blockDim.x) {
@@ -1532,19 +1608,36 @@ __device__ int lb_abort(LbCtxT<SY>& c) {
   return LB_RET_DONE;
 }
 
-// x = t + stp d, or z when stp == 1 (lnsrlb, lbfgsb.f:2562-2570)
+// x = t + stp d, or z when stp == 1 (lnsrlb, lbfgsb.f:2562-2570); at the start
+// of a line search also r = g
 template <typename SY>
-__device__ void lb_set_trial_x(LbCtxT<SY>& c) {
+__device__ void lb_set_trial_x(LbCtxT<SY>& c, bool start) {
   const double stp = c.S->stp;
-  for (int i = c.lo + threadIdx.x; i < c.hi; i += blockDim.x)
-    c.x[i] = (stp == 1.0) ? c.z[i] : stp * c.d[i] + c.t[i];
+  constexpr int U = 4;
+  const int bd = blockDim.x;
+  for (int i0 = c.lo + threadIdx.x; i0 < c.hi; i0 += U * bd) {
+    double v[U], gi[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = i0 + u * bd;
+      v[u] = i >= c.hi ? 0.0 : (stp == 1.0) ? c.z[i] : stp * c.d[i] + c.t[i];
+      gi[u] = start && i < c.hi ? c.gv[i] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = i0 + u * bd;
+      if (i >= c.hi) continue;
+      c.x[i] = v[u];
+      if (start) c.r[i] = gi[u];
+    }
+  }
   __syncthreads();
 }
 
 // "info /= 0 or iback >= 20" branch of mainlb (lbfgsb.f:888-920)
 template <typename SY>
-__device__ int lb_ls_fail(LbCtxT<SY>& c) {
-  for (int i = c.lo + threadIdx.x; i < c.hi; i += blockDim.x) {
+__device__ int lb_ls_fail(LbCtxT<SY>& c, bool restore) {
+  for (int i = c.lo + threadIdx.x; restore && i < c.hi; i += blockDim.x) {
     c.x[i] = c.t[i];
     c.gv[i] = c.r[i];
   }
@@ -1577,36 +1670,51 @@ __device__ int lb_ls_fail(LbCtxT<SY>& c) {
 
 // label 555 + the first part of lnsrlb (lbfgsb.f:2480-2575)
 template <typename SY>
-__device__ __noinline__ int lb_lnsrch_start(LbCtxT<SY>& c) {
+__device__ __noinline__ int lb_lnsrch_start(LbCtxT<SY>& c, bool ready) {
   LbState& S = *c.S;
   const bool bounded_steps = S.cnstnd && S.iter > 0;
-  double acc[2] = {0.0, 0.0}, stm[1] = {-1.0e10};  // dtd, gd; -stpmx (max)
-  for (int i = c.lo + threadIdx.x; i < c.hi; i += blockDim.x) {
-    const double di = c.z[i] - c.x[i];
-    const double xi = c.x[i], gi = c.gv[i];
-    c.d[i] = di;
-    c.t[i] = xi;
-    c.r[i] = gi;
-    acc[0] += di * di;
-    acc[1] += gi * di;
-    if (bounded_steps && c.P->nonneg && di < 0.0) {
-      const double a2 = -xi;  // l - x with l = 0
-      stm[0] = fmax(stm[0], a2 >= 0.0 ? 0.0 : -(a2 / di));
+  // gd, dtd; (unused), -stpmx (maxima): the places lb_cmprlb_subsm leaves them in
+  double acc[2] = {0.0, 0.0}, stm[2] = {0.0, -1.0e10};
+  constexpr int U = 2;  // elements in flight per thread
+  const int bd = blockDim.x;
+  for (int i0 = ready ? c.hi : c.lo + threadIdx.x; i0 < c.hi; i0 += U * bd) {
+    double zv[U], xv[U], gi[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = i0 + u * bd;
+      const bool in = i < c.hi;
+      zv[u] = in ? c.z[i] : 0.0;
+      xv[u] = in ? c.x[i] : 0.0;
+      gi[u] = in ? c.gv[i] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = i0 + u * bd;
+      if (i >= c.hi) continue;
+      const double di = zv[u] - xv[u];
+      c.d[i] = di;
+      c.t[i] = xv[u];
+      acc[1] += di * di;
+      acc[0] += gi[u] * di;
+      if (bounded_steps && c.P->nonneg && di < 0.0) {
+        const double a2 = -xv[u];  // l - x with l = 0
+        stm[1] = fmax(stm[1], a2 >= 0.0 ? 0.0 : -(a2 / di));
+      }
     }
   }
-  if (!lb_reduce(c, acc, stm)) return LB_RET_ABORT;
+  if (!ready && !lb_reduce(c, acc, stm)) return LB_RET_ABORT;
   __shared__ int act_s;
   if (threadIdx.x == 0) {
-    S.dtd = c.red[0];
+    S.dtd = c.red[1];
     S.dnorm = sqrt(S.dtd);
     S.stpmx = 1.0e10;
-    if (S.cnstnd) S.stpmx = (S.iter == 0) ? 1.0 : -c.red[2];
+    if (S.cnstnd) S.stpmx = (S.iter == 0) ? 1.0 : -c.red[3];
     S.stp = (S.iter == 0 && !S.boxed) ? fmin(1.0 / S.dnorm, S.stpmx) : 1.0;
     S.fold = S.f;
     S.ifun = 0;
     S.iback = 0;
     S.csave = CS_START;
-    S.gd = c.red[1];
+    S.gd = c.red[0];
     S.gdold = S.gd;
     if (S.gd >= 0.0) {
       S.info = -4;  // ascent direction in projection
@@ -1624,10 +1732,10 @@ __device__ __noinline__ int lb_lnsrch_start(LbCtxT<SY>& c) {
   const int act = act_s;
   __syncthreads();
   if (!act) {
-    const int r = lb_ls_fail(c);
+    const int r = lb_ls_fail(c, false);  // x and g have not changed yet
     return r == LB_RET_RESTART ? LB_RET_RESTART : LB_RET_DONE;
   }
-  lb_set_trial_x(c);
+  lb_set_trial_x(c, true);
   if (threadIdx.x == 0) S.task = LB_TASK_FG_LN;
   __syncthreads();
   return LB_RET_FG;
@@ -1660,6 +1768,7 @@ __device__ __noinline__ int lb_iter(LbCtxT<SY>& c) {
       if (threadIdx.x == 0) S.nintol += S.nseg;
       __syncthreads();
     }
+    bool ls_ready = false;
     if (S.nfree != 0 && S.col != 0) {
       if (S.wrk) {
         c.prof->mark(PR_LB_POST);
@@ -1673,7 +1782,7 @@ __device__ __noinline__ int lb_iter(LbCtxT<SY>& c) {
         }
       }
       c.prof->mark(PR_LB_POST);
-      const int rc = lb_cmprlb_subsm(c);
+      const int rc = lb_cmprlb_subsm(c, ls_ready);
       c.prof->mark(PR_SUBSM);
       if (rc == -9) return lb_abort(c);
       if (rc != 0) {
@@ -1683,7 +1792,7 @@ __device__ __noinline__ int lb_iter(LbCtxT<SY>& c) {
       }
     }
     c.prof->mark(PR_LB_POST);
-    const int r = lb_lnsrch_start(c);
+    const int r = lb_lnsrch_start(c, ls_ready);
     c.prof->mark(PR_LNSRCH);
     if (r == LB_RET_ABORT) return lb_abort(c);
     if (r == LB_RET_RESTART) continue;
@@ -1737,11 +1846,11 @@ __device__ __noinline__ int lb_after_fg(LbCtxT<SY>& c, double f, double gd_fg, d
   const int act = act_s;
   __syncthreads();
   if (act == 1) {
-    lb_set_trial_x(c);
+    lb_set_trial_x(c, false);
     return LB_RET_FG;
   }
   if (act == 2) {
-    const int r = lb_ls_fail(c);
+    const int r = lb_ls_fail(c, true);
     return r == LB_RET_RESTART ? lb_iter(c) : LB_RET_DONE;
   }
   // NEW_X: iteration finished (lbfgsb.f:931-944), driver test, label 777
@@ -1804,20 +1913,39 @@ __device__ __noinline__ int lb_after_fg(LbCtxT<SY>& c, double f, double gd_fg, d
     double rr_acc = 0.0, ay[SMILI_MAXM_DEV], as[SMILI_MAXM_DEV];
 #pragma unroll
     for (int j = 0; j < SMILI_MAXM_DEV; ++j) ay[j] = as[j] = 0.0;
-    for (int i = c.lo + threadIdx.x; i < c.hi; i += blockDim.x) {
-      const double ri = c.gv[i] - c.r[i];
-      const double di = c.d[i] * sc;
-      rr_acc += ri * ri;
+    constexpr int U = sizeof(SY) == 8 ? 2 : 1;  // elements in flight per thread
+    const int bd = blockDim.x;
+    for (int i0 = c.lo + threadIdx.x; i0 < c.hi; i0 += U * bd) {
+      double ri[U], di[U];
+      SY wy[U][SMILI_MAXM_DEV], ws[U][SMILI_MAXM_DEV];
 #pragma unroll
-      for (int j = 0; j < SMILI_MAXM_DEV; ++j) {
-        if (j < m) {
-          ay[j] += di * ld_wy(c, (size_t)j * n + i);
-          as[j] += ld_ws(c, (size_t)j * n + i) * di;
+      for (int u = 0; u < U; ++u) {
+        const int i = i0 + u * bd;
+        const bool in = i < c.hi;
+        ri[u] = in ? c.gv[i] - c.r[i] : 0.0;
+        di[u] = in ? c.d[i] * sc : 0.0;
+#pragma unroll
+        for (int j = 0; j < SMILI_MAXM_DEV; ++j) {
+          wy[u][j] = in && j < m ? c.wy[(size_t)j * n + i] : (SY)0;
+          ws[u][j] = in && j < m ? c.ws[(size_t)j * n + i] : (SY)0;
         }
       }
-      st_sy(c, (size_t)itail * n + i, di, ri);
-      c.r[i] = ri;
-      c.d[i] = di;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int i = i0 + u * bd;
+        if (i >= c.hi) continue;
+        rr_acc += ri[u] * ri[u];
+#pragma unroll
+        for (int j = 0; j < SMILI_MAXM_DEV; ++j) {
+          if (j < m) {
+            ay[j] += di[u] * (double)wy[u][j];
+            as[j] += (double)ws[u][j] * di[u];
+          }
+        }
+        st_sy(c, (size_t)itail * n + i, di[u], ri[u]);
+        c.r[i] = ri[u];
+        c.d[i] = di[u];
+      }
     }
     double acc[16];
 #pragma unroll

@@ -1527,7 +1527,8 @@ int finish_batch(smili_batch* b, std::vector<HostProb>& hps, const smili_options
       return cleanup(fail(SMILI_ERR_CUDA, "cudaStreamCreate failed"));
     b->own_stream = true;
   }
-  const cudaMemPool_t pool = device_pool(device);
+  // (buffers beyond what the pool keeps gain nothing from it)
+  const cudaMemPool_t pool = b->arena_bytes + aux <= kPoolKeep ? device_pool(device) : nullptr;
   b->pooled = pool != nullptr;
   auto alloc = [&](void** p, size_t n) {
     return (pool ? cudaMallocFromPoolAsync(p, n, pool, b->stream) : cudaMalloc(p, n)) == cudaSuccess;
