@@ -518,7 +518,10 @@ __global__ void __launch_bounds__(128) sum_partials_kernel(const float* partial,
 // access does not apply): each CTA owns 16 chains, all its threads bring
 // their pixels into shared memory (eight 16-byte loads in flight each, the
 // next ones while this batch is added), one thread per chain and channel
-// adds, and rank 0 gathers the chains over distributed shared memory.
+// adds, and rank 0 gathers the chains over distributed shared memory.  Nothing
+// may reach into rank 0's shared memory before its CTA has started: the cluster
+// barrier that says so is arrived at on entry and waited for before the stores,
+// behind the whole sum.
 // 24 channels of 32 x 128 x 128 pixels took 400 to 930 us with one CTA per
 // channel and 2-byte loads a row apart, 43 us with this and the mask.
 constexpr int BG_CTAS = 16, BG_THREADS = 512, BG_U = 8, BG_CHAINS = 256 / BG_CTAS;
@@ -542,6 +545,7 @@ __global__ void __launch_bounds__(BG_THREADS) bias_grad_kernel(const __nv_bfloat
   const size_t steps = (npix + 255) / 256;
   V v[BG_U], a[BG_U];
   memset(a, 0, sizeof(a));
+  cluster.barrier_arrive();  // this CTA runs
   auto pixel = [&](size_t k0, int u) { return (k0 + u * (BG_THREADS / BG_CHAINS) + lk) * 256 + rank * BG_CHAINS + lt; };
   auto load = [&](size_t k0) {
 #pragma unroll
@@ -582,6 +586,7 @@ __global__ void __launch_bounds__(BG_THREADS) bias_grad_kernel(const __nv_bfloat
     }
     __syncthreads();
   }
+  cluster.barrier_wait();  // and so do all others of the cluster
   if (threadIdx.x < BG_CHAINS * E)
     cluster.map_shared_rank(red, 0)[rank * BG_CHAINS * E + threadIdx.x] = s;
   cluster.sync();
