@@ -56,3 +56,19 @@ def test_other_ctas_shared_memory_is_reached_after_a_cluster_barrier():
         assert waits and waits[0] < remote[0], f"{name}: {kernel}"
         assert waits[-1] > remote[-1], f"{name}: {kernel}"
     assert seen
+
+
+def test_waits_before_warp_wide_instructions_answer_for_the_warp():
+    """A role that a whole warp plays issues .aligned instructions (tcgen05.ld,
+    elect, __syncwarp), so its bounded waits must end alike in every lane, also
+    when one runs out: only a role of a single lane may wait by itself."""
+    seen = 0
+    for name, kernel, body in _kernels():
+        if "tmem_ld16" not in body:
+            continue
+        seen += 1
+        for m in reversed(list(re.finditer(r"lane == 0\)\s*(?=\{)", body))):
+            block = _block(body, m.end())
+            body = body[:m.end()] + body[m.end():].replace(block, "", 1)
+        assert not re.search(r"\bmbar_wait\(", body), f"{name}: {kernel}"
+    assert seen
