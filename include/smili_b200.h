@@ -21,7 +21,8 @@ extern "C" {
 
 #define SMILI_OK 0
 #define SMILI_ERR_ARG (-1)         /* invalid size, index or option */
-#define SMILI_ERR_DATA (-2)        /* non-finite value or non-positive variance */
+#define SMILI_ERR_DATA (-2)        /* non-finite value, non-positive variance, or a uv coordinate
+                                    * beyond 2^30 cells of the fine grid (1e8 radians per pixel at 32 pixels) */
 #define SMILI_ERR_CUDA (-3)        /* CUDA runtime failure */
 #define SMILI_ERR_NODEV (-4)       /* no usable CUDA device */
 #define SMILI_ERR_TIMEOUT (-5)     /* a device-side wait gave up (solve aborted) */

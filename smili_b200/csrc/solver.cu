@@ -932,15 +932,20 @@ int pack_problem(const smili_imaging_args& a, int kind, int niter, int nonneg, i
   const bool bare = kind == PK_T1 || kind == PK_T2;  // points sorted on the device
   const R half = (R)0.5 * (R)w;
   auto coord = [](double u, int nf) { return (R)(u * nf / (2.0 * M_PI)); };
-  auto band = [&](const double* u, int nf, long& mn, long& mx) {
+  // False beyond 2^30 cells: the kernels find a point's cell in the band from
+  // differences of 32-bit cell numbers, which must not overflow.
+  auto band = [&](const double* u, int nf, long& mn, long& mx) -> bool {
     double lo, hi;
     range_of(u, nuv, lo, hi);
+    const R limit = (R)(1 << 30);
+    if (!(coord(lo, nf) >= -limit && coord(hi, nf) <= limit)) return false;
     mn = (long)std::ceil(coord(lo, nf) - half);
     mx = (long)std::ceil(coord(hi, nf) - half) + w - 1;
+    return true;
   };
   long mn1, mx1, mn2, mx2;
-  band(a.u, d.nf1, mn1, mx1);
-  band(a.v, d.nf2, mn2, mx2);
+  if (!band(a.u, d.nf1, mn1, mx1) || !band(a.v, d.nf2, mn2, mx2))
+    return fail(SMILI_ERR_DATA, "uv coordinates beyond 2^30 cells of the fine grid");
   if (mx1 - mn1 + 1 >= d.nf1) {
     d.b1s = 0;
     d.b1n = d.nf1;

@@ -61,9 +61,8 @@ __global__ void uvsort_count(const ProbDesc* desc, char* base, UvSort q) {
   int *key = at<int>(base, q.o_key), *hist = at<int>(base, q.o_hist);
   const R half = (R)0.5 * (R)P.w;
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < P.nuv; j += gridDim.x * blockDim.x) {
-    // inside the band but for coordinates beyond the integers
-    const int c1 = min(imod((int)ceil(grid_coord<R>(u[j], P.nf1) - half) - P.b1s, P.nf1), P.b1n - 1);
-    const int c2 = min(imod((int)ceil(grid_coord<R>(v[j], P.nf2) - half) - P.b2s, P.nf2), P.b2n - 1);
+    const int c1 = imod((int)ceil(grid_coord<R>(u[j], P.nf1) - half) - P.b1s, P.nf1);  // inside the band
+    const int c2 = imod((int)ceil(grid_coord<R>(v[j], P.nf2) - half) - P.b2s, P.nf2);
     const int t1 = c1 / P.bin, t2 = c2 / P.bin;
     const int k = ((t2 * q.nb1 + t1) * P.bin + (c2 - t2 * P.bin)) * P.bin + (c1 - t1 * P.bin);
     key[j] = k;
