@@ -72,3 +72,16 @@ def test_waits_before_warp_wide_instructions_answer_for_the_warp():
             body = body[:m.end()] + body[m.end():].replace(block, "", 1)
         assert not re.search(r"\bmbar_wait\(", body), f"{name}: {kernel}"
     assert seen
+
+
+def test_build_watches_every_included_file():
+    """A library is rebuilt when any file its source includes has changed."""
+    from smili_b200 import build
+    for src, deps, hdrs in build.LIBS.values():
+        found, todo = set(), [src]
+        while todo:
+            with open(os.path.join(CSRC, todo.pop())) as f:
+                inc = {os.path.basename(i) for i in re.findall(r'#include\s+"([^"]+)"', f.read())}
+            todo += [i for i in inc - found if os.path.exists(os.path.join(CSRC, i))]
+            found |= inc
+        assert found == set(deps) | set(hdrs)
