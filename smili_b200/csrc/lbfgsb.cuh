@@ -464,13 +464,13 @@ struct CauchySmem {
 // Bytes of dynamic shared memory; the launch gives every CTA at least this much.
 constexpr size_t SMILI_CAUCHY_SMEM = sizeof(CauchySmem);
 
-// Select the next batch (<= SMILI_KC elements, the smallest composites above
-// lo_key) from the unordered range [r0, r1) of the bucketed arrays into cand,
+// Select the next batch (<= SMILI_KC elements, the smallest composites from
+// first on) from the unordered range [r0, r1) of the bucketed arrays into cand,
 // by radix selection on 8-bit digits of the 96-bit composite (key, index).
 // Used for a bucket that holds more than SMILI_KC breakpoints.
 template <typename SY>
 __device__ __noinline__ int select_from_range(LbCtxT<SY>& c, const unsigned long long* sbk, const int* sbi, int r0,
-                                              int r1, u128 lo_key, u128* cand, unsigned* hist) {
+                                              int r1, u128 first, u128* cand, unsigned* hist) {
   __shared__ int cnt_s, vstar_s, cum_s;
   u128 prefix = 0;
   int level = 0, budget = SMILI_KC;
@@ -482,7 +482,7 @@ __device__ __noinline__ int select_from_range(LbCtxT<SY>& c, const unsigned long
     __syncthreads();
     for (int i = r0 + threadIdx.x; i < r1; i += blockDim.x) {
       const u128 ck = comp_key(sbk[i], sbi[i]);
-      if (ck <= lo_key) continue;
+      if (ck < first) continue;
       if (level > 0 && (ck >> (96 - 8 * level)) != prefix) continue;
       atomicAdd(&hist[(unsigned)((ck >> shift) & 0xffu)], 1u);
     }
@@ -526,7 +526,7 @@ __device__ __noinline__ int select_from_range(LbCtxT<SY>& c, const unsigned long
     u128 ck = 0;
     if (i < r1) {
       ck = comp_key(sbk[i], sbi[i]);
-      take = ck > lo_key && !(have_hi && ck >= sel_hi);
+      take = ck >= first && !(have_hi && ck >= sel_hi);
     }
     const unsigned bal = __ballot_sync(0xffffffffu, take);
     if (bal) {
@@ -837,8 +837,10 @@ __device__ __noinline__ int cauchy_search(LbCtxT<SY>& c, double f1_0, const doub
         }
       }
       if (big_r0 >= 0) {
-        const u128 lo_key = ((u128)bnd_hi_s << 64) | (u128)bnd_lo_s;
-        cnt = select_from_range(c, sbk, sbi, big_r0, big_r1, lo_key, sm.cand, sm.hist2);
+        // past the last element taken; none yet: from the least composite, 0 (a
+        // time that underflowed, at index 0)
+        const u128 first = kdone == 0 ? 0 : (((u128)bnd_hi_s << 64) | (u128)bnd_lo_s) + 1;
+        cnt = select_from_range(c, sbk, sbi, big_r0, big_r1, first, sm.cand, sm.hist2);
       }
       __syncthreads();
       pf.count(PR_C_ROUNDS);
