@@ -75,7 +75,8 @@ int smili_unet_adam(float* w, void* w16, const float* g, float* m, float* v, lon
 int smili_unet_f32_to_bf16(const float* x, void* y, long long n, void* stream);
 
 /* Convolution path (forward, data gradient and weight gradient): 0 (default)
- * tcgen05 where it applies, 1 mma.sync always, 2 tcgen05 with one 128-pixel
+ * tcgen05 where it applies, 1 mma.sync always (and the bias gradients of a
+ * device without room for a 16-CTA cluster), 2 tcgen05 with one 128-pixel
  * tile per group in the forward convolution (the default gives a group up to
  * four).  Process-wide; for comparisons and tests. */
 int smili_unet_set_conv_path(int path);

@@ -27,6 +27,7 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <atomic>
 #include <type_traits>
 
 #include "../../include/smili_unet.h"
@@ -598,6 +599,23 @@ __global__ void __launch_bounds__(BG_THREADS) bias_grad_kernel(const __nv_bfloat
   if (threadIdx.x < E) db[c0 + threadIdx.x] = accumulate ? db[c0 + threadIdx.x] + red[threadIdx.x] : red[threadIdx.x];
 }
 
+// The same sum, in the same order, by one CTA per channel: where the device
+// has no room for a cluster of 16 (a partition of a few SMs, say).
+__global__ void __launch_bounds__(256) bias_grad_block_kernel(const __nv_bfloat16* dy, int ld, size_t npix, float* db,
+                                                              int accumulate) {
+  __shared__ float red[256];
+  const int c = blockIdx.x;
+  float s = 0.f;
+  for (size_t p = threadIdx.x; p < npix; p += 256) s += __bfloat162float(dy[p * ld + c]);
+  red[threadIdx.x] = s;
+  __syncthreads();
+  for (int w = 128; w > 0; w >>= 1) {
+    if ((int)threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) db[c] = accumulate ? db[c] + red[0] : red[0];
+}
+
 // wt[ci][ky][kx][co] = w[co][2-ky][2-kx][ci]
 __global__ void flip_weights_kernel(const __nv_bfloat16* w, __nv_bfloat16* wt, int Cout, int Cin) {
   const size_t total = (size_t)Cout * 9 * Cin;
@@ -830,7 +848,7 @@ __global__ void f32_to_bf16_kernel(const float* x, __nv_bfloat16* y, size_t n) {
 }
 
 // 0: tensor-core (tcgen05) path where it applies, else mma.sync; 1: always
-// mma.sync; 2: tcgen05 with one 128-pixel tile per group (for comparisons)
+// mma.sync, and bias gradients without clusters; 2: tcgen05 with one 128-pixel tile per group (for comparisons)
 int g_conv_path = 0;
 
 int grid_for(size_t n, int block = 256) {
@@ -861,6 +879,22 @@ int check_launch() {
   return e == cudaSuccess ? 0 : SMILI_UNET_ERR_CUDA;
 }
 
+// Whether the current device can hold a cluster of this launch: 16 CTAs are
+// beyond the portable 8.  Asked once per device.
+bool cluster_fits(const void* fn, const cudaLaunchConfig_t& cfg) {
+  constexpr int kDevs = 64;
+  static std::atomic<int> known[kDevs];  // 0: not asked, 1: no, 2: yes
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kDevs) return false;
+  int k = known[dev].load();
+  if (k == 0) {
+    k = cudaOccupancyMaxActiveClusters(&n, fn, &cfg) == cudaSuccess && n > 0 ? 2 : 1;
+    if (k == 1) cudaGetLastError();
+    known[dev].store(k);
+  }
+  return k == 2;
+}
+
 // bias gradient, after masking dy by y > 0 where y is given
 int launch_bias_grad(const void* y, int ldy, void* dy, int lddy, long long npix, int C, float* db, int accumulate,
                      void* stream) {
@@ -870,9 +904,6 @@ int launch_bias_grad(const void* y, int ldy, void* dy, int lddy, long long npix,
   // 16 CTAs of a cluster, beyond the portable 8, and 64 KB of shared memory:
   // both opted into, per device
   const int smem = vec ? bg_smem<8>() : bg_smem<1>();
-  if (cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
-      cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-    return SMILI_UNET_ERR_CUDA;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
@@ -888,8 +919,21 @@ int launch_bias_grad(const void* y, int ldy, void* dy, int lddy, long long npix,
   const __nv_bfloat16* yp = static_cast<const __nv_bfloat16*>(y);
   __nv_bfloat16* dp = static_cast<__nv_bfloat16*>(dy);
   size_t n = (size_t)npix;
-  void* args[] = {&yp, &ldy, &dp, &lddy, &n, &db, &accumulate};
-  if (cudaLaunchKernelExC(&cfg, fn, args) != cudaSuccess) return SMILI_UNET_ERR_CUDA;
+  if (g_conv_path != 1) {
+    if (cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+      return SMILI_UNET_ERR_CUDA;
+    if (cluster_fits(fn, cfg)) {
+      void* args[] = {&yp, &ldy, &dp, &lddy, &n, &db, &accumulate};
+      if (cudaLaunchKernelExC(&cfg, fn, args) != cudaSuccess) return SMILI_UNET_ERR_CUDA;
+      return check_launch();
+    }
+  }
+  if (y) {
+    const int rc = smili_unet_relu_mask(y, ldy, dy, lddy, npix, C, stream);
+    if (rc != 0) return rc;
+  }
+  bias_grad_block_kernel<<<C, 256, 0, cfg.stream>>>(dp, lddy, n, db, accumulate);
   return check_launch();
 }
 

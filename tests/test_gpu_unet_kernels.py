@@ -168,3 +168,23 @@ def test_tensor_core_weight_gradient(N, H, W, Cin, Cout, nsplit):
     xs, ds = x[..., :Cin], dy[..., :Cout]
     bound = (N * H * W + nsplit) * 2.0 ** -23 * grad(xs.abs(), ds.abs())
     assert ((dw.double() - grad(xs, ds)).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("C,ld,npix", [(24, 24, 1000), (8, 8, 1), (5, 7, 70001), (192, 288, 4097)])
+@pytest.mark.parametrize("masked", [False, True])
+def test_bias_grad_without_clusters(C, ld, npix, masked):
+    """The kernels for a device that cannot hold a 16-CTA cluster add in the
+    same order: equal results."""
+    import torch
+    from smili_b200.warmstart import kernels as K
+    y, got = _rand((npix, ld), 2), []
+    for path in (0, 1):
+        K.set_conv_path(path)
+        dy, db = _rand((npix, ld), 1), torch.full((C,), 3.0, device="cuda")
+        if masked:
+            K.relu_bias_grad(y, ld, dy, ld, npix, C, db, accumulate=True)
+        else:
+            K.bias_grad(dy, ld, npix, C, db, accumulate=True)
+        got.append((dy, db))
+    K.set_conv_path(0)
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
