@@ -5,6 +5,7 @@
 // function/gradient evaluation (fg.cuh) and L-BFGS-B (lbfgsb.cuh) until the
 // problem stops, then takes the next one.  Stages inside a group are
 // separated by group barriers (common.cuh).
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -546,39 +547,64 @@ void gl_positive(int q, std::vector<double>& x, std::vector<double>& wt) {
   }
 }
 
+// The id of the current device's context, different after every
+// cudaDeviceReset; 0 where the driver does not tell.
+unsigned long long context_id() {
+  typedef CUresult (*GetIdFn)(CUcontext, unsigned long long*);
+  static const GetIdFn get_id = [] {
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuCtxGetId", &fn, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      fn = nullptr;
+    }
+    return reinterpret_cast<GetIdFn>(fn);
+  }();
+  unsigned long long id = 0;
+  return get_id && get_id(nullptr, &id) == CUDA_SUCCESS ? id : 0;
+}
+
 // A batch's two device buffers come from a memory pool of this library, one
 // per device, that keeps up to kPoolKeep bytes of freed buffers for the next
 // batch and returns the rest to the device when a batch is destroyed.  A
 // one-shot call (fftim2d.imaging, calc_cost, the bare transforms) spent 0.9 to
 // 1.3 ms, and now and then 14, in cudaMalloc and cudaFree.  Stream ordered and
-// safe from several threads (the driver's pool).  Null where the device has no
-// pools: plain cudaMalloc then.
+// safe from several threads (the driver's pool).  A pool goes with the context
+// it was made in: after a cudaDeviceReset the next batch makes another.  Null
+// where the device has no pools: plain cudaMalloc then.
 constexpr unsigned long long kPoolKeep = 256ull << 20;
 constexpr int kPoolMaxDev = 64;
 
 cudaMemPool_t device_pool(int device) {
+  struct Pool {
+    cudaMemPool_t pool;
+    unsigned long long context;  // 0: not tried
+  };
   static std::mutex mu;
-  static cudaMemPool_t pools[kPoolMaxDev] = {};
-  static bool tried[kPoolMaxDev] = {};
+  static Pool pools[kPoolMaxDev] = {};
   if (device < 0 || device >= kPoolMaxDev) return nullptr;
+  const unsigned long long context = context_id();
+  if (context == 0) return nullptr;
   std::lock_guard<std::mutex> lock(mu);
-  if (!tried[device]) {
-    tried[device] = true;
+  Pool& p = pools[device];
+  if (p.context != context) {
+    p = {nullptr, context};
     int have = 0;
-    cudaMemPool_t p = nullptr;
+    cudaMemPool_t made = nullptr;
     cudaMemPoolProps props = {};
     props.allocType = cudaMemAllocationTypePinned;
     props.location.type = cudaMemLocationTypeDevice;
     props.location.id = device;
     unsigned long long keep = kPoolKeep;
     if (cudaDeviceGetAttribute(&have, cudaDevAttrMemoryPoolsSupported, device) == cudaSuccess && have &&
-        cudaMemPoolCreate(&p, &props) == cudaSuccess &&
-        cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess)
-      pools[device] = p;
+        cudaMemPoolCreate(&made, &props) == cudaSuccess &&
+        cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess)
+      p.pool = made;
     else
       cudaGetLastError();
   }
-  return pools[device];
+  return p.pool;
 }
 
 // Calls pack(0), ..., pack(n - 1) on the host cores; the first (by index)
