@@ -1915,38 +1915,60 @@ __device__ __noinline__ int lb_after_fg(LbCtxT<SY>& c, double f, double gd_fg, d
     double rr_acc = 0.0, ay[SMILI_MAXM_DEV], as[SMILI_MAXM_DEV];
 #pragma unroll
     for (int j = 0; j < SMILI_MAXM_DEV; ++j) ay[j] = as[j] = 0.0;
-    constexpr int U = sizeof(SY) == 8 ? 2 : 1;  // elements in flight per thread
-    const int bd = blockDim.x;
-    for (int i0 = c.lo + threadIdx.x; i0 < c.hi; i0 += U * bd) {
-      double ri[U], di[U];
-      SY wy[U][SMILI_MAXM_DEV], ws[U][SMILI_MAXM_DEV];
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int i = i0 + u * bd;
-        const bool in = i < c.hi;
-        ri[u] = in ? c.gv[i] - c.r[i] : 0.0;
-        di[u] = in ? c.d[i] * sc : 0.0;
-#pragma unroll
-        for (int j = 0; j < SMILI_MAXM_DEV; ++j) {
-          wy[u][j] = in && j < m ? c.wy[(size_t)j * n + i] : (SY)0;
-          ws[u][j] = in && j < m ? c.ws[(size_t)j * n + i] : (SY)0;
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int i = i0 + u * bd;
-        if (i >= c.hi) continue;
-        rr_acc += ri[u] * ri[u];
+    // FP32 (64 registers): one element at a time, its loads where they are
+    // used.  With all 13 loads of an element before its arithmetic every
+    // stage of the launch came out slower: 74 problems of 256 x 256, 20
+    // iterations, 74.5 ms against 72.8; 1 to 3 % at 1 to 12 CTAs per problem.
+    if constexpr (sizeof(SY) == 4) {
+      for (int i = c.lo + threadIdx.x; i < c.hi; i += blockDim.x) {
+        const double ri = c.gv[i] - c.r[i];
+        const double di = c.d[i] * sc;
+        rr_acc += ri * ri;
 #pragma unroll
         for (int j = 0; j < SMILI_MAXM_DEV; ++j) {
           if (j < m) {
-            ay[j] += di[u] * (double)wy[u][j];
-            as[j] += (double)ws[u][j] * di[u];
+            ay[j] += di * ld_wy(c, (size_t)j * n + i);
+            as[j] += ld_ws(c, (size_t)j * n + i) * di;
           }
         }
-        st_sy(c, (size_t)itail * n + i, di[u], ri[u]);
-        c.r[i] = ri[u];
-        c.d[i] = di[u];
+        st_sy(c, (size_t)itail * n + i, di, ri);
+        c.r[i] = ri;
+        c.d[i] = di;
+      }
+    } else {
+      constexpr int U = 2;  // elements in flight per thread
+      const int bd = blockDim.x;
+      for (int i0 = c.lo + threadIdx.x; i0 < c.hi; i0 += U * bd) {
+        double ri[U], di[U];
+        SY wy[U][SMILI_MAXM_DEV], ws[U][SMILI_MAXM_DEV];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const int i = i0 + u * bd;
+          const bool in = i < c.hi;
+          ri[u] = in ? c.gv[i] - c.r[i] : 0.0;
+          di[u] = in ? c.d[i] * sc : 0.0;
+#pragma unroll
+          for (int j = 0; j < SMILI_MAXM_DEV; ++j) {
+            wy[u][j] = in && j < m ? c.wy[(size_t)j * n + i] : (SY)0;
+            ws[u][j] = in && j < m ? c.ws[(size_t)j * n + i] : (SY)0;
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const int i = i0 + u * bd;
+          if (i >= c.hi) continue;
+          rr_acc += ri[u] * ri[u];
+#pragma unroll
+          for (int j = 0; j < SMILI_MAXM_DEV; ++j) {
+            if (j < m) {
+              ay[j] += di[u] * (double)wy[u][j];
+              as[j] += (double)ws[u][j] * di[u];
+            }
+          }
+          st_sy(c, (size_t)itail * n + i, di[u], ri[u]);
+          c.r[i] = ri[u];
+          c.d[i] = di[u];
+        }
       }
     }
     double acc[16];
