@@ -1918,7 +1918,7 @@ __device__ __noinline__ int lb_after_fg(LbCtxT<SY>& c, double f, double gd_fg, d
     // FP32 (64 registers): one element at a time, its loads where they are
     // used.  With all 13 loads of an element before its arithmetic every
     // stage of the launch came out slower: 74 problems of 256 x 256, 20
-    // iterations, 74.5 ms against 72.8; 1 to 3 % at 1 to 12 CTAs per problem.
+    // iterations, 74.5 ms against 72.8; 0.5 to 1.5 % at 1 to 12 CTAs per problem.
     if constexpr (sizeof(SY) == 4) {
       for (int i = c.lo + threadIdx.x; i < c.hi; i += blockDim.x) {
         const double ri = c.gv[i] - c.r[i];

@@ -504,9 +504,11 @@ int next235even(int n) {
   }
 }
 
+// NUFFT tolerance of a call
+double eps_of(const smili_options* opt) { return (opt && opt->nufft_eps > 0) ? opt->nufft_eps : 1e-6; }
+
 void es_params(double eps, int& w, double& beta) {
-  w = (int)std::ceil(std::log10(10.0 / eps));
-  w = std::max(2, std::min(SMILI_MAXW, w));
+  w = (int)std::max(2.0, std::min((double)SMILI_MAXW, std::ceil(std::log10(10.0 / eps))));
   double c = 2.30;
   if (w == 2) c = 2.20;
   else if (w == 3) c = 2.26;
@@ -705,7 +707,8 @@ enum { PK_SOLVE = 0, PK_FG = 1, PK_T2 = 2, PK_T1 = 3, PK_FRAME = 4, PK_MODEL = 5
 
 // Whether the problems of a launch keep their kernel weights (fg_taps):
 // launches that use them at least twice (a bare transform uses them once),
-// unless the tables would take more than 16 GB of the device's memory.
+// unless the tables would take more than 16 GB of the device's memory.  Where
+// the device has no room for them the launch goes without (make_batch).
 template <typename R>
 bool keep_taps(int kind, double eps, double nuv_total) {
   int w;
@@ -1448,14 +1451,24 @@ int launch_batch(smili_batch* b, int mode, float* ms) {
 }
 
 template <typename R>
-int finish_batch(smili_batch* b, std::vector<HostProb>& hps, const smili_options* opt, smili_batch** out);
+int finish_batch(smili_batch* b, std::vector<HostProb>& hps, const smili_options* opt, smili_batch** out,
+                 bool& no_room);
+
+// make(taps, no_room) packs and uploads a batch; again without the kernel
+// weights' tables where the device had no room for it with them.
+template <class F>
+int make_batch(bool taps, F make) {
+  bool no_room = false;
+  const int rc = make(taps, no_room);
+  return rc != SMILI_OK && taps && no_room ? make(false, no_room) : rc;
+}
 
 template <typename R>
 int create_batch(int nprob, const smili_imaging_args* const* probs, const int* niter, int nonneg,
                  int m, double factr, double pgtol, const smili_options* opt, int kind,
                  const double* const* x_over, const double* c_re, const double* c_im,
-                 smili_batch** out) {
-  const double eps = (opt && opt->nufft_eps > 0) ? opt->nufft_eps : 1e-6;
+                 smili_batch** out, bool taps, bool& no_room) {
+  const double eps = eps_of(opt);
   const int device = opt ? opt->device : 0;
   if (!(eps < 1.0)) return fail(SMILI_ERR_ARG, "nufft_eps must be in (0, 1)");
   smili_batch* b = new smili_batch();
@@ -1469,9 +1482,6 @@ int create_batch(int nprob, const smili_imaging_args* const* probs, const int* n
   // to end and every offset moved by its region's start.
   std::vector<Arena> ars(nprob);
   std::vector<HostProb> hps(nprob);
-  double nuv_total = 0;
-  for (int p = 0; p < nprob; ++p) nuv_total += std::max(probs[p]->nuv, 0);
-  const bool taps = keep_taps<R>(kind, eps, nuv_total);
   const int rc = pack_parallel(nprob, [&](int p) -> int {
     ars[p].take(256);
     return pack_problem<R>(*probs[p], kind, niter ? niter[p] : 0, nonneg, m, factr, pgtol, eps, ars[p], hps[p],
@@ -1489,13 +1499,14 @@ int create_batch(int nprob, const smili_imaging_args* const* probs, const int* n
     b->descs.push_back(hps[p].d);
   }
   b->arena_bytes = base;
-  return finish_batch<R>(b, hps, opt, out);
+  return finish_batch<R>(b, hps, opt, out, no_room);
 }
 
 // Device side of a batch whose problems are packed (descs, arena size, host
 // blobs): launch geometry, buffers, upload.  Takes ownership of b.
 template <typename R>
-int finish_batch(smili_batch* b, std::vector<HostProb>& hps, const smili_options* opt, smili_batch** out) {
+int finish_batch(smili_batch* b, std::vector<HostProb>& hps, const smili_options* opt, smili_batch** out,
+                 bool& no_room) {
   const int device = b->device;
   const int nprob = b->nprob;
   b->niter_cap.clear();
@@ -1564,9 +1575,10 @@ int finish_batch(smili_batch* b, std::vector<HostProb>& hps, const smili_options
   auto alloc = [&](void** p, size_t n) {
     return (pool ? cudaMallocFromPoolAsync(p, n, pool, b->stream) : cudaMalloc(p, n)) == cudaSuccess;
   };
-  if (!alloc((void**)&b->d_arena, std::max<size_t>(b->arena_bytes, 256)))
-    return cleanup(fail(SMILI_ERR_CUDA, "allocation of the problem arena failed"));
-  if (!alloc((void**)&b->d_aux, aux)) return cleanup(fail(SMILI_ERR_CUDA, "allocation of the launch's buffers failed"));
+  if (!alloc((void**)&b->d_arena, std::max<size_t>(b->arena_bytes, 256)) || !alloc((void**)&b->d_aux, aux)) {
+    no_room = cudaGetLastError() == cudaErrorMemoryAllocation;
+    return cleanup(fail(SMILI_ERR_CUDA, "allocation of the problem arena or of the launch's buffers failed"));
+  }
   b->d_descs = reinterpret_cast<ProbDesc*>(b->d_aux + o_desc);
   b->d_results = reinterpret_cast<ProbResult*>(b->d_aux + o_res);
   b->d_queue = reinterpret_cast<int*>(b->d_aux + o_q);
@@ -1635,7 +1647,7 @@ int finish_batch(smili_batch* b, std::vector<HostProb>& hps, const smili_options
 template <typename R>
 int pack_movie(const smili_imaging3d_args& a, int kind, int niter, int nonneg, int m, double factr,
                double pgtol, double eps, Arena& ar, HostProb& hp, const double* x_override, int spread_bin,
-               int transform) {
+               int transform, bool taps) {
   const int N = a.npix, Nz = a.nz, nuv = a.nuv;
   if (N < 1 || Nz < 1 || nuv < 0 || a.nx < 1 || a.ny < 1 || (long)N * Nz > 0x7fffffffL)
     return fail(SMILI_ERR_ARG, "invalid movie sizes");
@@ -1867,7 +1879,7 @@ int pack_movie(const smili_imaging3d_args& a, int kind, int niter, int nonneg, i
     fa.wca = a.wca;
     fa.inormfactr = a.inormfactr;
     return pack_problem<R>(fa, PK_FRAME, 0, nonneg, m, factr, pgtol, eps, fa_ar[z], fh[z], nullptr, nullptr, nullptr,
-                           wtotal, spread_bin, transform, keep_taps<R>(PK_FRAME, eps, nuv), &tables);
+                           wtotal, spread_bin, transform, taps, &tables);
   };
   if ((rc = pack_parallel(Nz, pack_frame)) != SMILI_OK) return rc;
   for (int z = 0; z < Nz; ++z) {
@@ -1895,8 +1907,9 @@ int pack_movie(const smili_imaging3d_args& a, int kind, int niter, int nonneg, i
 
 template <typename R>
 int create_movie(const smili_imaging3d_args* a, int kind, int niter, int nonneg, int m, double factr,
-                 double pgtol, const smili_options* opt, const double* x_over, smili_batch** out) {
-  const double eps = (opt && opt->nufft_eps > 0) ? opt->nufft_eps : 1e-6;
+                 double pgtol, const smili_options* opt, const double* x_over, smili_batch** out, bool taps,
+                 bool& no_room) {
+  const double eps = eps_of(opt);
   if (!(eps < 1.0)) return fail(SMILI_ERR_ARG, "nufft_eps must be in (0, 1)");
   if (m < 1 || m > SMILI_MAXM_DEV) return fail(SMILI_ERR_UNSUPPORTED, "L-BFGS-B memory m must be 1..6");
   smili_batch* b = new smili_batch();
@@ -1907,22 +1920,23 @@ int create_movie(const smili_imaging3d_args* a, int kind, int niter, int nonneg,
   Arena ar;
   std::vector<HostProb> hps(1);
   const int rc = pack_movie<R>(*a, kind, niter, nonneg, m, factr, pgtol, eps, ar, hps[0], x_over,
-                               opt && opt->spread_bin ? opt->spread_bin : 8, opt ? opt->transform : 0);
+                               opt && opt->spread_bin ? opt->spread_bin : 8, opt ? opt->transform : 0, taps);
   if (rc != SMILI_OK) {
     delete b;
     return rc;
   }
   b->descs.push_back(hps[0].d);
   b->arena_bytes = ar.bytes;
-  return finish_batch<R>(b, hps, opt, out);
+  return finish_batch<R>(b, hps, opt, out, no_room);
 }
 
 // One evaluation of a single data term with unit weight and no
 // regularizer: the raw chi-square sum and gradient of model_fcv / amp / cp /
 // ca (fftlib.f90:744-1254), with every datum's model and residual.
 template <typename R>
-int create_model(const smili_imaging_args& a, const double* x, const smili_options* opt, smili_batch** out) {
-  const double eps = (opt && opt->nufft_eps > 0) ? opt->nufft_eps : 1e-6;
+int create_model(const smili_imaging_args& a, const double* x, const smili_options* opt, smili_batch** out, bool taps,
+                 bool& no_room) {
+  const double eps = eps_of(opt);
   if (!(eps < 1.0)) return fail(SMILI_ERR_ARG, "nufft_eps must be in (0, 1)");
   const int nterm = (a.isfcv != 0) + (a.isamp != 0) + (a.iscp != 0) + (a.isca != 0);
   if (nterm != 1) return fail(SMILI_ERR_ARG, "exactly one data term must be given");
@@ -1938,15 +1952,29 @@ int create_model(const smili_imaging_args& a, const double* x, const smili_optio
   Arena ar;
   std::vector<HostProb> hps(1);
   const int rc = pack_problem<R>(b0, PK_MODEL, 0, 0, 5, 1e1, 0.0, eps, ar, hps[0], x, nullptr, nullptr, w,
-                                 opt && opt->spread_bin ? opt->spread_bin : 8, opt ? opt->transform : 0,
-                                 keep_taps<R>(PK_MODEL, eps, std::max(a.nuv, 0)));
+                                 opt && opt->spread_bin ? opt->spread_bin : 8, opt ? opt->transform : 0, taps);
   if (rc != SMILI_OK) {
     delete b;
     return rc;
   }
   b->descs.push_back(hps[0].d);
   b->arena_bytes = ar.bytes;
-  return finish_batch<R>(b, hps, opt, out);
+  return finish_batch<R>(b, hps, opt, out, no_room);
+}
+
+template <typename R>
+int make_movie(const smili_imaging3d_args* a, int kind, int niter, int nonneg, int m, double factr, double pgtol,
+               const smili_options* opt, const double* x_over, smili_batch** out) {
+  return make_batch(keep_taps<R>(kind, eps_of(opt), a->nuv), [&](bool taps, bool& no_room) {
+    return create_movie<R>(a, kind, niter, nonneg, m, factr, pgtol, opt, x_over, out, taps, no_room);
+  });
+}
+
+template <typename R>
+int make_model(const smili_imaging_args& a, const double* x, const smili_options* opt, smili_batch** out) {
+  return make_batch(keep_taps<R>(PK_MODEL, eps_of(opt), a.nuv), [&](bool taps, bool& no_room) {
+    return create_model<R>(a, x, opt, out, taps, no_room);
+  });
 }
 
 int create_movie_any(const smili_imaging3d_args* a, int kind, int niter, int nonneg, int m, double factr,
@@ -1954,8 +1982,8 @@ int create_movie_any(const smili_imaging3d_args* a, int kind, int niter, int non
   if (!a || !out) return fail(SMILI_ERR_ARG, "null argument");
   const int prec = opt && opt->precision ? opt->precision : 64;
   if (prec != 64 && prec != 32) return fail(SMILI_ERR_ARG, "precision must be 64 or 32");
-  return prec == 64 ? create_movie<double>(a, kind, niter, nonneg, m, factr, pgtol, opt, x_over, out)
-                    : create_movie<float>(a, kind, niter, nonneg, m, factr, pgtol, opt, x_over, out);
+  return prec == 64 ? make_movie<double>(a, kind, niter, nonneg, m, factr, pgtol, opt, x_over, out)
+                    : make_movie<float>(a, kind, niter, nonneg, m, factr, pgtol, opt, x_over, out);
 }
 
 int run(smili_batch* b, int mode, float* ms) {
@@ -1968,6 +1996,7 @@ int run(smili_batch* b, int mode, float* ms) {
 template <typename R>
 int launch_bare(smili_batch* b, int mode) {
   const UvSort& q = b->sort;
+  cudaGetLastError();  // an earlier call's error, if any, was reported by that call
   const int nb = std::min(4 * 148, (b->descs[0].nuv + 255) / 256), nchunk = (q.nkey + UVSORT_CHUNK - 1) / UVSORT_CHUNK;
   uvsort_count<R><<<nb, 256, 0, b->stream>>>(b->d_descs, b->d_arena, q);
   uvsort_sums<<<nchunk, UVSORT_T, 0, b->stream>>>(b->d_arena, q);
@@ -1994,9 +2023,15 @@ int create_any(int nprob, const smili_imaging_args* const* probs, const int* nit
   if (nprob < 1 || !probs || !out) return fail(SMILI_ERR_ARG, "invalid batch arguments");
   const int prec = opt && opt->precision ? opt->precision : 64;
   if (prec != 64 && prec != 32) return fail(SMILI_ERR_ARG, "precision must be 64 or 32");
-  if (prec == 64)
-    return create_batch<double>(nprob, probs, niter, nonneg, m, factr, pgtol, opt, kind, x_over, c_re, c_im, out);
-  return create_batch<float>(nprob, probs, niter, nonneg, m, factr, pgtol, opt, kind, x_over, c_re, c_im, out);
+  double nuv = 0;
+  for (int p = 0; p < nprob; ++p) nuv += std::max(probs[p]->nuv, 0);
+  return make_batch(prec == 64 ? keep_taps<double>(kind, eps_of(opt), nuv) : keep_taps<float>(kind, eps_of(opt), nuv),
+                    [&](bool taps, bool& no_room) {
+    return prec == 64 ? create_batch<double>(nprob, probs, niter, nonneg, m, factr, pgtol, opt, kind, x_over, c_re,
+                                             c_im, out, taps, no_room)
+                      : create_batch<float>(nprob, probs, niter, nonneg, m, factr, pgtol, opt, kind, x_over, c_re,
+                                            c_im, out, taps, no_room);
+  });
 }
 
 }  // namespace
@@ -2383,7 +2418,7 @@ int smili_model_terms(const smili_imaging_args* a, const double* x, const smili_
     const int prec = opt && opt->precision ? opt->precision : 64;
     if (prec != 64 && prec != 32) return fail(SMILI_ERR_ARG, "precision must be 64 or 32");
     smili_batch* b = nullptr;
-    int rc = prec == 64 ? create_model<double>(*a, x, opt, &b) : create_model<float>(*a, x, opt, &b);
+    int rc = prec == 64 ? make_model<double>(*a, x, opt, &b) : make_model<float>(*a, x, opt, &b);
     if (rc != SMILI_OK) return rc;
     rc = run(b, MODE_FG, nullptr);
     double terms[SMILI_NTERMS];
@@ -2558,7 +2593,7 @@ size_t round256(size_t n) { return (n + 255) / 256 * 256; }
 template <typename R>
 int calc_cost_noalloc(const smili_imaging_args* a, const double* x, const smili_options* opt, double* terms,
                       double* grad) {
-  const double eps = (opt && opt->nufft_eps > 0) ? opt->nufft_eps : 1e-6;
+  const double eps = eps_of(opt);
   const int device = opt ? opt->device : 0;
   if (!(eps < 1.0)) return fail(SMILI_ERR_ARG, "nufft_eps must be in (0, 1)");
   Arena ar;
