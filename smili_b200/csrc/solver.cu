@@ -629,7 +629,10 @@ int pack_parallel(int n, F pack) {
   };
   const int nth = std::max(1, std::min(n, (int)std::thread::hardware_concurrency()));
   std::vector<std::thread> pool;
-  for (int t = 1; t < nth; ++t) pool.emplace_back(work);
+  try {
+    for (int t = 1; t < nth; ++t) pool.emplace_back(work);
+  } catch (const std::exception&) {  // no further thread to be had: those there are share the work
+  }
   work();
   for (auto& th : pool) th.join();
   for (int p = 0; p < n; ++p)
