@@ -1751,6 +1751,7 @@ int pack_movie(const smili_imaging3d_args& a, int kind, int niter, int nonneg, i
   d.prec64 = sizeof(R) == 8;
   d.nxref = a.nxref;
   d.nyref = a.nyref;
+  d.nuv = nuv;  // of all frames, for the size of its group
   d.nframes = Nz;
   d.frame_npix = N;
   d.nfcv = nfcv;

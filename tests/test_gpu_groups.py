@@ -174,3 +174,26 @@ def test_batch_refuses_a_capturing_stream(lib):
     g.replay()
     torch.cuda.synchronize()
     assert float(x) == 1.0
+
+
+def test_movie_group_counts_its_points():
+    """4 frames of 32^2 pixels with 2000 points each: 16 CTAs for the pixels
+    and 10 for the points.  Sums depend on the group size in their last bits
+    and on nothing else, so the automatic size shows in the cost terms."""
+    from smili_b200 import synth
+    from smili_b200.fortlib import fftim3d
+    from smili_b200.imaging.lbfgs3d import prepare_imaging3d
+    m = synth.dynamic_problem(seed=4, nframes=4, nx=32, nst=16, vis_per_frame=2000, niter=1)
+    kw, _ = prepare_imaging3d(m.frames, vistable=m.vistable, bstable=m.bstable, niter=1, l1_lambda=1.0,
+                              tsv_lambda=1.0, rt_lambda=1.0)
+    x = np.asarray(kw["iin"], dtype=np.float64) * np.random.default_rng(5).uniform(0.5, 1.5, np.size(kw["iin"]))
+    points = np.size(kw["u"])
+    want = int(4096 / 256 + points / 800)
+    assert want >= 20
+
+    def terms(ctas):
+        return fftim3d.calc_cost(x, nufft_eps=1e-6, ctas_per_problem=ctas, **kw)[0]
+
+    auto = terms(0)
+    assert auto == terms(0) == terms(want)
+    assert auto != terms(16)  # four CTAs per frame instead of six
