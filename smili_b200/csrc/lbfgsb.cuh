@@ -24,6 +24,7 @@
 #include <cfloat>
 
 #include "common.cuh"
+#include "quotient.cuh"
 
 #define SMILI_MAXM_DEV 6  // largest L-BFGS-B memory the device solver accepts
 #define SMILI_KC 1024     // breakpoints of one sorted batch of the Cauchy search
@@ -72,20 +73,6 @@ __device__ __forceinline__ void st_sy(const LbCtxT<SY>& c, size_t i, double s, d
 // loops / a column per lane, unrolled / as here: formk 22 / 13 / 8 us, the
 // two solves of subsm 9 / 7 / 2.8, an update 9 / 6 / 5 (B200).
 // ---------------------------------------------------------------------------
-// 1 / t for div_by, or 0 near the ends of the exponent range
-__device__ __forceinline__ double rcp_of(double t) {
-  const double a = fabs(t);
-  return a > 1e-280 && a < 1e280 ? 1.0 / t : 0.0;
-}
-
-// b / t from r = rcp_of(t): the product and one residual step, as accurate as
-// the division and a third of its latency
-__device__ __forceinline__ double div_by(double b, double t, double r) {
-  if (r == 0.0) return b / t;
-  const double q = b * r, c = fma(fma(-q, t, b), r, q);
-  return fabs(q) <= DBL_MAX ? c : q;
-}
-
 // Cholesky factor of the symmetric matrix in the upper triangle of a (shared,
 // column major, leading dimension ld).  The first n1 columns eliminate with
 // the opposite sign beyond row n1: [A B; B' C] becomes the factors of A and of
