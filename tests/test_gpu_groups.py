@@ -197,3 +197,37 @@ def test_movie_group_counts_its_points():
     auto = terms(0)
     assert auto == terms(0) == terms(want)
     assert auto != terms(16)  # four CTAs per frame instead of six
+
+
+@pytest.mark.parametrize("ctas", [1, 3, 16, 148])
+@pytest.mark.parametrize("eps", [1e-6, 1e-7, 1e-8])
+def test_register_spreading_over_group_sizes(odd, oracle, lib, eps, ctas):
+    """FP64 kernel widths 7, 8 and 9 spread with the subgrid in registers,
+    the points cut into one range per warp: the objective and the gradient of
+    the oracle at the same width (rounding only, at the bounds above)."""
+    kw, x, _ = odd
+    t, g = oracle.calc_cost(kw, x, eps=eps)
+    b = lib.Batch([lib.Problem(dict(kw, iin=x))], niter=1, options=lib.make_options(64, eps, ctas))
+    b.run(fg_only=1)
+    _, tb, gb, _ = b.fetch(0)
+    b.close()
+    assert abs(tb["cost"] - t["cost"]) <= 1e-9 * abs(t["cost"])
+    assert _rel(gb, g) <= 1e-8
+
+
+@pytest.mark.parametrize("ctas", [1, 3, 148])
+@pytest.mark.parametrize("eps", [0.5, 1e-2, 1e-6, 1e-8])
+def test_register_spreading_equals_general_spreading(odd, lib, eps, ctas):
+    """Widths 2, 3, 7 and 9 against the general spreading (16 x 16 tiles) at
+    the same group size: the gradient differs by the order of at most 2016
+    additions per cell and 64 per transform."""
+    kw, x, _ = odd
+    got = []
+    for spread_bin in (8, 16):
+        b = lib.Batch([lib.Problem(dict(kw, iin=x))], niter=1,
+                      options=lib.make_options(64, eps, ctas, spread_bin=spread_bin))
+        b.run(fg_only=1)
+        got.append(b.fetch(0))
+        b.close()
+    assert abs(got[0][1]["cost"] - got[1][1]["cost"]) <= 1e-13 * abs(got[1][1]["cost"])
+    assert _rel(got[0][2], got[1][2]) <= 1e-11
