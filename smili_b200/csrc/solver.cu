@@ -609,6 +609,17 @@ cudaMemPool_t device_pool(int device) {
   return p.pool;
 }
 
+// cudaMalloc on the current device; where it has no room, once more with the
+// pool's idle memory given back to it.
+cudaError_t malloc_or_trim(void** p, size_t n, int device) {
+  cudaError_t e = cudaMalloc(p, n);
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
+  const cudaMemPool_t pool = device_pool(device);
+  if (pool && cudaMemPoolTrimTo(pool, 0) != cudaSuccess) cudaGetLastError();
+  return cudaMalloc(p, n);
+}
+
 // Calls pack(0), ..., pack(n - 1) on the host cores; the first (by index)
 // error code with its message, or SMILI_OK.
 template <class F>
@@ -1340,6 +1351,17 @@ struct smili_batch {
 
 namespace {
 
+// Frees a batch's two device buffers.
+void free_buffers(smili_batch* b) {
+  for (char** p : {&b->d_arena, &b->d_aux}) {
+    if (*p && (!b->pooled || cudaFreeAsync(*p, b->stream) != cudaSuccess)) cudaFree(*p);
+    *p = nullptr;
+  }
+  // what the pool does not keep goes back to the device with this wait
+  if (b->pooled && b->stream) cudaStreamSynchronize(b->stream);
+  b->pooled = false;
+}
+
 // CTAs that one problem is worth when the device has it to itself.  Per CTA a
 // pixel or a uv point costs little against a stage's fixed latency, so a group
 // grows until its barriers and group sums cost what a larger one saves.  Ten
@@ -1573,14 +1595,23 @@ int finish_batch(smili_batch* b, std::vector<HostProb>& hps, const smili_options
     b->own_stream = true;
   }
   // (buffers beyond what the pool keeps gain nothing from it)
+  const size_t arena_bytes = std::max<size_t>(b->arena_bytes, 256);
   const cudaMemPool_t pool = b->arena_bytes + aux <= kPoolKeep ? device_pool(device) : nullptr;
-  b->pooled = pool != nullptr;
-  auto alloc = [&](void** p, size_t n) {
-    return (pool ? cudaMallocFromPoolAsync(p, n, pool, b->stream) : cudaMalloc(p, n)) == cudaSuccess;
-  };
-  if (!alloc((void**)&b->d_arena, std::max<size_t>(b->arena_bytes, 256)) || !alloc((void**)&b->d_aux, aux)) {
-    no_room = cudaGetLastError() == cudaErrorMemoryAllocation;
-    return cleanup(fail(SMILI_ERR_CUDA, "allocation of the problem arena or of the launch's buffers failed"));
+  if (pool) {
+    b->pooled = true;
+    if (cudaMallocFromPoolAsync((void**)&b->d_arena, arena_bytes, pool, b->stream) != cudaSuccess ||
+        cudaMallocFromPoolAsync((void**)&b->d_aux, aux, pool, b->stream) != cudaSuccess) {
+      // the pool grows by 32 MB at a time; less may be left for plain buffers
+      cudaGetLastError();
+      free_buffers(b);
+    }
+  }
+  if (!b->pooled) {
+    if (malloc_or_trim((void**)&b->d_arena, arena_bytes, device) != cudaSuccess ||
+        malloc_or_trim((void**)&b->d_aux, aux, device) != cudaSuccess) {
+      no_room = cudaGetLastError() == cudaErrorMemoryAllocation;
+      return cleanup(fail(SMILI_ERR_CUDA, "allocation of the problem arena or of the launch's buffers failed"));
+    }
   }
   b->d_descs = reinterpret_cast<ProbDesc*>(b->d_aux + o_desc);
   b->d_results = reinterpret_cast<ProbResult*>(b->d_aux + o_res);
@@ -2158,7 +2189,7 @@ int save_starts(smili_batch* b) {
     b->x0_saved_off[p] = total;
     if (b->descs[p].o_x0 && b->descs[p].nframes == 0) total += (size_t)b->descs[p].npix;
   }
-  CUDA_TRY(cudaMalloc(&b->d_x0_saved, sizeof(double) * std::max<size_t>(total, 1)));
+  CUDA_TRY(malloc_or_trim((void**)&b->d_x0_saved, sizeof(double) * std::max<size_t>(total, 1), b->device));
   for (int p = 0; p < b->nprob; ++p) {
     const ProbDesc& d = b->descs[p];
     if (!d.o_x0 || d.nframes > 0) continue;
@@ -2289,7 +2320,7 @@ int smili_batch_set_starts_from_images(smili_batch* b, const float* img, int nx,
     CUDA_TRY(cudaSetDevice(b->device));
     if ((rc = save_starts(b)) != SMILI_OK) return rc;
     if (keep) {
-      if (!b->d_keep) CUDA_TRY(cudaMalloc(&b->d_keep, b->nprob));
+      if (!b->d_keep) CUDA_TRY(malloc_or_trim((void**)&b->d_keep, b->nprob, b->device));
       CUDA_TRY(cudaMemcpyAsync(b->d_keep, keep, b->nprob, cudaMemcpyHostToDevice, b->stream));
     }
     batch_starts_kernel<<<b->nprob, kWarmThreads, 0, b->stream>>>(b->d_descs, b->d_arena, img, nx, ny,
@@ -2333,12 +2364,7 @@ void smili_batch_destroy(smili_batch* b) {
   if (!b) return;
   cudaSetDevice(b->device);
   if (b->stream) cudaStreamSynchronize(b->stream);
-  for (char* p : {b->d_arena, b->d_aux})
-    if (p) {
-      if (!b->pooled || cudaFreeAsync(p, b->stream) != cudaSuccess) cudaFree(p);
-    }
-  // what the pool does not keep goes back to the device with this wait
-  if (b->pooled && b->stream) cudaStreamSynchronize(b->stream);
+  free_buffers(b);
   if (b->d_x0_saved) cudaFree(b->d_x0_saved);
   if (b->d_keep) cudaFree(b->d_keep);
   if (b->own_stream && b->stream) cudaStreamDestroy(b->stream);
