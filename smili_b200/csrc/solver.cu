@@ -609,17 +609,6 @@ cudaMemPool_t device_pool(int device) {
   return p.pool;
 }
 
-// cudaMalloc on the current device; where it has no room, once more with the
-// pool's idle memory given back to it.
-cudaError_t malloc_or_trim(void** p, size_t n, int device) {
-  cudaError_t e = cudaMalloc(p, n);
-  if (e != cudaErrorMemoryAllocation) return e;
-  cudaGetLastError();
-  const cudaMemPool_t pool = device_pool(device);
-  if (pool && cudaMemPoolTrimTo(pool, 0) != cudaSuccess) cudaGetLastError();
-  return cudaMalloc(p, n);
-}
-
 // Calls pack(0), ..., pack(n - 1) on the host cores; the first (by index)
 // error code with its message, or SMILI_OK.
 template <class F>
@@ -1607,8 +1596,8 @@ int finish_batch(smili_batch* b, std::vector<HostProb>& hps, const smili_options
     }
   }
   if (!b->pooled) {
-    if (malloc_or_trim((void**)&b->d_arena, arena_bytes, device) != cudaSuccess ||
-        malloc_or_trim((void**)&b->d_aux, aux, device) != cudaSuccess) {
+    if (cudaMalloc((void**)&b->d_arena, arena_bytes) != cudaSuccess ||
+        cudaMalloc((void**)&b->d_aux, aux) != cudaSuccess) {
       no_room = cudaGetLastError() == cudaErrorMemoryAllocation;
       return cleanup(fail(SMILI_ERR_CUDA, "allocation of the problem arena or of the launch's buffers failed"));
     }
@@ -2189,7 +2178,7 @@ int save_starts(smili_batch* b) {
     b->x0_saved_off[p] = total;
     if (b->descs[p].o_x0 && b->descs[p].nframes == 0) total += (size_t)b->descs[p].npix;
   }
-  CUDA_TRY(malloc_or_trim((void**)&b->d_x0_saved, sizeof(double) * std::max<size_t>(total, 1), b->device));
+  CUDA_TRY(cudaMalloc(&b->d_x0_saved, sizeof(double) * std::max<size_t>(total, 1)));
   for (int p = 0; p < b->nprob; ++p) {
     const ProbDesc& d = b->descs[p];
     if (!d.o_x0 || d.nframes > 0) continue;
@@ -2320,7 +2309,7 @@ int smili_batch_set_starts_from_images(smili_batch* b, const float* img, int nx,
     CUDA_TRY(cudaSetDevice(b->device));
     if ((rc = save_starts(b)) != SMILI_OK) return rc;
     if (keep) {
-      if (!b->d_keep) CUDA_TRY(malloc_or_trim((void**)&b->d_keep, b->nprob, b->device));
+      if (!b->d_keep) CUDA_TRY(cudaMalloc(&b->d_keep, b->nprob));
       CUDA_TRY(cudaMemcpyAsync(b->d_keep, keep, b->nprob, cudaMemcpyHostToDevice, b->stream));
     }
     batch_starts_kernel<<<b->nprob, kWarmThreads, 0, b->stream>>>(b->d_descs, b->d_arena, img, nx, ny,

@@ -242,7 +242,7 @@ static int uvlist_run(int n, const double* u, const double* v, int device, cudaS
     wk.d = nullptr;
     wk.cap = 0;
     const size_t want = off + off / 4;  // headroom for slightly larger lists
-    if (malloc_or_trim((void**)&wk.d, want, device) != cudaSuccess) {
+    if (cudaMalloc(&wk.d, want) != cudaSuccess) {
       wk.d = nullptr;
       return fail(SMILI_ERR_CUDA, "get_uvlist: cudaMalloc of the work space failed");
     }
