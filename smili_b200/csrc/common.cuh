@@ -76,7 +76,7 @@ struct GroupCtx {
 
 // largest reduction: the Gram blocks of formk, 2 m (m + 1) / 2 + 2 m m at m = 6
 #define SMILI_REDK 128
-// reductions of one evaluation (no L-BFGS-B step): at most 16 sums and 3 maxima
+// reductions of one evaluation (no L-BFGS-B step): at most 16 sums and one maximum
 #define SMILI_REDK_FG 32
 
 // Spin budget of one barrier wait.  A healthy barrier completes in

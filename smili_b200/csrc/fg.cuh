@@ -114,7 +114,9 @@ struct KSumF {
 // As register tiles of 64 rows, 512 cells, 8 band rows and 4 image rows the
 // stages had work for 4 to 16 CTAs only: 256 x 256, 44 x 21 cells, FP64 on 64
 // CTAs, 70 + 40 + 24 + 14 us per evaluation, 18 + 7 + 21 on 96 now; FP32 on
-// groups of 2 CTAs (148 problems) 100 + 40 + 44 + 141, now 112 + 42 + 96.
+// groups of 2 CTAs (148 problems) 100 + 40 + 44 + 141, now 112 + 42 + 96.  (On
+// groups of 4 the FP32 rows take 106 us; with the earlier tiles back, 2 rows by 4
+// cells on all 512 threads, 94, but the launch of 74 problems 73.6 ms against 73.4.)
 // ---------------------------------------------------------------------------
 constexpr int DFT_NB = 64;  // largest band side on this path (and 2048 cells in all)
 constexpr int DFT_KC = 32;  // image columns per staged chunk of the FP32 F1
@@ -147,7 +149,7 @@ __device__ __forceinline__ R dense_pixel(const ProbDesc& P, const double* x, con
 }
 
 // Sum of each of v[0..N) over the warp (N a power of two up to 32): lane l
-// returns the sum of value l / (32 / N), as warp_fold in the compute type.
+// returns the sum of value l / (32 / N).
 template <int N, typename R>
 __device__ __forceinline__ R warp_fold_r(R (&v)[N], int lane) {
   int b = 16;
@@ -837,19 +839,6 @@ __device__ __noinline__ void fg_chisq(FgCtx<R>& c, const GroupCtx& g, double (&c
 __device__ __forceinline__ void atomic_add_r(double* p, double v) { atomicAdd(p, v); }
 __device__ __forceinline__ void atomic_add_r(float* p, float v) { atomicAdd(p, v); }
 
-template <typename R>
-__device__ __forceinline__ R warp_sum(R v) {
-  for (int s = 16; s > 0; s >>= 1) v += __shfl_xor_sync(0xffffffffu, v, s);
-  return v;
-}
-
-// Subproblem spreading.  The bin-sorted points are cut into work items of
-// at most 128 points that share one 8x8 bin of the band.  A warp owns an item
-// and a private (8+w-1)^2 subgrid in shared memory: for every point the
-// lanes cover the w*w taps (all lanes hit different cells, and consecutive
-// points are ordered by __syncwarp), so the inner loop needs no atomics.  The
-// finished subgrid is added to the CTA's band copy (shared atomics, only the
-// overlapping halos collide) and the CTA's band to the global band at the end.
 // The work item that holds point p0 (items cover the points in order)
 __device__ __forceinline__ int item_of(const int4* items, int nitems, int p0) {
   int it = 0;
@@ -1147,6 +1136,14 @@ __device__ __noinline__ void fg_spread_tc(FgCtx<float>& c, const GroupCtx& g) {
   }
 }
 
+// F5 for any bin and width (the two above where they apply): subproblem
+// spreading.  The bin-sorted points are cut into work items of at most 128
+// points that share one bin of the band.  A warp owns an item and a private
+// (bin+w-1)^2 subgrid in shared memory: for every point the lanes cover the w*w
+// taps (all lanes hit different cells, and consecutive points are ordered by
+// __syncwarp), so the inner loop needs no atomics.  The finished subgrid is
+// added to the CTA's band copy (shared atomics, only the overlapping halos
+// collide) and the CTA's band to the global band at the end.
 template <typename R>
 __device__ __noinline__ void fg_spread(FgCtx<R>& c, const GroupCtx& g) {
   if (c.P->bin == 8) {

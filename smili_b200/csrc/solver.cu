@@ -1354,12 +1354,16 @@ void free_buffers(smili_batch* b) {
 // CTAs that one problem is worth when the device has it to itself.  Per CTA a
 // pixel or a uv point costs little against a stage's fixed latency, so a group
 // grows until its barriers and group sums cost what a larger one saves.  Ten
-// iterations on a B200 in FP64 (the FP32 optima are close), kernel ms at four
+// iterations on a B200 in FP64, kernel ms at four
 // pixels per thread / at this rule: 64^2 px, 2.0 k points 3.58 at 4 CTAs /
 // 2.65 at 19; 7.6 k px, 4.2 k points 4.16 at 8 / 3.00 at 35; 64^2 px, 50 k
 // points 8.85 at 4 / 3.18 at 66; 128^2 px, 50 k points 4.71 at 16 / 3.28 at
 // 72; 256^2 px 5.21 at 64 / 4.91 at 96; 512^2 px 4.3 at 256 / 3.85 at 148.
 // Two CTAs on an SM only pay from about 2^19 pixels (1024^2: 148 8.9, 296 8.4).
+// FP32 takes the same rule: us per evaluation and iteration at this size / at the
+// best of 15 sizes: 64^2 px, 2.0 k points 197 / 197; 50 k points 195 / 193 (48
+// CTAs); 128^2, 50 k 238 / 227 (48); 256^2, 97 k 330 / 322 (64); 512^2, 99 k 441 / 434
+// (128); 1024^2, 240 k 810 / 810.
 int group_size(double npix, double nuv, int nsm, int maxres) {
   double G = std::min(npix / 256 + nuv / 800, 64 + npix / 2048);
   if (npix <= 1 << 19) G = std::min(G, (double)nsm);
@@ -2021,7 +2025,9 @@ template <typename R>
 int launch_bare(smili_batch* b, int mode) {
   const UvSort& q = b->sort;
   cudaGetLastError();  // an earlier call's error, if any, was reported by that call
-  const int nb = std::min(4 * 148, (b->descs[0].nuv + 255) / 256), nchunk = (q.nkey + UVSORT_CHUNK - 1) / UVSORT_CHUNK;
+  int nsm = 0;
+  CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, b->device));
+  const int nb = std::min(4 * nsm, (b->descs[0].nuv + 255) / 256), nchunk = (q.nkey + UVSORT_CHUNK - 1) / UVSORT_CHUNK;
   uvsort_count<R><<<nb, 256, 0, b->stream>>>(b->d_descs, b->d_arena, q);
   uvsort_sums<<<nchunk, UVSORT_T, 0, b->stream>>>(b->d_arena, q);
   uvsort_scan<<<nchunk, UVSORT_T, 0, b->stream>>>(b->d_arena, q);
